@@ -356,6 +356,8 @@ static cudaError_t run_int4(const void *x, const void *w, const void *scales, co
   if (group % 32 != 0 || K % group != 0 || N % 8 != 0) return cudaErrorInvalidValue;
   if (qzeros != nullptr && N % 32 != 0) return cudaErrorInvalidValue;   // zero-point rows travel as 16-byte bulk copies
   if (wa_refused(x, w, K, dtype, e)) return e;
+  // scale and zero-point rows travel as bulk copies, which start on 16-byte boundaries (N makes their rows multiples of 16 bytes)
+  if (((uintptr_t)scales & 15) || ((uintptr_t)qzeros & 15)) return cudaErrorMisalignedAddress;
   const TsDevice &d = ts_device();
   // (a span of a row: 128 B of nibbles and its scales; the dequantisers take two operations a weight, some 800 clocks a span)
   const TsPlan plan = ts_plan(M, N, K, 128 + 2 * ((TS_SPAN_K + group - 1) / group), 800, 0, d);
