@@ -23,7 +23,8 @@
 // after (before: one kernel for Q8_0, Q4_K and Q6_K with 128 or 256 tokens a tile and K whole, per-element decoding for the other types,
 // a kernel with 8 dequantising warps for int4): Q4_K 14336 x 4096, 24 tokens 29.2 / 18.4; Q5_K 4096 x 4096, 200 tokens 2516 / 20; Q8_0
 // 14336 x 4096, 4096 tokens 488 / 429; int4 14336 x 4096, 32 tokens 21.9 / 18.4; int4 with zero points 4096 x 14336, 500 tokens 170 / 69.
-// Every wait has a limit; one that runs out sets a device flag (mrs_mmq_timeouts) and ends the CTA.
+// Every wait has a limit; one that runs out sets a device flag (mrs_mmq_timeouts) and ends the CTA.  What a limit counts is this grid's
+// own work: in a programmatic-dependent-launch chain a warp passes pdl_wait before its first wait that the activations hold up.
 #pragma once
 #include "dequant.cuh"
 #include "tc_common.cuh"
@@ -582,6 +583,7 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
     for (int t = first; ok && t < n_tiles; t += step) {
       const int n0 = (t % p.tiles_n) * TS_BM;
       for (int s = s0; s < s1; s++, it++) {
+        if (p.pdl && it == RS) pdl_wait();             // the ring is full: from here on its stages are freed at the grid before's pace
         ok = ts_wait(raw_empty + st, ph ^ 1, late);
         if (!ok) break;
         if constexpr (TYPE == TS_INT4) {
@@ -645,6 +647,7 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
     const uint32_t x0 = __reduce_max_sync(0xffffffffu, smem_u32(x_ring)), xe0 = __reduce_max_sync(0xffffffffu, smem_u32(x_empty));
     int it = 0, xs = 0, xph = 0, j = 0;
     bool ok = true;
+    if (p.pdl) pdl_wait();                   // (x_full completes behind it)
     for (int t = first; ok && t < n_tiles; t += step, j++) {
       const int b = j % n_acc;
       const uint32_t acc = tmem_base + (uint32_t)b * 128u;
@@ -717,6 +720,7 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
           u.load(row0 + stage + phase, part);
           u.template half<0>(part, o);
         }
+        if (p.pdl && it == TS_AS) pdl_wait();          // (a stage is freed by products, which need x)
         ok = ts_wait(a_empty + as, ((it / TS_AS) & 1) ^ 1, late);   // the MMAs that read this A stage have retired
         if (!ok) break;
         tc_fence_after();
