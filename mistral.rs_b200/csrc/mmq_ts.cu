@@ -1,6 +1,8 @@
 // mmq_ts.cu — plan and entry point of the dequant-GEMM of mmq_ts.cuh (its kernels: mmq_ts_*.cu, two block types each).
 #include "mmq_ts.cuh"
 
+#include <mutex>
+
 namespace mrs {
 
 #define MRS_TS_TYPES(X) X(MRS_Q4_0) X(MRS_Q4_1) X(MRS_Q5_0) X(MRS_Q5_1) X(MRS_Q8_0) X(MRS_Q2_K) X(MRS_Q3_K) X(MRS_Q4_K) X(MRS_Q5_K) X(MRS_Q6_K)
@@ -12,17 +14,18 @@ static __device__ int g_ts_timeouts = 0;
 const TsDevice &ts_device() {
   constexpr int MAX = 64;
   static TsDevice devs[MAX] = {};
+  static std::once_flag once[MAX];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= MAX) dev = 0;
   TsDevice &d = devs[dev];
-  if (d.sms == 0) {                          // (several threads may get here: they write the same values, the count last)
+  std::call_once(once[dev], [&d, dev] {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    d.sms = sms > 0 ? sms : 148;
     ts_count_clusters(d.clusters);
     cudaGetSymbolAddress((void **)&d.timeouts, g_ts_timeouts);
-    d.sms = sms > 0 ? sms : 148;
-  }
+  });
   return d;
 }
 
