@@ -2,6 +2,7 @@
 #include "mmq_ts.cuh"
 
 #include <mutex>
+#include <string.h>
 
 namespace mrs {
 
@@ -9,24 +10,51 @@ namespace mrs {
 #define MRS_TS_EXTERN(T) extern template cudaError_t ts_launch<T>(const TsCall &);
 MRS_TS_TYPES(MRS_TS_EXTERN)
 
-static __device__ int g_ts_timeouts = 0;
+// A word a device that a kernel sets when a wait runs out: page-locked memory, so that the host sees it without waiting for anything.
+// Allocated once for the process (the first call may be inside a capture, which forbids allocations in its own mode).
+constexpr int TS_MAX_DEVICES = 64;
+static int32_t *ts_flags() {
+  static std::once_flag once;
+  static int32_t *flags = nullptr;
+  std::call_once(once, [] {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    const bool relaxed = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, TS_MAX_DEVICES * sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+      memset(p, 0, TS_MAX_DEVICES * sizeof(int32_t));
+      flags = (int32_t *)p;
+    } else {
+      (void)cudaGetLastError();
+    }
+    if (relaxed) cudaThreadExchangeStreamCaptureMode(&mode);
+  });
+  return flags;
+}
 
 const TsDevice &ts_device() {
-  constexpr int MAX = 64;
-  static TsDevice devs[MAX] = {};
-  static std::once_flag once[MAX];
+  static TsDevice devs[TS_MAX_DEVICES] = {};
+  static std::once_flag once[TS_MAX_DEVICES];
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= MAX) dev = 0;
+  if (dev < 0 || dev >= TS_MAX_DEVICES) dev = 0;
   TsDevice &d = devs[dev];
   std::call_once(once[dev], [&d, dev] {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     d.sms = sms > 0 ? sms : 148;
     ts_count_clusters(d.clusters);
-    cudaGetSymbolAddress((void **)&d.timeouts, g_ts_timeouts);
+    if (int32_t *flags = ts_flags()) {
+      void *seen = nullptr;
+      if (cudaHostGetDevicePointer(&seen, flags + dev, 0) == cudaSuccess) { d.timeouts = (int *)seen; d.flag = flags + dev; }
+      else (void)cudaGetLastError();
+    }
   });
   return d;
+}
+
+cudaError_t ts_refused(const TsDevice &d) {
+  if (d.flag == nullptr) return cudaErrorNotSupported;
+  return *(volatile const int32_t *)d.flag != 0 ? cudaErrorLaunchTimeout : cudaSuccess;
 }
 
 // Matrices of fewer rows are not split: results then stay bit for bit those of csrc/mmq_tc.cu, and so small a product is short
@@ -71,12 +99,15 @@ using namespace mrs;
 static int g_mmq_path = 0;
 extern "C" void mrs_mmq_set_path(int32_t path) { g_mmq_path = path; }
 
-// non-zero when a wait inside the kernel ever ran out on the current device (synchronises)
+// non-zero when a wait inside a kernel ever ran out on the current device (synchronises)
 extern "C" int32_t mrs_mmq_timeouts(void) {
-  int v = 0;
-  const cudaError_t e = cudaMemcpyFromSymbol(&v, g_ts_timeouts, sizeof(int));
-  return e == cudaSuccess ? v : -(int)e;
+  const cudaError_t e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) return -(int32_t)e;
+  const TsDevice &d = ts_device();
+  return d.flag != nullptr ? *(volatile const int32_t *)d.flag : -(int32_t)cudaErrorNotSupported;
 }
+// the word behind it, for callers that know the stream to be done (null without a device)
+extern "C" int32_t *mrs_mmq_timeout_flag(void) { return ts_device().flag; }
 
 // returns cudaErrorNotSupported when the launch does not fit this kernel (the caller falls back to mmq_tc.cu)
 extern "C" int32_t mrs_mmq_gguf_ts(int32_t ggml_type, const void *w, const void *x, void *y, int32_t M, int32_t N, int32_t K,
@@ -89,6 +120,8 @@ extern "C" int32_t mrs_mmq_gguf_ts(int32_t ggml_type, const void *w, const void 
   const bool common = ggml_type == MRS_Q8_0 || ggml_type == MRS_Q4_K || ggml_type == MRS_Q6_K;
   if (((uintptr_t)y & 15) && !(common && K % TS_SPAN_K == 0 && (K / elems * bytes) % 16 == 0)) return (int32_t)cudaErrorNotSupported;
   const TsDevice &d = ts_device();
+  const cudaError_t refused = ts_refused(d);
+  if (refused != cudaSuccess) return (int32_t)refused;
   // clocks that the dequantisers take for a span
   const int clocks = ggml_type == MRS_Q6_K ? 1500 : ggml_type == MRS_Q5_K || ggml_type == MRS_Q3_K || ggml_type == MRS_Q5_0 || ggml_type == MRS_Q5_1 ? 1350 : 1150;
   const TsPlan plan = ts_plan(M, N, K, bytes * (256 / elems), clocks, TS_SPLIT_MIN_ROWS, d);

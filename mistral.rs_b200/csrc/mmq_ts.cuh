@@ -23,7 +23,8 @@
 // after (before: one kernel for Q8_0, Q4_K and Q6_K with 128 or 256 tokens a tile and K whole, per-element decoding for the other types,
 // a kernel with 8 dequantising warps for int4): Q4_K 14336 x 4096, 24 tokens 29.2 / 18.4; Q5_K 4096 x 4096, 200 tokens 2516 / 20; Q8_0
 // 14336 x 4096, 4096 tokens 488 / 429; int4 14336 x 4096, 32 tokens 21.9 / 18.4; int4 with zero points 4096 x 14336, 500 tokens 170 / 69.
-// Every wait has a limit; one that runs out sets a device flag (mrs_mmq_timeouts) and ends the CTA.  What a limit counts is this grid's
+// Every wait has a limit; one that runs out ends the CTA and sets a word in host memory, after which the entry points refuse every call
+// on that device with cudaErrorLaunchTimeout (the word itself: mrs_mmq_timeout_flag, mrs_mmq_timeouts).  What a limit counts is this grid's
 // own work: in a programmatic-dependent-launch chain a warp passes pdl_wait before its first wait that the activations hold up.
 #pragma once
 #include "dequant.cuh"
@@ -95,7 +96,8 @@ __device__ __forceinline__ bool ts_wait(uint64_t *bar, uint32_t parity, int *tim
                  : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     if (__all_sync(0xffffffffu, done)) return true;
   } while (++n < TS_WAIT_LIMIT);
-  atomicExch(timeouts, 1);
+  *(volatile int *)timeouts = 1;
+  __threadfence_system();
   return false;
 }
 
@@ -906,8 +908,10 @@ template <int TYPE> cudaError_t ts_launch(const TsCall &c) {
 }
 
 // what a plan is made for and from: the current device, and the choice of token tile and split (mmq_ts.cu)
-struct TsDevice { int sms, clusters[9]; int *timeouts; };
+struct TsDevice { int sms, clusters[9]; int *timeouts; int32_t *flag; };   // the timeout word as the device and as the host address it
 const TsDevice &ts_device();
+// cudaErrorLaunchTimeout once a wait has run out on the device, cudaErrorNotSupported when there is no word to report it in
+cudaError_t ts_refused(const TsDevice &d);
 struct TsPlan { int nt, tiles_m, ksplit; };
 TsPlan ts_plan(int M, int N, int K, int span_bytes, int dequant_clocks, int split_min_rows, const TsDevice &d);
 

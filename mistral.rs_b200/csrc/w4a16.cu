@@ -359,6 +359,7 @@ static cudaError_t run_int4(const void *x, const void *w, const void *scales, co
   // scale and zero-point rows travel as bulk copies, which start on 16-byte boundaries (N makes their rows multiples of 16 bytes)
   if (((uintptr_t)scales & 15) || ((uintptr_t)qzeros & 15)) return cudaErrorMisalignedAddress;
   const TsDevice &d = ts_device();
+  if ((e = ts_refused(d)) != cudaSuccess) return e;
   // (a span of a row: 128 B of nibbles and its scales; the dequantisers take two operations a weight, some 800 clocks a span)
   const TsPlan plan = ts_plan(M, N, K, 128 + 2 * ((TS_SPAN_K + group - 1) / group), 800, 0, d);
   const TsCall c = {w, x, y, M, N, K, 0, dtype, plan.nt, plan.tiles_m, plan.ksplit, d.sms, d.timeouts, st, scales, qzeros, group, scale_perm, pdl ? 1 : 0};

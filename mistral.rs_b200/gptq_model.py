@@ -16,7 +16,7 @@ from dataclasses import dataclass
 import numpy as np
 import torch
 
-from . import kv_index, lib
+from . import kv_index, lib, mmq
 from .model import rope_tables, runner_split_pages
 
 
@@ -234,6 +234,12 @@ class GptqRunner:
     def reset(self, context_len=0):
         self.context_lens.fill_(context_len)
         self.error_flag.zero_()
+
+    def check_overflow(self):
+        """raises when a sequence ran past its context or a linear gave up waiting; synchronises"""
+        if int(self.error_flag.item()) & 1:
+            raise RuntimeError("GptqRunner: a sequence ran past its allocated context (KV write skipped)")
+        mmq.check_timeouts(self.dev)
 
     def capture(self):
         self.step(); self.reset()

@@ -1,7 +1,7 @@
 """Prefill (batch > 8) quantized GEMM — mirror of `fast_mmq::plain`
 (REF mistralrs-quant/src/gguf/fast_mmq.rs:762-826) on the tcgen05 dequant-GEMM kernel
-(`mrs_mmq_gguf`, csrc/mmq_tc.cu).  Unlike the reference there is no activation quantisation
-pass: activations stay bf16/f16 and weights are dequantised on the fly into shared memory."""
+(`mrs_mmq_gguf`, csrc/mmq_ts.cu).  Unlike the reference there is no activation quantisation
+pass: activations stay bf16/f16 and weights are dequantised on the fly into tensor memory."""
 import ctypes
 
 import torch
@@ -31,6 +31,18 @@ def forward(w, xs: torch.Tensor) -> torch.Tensor:
     if rc != 0:
         raise RuntimeError(f"mrs_mmq_gguf failed with cudaError {rc}")
     return out
+
+
+def check_timeouts(device):
+    """Raises when a wait inside the dequantising GEMM (ggml and int4 linears) ever ran out on `device`: results since then are incomplete.
+    Reads a word in host memory, so call it once the work in question is done.  Calls refuse to launch by themselves from then on; replays of a
+    graph pass no entry point and need this."""
+    with torch.cuda.device(device):
+        fn = lib().mrs_mmq_timeout_flag
+        fn.restype = ctypes.POINTER(ctypes.c_int32)
+        flag = fn()
+    if flag and flag[0]:
+        raise RuntimeError("a wait inside the dequantising GEMM ran out: the results of this device are incomplete")
 
 
 def set_path(path: str):

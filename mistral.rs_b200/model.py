@@ -16,7 +16,7 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
-from . import BLOCK_BYTES, BLOCK_ELEMS, GGML, kv_index, lib
+from . import BLOCK_BYTES, BLOCK_ELEMS, GGML, kv_index, lib, mmq
 
 F16_FIELDS = {"q4_0": [0], "q4_1": [0, 2], "q5_0": [0], "q5_1": [0, 2], "q8_0": [0],
               "q2_k": [80, 82], "q3_k": [108], "q4_k": [0, 2], "q5_k": [0, 2], "q6_k": [208]}
@@ -633,6 +633,7 @@ class LlamaRunner:
     def check_overflow(self):
         if int(self.error_flag.item()) & 1:
             raise RuntimeError("LlamaRunner: a sequence ran past its allocated context (KV write skipped)")
+        mmq.check_timeouts(self.dev)      # (of prompts read on the same device; the flag above was read behind them)
 
     def capture(self):
         self.step(); self.reset()  # warm-up outside capture (module load, attributes)

@@ -39,6 +39,8 @@ extern "C" {
     pub fn mrs_mmq_set_weight_format(fmt: i32);
     pub fn mrs_mmq_set_path(path: i32);
     pub fn mrs_mmq_gguf_ts(ggml_type: i32, w: *const c_void, x: *const c_void, y: *mut c_void, M: i32, N: i32, K: i32, dtype: i32, stream: *mut c_void) -> i32;
+    pub fn mrs_mmq_timeouts() -> i32;
+    pub fn mrs_mmq_timeout_flag() -> *mut i32;
     pub fn mrs_gptq_gemm(x: *const c_void, qweight: *const i32, scales: *const c_void, qzeros: *const i32, g_idx: *const i32, y: *mut c_void, M: i32, K: i32, N: i32, group_size: i32, is_awq: i32, stream: *mut c_void) -> i32;
     pub fn mrs_w4a16_gemm(x: *const c_void, w_tiles: *const c_void, scales: *const c_void, qzeros: *const i32, y: *mut c_void, M: i32, K: i32, N: i32, group: i32, dtype: i32, scale_perm: i32, stream: *mut c_void) -> i32;
     pub fn mrs_dense_linear(x: *const c_void, w: *const c_void, y: *mut c_void, M: i32, K: i32, N: i32, dtype: i32, stream: *mut c_void) -> i32;

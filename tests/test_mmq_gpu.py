@@ -1,6 +1,8 @@
 """Prefill tcgen05 dequant-GEMM vs the oracle's EXACT product (f64 sum of deq(w)*x) — the
 known-answer structure of the reference's own GEMM test (packed_affine.rs:967-1000:
 quantized product == dequantize() . x, max abs <= 0.08, mean <= 0.01 on patterned inputs)."""
+import os
+
 import numpy as np
 import pytest
 import torch
@@ -108,3 +110,54 @@ def test_every_type_at_tile_edges(cuda, dtype, dt, M, N, K):
 def test_ragged_last_span(cuda, dtype, K):
     """32-wide types take any multiple of 64 columns: the last 256 are partly past the row."""
     _check(dtype, 33, 1100, K, "bf16", 13)
+
+
+def test_calls_are_refused_once_a_wait_has_run_out(cuda):
+    """The word that a kernel sets when a wait runs out, set here by the host: ggml and int4 calls and the runners' check report it."""
+    import ctypes
+    from mistralrs_b200 import gptq, lib
+    K, N = 256, 64
+    w = quant.QTensor(to_dev(make_weight("q4_k", N, K, 1).reshape(-1), cuda), "q4_k", (N, K))
+    int4 = gptq.GptqMarlinLayer(torch.zeros(K // 8, N, dtype=torch.int32, device=cuda), torch.ones(K // 64, N, dtype=torch.float16, device=cuda), group_size=64)
+    x = torch.ones(9, K, dtype=torch.float16, device=cuda)
+    want = [mmq.forward(w, x), int4.forward_raw(x)]
+    assert lib().mrs_mmq_timeouts() == 0
+    fn = lib().mrs_mmq_timeout_flag
+    fn.restype = ctypes.POINTER(ctypes.c_int32)
+    flag = fn()
+    try:
+        flag[0] = 1
+        for call in (lambda: mmq.forward(w, x), lambda: int4.forward_raw(x)):
+            with pytest.raises(RuntimeError, match="702"):
+                call()
+        with pytest.raises(RuntimeError, match="ran out"):
+            mmq.check_timeouts(cuda)
+        assert lib().mrs_mmq_timeouts() == 1
+    finally:
+        flag[0] = 0
+    mmq.check_timeouts(cuda)
+    assert torch.equal(mmq.forward(w, x), want[0]) and torch.equal(int4.forward_raw(x), want[1])
+
+
+def test_first_call_of_a_process_inside_a_capture(cuda):
+    """The first call sets up what calls on a device share; a capture does not forbid it."""
+    import subprocess
+    import sys
+    code = """
+import torch
+from __graft_entry__ import load_package
+load_package()
+from mistralrs_b200 import mmq, quant
+w = quant.QTensor(torch.randint(0, 64, (64 * 144,), dtype=torch.uint8, device='cuda'), 'q4_k', (64, 256))
+x = torch.ones(9, 256, dtype=torch.bfloat16, device='cuda')
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    y = mmq.forward(w, x)
+g.replay()
+torch.cuda.synchronize()
+assert torch.equal(y, mmq.forward(w, x))
+mmq.check_timeouts(x.device)
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]
