@@ -699,10 +699,13 @@ class RoutedExperts:
         if self.n_routes > self.n_experts and not gated:
             raise NotImplementedError("identity experts come beside gated experts")
 
-    def groups_weights(self, n_tok):
+    def grouped_fits(self):
         if self._grouped is None:
             self._grouped = K.moe_grouped_fits(self.w_down.dtype, self.w_down.shape[1], self.w_down.shape[2])
-        return (self._grouped and n_tok >= self.GROUPED_MIN_TOKENS and n_tok * self.top <= self.GROUPED_PER_EXPERT * self.n_experts
+        return self._grouped
+
+    def groups_weights(self, n_tok):
+        return (self.grouped_fits() and n_tok >= self.GROUPED_MIN_TOKENS and n_tok * self.top <= self.GROUPED_PER_EXPERT * self.n_experts
                 and not self.outgrows_groups(n_tok))
 
     def outgrows_groups(self, n_tok):
@@ -724,7 +727,7 @@ class RoutedExperts:
 
     def streams_weights(self, n_tok):
         per_expert = 4 if self.expert_bytes() <= self.SMALL_EXPERT_BYTES else 2
-        return n_tok * self.top <= per_expert * self.n_experts and not (self._grouped and self.outgrows_groups(n_tok))
+        return n_tok * self.top <= per_expert * self.n_experts and not (self.grouped_fits() and self.outgrows_groups(n_tok))
 
     def route(self, h):
         logits = K.router_logits(h, self.w_router, self.w_router16)
