@@ -8,7 +8,8 @@
  *     [RMSNorm + Q8_1 + fused QKV GEMV] -> RoPE -> KV-cache write -> paged decode attention
  *     -> [Q8_1 + o_proj GEMV + residual] -> [RMSNorm + Q8_1 + gate/up GEMV + SiLU*mul]
  *     -> [Q8_1 + down GEMV + residual]
- * with the bracketed groups being single `mrs_mmvq_fused` launches.
+ * with the bracketed groups being single `mrs_mmvq_fused` launches (larger steps: one launch for the norm and the
+ * quantisation, then the GEMVs; see `q8`).
  */
 #ifndef MRS_B200_MODEL_H
 #define MRS_B200_MODEL_H
@@ -60,7 +61,7 @@ typedef struct {
   int32_t batch, padded_tiles, max_blocks_per_seq;
   int32_t skip_mask;         /* measurement only: bit0 skip rope/cache/attention, bit1 skip the GEMVs */
   int32_t fused_attention;   /* 1: mrs_paged_decode_fused; 0: rotary + reshape_and_cache + flashinfer_decode */
-  int32_t reserved0;
+  int32_t extension;         /* 0, or MRS_LLAMA_STEP_Q8: the fields behind `tp` are there */
   int32_t *token_ids;        /* [batch] in: token to process; out_token may alias it */
   int32_t *positions;        /* [batch] */
   int64_t *slot_mapping;     /* [batch] */
@@ -77,7 +78,13 @@ typedef struct {
   void (*all_reduce)(void *buf, int64_t count, int32_t dtype, void *stream, void *user);
   void *all_reduce_user;
   const mrs_tp_ctx *tp;      /* non-NULL with world > 1: peer-memory sum (takes precedence over all_reduce) */
+  /* Only read when `extension` is MRS_LLAMA_STEP_Q8.  Scratch for Q8_1 rows, 4-byte aligned: from five sequences on, and for fewer from
+   * batch x columns = 16384 on, a projection's input is quantised once into it (batch * columns / 32 * 36 bytes) instead of by every CTA of the
+   * GEMVs that read it; same bits, less time.  Where the buffer is absent or too small the fused launch serves.  The step uses none of its
+   * other buffers for this: the logits of a step are valid until the next step's head writes them. */
+  void *q8; int64_t q8_bytes;
 } mrs_llama_step;
+#define MRS_LLAMA_STEP_Q8 0x51380001
 
 /* Enqueue one decode step (all layers + lm_head + argmax) on `stream`. Returns cudaError. */
 int32_t mrs_llama_decode_step(const mrs_llama_step *s, void *stream);

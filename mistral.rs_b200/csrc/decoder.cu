@@ -390,17 +390,18 @@ extern "C" int32_t mrs_llama_decode_step(const mrs_llama_step *s, void *stream) 
   // without it: four layers 4096 wide (K = 4096 and 14336), Q4_K_M, 2 sequences 358 (down projection alone) / 376, all products 402;
   // 3 sequences 484 (down alone) / 529, all 491; 4: 507 / 573; 8: 751 / 1028.  Six layers 2048 wide (K = 2048 and 5632): 2 sequences 298
   // (down alone) / 288; 3: 375 (down alone) / 384, all 416; 4: 408 (down alone) / 417, all 433; 5: 543 / 610; 8: 587 / 716.  (A single row
-  // stays fused, however long: behind the GEMV before it the launch is not free.)  The quantised rows' place is a buffer that is not in
-  // use yet: the logits, for the head itself the feed-forward's.
+  // stays fused, however long: behind the GEMV before it the launch is not free.)  The rows go to a buffer of their own: nothing else of the
+  // step is overwritten, the last step's logits among them.
+  const bool extended = s->extension == MRS_LLAMA_STEP_Q8 && ((uintptr_t)s->q8 & 3) == 0;
+  void *const q8 = extended ? s->q8 : nullptr;
+  const int64_t q8_bytes = q8 != nullptr ? s->q8_bytes : 0;
   auto gemv = [&](const mrs_qweight &w0, int mode, const void *w1, const void *w2, const void *x, const void *norm_w, const void *residual, void *d0,
-                  void *d1, void *d2, int K, int n0, int n1, int n2, void *place, int64_t place_bytes, bool quantised) -> int {
-    if (!((B >= 5 || (B >= 2 && (int64_t)B * K >= 16384)) && K % 32 == 0 && ((uintptr_t)place & 3) == 0 && (int64_t)B * (K / 32) * 36 <= place_bytes))
+                  void *d1, void *d2, int K, int n0, int n1, int n2, bool quantised) -> int {
+    if (!((B >= 5 || (B >= 2 && (int64_t)B * K >= 16384)) && K % 32 == 0 && (int64_t)B * (K / 32) * 36 <= q8_bytes))
       return mrs_mmvq_fused(w0.ggml_type, mode, dt, w0.data, w1, w2, x, norm_w, s->rms_eps, residual, d0, d1, d2, K, n0, n1, n2, B, 0, pdl, stream);
-    if (!quantised) MRS_TRY(mrs_rms_quantize_q8_1(dt, x, norm_w, s->rms_eps, K, B, place, pdl, stream));
-    return mrs_mmvq_q8(w0.ggml_type, mode, dt, w0.data, w1, w2, place, residual, d0, d1, d2, K, n0, n1, n2, B, 0, pdl, stream);
+    if (!quantised) MRS_TRY(mrs_rms_quantize_q8_1(dt, x, norm_w, s->rms_eps, K, B, q8, pdl, stream));
+    return mrs_mmvq_q8(w0.ggml_type, mode, dt, w0.data, w1, w2, q8, residual, d0, d1, d2, K, n0, n1, n2, B, 0, pdl, stream);
   };
-  void *const place = s->logits;
-  const int64_t place_bytes = (int64_t)B * s->vocab * 2, act_bytes = s->n_layers > 0 ? (int64_t)B * s->layers[0].w_gate.rows * 2 : 0;
   MRS_TRY(mrs_embedding_gather(s->tok_embd.ggml_type, s->tok_embd.data, H, s->token_ids, B, s->x, dt, stream));
   void *hidden = s->x, *hidden2 = s->x2;
   for (int l = 0; l < s->n_layers; l++) {
@@ -410,17 +411,17 @@ extern "C" int32_t mrs_llama_decode_step(const mrs_llama_step *s, void *stream) 
     // overrides (GGUF --tensor-type, per-layer UQFF topologies) take separate launches
     if (!do_gemv) {
     } else if (L.wq.ggml_type != L.wk.ggml_type) {
-      MRS_TRY(gemv(L.wq, 0, nullptr, nullptr, hidden, L.attn_norm, nullptr, s->q, nullptr, nullptr, H, nq, 0, 0, place, place_bytes, false));
-      MRS_TRY(gemv(L.wk, 0, nullptr, nullptr, hidden, L.attn_norm, nullptr, s->k, nullptr, nullptr, H, nkv, 0, 0, place, place_bytes, true));
-      MRS_TRY(gemv(L.wv, 0, nullptr, nullptr, hidden, L.attn_norm, nullptr, s->v, nullptr, nullptr, H, nkv, 0, 0, place, place_bytes, true));
+      MRS_TRY(gemv(L.wq, 0, nullptr, nullptr, hidden, L.attn_norm, nullptr, s->q, nullptr, nullptr, H, nq, 0, 0, false));
+      MRS_TRY(gemv(L.wk, 0, nullptr, nullptr, hidden, L.attn_norm, nullptr, s->k, nullptr, nullptr, H, nkv, 0, 0, true));
+      MRS_TRY(gemv(L.wv, 0, nullptr, nullptr, hidden, L.attn_norm, nullptr, s->v, nullptr, nullptr, H, nkv, 0, 0, true));
     } else if (L.wk.ggml_type == L.wv.ggml_type) {
-      MRS_TRY(gemv(L.wq, 2, L.wk.data, L.wv.data, hidden, L.attn_norm, nullptr, s->q, s->k, s->v, H, nq, nkv, nkv, place, place_bytes, false));
+      MRS_TRY(gemv(L.wq, 2, L.wk.data, L.wv.data, hidden, L.attn_norm, nullptr, s->q, s->k, s->v, H, nq, nkv, nkv, false));
     } else {
       // Q4_K_M keeps attn_v in Q6_K on some layers: q∥k fused, v on its own.  (The one-grid form,
       // mrs_mmvq_fused_qkv_mixed, measured 0.7 % slower here: under PDL the small v launch already
       // hides behind the q∥k tail, and q∥k loses the CTAs it hands to v.)
-      MRS_TRY(gemv(L.wq, 2, L.wk.data, nullptr, hidden, L.attn_norm, nullptr, s->q, s->k, nullptr, H, nq, nkv, 0, place, place_bytes, false));
-      MRS_TRY(gemv(L.wv, 0, nullptr, nullptr, hidden, L.attn_norm, nullptr, s->v, nullptr, nullptr, H, nkv, 0, 0, place, place_bytes, true));
+      MRS_TRY(gemv(L.wq, 2, L.wk.data, nullptr, hidden, L.attn_norm, nullptr, s->q, s->k, nullptr, H, nq, nkv, 0, false));
+      MRS_TRY(gemv(L.wv, 0, nullptr, nullptr, hidden, L.attn_norm, nullptr, s->v, nullptr, nullptr, H, nkv, 0, 0, true));
     }
     if (do_attn && s->fused_attention) {
       MRS_TRY(mrs_paged_decode_fused(s->q, s->k, s->v, L.k_cache, L.v_cache, s->rope_cos, s->rope_sin, s->positions,
@@ -447,32 +448,32 @@ extern "C" int32_t mrs_llama_decode_step(const mrs_llama_step *s, void *stream) 
     if (s->tp != nullptr && s->tp->world > 1) {
       // row-parallel partial -> this rank's slot buffer -> peer-memory sum + residual (one kernel, on the PDL chain)
       void *part = (uint8_t *)s->tp->peer_base[s->tp->rank] + s->tp->slot_offset[0];
-      MRS_TRY(gemv(L.wo, 0, nullptr, nullptr, s->attn_out, nullptr, nullptr, part, nullptr, nullptr, nq, H, 0, 0, place, place_bytes, false));
+      MRS_TRY(gemv(L.wo, 0, nullptr, nullptr, s->attn_out, nullptr, nullptr, part, nullptr, nullptr, nq, H, 0, 0, false));
       MRS_TRY(mrs_tp_allreduce_residual(s->tp, 0, hidden, hidden2, B * H, dt, pdl, stream));
     } else if (s->all_reduce == nullptr) {
-      MRS_TRY(gemv(L.wo, 0, nullptr, nullptr, s->attn_out, nullptr, hidden, hidden2, nullptr, nullptr, nq, H, 0, 0, place, place_bytes, false));
+      MRS_TRY(gemv(L.wo, 0, nullptr, nullptr, s->attn_out, nullptr, hidden, hidden2, nullptr, nullptr, nq, H, 0, 0, false));
     } else {  // row-parallel: partial sums -> all-reduce -> residual add (REF distributed/layers.rs:965-975)
-      MRS_TRY(gemv(L.wo, 0, nullptr, nullptr, s->attn_out, nullptr, nullptr, hidden2, nullptr, nullptr, nq, H, 0, 0, place, place_bytes, false));
+      MRS_TRY(gemv(L.wo, 0, nullptr, nullptr, s->attn_out, nullptr, nullptr, hidden2, nullptr, nullptr, nq, H, 0, 0, false));
       s->all_reduce(hidden2, (int64_t)B * H, dt, stream, s->all_reduce_user);
       add_residual_kernel<<<(unsigned)(((int64_t)B * H + 255) / 256), 256, 0, st>>>(hidden2, hidden, (int64_t)B * H, dt);
     }
     // --- MLP block: x = x + down(silu(gate(norm(x))) * up(norm(x)))
     if (L.w_gate.ggml_type != L.w_up.ggml_type || L.w_gate.rows != L.w_up.rows) return (int32_t)cudaErrorInvalidValue;
-    MRS_TRY(gemv(L.w_gate, 1, L.w_up.data, nullptr, hidden2, L.ffn_norm, nullptr, s->act, nullptr, nullptr, H, L.w_gate.rows, L.w_gate.rows, 0, place, place_bytes, false));
+    MRS_TRY(gemv(L.w_gate, 1, L.w_up.data, nullptr, hidden2, L.ffn_norm, nullptr, s->act, nullptr, nullptr, H, L.w_gate.rows, L.w_gate.rows, 0, false));
     if (s->tp != nullptr && s->tp->world > 1) {
       void *part = (uint8_t *)s->tp->peer_base[s->tp->rank] + s->tp->slot_offset[1];
-      MRS_TRY(gemv(L.w_down, 0, nullptr, nullptr, s->act, nullptr, nullptr, part, nullptr, nullptr, L.w_down.cols, H, 0, 0, place, place_bytes, false));
+      MRS_TRY(gemv(L.w_down, 0, nullptr, nullptr, s->act, nullptr, nullptr, part, nullptr, nullptr, L.w_down.cols, H, 0, 0, false));
       MRS_TRY(mrs_tp_allreduce_residual(s->tp, 1, hidden2, hidden, B * H, dt, pdl, stream));
     } else if (s->all_reduce == nullptr) {
-      MRS_TRY(gemv(L.w_down, 0, nullptr, nullptr, s->act, nullptr, hidden2, hidden, nullptr, nullptr, L.w_down.cols, H, 0, 0, place, place_bytes, false));
+      MRS_TRY(gemv(L.w_down, 0, nullptr, nullptr, s->act, nullptr, hidden2, hidden, nullptr, nullptr, L.w_down.cols, H, 0, 0, false));
     } else {
-      MRS_TRY(gemv(L.w_down, 0, nullptr, nullptr, s->act, nullptr, nullptr, hidden, nullptr, nullptr, L.w_down.cols, H, 0, 0, place, place_bytes, false));
+      MRS_TRY(gemv(L.w_down, 0, nullptr, nullptr, s->act, nullptr, nullptr, hidden, nullptr, nullptr, L.w_down.cols, H, 0, 0, false));
       s->all_reduce(hidden, (int64_t)B * H, dt, stream, s->all_reduce_user);
       add_residual_kernel<<<(unsigned)(((int64_t)B * H + 255) / 256), 256, 0, st>>>(hidden, hidden2, (int64_t)B * H, dt);
     }
   }
   if (do_gemv)
-  MRS_TRY(gemv(s->lm_head, 0, nullptr, nullptr, hidden, s->final_norm, nullptr, s->logits, nullptr, nullptr, H, s->vocab, 0, 0, s->act, act_bytes, false));
+  MRS_TRY(gemv(s->lm_head, 0, nullptr, nullptr, hidden, s->final_norm, nullptr, s->logits, nullptr, nullptr, H, s->vocab, 0, 0, false));
   MRS_TRY(mrs_argmax(s->logits, B, s->vocab, dt, s->out_token, s->argmax_scratch, pdl, stream));
   return 0;
 }

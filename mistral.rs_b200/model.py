@@ -125,13 +125,17 @@ class _Step(ctypes.Structure):
                 ("pdl", ctypes.c_int32), ("layers", ctypes.POINTER(_Layer)), ("tok_embd", _QW), ("lm_head", _QW),
                 ("final_norm", ctypes.c_void_p), ("rope_cos", ctypes.c_void_p), ("rope_sin", ctypes.c_void_p),
                 ("batch", ctypes.c_int32), ("padded_tiles", ctypes.c_int32), ("max_blocks_per_seq", ctypes.c_int32),
-                ("skip_mask", ctypes.c_int32), ("fused_attention", ctypes.c_int32), ("reserved0", ctypes.c_int32)] + \
+                ("skip_mask", ctypes.c_int32), ("fused_attention", ctypes.c_int32), ("extension", ctypes.c_int32)] + \
                [(n, ctypes.c_void_p) for n in ("token_ids", "positions", "slot_mapping", "kv_indptr", "kv_indices",
                                                "kv_last_page_len", "request_indices", "kv_tile_indices", "o_indptr",
                                                "kv_chunk_size", "block_valid_mask", "x", "x2", "q", "k", "v",
                                                "attn_out", "act", "logits", "tmp_v", "tmp_s", "out_token",
                                                "attn_counters", "argmax_scratch")] + \
-               [("all_reduce", _AR_FN), ("all_reduce_user", ctypes.c_void_p), ("tp", ctypes.c_void_p)]
+               [("all_reduce", _AR_FN), ("all_reduce_user", ctypes.c_void_p), ("tp", ctypes.c_void_p),
+                ("q8", ctypes.c_void_p), ("q8_bytes", ctypes.c_int64)]
+
+
+STEP_Q8 = 0x51380001       # MRS_LLAMA_STEP_Q8: q8 and q8_bytes are set
 
 
 class _TpCtx(ctypes.Structure):
@@ -579,6 +583,9 @@ class LlamaRunner:
             setattr(s, n, t.data_ptr())
         for n, t in self.buf.items():
             setattr(s, n, t.data_ptr())
+        # the projections' inputs as Q8_1 rows (36 bytes for 32 columns), quantised once for a step of several sequences
+        self.q8 = torch.empty(batch * max(H, self.n_heads * cfg.head_dim, cfg.inter // tp) // 32 * 36, dtype=torch.uint8, device=dev)
+        s.extension, s.q8, s.q8_bytes = STEP_Q8, self.q8.data_ptr(), self.q8.numel()
         self._ar_cb, self._peer = None, peer_allreduce
         if peer_allreduce is not None:     # in-graph peer-memory sum (takes precedence over the callback)
             s.tp = peer_allreduce.pointer()
