@@ -199,3 +199,39 @@ def test_one_row_at_any_address(cuda, offset):
     aligned = x.clone().reshape(1, K)
     assert torch.equal(quant.plain(w, x).reshape(1, -1), quant.plain(w, aligned))
     assert torch.equal(quant.plain(w, torch.cat([aligned, aligned]))[:1], quant.plain(w, aligned))
+
+
+@pytest.mark.parametrize("pdl", [0, 1])
+@pytest.mark.parametrize("dtype", ["q4_k", "q6_k", "q8_0"])
+@pytest.mark.parametrize("rows,K", [(2, 2304), (5, 1024), (8, 2048)])
+def test_every_mode_over_rows_quantised_apart(cuda, dtype, rows, K, pdl):
+    """QKV, GLU and a residual over rows that a launch before quantised, in the chain of a decode step: one buffer, quantised again behind every
+    GEMV that reads it, with and without programmatic launches.  The bits of mrs_mmvq_fused."""
+    import ctypes
+    from mistralrs_b200 import GGML, lib
+    gen = torch.Generator(device=cuda).manual_seed(K + rows)
+    rand = lambda *s: torch.randn(*s, device=cuda, generator=gen).to(torch.bfloat16)
+    weight = lambda n, seed: quant.QTensor(to_dev(make_weight(dtype, n, K, seed).reshape(-1), cuda), dtype, (n, K))
+    x, h, nw = rand(rows, K), rand(rows, K), (1 + 0.1 * rand(K).float()).to(torch.bfloat16)
+    wq, wk, wv, gate, up, wo = (weight(n, i) for i, n in enumerate((160, 64, 64, 96, 96, K)))
+    res = rand(rows, K)
+    want = [*quant.mmvq_fused(wq, x, mode=2, w1=wk, w2=wv, norm_w=nw), quant.mmvq_fused(gate, h, mode=1, w1=up, norm_w=nw),
+            quant.mmvq_fused(wo, h, residual=res)]
+    got = [torch.empty_like(w) for w in want]
+    q8 = torch.empty(rows * (K // 32) * 36, dtype=torch.uint8, device=cuda)
+    P, I = (lambda t: ctypes.c_void_p(t.data_ptr() if t is not None else 0)), ctypes.c_int
+    st = ctypes.c_void_p(torch.cuda.current_stream(cuda).cuda_stream)
+
+    def apart(mode, inp, norm, ws, residual, outs):
+        ws, outs = list(ws) + [None] * (3 - len(ws)), list(outs) + [None] * (3 - len(outs))
+        n = [0 if w is None else w.shape[0] for w in ws]
+        assert lib().mrs_rms_quantize_q8_1(I(1), P(inp), P(norm), ctypes.c_float(1e-5), I(K), I(rows), P(q8), I(pdl), st) == 0
+        assert lib().mrs_mmvq_q8(I(GGML[dtype]), I(mode), I(1), *(P(w.data if w is not None else None) for w in ws), P(q8), P(residual),
+                                 *(P(o) for o in outs), I(K), *(I(v) for v in n), I(rows), I(0), I(pdl), st) == 0
+
+    for _ in range(3):
+        apart(2, x, nw, (wq, wk, wv), None, got[:3])
+        apart(1, h, nw, (gate, up), None, got[3:4])
+        apart(0, h, None, (wo,), res, got[4:])
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, w) for g, w in zip(got, want))
