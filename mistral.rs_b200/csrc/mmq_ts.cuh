@@ -58,6 +58,7 @@ struct TsParams {
   const uint8_t *scales;
   const uint8_t *qzeros;      // AWQ [K/group][N/8] words, or null: zero point 8
   int group, scale_perm;      // scale_perm: columns 0 plain, 1 / 2 Marlin-permuted 64 / 32 wide
+  int group32, group_shift;   // group / 32, and its logarithm or -1
   int pdl;                    // link of a programmatic-dependent-launch chain: x comes from, y may be read by, the grid before
 };
 
@@ -710,13 +711,14 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
         typename std::conditional<TYPE == TS_INT4, TsInt4<BF>, TsUnit<TYPE, ALIGNED, BF>>::type u;
         if constexpr (TYPE == TS_INT4) {
           u.a = lds128(row0 + stage + (uint32_t)(part * TS_I4_CHUNK)); u.b = lds128(row0 + stage + (uint32_t)(part * TS_I4_CHUNK) + 16u);
-          // each 32 weights' group, counted from the span's first (uniform)
-          int k_in_g = (s * TS_SPAN_K) % p.group + 64 * part, g = 0;
+          // each 32 weights' group, counted from the span's first (uniform); in units of 32 weights, by shifts where a group is a power of two
+          const uint32_t u0 = (uint32_t)(s * (TS_SPAN_K / 32)), u1 = u0 + 2u * (uint32_t)part;
+          const uint32_t g0 = p.group_shift >= 0 ? u0 >> p.group_shift : u0 / (uint32_t)p.group32;
 #pragma unroll
-          for (int h = 0; h < 2; h++, k_in_g += 32) {
-            for (; k_in_g >= p.group; g++) k_in_g -= p.group;
-            u.s[h] = lds_u16s(scale0 + stage + (uint32_t)(g * TS_BM * 2));
-            u.z[h] = p.qzeros != nullptr ? (lds32(zero0 + stage + (uint32_t)(g * 64)) >> zero_shift) & 0xFu : 8u;
+          for (uint32_t h = 0; h < 2; h++) {
+            const uint32_t g = (p.group_shift >= 0 ? (u1 + h) >> p.group_shift : (u1 + h) / (uint32_t)p.group32) - g0;
+            u.s[h] = lds_u16s(scale0 + stage + g * (TS_BM * 2));
+            u.z[h] = p.qzeros != nullptr ? (lds32(zero0 + stage + g * 64u) >> zero_shift) & 0xFu : 8u;
           }
           u.template half<0>(o);
         } else {
@@ -866,6 +868,8 @@ template <int TYPE, bool ALIGNED> static cudaError_t ts_launch_as(const TsCall &
   TsParams p = {};
   p.w = (const uint8_t *)c.w; p.y = c.y; p.timeouts = c.timeouts; p.M = c.M; p.N = c.N; p.K = c.K; p.row_bytes = c.row_bytes;
   p.scales = (const uint8_t *)c.scales; p.qzeros = (const uint8_t *)c.qzeros; p.group = c.group; p.scale_perm = c.scale_perm; p.pdl = c.pdl;
+  p.group32 = c.group / 32; p.group_shift = -1;
+  for (int i = 0; i < 26; i++) if (p.group32 == 1 << i) p.group_shift = i;
   p.nt = c.nt; p.tiles_m = c.tiles_m; p.tiles_n = (c.N + TS_BM - 1) / TS_BM; p.ksplit = c.ksplit;
   // Fewer and larger X stages where the tokens are few: each costs the issuer a wait and a commit.  Three raw stages (two where three do
   // not fit), the rest of the memory first to X up to its limit: a stage's round trip (products retire, copy from L2) takes some 2500
