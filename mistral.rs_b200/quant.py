@@ -132,15 +132,20 @@ def _fused_entry():
     return typed("mrs_mmvq_fused", _I, _I, _I, _P, _P, _P, _P, _P, _F, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P)
 
 
-# One row of up to this many columns is quantised inside the GEMV (`mrs_mmvq_fused`, the same bits) instead of by a launch before it: every CTA
-# repeats the work, which is the smaller cost while the row is short.  us, two launches / one, Q4_K on one B200: 2048 columns 4.5 / 3.3,
-# 4096 7.1 / 5.7 (14336 rows 12.3 / 11.1), 14336 12.0 / 14.7; two rows of 4096 7.8 / 8.1, eight 13.9 / 22.6.
-ONE_LAUNCH_MAX_K = 8192
+# One row of up to so many columns is quantised inside the GEMV (`mrs_mmvq_fused`, the same bits) instead of by a launch before it: every CTA
+# repeats the work, which is the smaller cost while the row is short.  One B200, device time of one launch / two, mean and worst of ten block
+# types, 1024 / 4096 / 14336 rows: 2048 columns 0.78 / 0.83 / 0.90 (worst 0.98), 4096 columns 0.88 / 0.85 / 0.92 (0.98), 5120 and 6144
+# columns 0.97 (1.07) / 0.92 (0.98) / 0.96 (0.99), 7168 columns 1.05 (1.20) / 0.99 (1.05) / 1.00 (1.03), 8192 columns 1.04 (1.18) / 1.01 (1.08) /
+# 1.01 (1.06); Q4_K 14336 columns 1.23.  Two rows of 4096 7.8 us / 8.1, eight 13.9 / 22.6.  Outside a graph the host is the bound, 14 us a call
+# against 23, so there the line is where the device's loss would outgrow that.
+ONE_LAUNCH_MAX_K, ONE_LAUNCH_CAPTURED = 8192, ((4096, 0), (6144, 4096))      # captured: (columns, from so many rows on)
 
 
-def _one_launch(b_size, k, xs):
+def _one_launch(b_size, k, nrows, xs):
     # (the fused prologue reads 16 bytes at a time; the quantising launch takes any element address)
-    return b_size == 1 and k <= ONE_LAUNCH_MAX_K and xs.data_ptr() % 16 == 0
+    if b_size != 1 or k > ONE_LAUNCH_MAX_K or xs.data_ptr() % 16 != 0:
+        return False
+    return any(k <= most and nrows >= least for most, least in ONE_LAUNCH_CAPTURED) or not torch.cuda.is_current_stream_capturing()
 
 
 def _fused_one_row(mode, ws, xs, outs, k, activation=0):
@@ -205,7 +210,7 @@ def plain(w: QTensor, xs: torch.Tensor) -> torch.Tensor:
     nrows, ncols, k, b_size = _check_common("fast_mmvq", w, xs)
     xs = xs.contiguous()
     out = xs.new_empty((*xs.shape[:-1], nrows))
-    if _one_launch(b_size, k, xs):
+    if _one_launch(b_size, k, nrows, xs):
         _fused_one_row(0, (w,), xs, (out,), k)
         return out
     scratch, stride_col_y = _quantize_into_workspace(xs, k, b_size)
@@ -224,7 +229,7 @@ def fused_glu(gate_w: QTensor, up_w: QTensor, xs: torch.Tensor, activation: GluA
     nrows, ncols, k, b_size = _check_common("fast_mmvq fused_glu", gate_w, xs)
     xs = xs.contiguous()
     out = xs.new_empty((*xs.shape[:-1], nrows))
-    if _one_launch(b_size, k, xs):
+    if _one_launch(b_size, k, nrows, xs):
         _fused_one_row(1, (gate_w, up_w), xs, (out,), k, int(activation))
         return out
     scratch, stride_col_y = _quantize_into_workspace(xs, k, b_size)
@@ -244,7 +249,7 @@ def fused_qkv(q_w: QTensor, k_w: QTensor, v_w: QTensor, xs: torch.Tensor):
     _, _, k, b_size = _check_common("fast_mmvq fused_qkv", q_w, xs)
     xs = xs.contiguous()
     outs = [xs.new_empty((*xs.shape[:-1], w.shape[0])) for w in (q_w, k_w, v_w)]
-    if _one_launch(b_size, k, xs):
+    if _one_launch(b_size, k, sum(w.shape[0] for w in (q_w, k_w, v_w)), xs):
         _fused_one_row(2, (q_w, k_w, v_w), xs, outs, k)
         return tuple(outs)
     scratch, stride_col_y = _quantize_into_workspace(xs, k, b_size)

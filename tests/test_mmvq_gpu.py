@@ -235,3 +235,18 @@ def test_every_mode_over_rows_quantised_apart(cuda, dtype, rows, K, pdl):
         apart(0, h, None, (wo,), res, got[4:])
     torch.cuda.synchronize()
     assert all(torch.equal(g, w) for g, w in zip(got, want))
+
+
+@pytest.mark.parametrize("K,N", [(4096, 64), (5120, 64), (6144, 4096), (8192, 64)])
+def test_one_row_captured_and_not(cuda, K, N):
+    """In a graph long rows of few results take the two launches, outside one launch: the same bits."""
+    ws = [quant.QTensor(to_dev(make_weight("q4_k", N, K, i).reshape(-1), cuda), "q4_k", (N, K)) for i in range(3)]
+    x = torch.randn(1, K, device=cuda, generator=torch.Generator(device=cuda).manual_seed(K)).to(torch.bfloat16)
+    call = lambda: [quant.plain(ws[0], x), quant.fused_glu(ws[0], ws[1], x, quant.GluActivationType.Silu), *quant.fused_qkv(*ws, x)]
+    want = call()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = call()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
