@@ -4,8 +4,8 @@ import pytest
 import torch
 
 import oracle
-from mistralrs_b200 import ops, paged_attn
-from util import TORCH_DT, make_acts, to_dev
+from mistralrs_b200 import ops, paged_attn, quant
+from util import TORCH_DT, make_acts, make_weight, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -235,3 +235,12 @@ def test_norms_and_glu_by_vectors_and_by_elements(cuda, dt, rows, cols, shift):
     got, want = ops.fused_glu(at(a), at(b), 0).float().cpu().numpy(), oracle.fused_glu(a, b, 0, dt)
     # (the activation is rounded, then the product: a last place of the first and one of the second)
     assert (np.abs(got - want) <= 2 * ulp * np.abs(want) + 1e-6).all()
+
+
+@pytest.mark.parametrize("n,cols", [(1, 14336), (5, 2560), (300, 2816), (2367, 1280), (2368, 1280)])
+def test_embedding_rows_in_pieces_and_whole(cuda, n, cols):
+    """Few rows are split over several CTAs, many are not: each row is what a gather of it alone gives."""
+    w = quant.QTensor(to_dev(make_weight("q4_k", 7, cols, 3).reshape(-1), cuda), "q4_k", (7, cols))
+    ids = torch.randint(0, 7, (n,), device=cuda, dtype=torch.int32, generator=torch.Generator(device=cuda).manual_seed(n))
+    rows = torch.cat([ops.embedding_gather(w, torch.tensor([i], device=cuda, dtype=torch.int32), torch.float32) for i in range(7)])
+    assert torch.equal(ops.embedding_gather(w, ids, torch.float32), rows[ids.long()])
