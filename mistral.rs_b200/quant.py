@@ -137,15 +137,15 @@ def _fused_entry():
 # types, 1024 / 4096 / 14336 rows: 2048 columns 0.78 / 0.83 / 0.90 (worst 0.98), 4096 columns 0.88 / 0.85 / 0.92 (0.98), 5120 and 6144
 # columns 0.97 (1.07) / 0.92 (0.98) / 0.96 (0.99), 7168 columns 1.05 (1.20) / 0.99 (1.05) / 1.00 (1.03), 8192 columns 1.04 (1.18) / 1.01 (1.08) /
 # 1.01 (1.06); Q4_K 14336 columns 1.23.  Two rows of 4096 7.8 us / 8.1, eight 13.9 / 22.6.  Outside a graph the host is the bound, 14 us a call
-# against 23, so there the line is where the device's loss would outgrow that.
-ONE_LAUNCH_MAX_K, ONE_LAUNCH_CAPTURED = 8192, ((4096, 0), (6144, 4096))      # captured: (columns, from so many rows on)
+# against 23, so there the line is where the device's loss would outgrow that.  In a graph: up to 4096 columns, up to 6144 for matrices of at
+# least 4096 rows.
+ONE_LAUNCH_MAX_K = 8192
 
 
 def _one_launch(b_size, k, nrows, xs):
     # (the fused prologue reads 16 bytes at a time; the quantising launch takes any element address)
-    if b_size != 1 or k > ONE_LAUNCH_MAX_K or xs.data_ptr() % 16 != 0:
-        return False
-    return any(k <= most and nrows >= least for most, least in ONE_LAUNCH_CAPTURED) or not torch.cuda.is_current_stream_capturing()
+    return (b_size == 1 and k <= ONE_LAUNCH_MAX_K and xs.data_ptr() % 16 == 0
+            and (k <= 4096 or (k <= 6144 and nrows >= 4096) or not torch.cuda.is_current_stream_capturing()))
 
 
 def _fused_one_row(mode, ws, xs, outs, k, activation=0):
