@@ -237,6 +237,23 @@ def test_norms_and_glu_by_vectors_and_by_elements(cuda, dt, rows, cols, shift):
     assert (np.abs(got - want) <= 2 * ulp * np.abs(want) + 1e-6).all()
 
 
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("rows,cols,gap", [(65, 4104, 0), (70, 4104, 8), (40000, 8, 0), (64, 4096, 0), (33, 8000, 3), (3, 131072, 16), (50, 5632, 0),
+                                           (66000, 1536, 8)])
+def test_large_glu_by_vectors(cuda, dt, rows, cols, gap):
+    """Above 2^18 elements the GLU goes by vectors of eight where columns and row distances allow it (a gap of 8, 16 or none), numbered through or
+    (131072, 5632 and 1536 columns) row by row, else by elements (64 x 4096 is just not above, a gap of 3): the same arithmetic in an element,
+    so the same bits as a few rows give."""
+    a, b = (torch.randn(rows, cols + gap, device=cuda, generator=torch.Generator(device=cuda).manual_seed(i)).to({"bf16": torch.bfloat16, "f16": torch.float16}[dt])
+            for i in (1, 2))
+    for act in range(3):
+        got = ops.fused_glu(a[:, :cols], b[:, :cols], act)
+        n = max(1, min(rows, 200000 // cols))
+        for r in range(0, rows, max(1, rows // 16)):
+            part = slice(r, min(rows, r + n))
+            assert torch.equal(got[part], ops.fused_glu(a[part, :cols].contiguous(), b[part, :cols].contiguous(), act))
+
+
 @pytest.mark.parametrize("n,cols", [(1, 14336), (5, 2560), (300, 2816), (2367, 1280), (2368, 1280)])
 def test_embedding_rows_in_pieces_and_whole(cuda, n, cols):
     """Few rows are split over several CTAs, many are not: each row is what a gather of it alone gives."""
