@@ -1,8 +1,8 @@
 #!/usr/bin/env python
 """bench.py — the quantized-linear + paged-attention hot path of mistral.rs on B200.
 
-Headline (BASELINE.json configs[1], `--config 2`, the default): Llama-3-8B, GGUF Q4_K_M tensor types,
-decode batch 1, 128-token prompt -> +256 generated tokens, synthetic weights / prompts (SURVEY §8(d)),
+Headline (`--config 2`, the default): Llama-3-8B, GGUF Q4_K_M tensor types,
+decode batch 1, 128-token prompt -> +256 generated tokens, synthetic weights / prompts,
 paged KV cache block_size 16 (FlashInfer HND layout).  Metric definitions follow the reference's
 `mistralrs bench` (mistralrs-cli/src/commands/bench.rs:269-296): prefill tok/s = L / TTFT, decode
 tok/s = (G - 1) / (t_last_token - t_first_token).
@@ -12,7 +12,7 @@ the launching stream (max over ranks).  `value` replays the per-token CUDA graph
 resident in HBM; `e2e` drives the same graph the way a serving engine does (token id copied from
 pinned host memory before every step, sampled id read back after it).  The same JSON line carries
 `roofline` (dominant kernel, measured live), `cpu_baseline` (the reference's CPU arithmetic, whole
-tokens on all host cores), `prefill` (BASELINE config 3: 4096-token prompt on Q8_0 weights, TTFT
+tokens on all host cores), `prefill` (4096-token prompt on Q8_0 weights, TTFT
 including prompt attention) and `config4` (Mistral-7B GPTQ int4 decode at batch 32, both KV layouts).
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--config 2|3|4|5]
@@ -121,7 +121,7 @@ def cpu_decode_samples(cfg, M, seconds=10.0, min_tokens=2, threads=0, nsamples=1
     """The reference's CPU arithmetic (oracle/mrs_oracle.c: Q8_K / Q8_0 activations + integer block dots,
     the candle QMatMul algorithm) on WHOLE tokens of this model: all layers, every weight byte streamed
     from DRAM each token, attention / norms / GLU included, one pinned thread per usable host core
-    (oracle/cpu_decode_bench.c).  Compiled here, on the box that runs it, with -O3 -march=native.
+    (oracle/cpu_decode_bench.c).  Compiled where it runs, with -O3 -march=native.
     `nsamples` timed samples of about `seconds` each share ONE model allocation (one short-lived child process).
     Returns ([tok/s per sample], threads, description)."""
     src = os.path.join(ROOT, "oracle", "cpu_decode_bench.c")
@@ -210,7 +210,7 @@ def run_reference(args):
 
 
 def run_config1(args):
-    """BASELINE config 1: TinyLlama-1.1B GGUF Q4_K_M on the CPU, 128-token prompt + 64 decode tokens — plumbing
+    """TinyLlama-1.1B GGUF Q4_K_M on the CPU, 128-token prompt + 64 decode tokens — plumbing
     only (no GPU): the CPU port of the reference's arithmetic through every layer (oracle/cpu_decode_bench.c),
     the prompt fed token by token like the decode steps."""
     if int(os.environ.get("RANK", "0")) != 0:
@@ -305,7 +305,7 @@ def validate_first_tokens(weights, M, torch, n_tokens=6):
 
 # ------------------------------------------------------------------------------------------- config 3
 def bench_prefill_q8(M, torch, dev, peaks, prompt=4096, layers=0):
-    """BASELINE config 3: Llama-3-8B with Q8_0 blocks everywhere (UQFF q8), one 4096-token prompt.
+    """Llama-3-8B with Q8_0 blocks everywhere (UQFF q8), one 4096-token prompt.
     TTFT = embedding -> 32 x (norm, tcgen05 dequant-GEMMs, RoPE, causal prompt attention, KV scatter, GLU) ->
     lm_head on the last row -> argmax; prefill tok/s = L / TTFT (bench.rs:269-271)."""
     cfg = M.LlamaConfig.llama3_8b(quant="q8_0")
@@ -358,7 +358,7 @@ def bench_prefill_q8(M, torch, dev, peaks, prompt=4096, layers=0):
 
 # ------------------------------------------------------------------------------------------- config 4
 def bench_gptq_batch32(torch, dev, peaks, steps=2, layers=0, batch=32):
-    """BASELINE config 4: Mistral-7B GPTQ int4 (g128, symmetric) decode at batch 32, paged KV block 16,
+    """Mistral-7B GPTQ int4 (g128, symmetric) decode at batch 32, paged KV block 16,
     128-token prompts -> +256 tokens, in the HND (FlashInfer) and vLLM cache layouts."""
     from mistralrs_b200 import gptq_model as G
     cfg = G.GptqConfig.mistral_7b()
@@ -402,7 +402,7 @@ def bench_gptq_batch32(torch, dev, peaks, steps=2, layers=0, batch=32):
             lin_s = timed_graph(gg, 10, torch)
             run.step_struct.skip_mask = 0
             res["linears"] = {"ms_per_step": lin_s * 1e3, "achieved_gbs": w.nbytes / lin_s / 1e9, "hbm_frac": w.nbytes / lin_s / 1e9 / peak,
-                              "kernel": "w4a16_kernel<32> (swap-AB tcgen05) + dense lm_head"}
+                              "kernel": "mmq_ts_kernel<TS_INT4> (swap-AB tcgen05) + w16_dense_kernel (lm_head)"}
         del run, graph
     del w
     torch.cuda.empty_cache()

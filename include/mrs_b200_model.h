@@ -109,7 +109,7 @@ int32_t mrs_embedding_gather(int32_t ggml_type, const void *table, int32_t cols,
 int32_t mrs_argmax(const void *logits, int32_t rows, int32_t cols, int32_t act_dtype, int32_t *out, void *scratch,
                    int32_t pdl, void *stream);
 
-/* ---- GPTQ / AWQ int4 decode stack (Mistral-7B GPTQ g128, batch 32) --------------
+/* ---- GPTQ / AWQ int4 decode stack (measured on Mistral-7B GPTQ g128, batch 32) --------------
  * Linears are int4 tiles produced by gptq_marlin_repack / awq_marlin_repack (mrs_b200_quant.h) with
  * UNPERMUTED scales [K/group, N] in the activation dtype; q||k||v and gate||up are concatenated along
  * N at load time.  cache_layout 1: HND cache + fused RoPE/KV-write/attention; 0: vLLM layout

@@ -107,7 +107,7 @@ int32_t mrs_paged_decode_fused_strided(void *q, void *k_new, void *v_new, void *
                                int32_t num_qo_heads, int32_t num_kv_heads, int32_t head_size, int32_t page_size,
                                float sm_scale, uint32_t dtype, int32_t pdl, int64_t q_stride_n, int64_t kv_new_stride,
                                void *stream);
-/* ---- prompt attention over fresh q/k/v (SURVEY §8(f) rank 1; REF paged_attention.rs:1413-1475 ->
+/* ---- prompt attention over fresh q/k/v (REF paged_attention.rs:1413-1475 ->
  * flash_attn_varlen): causal [+ sliding window / soft-cap], GQA, var-len batches via cu_seqlens
  * (device i32 [batch+1], or NULL for one sequence).  q [total,H,D], k/v [total,KVH,D], strides in
  * elements between tokens; head_dim 64 | 128; dtype 0 f16 / 1 bf16.  csrc/prefill_attn.cu. */

@@ -3,7 +3,7 @@
  * Every `launch_mmvq_gguf_*` symbol below has exactly the name, argument order and meaning of
  * the reference launcher it replaces, so mistralrs-quant's `extern "C"` block
  * (mistralrs-quant/src/gguf/ffi.rs, consumed by src/gguf/fast_mmvq.rs:116-157) links against
- * this library unchanged.  Contract (SURVEY §8b): raw device pointers already offset by the
+ * this library unchanged.  Contract: raw device pointers already offset by the
  * tensor's start_offset; the caller owns all memory incl. the Q8_1 scratch; every call is
  * asynchronous on `stream`, allocation-free and CUDA-graph capturable; launchers return void and
  * do not check cudaGetLastError (like the reference); batch b_size outside 1..8 is a no-op.

@@ -1,5 +1,5 @@
 // gptq_decoder.cu — decode layer stack for GPTQ / AWQ int4 checkpoints (Mistral / Llama family)
-// at serving batch sizes (Mistral-7B GPTQ g128, batch 32, paged KV block 16).
+// at serving batch sizes (measured on Mistral-7B GPTQ g128, batch 32, paged KV block 16).
 //
 // REF structure mirrored: mistralrs-core/src/models/mistral.rs (Attention / MLP / DecoderLayer
 // forward over `QuantMethod` linears), with the linears on the reference's Marlin symbols

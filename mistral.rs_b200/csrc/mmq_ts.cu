@@ -57,13 +57,19 @@ cudaError_t ts_refused(const TsDevice &d) {
   return *(volatile const int32_t *)d.flag != 0 ? cudaErrorLaunchTimeout : cudaSuccess;
 }
 
-// Matrices of fewer rows are not split: results then stay bit for bit those of csrc/mmq_tc.cu, and so small a product is short
-// either way.
+// ggml matrices of fewer rows are not split: results then stay bit for bit those of csrc/mmq_tc.cu, and so small a product is short
+// either way.  (Where K is split, how depends on the number of tokens too: the bits of a token's results may depend on how many
+// tokens are beside it.)
 constexpr int TS_SPLIT_MIN_ROWS = 1024;
 
-// Token tile and split of K by estimated clocks.  A span (256 k) of a tile takes the longest of: the tensor pipe (8 clocks a token, 50 a
-// product at least), the dequantisers, and the weight stream at its share of the memory's rate; a CTA adds what it spends before the
-// first product and after the last.  K whole: persistent CTAs, so the tiles of one share the start.
+// Token tile and split of K by an estimate in clocks.  A span (256 k) of a tile takes the longest of: the tensor pipe (8 clocks a token),
+// the dequantisers, and the weight stream at its share of the memory's rate; a CTA adds what it spends before the first product and after
+// the last.  K whole: persistent CTAs, so the tiles of one share the start.
+// The weights rank plans and are no measured clocks: the dequantisers' 800 to 1500 (the callers') stand for spans that take 1300 by issue alone
+// (Q4_K) and up to 3300 in a kernel (Q6_K at 24 tokens).  What they are worth, against the fastest of all plans on one B200: ten block types at
+// five matrices and 9 to 512 tokens, 1.1 % slower on average and more than 5 % in 27 of 350 (2048 x 2048 at 300 and 512 tokens, up to 37 %;
+// 4096 x 4096 at 200 and 512, up to 12 %); int4 at eleven matrices, 1.9 % on average and more than 5 % in 22 of 154 (matrices 1024 columns
+// wide from 64 tokens on, up to 24 %; 4096 columns and more at 300 and 500 tokens, up to 10 %).
 TsPlan ts_plan(int M, int N, int K, int span_bytes, int dequant_clocks, int split_min_rows, const TsDevice &d) {
   constexpr int START = 4500, TILE_END = 1200, SPLIT_END = 2600;     // clocks
   const int tiles_n = (N + TS_BM - 1) / TS_BM, spans = (K + TS_SPAN_K - 1) / TS_SPAN_K;
@@ -122,7 +128,7 @@ extern "C" int32_t mrs_mmq_gguf_ts(int32_t ggml_type, const void *w, const void 
   const TsDevice &d = ts_device();
   const cudaError_t refused = ts_refused(d);
   if (refused != cudaSuccess) return (int32_t)refused;
-  // clocks that the dequantisers take for a span
+  // the dequantisers' weight in the plan's estimate
   const int clocks = ggml_type == MRS_Q6_K ? 1500 : ggml_type == MRS_Q5_K || ggml_type == MRS_Q3_K || ggml_type == MRS_Q5_0 || ggml_type == MRS_Q5_1 ? 1350 : 1150;
   const TsPlan plan = ts_plan(M, N, K, bytes * (256 / elems), clocks, TS_SPLIT_MIN_ROWS, d);
   const TsCall c = {w, x, y, M, N, K, K / elems * bytes, dtype, plan.nt, plan.tiles_m, plan.ksplit, d.sms, d.timeouts, (cudaStream_t)stream, nullptr, nullptr, 0, 0, 0};

@@ -1,9 +1,9 @@
 // paged_attn_mma.cuh — tensor-core decode attention over the HND paged cache (included by paged_attn.cu).
 //
 // The GQA group of one KV head is an MMA tile: the group's query heads (<= 16) are the M = 16 rows of
-// mma.m16n8k16, the tokens of the work tile are N.  Per 64-token step the whole CTA (4 warps) gathers
-// the K and V rows of the tile from their pages into XOR-swizzled shared memory with cp.async
-// (16-byte copies, page ids staged once); warp w copies and owns tokens 16w..16w+15 of the step:
+// mma.m16n8k16, the tokens of the work tile are N.  Of each 64-token step, warp w (of 4) gathers the K and
+// V rows of tokens 16w..16w+15 from their pages into XOR-swizzled shared memory with cp.async (16-byte
+// copies, page ids staged once) and computes with them, waiting for no copies but its own:
 // S = Q K^T (16 MMAs for D = 128), online softmax in f32 (base 2), O += P V (16 MMAs, V^T fragments
 // through ldmatrix.trans).  ~4 warp-instructions per token where the SIMT kernel needs ~85.
 //

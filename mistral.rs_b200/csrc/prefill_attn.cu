@@ -4,7 +4,7 @@
 //   REF mistralrs-core/src/paged_attention/layers/paged_attention.rs:1413-1475 (prompt path: attention over
 //   the just-projected q/k/v, then reshape_and_cache), mistralrs-flash-attn/kernels/flash_fwd_*_sm80.cu,
 //   API flash_attn_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, max_q, max_k, softmax_scale, causal).
-// SURVEY §8(f) rank 1.  This is an original kernel with the same arithmetic class: S = QK^T and O = PV on
+// This is an original kernel with the same arithmetic class: S = QK^T and O = PV on
 // 16-bit tensor-core MMAs with f32 accumulation, online softmax in f32 (base-2 exponent, scale folded),
 // P rounded to the activation dtype before the second GEMM.
 //

@@ -1,7 +1,7 @@
 // prefill_attn_tc.cu — causal (var-len) prompt attention on the 5th-gen tensor cores (tcgen05 + TMEM), head size 128.
 //
 // Same contract and arithmetic class as prefill_attn.cu (REF mistralrs-core/src/paged_attention/layers/
-// paged_attention.rs:1413-1475 -> flash_attn_varlen; SURVEY §8(f) rank 1): S = QK^T and O = PV on 16-bit MMAs with
+// paged_attention.rs:1413-1475 -> flash_attn_varlen): S = QK^T and O = PV on 16-bit MMAs with
 // f32 accumulation, online softmax in f32 (base-2 exponent, scale folded), P rounded to the activation dtype before
 // the second GEMM.  mrs_prefill_attention routes here for head_dim 128 without window / softcap; prefill_attn.cu
 // (mma.sync) keeps every other case.

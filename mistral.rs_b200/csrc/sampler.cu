@@ -3,7 +3,7 @@
 //   topk_large_f32, topk_large_f32_packed, topk_large_f32_packed_batched,
 //   top1_large_f32_packed, top1_large_f32_packed_batched
 // REF mistralrs-core/src/cuda/ffi.rs:581-665, kernels mistralrs-core/src/cuda/sort.cu:1503-2262, callers
-// mistralrs-core/src/ops.rs:690-830,1915 (chunk_size 2048, k <= 128).  SURVEY §8(f) rank 3.
+// mistralrs-core/src/ops.rs:690-830,1915 (chunk_size 2048, k <= 128).
 //
 // Output contract restated from the reference kernels (bit-exact for values and indices):
 //   top-k  : the k largest RAW logits in (value descending, token index ascending) order — NaN and

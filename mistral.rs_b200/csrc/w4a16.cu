@@ -41,9 +41,6 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait_acquire() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t local_smem_addr, uint32_t rank) {
@@ -360,7 +357,7 @@ static cudaError_t run_int4(const void *x, const void *w, const void *scales, co
   if (((uintptr_t)scales & 15) || ((uintptr_t)qzeros & 15)) return cudaErrorMisalignedAddress;
   const TsDevice &d = ts_device();
   if ((e = ts_refused(d)) != cudaSuccess) return e;
-  // (a span of a row: 128 B of nibbles and its scales; the dequantisers take two operations a weight, some 800 clocks a span)
+  // (a span of a row: 128 B of nibbles and its scales; 800: the dequantisers' weight in the plan's estimate, two operations a weight)
   const TsPlan plan = ts_plan(M, N, K, 128 + 2 * ((TS_SPAN_K + group - 1) / group), 800, 0, d);
   const TsCall c = {w, x, y, M, N, K, 0, dtype, plan.nt, plan.tiles_m, plan.ksplit, d.sms, d.timeouts, st, scales, qzeros, group, scale_perm, pdl ? 1 : 0};
   return ts_launch<TS_INT4>(c);

@@ -1,4 +1,4 @@
-"""GGUF archives -> device-resident ggml block tensors (SURVEY §8(f) rank 2).
+"""GGUF archives -> device-resident ggml block tensors.
 
 Python mirror of the reference's archive layer (`mistralrs-quant/src/gguf/archive.rs`:
 `GgufArchive::{open, metadata, tensors, tensor_info, contains_tensor, tensor_data, load_qtensor}`)

@@ -1,10 +1,10 @@
 """GPTQ / AWQ int4 decode runner over the C ABI (`mrs_gptq_decode_step`, include/mrs_b200_model.h) —
-BASELINE config 4 (Mistral-7B GPTQ int4 g128, decode batch 32, paged KV block_size 16).
+Mistral-7B GPTQ int4 g128 at decode batch 32 over a paged KV cache of 16-token blocks is what it is measured on.
 
 Python is the harness only (device memory, struct filling, CUDA-graph capture); the layer stack is
 C++ (csrc/gptq_decoder.cu) over the reference's Marlin symbols' kernel (csrc/w4a16.cu).
 
-Synthetic checkpoints follow SURVEY §8(d): `qweight` uniform u4 packed [K/8, N] i32, `scales` f16
+Synthetic checkpoints: `qweight` uniform u4 packed [K/8, N] i32, `scales` f16
 2^U(-8,-6) [K/128, N], symmetric (`qzeros` = 0x77777777 in the checkpoint, ignored by the Marlin
 path), `g_idx[k] = k/128`; dense f16 embeddings / lm_head / norms.  Load flow = the reference's
 `gptq_linear` (gptq_cuda.rs:451-623): `gptq_marlin_repack` per tensor (q/k/v and gate/up are
@@ -78,7 +78,7 @@ class _Step(ctypes.Structure):
 
 
 def synth_gptq(K, N, group, seed, scale_exp=(-8, -6)):
-    """(qweight [K/8, N] i32, scales [K/group, N] f16) per SURVEY §8(d)."""
+    """(qweight [K/8, N] i32 uniform, scales [K/group, N] f16 2^U(scale_exp))."""
     rng = np.random.Generator(np.random.PCG64(seed))
     qweight = rng.integers(0, 2 ** 32, size=(K // 8, N), dtype=np.uint64).astype(np.uint32).view(np.int32)
     scales = np.exp2(rng.uniform(scale_exp[0], scale_exp[1], size=(K // group, N))).astype(np.float16)

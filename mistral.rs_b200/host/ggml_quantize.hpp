@@ -2,10 +2,10 @@
 // quantisation (ISQ) runs on the host when a GGUF layer is re-quantised to another type.
 //   REF mistralrs-quant/src/gguf/mod.rs:633-708 (`GgufMatMul::apply_isq`: same type -> keep the blocks; otherwise
 //       dequantise and `QTensor::quantize` to the requested type), :601-604.
-// The arithmetic is candle-core `quantized::k_quants` `from_float` (third-party, pinned at candle 0.11.0 — not under
-// /root/reference), which follows ggml's `quantize_row_*_ref`; the offline pin used here is gguf-py's bit-exact
+// The arithmetic is candle-core `quantized::k_quants` `from_float` (third-party, pinned at candle 0.11.0 — not part of
+// the reference's tree), which follows ggml's `quantize_row_*_ref`; the offline pin used here is gguf-py's bit-exact
 // restatement of the same routines (tests/test_isq_host.py).  K-quant quantisation (Q2_K..Q6_K: iterative scale search)
-// is NOT provided: no offline reference to pin it against (SURVEY §8c lists it as unpinned).
+// is NOT provided: no offline reference to pin it against.
 // Compile with -ffp-contract=off: `x * id + 8.5f` must round twice, as the reference does.
 #pragma once
 #include <cmath>

@@ -1,6 +1,6 @@
 // gguf_reader.hpp — GGUF v2/v3 archive reader (mmap), the data-format side of the hot path:
 // real weights arrive as ggml blocks inside GGUF files and are uploaded to HBM *as stored* (the
-// kernels consume the block layout directly, DESIGN.md §3).
+// kernels consume the block layout directly).
 //
 // Mirrors the behaviour of the reference's archive layer — REF mistralrs-quant/src/gguf/archive.rs:
 //   * header / metadata / tensor catalogue parsing            (:351-611, parse_shards)

@@ -4,7 +4,7 @@ Python here is only the harness: it allocates device memory with torch, fills th
 raw pointers and drives CUDA-graph capture/replay.  The layer stack itself (which kernels run, in
 which order) is C++ inside libmrs_b200.so.
 
-Synthetic weights follow SURVEY §8(d): ggml blocks with uniformly random quants over their full
+Synthetic weights: ggml blocks with uniformly random quants over their full
 bit range, f16 scales d = 2^U(-9,-7), dmin = d*U(0,0.5); tensor-type map for Q4_K_M = the
 llama.cpp recipe (Q4_K everywhere; Q6_K for `output`, and for attn_v + ffn_down on layers
 i < n/8, i >= 7n/8 or (i - n/8) % 3 == 2).
@@ -40,11 +40,11 @@ class LlamaConfig:
     name: str = "llama-3-8b"
     rope_neox: bool = True     # rotate-half pairing; GGUF llama files use the interleaved pairing (False)
     rope_freq_factors: object = None   # optional per-frequency divisors (GGUF `rope_freqs.weight`, Llama-3.1 scaling)
-    synth_scale_exp: tuple = (-9, -7)  # synthetic weights: block scales d = 2^U(lo, hi) (SURVEY §8(d))
+    synth_scale_exp: tuple = (-9, -7)  # synthetic weights: block scales d = 2^U(lo, hi)
 
     # Real-size models take block super-scales 2^U(-15,-13): with the 6-bit sub-scales (1..63) and 4-bit
     # quants of the k-quants that gives |w| ~ 0.016, i.e. unit-scale activations at K = 4096 .. 28672.
-    # SURVEY §8(d)'s 2^U(-9,-7) (|w| ~ 1) sends the 14336-wide down projection past f16's range, and the
+    # 2^U(-9,-7) (|w| ~ 1) sends the 14336-wide down projection past f16's range, and the
     # Q8_1 block scale is a half (REF mmvq_gguf.cu:146-152): the reference itself would produce NaN.
     @staticmethod
     def llama3_8b(**kw):
@@ -70,7 +70,7 @@ class LlamaConfig:
 
 
 def tensor_type(cfg: LlamaConfig, name: str, layer: int = 0) -> str:
-    """ggml type of a tensor under cfg.quant (llama.cpp Q4_K_M recipe, SURVEY §8(d))."""
+    """ggml type of a tensor under cfg.quant (llama.cpp Q4_K_M recipe)."""
     if cfg.quant != "q4_k_m":
         return cfg.quant
     if name == "output":
@@ -87,7 +87,7 @@ TENSOR_IDS = {"attn_q": 0, "attn_k": 1, "attn_v": 2, "attn_output": 3, "ffn_gate
 
 
 def synth_blocks(dtype: str, nblocks: int, seed: int, scale_exp=(-9, -7)) -> np.ndarray:
-    """uint8 [nblocks, block_bytes] per SURVEY §8(d), numpy PCG64(seed)."""
+    """uint8 [nblocks, block_bytes] of uniformly random quants and scales 2^U(scale_exp), numpy PCG64(seed)."""
     rng = np.random.Generator(np.random.PCG64(seed))
     bb = BLOCK_BYTES[dtype]
     raw = rng.integers(0, 256, size=(nblocks, bb), dtype=np.uint8)
@@ -242,8 +242,8 @@ class LlamaWeights:
 
     def __init__(self, cfg: LlamaConfig, device, dtype=torch.bfloat16, tp_rank=0, tp_size=1, keep_host=False, fast_synth=False):
         """fast_synth: generate the (shard-shaped) blocks on the device with torch's RNG instead of numpy
-        PCG64 on the host — same distribution, not the SURVEY §8(d) byte stream; for throughput runs of
-        large models (config 3's 8 GB, config 5's 40 GB) where no oracle comparison is made."""
+        PCG64 on the host — same distribution, not the same byte stream; for throughput runs of
+        large models (8 GB of Q8_0, 40 GB of a 70B model) where no oracle comparison is made."""
         self.cfg, self.device, self.dtype = cfg, device, dtype
         self.tp_rank, self.tp_size = tp_rank, tp_size
         self.fast_synth = bool(fast_synth)
@@ -665,7 +665,7 @@ class LlamaPrefill:
     RMSNorm -> tcgen05 dequant-GEMMs (`mmq.forward`, the `fast_mmq` path) -> RoPE -> causal prompt
     attention over the fresh q/k/v (`paged_attn.prefill_attention`, the reference's flash-attn call,
     paged_attention.rs:1413-1475) -> KV scatter into the paged HND cache -> o_proj -> add+RMSNorm ->
-    GLU -> down -> add.  TTFT of BASELINE config 3 is the time of `forward` on a 4096-token prompt."""
+    GLU -> down -> add.  Time to first token is the time of `forward`."""
 
     def __init__(self, weights: "LlamaWeights", max_tokens=4096, runner: "LlamaRunner" = None):
         """runner: write the prompt's K/V into sequence 0 of this decode runner's paged cache (its block

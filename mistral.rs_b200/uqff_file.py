@@ -1,4 +1,4 @@
-"""UQFF artifacts -> device-resident ggml block tensors (SURVEY §8(f) rank 2).
+"""UQFF artifacts -> device-resident ggml block tensors.
 
 UQFF is the reference's native quantized format: a directory of `<stem>-<n>.uqff` shards (each a
 safetensors file whose entries follow naming conventions), `residual.safetensors` for the

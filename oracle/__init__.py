@@ -2,7 +2,7 @@
 
 ctypes front-end of oracle/liboracle.so (oracle/mrs_oracle.c: a plain-C restatement of the
 reference's arithmetic, every function citing the reference file:line it follows) and of the
-unmodified reference CUDA kernels built from /root/reference into oracle/_ref/ (build_ref.sh).
+unmodified reference CUDA kernels built from its tree into oracle/_ref/ (build_ref.sh).
 
 Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / `--impl reference` legs may
 import this package, and only as the checker or the CPU timing baseline.  The product package
@@ -57,7 +57,7 @@ def _p(a):
 
 
 def random_blocks(dtype, nblocks, rng, scale_exp=(-9, -7)):
-    """Synthetic ggml blocks per SURVEY §8(d): quants uniform over their full bit range, f16
+    """Synthetic ggml blocks: quants uniform over their full bit range, f16
     scales 2^U(lo,hi) (dmin = d*U(0,0.5)); K-quant 6-bit scales/mins uniform."""
     bb = BLOCK_BYTES[dtype]
     raw = rng.integers(0, 256, size=(nblocks, bb), dtype=np.uint8)

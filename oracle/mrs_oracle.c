@@ -2,7 +2,7 @@
  * mrs_oracle.c — CPU ORACLE (TEST INFRASTRUCTURE, NOT PRODUCT).  See mrs_oracle.h.
  *
  * Every function cites the reference file:line whose behaviour it restates.  `REF:` paths are
- * relative to /root/reference (EricLBuehler/mistral.rs @ 9e92262).
+ * relative to the reference's tree (EricLBuehler/mistral.rs @ 9e92262).
  * Build: gcc -O2 -ffp-contract=off -fPIC -shared -pthread (oracle/Makefile).  -ffp-contract=off
  * matters: the quantiser's f32 butterfly sums must not be fused.
  */
@@ -322,8 +322,8 @@ void mrs_quantize_q8_1(const float *x, void *y, int kx, int kx_padded, int rows)
 
 /* ------------------------------------------------------------------ Q8_1 GEMV arithmetic
  * REF: mmvq_gguf.cu:244-450 (vec_dot_*_impl) and :458-684 (per-type wrappers).  Written in
- * "sum over scale groups" form; the derivation that each reference thread-partial adds up to
- * exactly these integer dots is in DESIGN.md §Oracle.  Integer dots are exact; the float
+ * "sum over scale groups" form; the thread-partials of a reference warp add up to exactly these
+ * integer dots (each covers its own quants of the group).  Integer dots are exact; the float
  * factors (half d/dmin/d8, 6-bit scales) are multiplied exactly in double, so this is the
  * infinitely-precise value of the reference's arithmetic — the reference and our kernels
  * differ from it only by f32 accumulation order. */
@@ -424,7 +424,7 @@ int mrs_matmul_exact(int type, const void *w, const float *x, double *out, int n
 
 /* ------------------------------------------------------------------ reference CPU path
  * REF call site: mistralrs-quant/src/gguf/mod.rs:465-478 -> candle QMatMul::forward (candle
- * v0.11.0 @35d7ae7c, candle-core/src/quantized/k_quants.rs — NOT under /root/reference).
+ * v0.11.0 @35d7ae7c, candle-core/src/quantized/k_quants.rs — not part of the reference's tree).
  * Algorithm restated from the published llama.cpp/candle k-quants: activations quantised per
  * 256 to Q8_K (iscale=-128/max, bsums per 16) for K-quants, per 32 to Q8_0 (d=amax/127) for
  * the 32-wide types; integer block dots; f32 accumulation.  Parity vs candle: UNPINNED. */

@@ -9,10 +9,9 @@
  * Pinning status: the block decoders are pinned against gguf-py 0.19.0 `gguf.quants.dequantize`
  * (tests/golden/gguf_dequant_*.npz, generated by tests/golden/make_gguf_golden.py) and the
  * Q8_1 arithmetic, cache scatter, RoPE, GLU and RMSNorm functions are pinned against the
- * reference's own CUDA kernels compiled from /root/reference (oracle/_ref, built by
- * oracle/build_ref.sh) both live on the GPU box (tests/test_ref_kernels_gpu.py) and through
- * the committed fixtures tests/golden/ref_*.npz produced by tests/golden/make_ref_golden.py.
- * The candle CPU path (Q8_K activations) is NOT in /root/reference (git dependency
+ * reference's own CUDA kernels (oracle/_ref, built from its tree by oracle/build_ref.sh) through
+ * the committed fixture tests/golden/ref_golden.npz produced by tests/golden/make_ref_golden.py.
+ * The candle CPU path (Q8_K activations) is NOT in the reference's tree (git dependency
  * huggingface/candle@35d7ae7c, v0.11.0): mrs_qmatmul_cpu restates the published
  * llama.cpp/candle k-quants algorithm and is "parity unpinned" against candle itself.
  */

@@ -1,4 +1,4 @@
-"""BASELINE config 1 (TinyLlama-1.1B Q4_K_M, CPU, 128-token prompt + 64 generated): the CPU port of
+"""TinyLlama-1.1B Q4_K_M on the CPU, 128-token prompt + 64 generated: the CPU port of
 the reference's CPU path (oracle/: Q8_K / Q8_0 activations + integer block dots) end to end — full
 layer stack incl. RMSNorm, RoPE and attention — on synthetic weights of that shape.
 usage: python scripts/cpu_config1.py [prompt_len] [gen_len]     (plumbing + CPU tok/s; no GPU)"""

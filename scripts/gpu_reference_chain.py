@@ -10,7 +10,7 @@ the reference's `pipeline/cuda_graph.rs`:
     -> quantize_q8_1 -> mmvq plain (down_proj)                                          [13-15 launches / layer]
     ... final add_rms_norm -> quantize_q8_1 -> mmvq plain (lm_head) -> argmax
 
-This is "the recompiled Ampere-class kernel path on the same B200" (BASELINE.md §1), not our product: bench.py
+This is the reference's own kernel path recompiled for the same GPU, not our product: bench.py
 reports it as `gpu_reference` next to `value`.  Only the KV-index advance, the embedding gather and the argmax
 are ours (plumbing the reference does on the host / in candle)."""
 import ctypes

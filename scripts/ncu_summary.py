@@ -1,4 +1,4 @@
-"""Summarise an ncu report (read on the CPU box): python scripts/ncu_summary.py file.ncu-rep"""
+"""Summarise an ncu report (needs no GPU): python scripts/ncu_summary.py file.ncu-rep"""
 import csv, subprocess, sys, io
 rep = sys.argv[1]
 raw = subprocess.run(["ncu", "-i", rep, "--page", "raw", "--csv"], capture_output=True, text=True).stdout
