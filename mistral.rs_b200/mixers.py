@@ -677,7 +677,9 @@ class RoutedExperts:
     # per megabyte of weights that a pair reads), the one-launch products' does not: above one pair per expert and GROUPED_PAIR_BYTES they take
     # over.  One B200, us of the block, grouped / one-launch: 16 experts, top 4, width and ff 2048 (25 MB each): 4 tokens 84 / 95,
     # 8: 113 / 102, 16: 154 / 106, 32: 242 / 107; 8 experts, top 2, 2048 x 1024 (13 MB): 16 tokens 69 / 88, 32: 91 / 89; 32 experts, top 2,
-    # 1024 x 768 (5 MB): 64 tokens 100 / 89, 128: 140 / 99; 16 experts, top 4, 4096 x 2048 (50 MB): 4 tokens 127 / 147, 8: 165 / 164.
+    # 1024 x 768 (5 MB): 64 tokens 100 / 89, 128: 140 / 99; 16 experts, top 4, 4096 x 2048 (50 MB): 4 tokens 127 / 147, 8: 165 / 164.  At the
+    # line (805 MB) with few experts the two are even for calls from the host (8 experts of 25 MB, top 8, 4 tokens: 91 / 92) and the one-launch
+    # products ahead in a graph (79 / 67).  The same line for steps that stream per pair: 8 experts of 100 MB, top 8, 2 tokens 657 / 186.
     # Elsewhere weights are streamed per pair up to 4 pairs per expert while an expert is small enough that repeated reads hit L2, up to
     # 2 above that.
     GROUPED_MIN_TOKENS, GROUPED_PER_EXPERT, GROUPED_PAIR_BYTES = 4, 8, 700 << 20
