@@ -98,7 +98,6 @@ __device__ __forceinline__ bool ts_wait(uint64_t *bar, uint32_t parity, int *tim
     if (__all_sync(0xffffffffu, done)) return true;
   } while (++n < TS_WAIT_LIMIT);
   *(volatile int *)timeouts = 1;
-  __threadfence_system();
   return false;
 }
 
@@ -540,7 +539,7 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
   uint64_t *bars = (uint64_t *)(r_ring + (size_t)RS * RAW_BYTES);
   uint64_t *raw_full = bars, *raw_empty = raw_full + TS_RS_MAX, *x_full = raw_empty + TS_RS_MAX, *x_empty = x_full + TS_XS_MAX,
            *a_full = x_empty + TS_XS_MAX, *a_empty = a_full + TS_AS, *acc_full = a_empty + TS_AS, *acc_empty = acc_full + 2, *drain = acc_empty + 2;
-  uint32_t *tmem_slot = (uint32_t *)(bars + TS_N_BARS), *lost = tmem_slot + 1;      // lost: a rank of the cluster has no partial tile
+  uint32_t *tmem_slot = (uint32_t *)(bars + TS_N_BARS);
   int *const late = p.timeouts;
 
   // (taken from lane 0: the compiler then knows that the warp's branches are uniform and keeps their operands in uniform registers)
@@ -568,7 +567,6 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
     if (warp == 1) {
       if (lane < 2 * TS_AS + 5)
         mbar_init(&a_full[lane], lane < TS_AS ? (uint32_t)TS_DQ_WARPS : lane >= 2 * TS_AS + 2 && lane < 2 * TS_AS + 4 ? (uint32_t)TS_EPI_WARPS : 1u);
-      if (lane == 0) *lost = 0u;
       fence_mbar_init();
       __syncwarp();
       tmem_alloc(tmem_slot, 512);
@@ -795,17 +793,12 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
     float *red = (float *)smem;                        // [rank][C][128 rows]
     __syncwarp();
     if (p.pdl) pdl_wait();
-    bool ok = true;
+    uint32_t lost = 0u;                                // a rank whose products did not come sends NaNs: no sum without its part looks like one
     if (warp >= 4) {
-      ok = ts_wait(acc_full, 0, late);
+      lost = ts_wait(acc_full, 0, late) ? 0u : 0x7fffffffu;
       tc_fence_after();
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (warp >= 4 && !ok && lane < p.ksplit) {         // no rank stores a sum that lacks this partial tile
-      uint32_t to;
-      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_u32(lost)), "r"(lane));
-      asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(to), "r"(1u) : "memory");
-    }
     if (warp >= 4) {
       for (int c0 = 8 * g; c0 < p.nt; c0 += 8 * G) {
         uint32_t v[8];
@@ -814,12 +807,12 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
         uint32_t to;
         asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_u32(red + (rank * C + c0 - (int)owner * C) * TS_BM + row)), "r"(owner));
 #pragma unroll
-        for (int i = 0; i < 8; i++) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(to + (uint32_t)i * (TS_BM * 4)), "r"(v[i]) : "memory");
+        for (int i = 0; i < 8; i++) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(to + (uint32_t)i * (TS_BM * 4)), "r"(v[i] | lost) : "memory");
       }
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     const int m0 = (first / p.tiles_n) * p.nt + rank * C, nrow = (first % p.tiles_n) * TS_BM + row;
-    if (warp >= 4 && *(volatile uint32_t *)lost == 0u && nrow < p.N) {
+    if (warp >= 4 && nrow < p.N) {
       const int cols = min(min(C, p.nt - rank * C), p.M - m0);
       for (int c = g; c < cols; c += G) {
         float v = red[(size_t)c * TS_BM + row];
