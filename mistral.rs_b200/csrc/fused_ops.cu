@@ -135,8 +135,9 @@ __global__ void __launch_bounds__(256) glu_vec_kernel(const T *__restrict__ a, c
 }
 // Eight activations in one thread are a longer chain than one: up to this many elements, where the GPU has room for a thread an element, the
 // kernel by elements is the faster one.  us, by elements / by vectors: 512 x 64 1.90 / 2.62, 64 x 4096 2.43 / 2.69, 64 x 5632 2.84 / 2.64,
-// 256 x 2048 3.41 / 2.74 (bf16, one B200).
-constexpr uint64_t GLU_VEC_MIN = 1u << 18;
+// 256 x 2048 3.41 / 2.74 (bf16, one B200).  As a link of a launch chain fewer blocks count for more, since the links beside it take whole SMs: a
+// decode step of four layers of a GPTQ 7B model, rows of 14336, 2 sequences 360 / 364, 4 376 / 370, 16 395 / 388.
+constexpr uint64_t GLU_VEC_MIN = 1u << 18, GLU_VEC_MIN_PDL = 1u << 15;
 
 template <typename T>
 static void launch_glu(const void *a, const void *b, void *out, uint32_t rows, uint32_t cols, uint32_t as, uint32_t bs,
@@ -145,7 +146,7 @@ static void launch_glu(const void *a, const void *b, void *out, uint32_t rows, u
   const uint64_t n = (uint64_t)rows * cols;
   cudaLaunchConfig_t cfg = {};
   if constexpr (sizeof(T) == 2) {
-    if (n > GLU_VEC_MIN && n / 8 < (1ull << 31) && cols % 8 == 0 && as % 8 == 0 && bs % 8 == 0 &&
+    if (n > (pdl ? GLU_VEC_MIN_PDL : GLU_VEC_MIN) && n / 8 < (1ull << 31) && cols % 8 == 0 && as % 8 == 0 && bs % 8 == 0 &&
         (((uintptr_t)a | (uintptr_t)b | (uintptr_t)out) & 15) == 0) {
       const uint32_t chunks = cols / 8, across = (chunks + 255) / 256;
       const bool wide = chunks * 4ull >= across * 256ull * 3;      // (at most a quarter of the threads past the row's end)
