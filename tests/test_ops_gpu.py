@@ -211,9 +211,10 @@ def test_embedding_gather_matches_dequantized_rows(cuda, dtype):
 
 
 @pytest.mark.parametrize("dt", ["bf16", "f16"])
-@pytest.mark.parametrize("rows,cols,shift", [(3, 8, 0), (5, 1000, 0), (2, 4104, 0), (1, 8200, 0), (2, 16384, 0), (2, 1000, 1), (2, 1001, 0), (2, 16392, 0)])
+@pytest.mark.parametrize("rows,cols,shift", [(3, 8, 0), (4, 248, 0), (4, 256, 0), (5, 1000, 0), (2, 4104, 0), (1, 8200, 0), (2, 16384, 0), (2, 1000, 1), (2, 1001, 0), (2, 16392, 0)])
 def test_norms_and_glu_by_vectors_and_by_elements(cuda, dt, rows, cols, shift):
-    """16-bit rows of multiples of 8 elements on 16-byte boundaries go eight elements at a time (norms up to 16384 columns), others one by one."""
+    """Norms of 16-bit rows of multiples of 8 elements on 16-byte boundaries go eight elements at a time from 256 to 16384 columns, others one by
+    one.  (A GLU of these sizes goes by elements: test_large_glu_by_vectors.)"""
     rng = np.random.default_rng(cols + shift)
     a, b = (oracle.round_dtype(rng.standard_normal((rows, cols)).astype(np.float32), dt) for _ in range(2))
     w = oracle.round_dtype((1 + 0.1 * rng.standard_normal(cols)).astype(np.float32), dt)
