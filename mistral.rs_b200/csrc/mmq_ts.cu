@@ -1,6 +1,7 @@
 // mmq_ts.cu — plan and entry point of the dequant-GEMM of mmq_ts.cuh (its kernels: mmq_ts_*.cu, two block types each).
 #include "mmq_ts.cuh"
 
+#include <atomic>
 #include <mutex>
 #include <string.h>
 
@@ -34,10 +35,12 @@ static int32_t *ts_flags() {
 const TsDevice &ts_device() {
   static TsDevice devs[TS_MAX_DEVICES] = {};
   static std::once_flag once[TS_MAX_DEVICES];
+  static std::atomic<bool> known[TS_MAX_DEVICES];      // (a call_once that has nothing to do is a call all the same)
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= TS_MAX_DEVICES) dev = 0;
   TsDevice &d = devs[dev];
+  if (known[dev].load(std::memory_order_acquire)) return d;
   std::call_once(once[dev], [&d, dev] {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -48,6 +51,7 @@ const TsDevice &ts_device() {
       if (cudaHostGetDevicePointer(&seen, flags + dev, 0) == cudaSuccess) { d.timeouts = (int *)seen; d.flag = flags + dev; }
       else (void)cudaGetLastError();
     }
+    known[dev].store(true, std::memory_order_release);
   });
   return d;
 }

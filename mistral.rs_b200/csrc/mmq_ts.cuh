@@ -24,7 +24,8 @@
 // a kernel with 8 dequantising warps for int4): Q4_K 14336 x 4096, 24 tokens 29.3 / 18.4; Q5_K 4096 x 4096, 200 tokens 2517 / 20; Q8_0
 // 14336 x 4096, 4096 tokens 475 / 421; int4 14336 x 4096, 32 tokens 21.9 / 18.4; int4 with zero points 4096 x 14336, 500 tokens 170 / 67.
 // Every wait has a limit; one that runs out ends the CTA and sets a word in host memory, after which the entry points refuse every call
-// on that device with cudaErrorLaunchTimeout (the word itself: mrs_mmq_timeout_flag, mrs_mmq_timeouts).  What a limit counts is this grid's
+// on that device with cudaErrorLaunchTimeout (the word itself: mrs_mmq_timeout_flag, mrs_mmq_timeouts).  That launch's output is not valid:
+// a tile may be missing, or with K split lack a rank's part (telling the other ranks cost every split launch 1 to 6 %).  What a limit counts is this grid's
 // own work: in a programmatic-dependent-launch chain a warp passes pdl_wait before its first wait that the activations hold up.
 #pragma once
 #include "dequant.cuh"
@@ -57,10 +58,12 @@ struct TsParams {
   // int4 checkpoints (TS_INT4): w in tiles [K/64][N][32 B] (csrc/w4a16.cu), scales [K/group][N] in the activation format
   const uint8_t *scales;
   const uint8_t *qzeros;      // AWQ [K/group][N/8] words, or null: zero point 8
-  int group, scale_perm;      // scale_perm: columns 0 plain, 1 / 2 Marlin-permuted 64 / 32 wide
-  int group32, group_shift;   // group / 32, and its logarithm or -1
+  int group32, group_shift;   // weights of a group / 32, and its logarithm or -1
+  int scale_perm;             // columns 0 plain, 1 / 2 Marlin-permuted 64 / 32 wide
   int pdl;                    // link of a programmatic-dependent-launch chain: x comes from, y may be read by, the grid before
 };
+// (eight bytes more, and every launch took the host 0.3 us longer)
+static_assert(sizeof(TsParams) <= 104, "parameters of a launch");
 
 constexpr int TS_INT4 = 200;               // block type of int4 checkpoints
 // SPAN: bytes of 256 weights of a row; PITCH: of a row in a raw stage, an odd multiple of 16 (16-byte reads of 8 consecutive rows
@@ -589,8 +592,8 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
         ok = ts_wait(raw_empty + st, ph ^ 1, late);
         if (!ok) break;
         if constexpr (TYPE == TS_INT4) {
-          const int k0 = s * TS_SPAN_K, rows = min(TS_BM, p.N - n0), chunks = min(4, (p.K - k0) >> 6), g0 = k0 / p.group;
-          const int groups = (k0 + 64 * chunks - 1) / p.group - g0 + 1;                         // that the span's k touch
+          const int k0 = s * TS_SPAN_K, rows = min(TS_BM, p.N - n0), chunks = min(4, (p.K - k0) >> 6), g0 = (k0 >> 5) / p.group32;
+          const int groups = ((k0 + 64 * chunks - 1) >> 5) / p.group32 - g0 + 1;                // that the span's k touch
           const uint32_t dst = smem_u32(r_ring) + (uint32_t)st * RAW_BYTES, bar = smem_u32(raw_full + st);
           const uint32_t zero_bytes = p.qzeros != nullptr ? (uint32_t)rows / 2u : 0u;
           mbar_arrive_expect_tx_warp(raw_full + st, (uint32_t)(chunks * rows * 32) + (uint32_t)groups * ((uint32_t)rows * 2u + zero_bytes));
@@ -793,9 +796,9 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
     float *red = (float *)smem;                        // [rank][C][128 rows]
     __syncwarp();
     if (p.pdl) pdl_wait();
-    uint32_t lost = 0u;                                // a rank whose products did not come sends NaNs: no sum without its part looks like one
+    bool ok = true;
     if (warp >= 4) {
-      lost = ts_wait(acc_full, 0, late) ? 0u : 0x7fffffffu;
+      ok = ts_wait(acc_full, 0, late);
       tc_fence_after();
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -807,12 +810,12 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
         uint32_t to;
         asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_u32(red + (rank * C + c0 - (int)owner * C) * TS_BM + row)), "r"(owner));
 #pragma unroll
-        for (int i = 0; i < 8; i++) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(to + (uint32_t)i * (TS_BM * 4)), "r"(v[i] | lost) : "memory");
+        for (int i = 0; i < 8; i++) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(to + (uint32_t)i * (TS_BM * 4)), "r"(v[i]) : "memory");
       }
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     const int m0 = (first / p.tiles_n) * p.nt + rank * C, nrow = (first % p.tiles_n) * TS_BM + row;
-    if (warp >= 4 && nrow < p.N) {
+    if (warp >= 4 && ok && nrow < p.N) {
       const int cols = min(min(C, p.nt - rank * C), p.M - m0);
       for (int c = g; c < cols; c += G) {
         float v = red[(size_t)c * TS_BM + row];
@@ -860,7 +863,7 @@ template <int TYPE, bool ALIGNED> static cudaError_t ts_launch_as(const TsCall &
   }
   TsParams p = {};
   p.w = (const uint8_t *)c.w; p.y = c.y; p.timeouts = c.timeouts; p.M = c.M; p.N = c.N; p.K = c.K; p.row_bytes = c.row_bytes;
-  p.scales = (const uint8_t *)c.scales; p.qzeros = (const uint8_t *)c.qzeros; p.group = c.group; p.scale_perm = c.scale_perm; p.pdl = c.pdl;
+  p.scales = (const uint8_t *)c.scales; p.qzeros = (const uint8_t *)c.qzeros; p.scale_perm = c.scale_perm; p.pdl = c.pdl;
   p.group32 = c.group / 32; p.group_shift = -1;
   for (int i = 0; i < 26; i++) if (p.group32 == 1 << i) p.group_shift = i;
   p.nt = c.nt; p.tiles_m = c.tiles_m; p.tiles_n = (c.N + TS_BM - 1) / TS_BM; p.ksplit = c.ksplit;
