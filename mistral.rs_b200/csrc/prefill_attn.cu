@@ -13,8 +13,8 @@
 // ring with cp.async (16-byte copies, two tiles in flight); B fragments come from ldmatrix
 // (transposed for V).  GQA: head h reads KV head h / (H / KVH).  Causal tiles beyond the diagonal
 // are skipped, the diagonal tile is masked in registers; heavy (late) query tiles are scheduled first.
-// Legacy mma.sync path.  Head size 128 without window / softcap now runs on prefill_attn_tc.cu (tcgen05);
-// this kernel keeps head size 64, sliding window, softcap, and is the A/B for the other one.
+// mma.sync path: calls without softcap run on prefill_attn_tc.cu (tcgen05); this kernel keeps softcap, strides and scales that the other
+// declines, and is the A/B for it.
 #include "mma_common.cuh"
 
 #include <stdio.h>
@@ -243,7 +243,7 @@ extern "C" int32_t mrs_prefill_attention(const void *q, const void *k, const voi
                                          int64_t o_stride, float softmax_scale, int32_t causal, int32_t window_left,
                                          float softcap, uint32_t dtype, void *stream) {
   if (total_tokens <= 0) return 0;
-  {   // the tcgen05 kernel when the call fits it (head size 128, no window, no softcap)
+  {   // the tcgen05 kernel when the call fits it (no softcap)
     const int32_t e = mrs_prefill_attention_tc(q, k, v, out, cu_seqlens, batch, total_tokens, max_seqlen, num_heads, num_kv_heads,
                                                head_dim, q_stride, kv_stride, o_stride, softmax_scale, causal, window_left, softcap,
                                                dtype, stream);

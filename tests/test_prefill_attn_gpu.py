@@ -91,3 +91,37 @@ def test_both_kernels_head_128(cuda, dt):
                 assert (got - want).abs().max().item() <= 3 * ulp * want.abs().max().item() + 1e-6, (enable, causal)
     finally:
         lib().mrs_prefill_attn_tc_debug(ctypes.c_int32(1), ctypes.c_uint32(0), ctypes.c_uint32(0))
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D,H,KVH", [(64, 14, 2), (128, 6, 2)])
+@pytest.mark.parametrize("T", [1, 127, 128, 129, 400])
+def test_tensor_memory_kernel_windows_and_head_64(cuda, dt, D, H, KVH, T):
+    """Windows and head size 64 on csrc/prefill_attn_tc.cu, at the edges of its tiles of 128 queries and 128 keys, from slices of one packed
+    q / k / v buffer, against the fp64 reference: 3 ulp as above (P and the result are each rounded once)."""
+    gen = torch.Generator(device=cuda).manual_seed(T + D)
+    qkv = torch.randn(T, (H + 2 * KVH) * D, device=cuda, generator=gen).to(dt)
+    q, k, v = (t.unflatten(1, (-1, D)) for t in qkv.split([H * D, KVH * D, KVH * D], 1))
+    scale = 1.0 / np.sqrt(D)
+    ulp = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11
+    for causal in (True, False):
+        for window in (None, 0, 1, 127, 128, 129, 2 ** 31 - 1):
+            got = paged_attn.prefill_attention(q, k, v, scale, causal=causal, window_left=window).double()
+            want = _ref(q, k, v, scale, causal, window=window)
+            assert (got - want).abs().max().item() <= 3 * ulp * want.abs().max().item() + 1e-6, (causal, window)
+
+
+@pytest.mark.parametrize("D,window", [(64, None), (64, 50), (128, None), (128, 50)])
+def test_sequences_do_not_see_their_neighbours(cuda, D, window):
+    """A last tile reaches into the next sequence's rows: what stands there, finite or not, leaves no trace."""
+    lens, H, KVH = [70, 128, 0, 200, 5], 4, 2
+    gen = torch.Generator(device=cuda).manual_seed(4)
+    q, k, v = (torch.randn(sum(lens), h, D, device=cuda, generator=gen).to(torch.bfloat16) for h in (H, KVH, KVH))
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device=cuda)
+    run = lambda kk, vv: paged_attn.prefill_attention(q, kk, vv, D ** -0.5, cu_seqlens=cu, max_seqlen=max(lens), window_left=window)  # noqa: E731
+    clean = run(k, v)
+    for keep in range(len(lens)):
+        at = slice(int(cu[keep]), int(cu[keep + 1]))
+        kk, vv = torch.full_like(k, float("nan")), torch.full_like(v, float("inf"))
+        kk[at], vv[at] = k[at], v[at]
+        assert torch.equal(run(kk, vv)[at], clean[at])
