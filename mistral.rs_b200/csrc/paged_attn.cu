@@ -19,6 +19,7 @@
 #include <cuda_fp8.h>
 #include <stdio.h>
 #include <stdlib.h>
+#include <type_traits>
 
 namespace mrs {
 
@@ -56,6 +57,7 @@ struct PagedParams {
   int heads_per_cta;        // GQA group may be processed in sub-groups (blockIdx.z)
   int batch_size;           // sequences in this launch (0: unknown)
   int pdl;                  // launched with programmatic stream serialisation
+  int leads;                // lets the launch behind start (which waits for this one's results)
   // FUSED (mrs_paged_decode_fused): un-rotated new-token K/V, RoPE tables, slots, merge counters
   const void *k_new, *v_new;
   int64_t kv_new_stride;
@@ -223,8 +225,9 @@ __global__ void __launch_bounds__(PA_THREADS) paged_decode_kernel(const PagedPar
   }
   int chunk = p.kv_chunk_size_ptr ? *p.kv_chunk_size_ptr : p.kv_chunk_size;
   if (chunk <= 0) chunk = kv_len > 0 ? kv_len : 1;
-  const int t_begin = chunk_idx * chunk;
-  int t_end = min(kv_len, t_begin + chunk);
+  const int win_lo = (p.window_left >= 0) ? max(0, kv_len - 1 - p.window_left) : 0;
+  const int t_begin = max(chunk_idx * chunk, win_lo);      // (what lies before the window is not read)
+  int t_end = min(kv_len, chunk_idx * chunk + chunk);
   const bool partial = p.tmp_o != nullptr;
 
   const int group = p.num_heads / p.num_kv_heads;
@@ -248,7 +251,6 @@ __global__ void __launch_bounds__(PA_THREADS) paged_decode_kernel(const PagedPar
   }
 
   const CT *kc = (const CT *)p.kc, *vc = (const CT *)p.vc;
-  const int win_lo = (p.window_left >= 0) ? max(0, kv_len - 1 - p.window_left) : 0;
 
   auto load_q = [&]() {
     if (p.pdl) pdl_wait();
@@ -573,6 +575,7 @@ __global__ void merge_partials_kernel(const T *__restrict__ tmp_o, const float *
                                       int num_heads, int D, const float *__restrict__ sinks,
                                       const int32_t *__restrict__ context_lens, int partition_size) {
   const int s = blockIdx.x, h = blockIdx.y;
+  pdl_wait();                                // (launched behind the tiles; where they let it start early, its launch costs 0.4 us less)
   int t0, t1;
   if (o_indptr != nullptr) { t0 = o_indptr[s]; t1 = o_indptr[s + 1]; }
   else {
@@ -601,7 +604,16 @@ __global__ void merge_partials_kernel(const T *__restrict__ tmp_o, const float *
 #include "paged_attn_mma.cuh"
 namespace mrs {
 
-static int g_pa_flags = 0;   // bit 0: keep HND decode on the SIMT kernel (A/B, debugging)
+static int g_pa_flags = 0;   // bit 0: keep HND decode on the SIMT kernel (A/B, debugging); bit 2 / 3: never / always pairs of CTAs a tile; bit 4: merge late
+
+// Pairs of CTAs a tile, each with half of its tokens: at up to one and a half CTAs an SM.  There a tile's time is its chain of stages (load, scores,
+// soft-max, product: ~1 us each), and half as many of them take 11.3 us where the whole took 13.8 (1 sequence of 300 tokens, 32 query and 8 KV heads of
+// 128), 13.9 against 15.4 (1 of 3000), 13.9 against 15.5 (16 of 300), 12.7 against 14.0 (8 of 500).  With more CTAs the pairs no longer run at one time
+// and each adds a head and an exchange: 256 CTAs take 19.4 us against 15.2, 376 take 25.3 against 19.2.
+static bool pm_pairs(long long ctas) {
+  if (g_pa_flags & 12) return (g_pa_flags & 8) != 0;
+  return 2 * ctas <= 3 * 148;
+}
 
 template <typename K>
 static cudaError_t launch_pa(K kern, dim3 grid, const PagedParams &p, cudaStream_t st, size_t dyn_smem, int threads = PA_THREADS) {
@@ -654,6 +666,22 @@ static cudaError_t launch_decode_g(PagedParams p, int tiles, cudaStream_t st) {
             cfg.numAttrs = p.pdl ? 2 : 1;
             return cudaLaunchKernelEx(&cfg, kern, p);
           }
+        }
+      }
+      if constexpr (!FUSED) {
+        if (pm_pairs((long long)tiles * p.num_kv_heads * nsub)) {
+          auto kern = paged_decode_mma_kernel<T, D, false, false, true>;
+          const size_t dyn = pm_smem_bytes<D>(false, false);
+          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+          cudaLaunchConfig_t cfg = {};
+          cfg.gridDim = dim3(2 * tiles, p.num_kv_heads, nsub); cfg.blockDim = dim3(PM_THREADS); cfg.dynamicSmemBytes = dyn; cfg.stream = st;
+          cudaLaunchAttribute attr[2];
+          attr[0].id = cudaLaunchAttributeClusterDimension;
+          attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+          attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+          attr[1].val.programmaticStreamSerializationAllowed = 1;
+          cfg.attrs = attr; cfg.numAttrs = p.pdl ? 2 : 1;
+          return cudaLaunchKernelEx(&cfg, kern, p);
         }
       }
       return launch_pa(paged_decode_mma_kernel<T, D, FUSED, false>, grid, p, st, pm_smem_bytes<D>(FUSED, false), PM_THREADS);
@@ -757,14 +785,23 @@ extern "C" int32_t flashinfer_decode(void *q, void *key_cache, void *value_cache
     p.request_indices = nullptr; p.kv_tile_indices = nullptr; p.block_valid_mask = nullptr;
   }
   const int tiles = split ? padded_batch_size : batch_size;
+  p.leads = split && !(g_pa_flags & 16);
   cudaError_t e = launch_decode_any<1>(p, dtype, cache_dtype, head_size, tiles, stream);
   if (e != cudaSuccess) { fprintf(stderr, "mrs_b200: flashinfer_decode failed: %s\n", cudaGetErrorString(e)); return (int32_t)e; }
   if (split) {
     dim3 grid(batch_size, num_qo_heads);
-    if (dtype == 0) merge_partials_kernel<__half><<<grid, 128, 0, stream>>>((const __half *)tmp_v, (const float *)tmp_s, (__half *)o, o_indptr, 0, num_qo_heads, head_size, nullptr, nullptr, 0);
-    else if (dtype == 1) merge_partials_kernel<__nv_bfloat16><<<grid, 128, 0, stream>>>((const __nv_bfloat16 *)tmp_v, (const float *)tmp_s, (__nv_bfloat16 *)o, o_indptr, 0, num_qo_heads, head_size, nullptr, nullptr, 0);
-    else merge_partials_kernel<float><<<grid, 128, 0, stream>>>((const float *)tmp_v, (const float *)tmp_s, (float *)o, o_indptr, 0, num_qo_heads, head_size, nullptr, nullptr, 0);
-    e = cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = dim3(128); cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = p.leads ? 1 : 0;
+    auto merge = [&](auto *t) {
+      using T = std::remove_pointer_t<decltype(t)>;
+      return cudaLaunchKernelEx(&cfg, merge_partials_kernel<T>, (const T *)tmp_v, (const float *)tmp_s, (T *)o, o_indptr, 0, (int)num_qo_heads,
+                                (int)head_size, (const float *)nullptr, (const int32_t *)nullptr, 0);
+    };
+    e = dtype == 0 ? merge((__half *)nullptr) : dtype == 1 ? merge((__nv_bfloat16 *)nullptr) : merge((float *)nullptr);
   }
   return (int32_t)e;
 }

@@ -47,7 +47,7 @@ __device__ __forceinline__ void pm_st_cluster_f32(const float *local_ptr, uint32
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
 }
 
-template <typename T, int D, bool FUSED, bool CLUSTER>
+template <typename T, int D, bool FUSED, bool CLUSTER, bool SPLIT = false>
 __global__ void __launch_bounds__(PM_THREADS, 3) paged_decode_mma_kernel(const PagedParams p) {
   constexpr int KSTEPS = D / 16, DT = D / 8, CPR = D / 8, LPT = D / 8;
   constexpr int TILE_BYTES = PM_BN * D * 2;
@@ -60,9 +60,10 @@ __global__ void __launch_bounds__(PM_THREADS, 3) paged_decode_mma_kernel(const P
   __shared__ int st_pages[2048 / 8 + 2];
   __shared__ int sm_last;
 
-  const int tile = blockIdx.x, kvh = blockIdx.y;
+  static_assert(!SPLIT || (!FUSED && !CLUSTER), "a tile's pair of CTAs merges for itself");
+  const int tile = SPLIT ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, kvh = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (p.pdl && tid == 0) pdl_launch_dependents();
+  if ((p.pdl || p.leads) && tid == 0) pdl_launch_dependents();
   const bool valid = p.block_valid_mask == nullptr || p.block_valid_mask[tile] != 0;
   if (!CLUSTER && !valid) return;
   int seq = tile, chunk_idx = 0;
@@ -72,13 +73,18 @@ __global__ void __launch_bounds__(PM_THREADS, 3) paged_decode_mma_kernel(const P
   const int kv_len = (p1 > p0) ? (p1 - p0 - 1) * p.page_size + p.kv_last_page_len[seq] : 0;
   int chunk = p.kv_chunk_size_ptr ? *p.kv_chunk_size_ptr : p.kv_chunk_size;
   if (chunk <= 0) chunk = kv_len > 0 ? kv_len : 1;
-  const int t_begin = chunk_idx * chunk;
-  const int t_end = valid ? min(kv_len, t_begin + chunk) : t_begin;
+  const int win_lo = (p.window_left >= 0) ? max(0, kv_len - 1 - p.window_left) : 0;
+  int t_begin = max(chunk_idx * chunk, win_lo);            // (what lies before the window is not read)
+  int t_end = valid ? min(kv_len, chunk_idx * chunk + chunk) : t_begin;
+  if constexpr (SPLIT) {                                   // the pair's first CTA takes the first half, in whole steps
+    const int mid = min(t_end, t_begin + (((max(0, t_end - t_begin) >> 1) + PM_BN - 1) & ~(PM_BN - 1)));
+    if (pm_cluster_rank() == 0) t_end = mid;
+    else t_begin = mid;
+  }
   const bool partial = p.tmp_o != nullptr;
   const int group = p.num_heads / p.num_kv_heads;
   const int h0 = kvh * group + blockIdx.z * p.heads_per_cta;
   const int gsize = min(p.heads_per_cta, group - (int)blockIdx.z * p.heads_per_cta);   // <= 16
-  const int win_lo = (p.window_left >= 0) ? max(0, kv_len - 1 - p.window_left) : 0;
   bool owns_new = false;
   if constexpr (FUSED) owns_new = valid && kv_len > 0 && (kv_len - 1) >= t_begin && (kv_len - 1) < t_end;
   const int t_cache_end = owns_new ? kv_len - 1 : t_end;   // the new token is attended from shared memory
@@ -280,12 +286,41 @@ __global__ void __launch_bounds__(PM_THREADS, 3) paged_decode_mma_kernel(const P
   }
   __syncthreads();
   uint32_t crank = 0;
-  if constexpr (CLUSTER) crank = pm_cluster_rank();
+  if constexpr (CLUSTER || SPLIT) crank = pm_cluster_rank();
+  // SPLIT: [16][D + 2] of the second CTA, in the first one's buffers behind the warps' states
+  [[maybe_unused]] float *other = (float *)(pm_smem + 2 * TILE_BYTES + TILE_BYTES / 2);
+  static_assert((size_t)(PM_WARPS * 16 * (D + 2)) * 4 <= (size_t)(2 * TILE_BYTES + TILE_BYTES / 2), "the warps' states lie in front");
+  static_assert((size_t)16 * (D + 2) * 4 <= (size_t)(TILE_BYTES + TILE_BYTES / 2), "and the other CTA's in the buffers too");
+  if constexpr (SPLIT) {
+    pm_cluster_sync();                             // both CTAs have left their buffers
+    if (crank == 1) {
+      for (int idx = tid; idx < gsize * D; idx += PM_THREADS) {
+        const int g = idx / D, d = idx % D;
+        float M = -INFINITY, L = 0.f, acc = 0.f;
+#pragma unroll
+        for (int w = 0; w < PM_WARPS; w++) M = fmaxf(M, mm[w * 16 + g]);
+        if (M > -INFINITY) {
+#pragma unroll
+          for (int w = 0; w < PM_WARPS; w++) {
+            const float c = exp2f(mm[w * 16 + g] - M);
+            L += ml[w * 16 + g] * c;
+            acc += mo[((size_t)w * 16 + g) * D + d] * c;
+          }
+        }
+        float *slot = other + (size_t)g * (D + 2);
+        pm_st_cluster_f32(slot + d, 0u, acc);
+        if (d == 0) { pm_st_cluster_f32(slot + D, 0u, M); pm_st_cluster_f32(slot + D + 1, 0u, L); }
+      }
+    }
+    pm_cluster_sync();
+    if (crank == 1) return;
+  }
   for (int idx = tid; idx < gsize * D; idx += PM_THREADS) {
     const int g = idx / D, d = idx % D;
     float M = -INFINITY;
 #pragma unroll
     for (int w = 0; w < PM_WARPS; w++) M = fmaxf(M, mm[w * 16 + g]);
+    if constexpr (SPLIT) M = fmaxf(M, other[(size_t)g * (D + 2) + D]);
     float L = 0.f, acc = 0.f;
     if (M > -INFINITY) {
 #pragma unroll
@@ -293,6 +328,11 @@ __global__ void __launch_bounds__(PM_THREADS, 3) paged_decode_mma_kernel(const P
         const float c = exp2f(mm[w * 16 + g] - M);
         L += ml[w * 16 + g] * c;
         acc += mo[((size_t)w * 16 + g) * D + d] * c;
+      }
+      if constexpr (SPLIT) {
+        const float *slot = other + (size_t)g * (D + 2), c = exp2f(slot[D] - M);
+        L += slot[D + 1] * c;
+        acc += slot[d] * c;
       }
     }
     if constexpr (CLUSTER) {

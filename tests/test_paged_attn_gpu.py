@@ -111,3 +111,33 @@ def test_softcap_window_and_errors(cuda):
     with pytest.raises(ValueError, match="i32"):
         paged_attn.flashinfer_decode(to_dev(q, cuda, dt), kct, vct, d(indptr).long(), d(indices), d(last), d(req), d(tile),
                                      d(o_indptr), d(chunk), d(mask), scale)
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("H,KVH,D", [(16, 1, 128), (8, 4, 64)])
+@pytest.mark.parametrize("window", [None, 0, 63, 64, 500])
+def test_pairs_of_ctas_and_windows(cuda, dt, H, KVH, D, window):
+    """A tile by one CTA and by a pair that halves its tokens in whole steps of 64, with the tokens before a window unread: 2.5 ulp as above."""
+    import ctypes
+    from mistralrs_b200 import lib
+    ctx, BS = [1, 63, 64, 65, 127, 129, 700], 16
+    q, kct, vct, _, _, bt, tables = _setup(cuda, len(ctx), H, KVH, D, BS, ctx, "hnd", dt, seed=5)
+    qt, want = to_dev(q, cuda, dt), []
+    for b, n in enumerate(ctx):
+        k, v = (t[torch.tensor(tables[b], device=cuda)].double().transpose(1, 2).reshape(-1, KVH, D)[:n].repeat_interleave(H // KVH, 1) for t in (kct, vct))
+        s = torch.einsum("hd,thd->ht", qt[b].double(), k) * D ** -0.5
+        if window is not None:
+            s[:, :max(0, n - 1 - window)] = -torch.inf
+        want.append(torch.einsum("ht,thd->hd", torch.softmax(s, -1), v))
+    want = torch.stack(want).cpu().numpy()
+    indptr, indices, last = kv_index.make_paged_kv_tensors(tables, ctx, BS, bt.size)
+    try:
+        for pages in (None, 16):
+            tiles = sum(-(-len(t) // pages) if pages else 1 for t in tables)
+            meta = [to_dev(np.ascontiguousarray(m), cuda) for m in (indptr, indices, last, *kv_index.make_paged_kv_decode_tensors(tables, ctx, BS, pages, tiles))]
+            for flags in (4, 8):
+                lib().mrs_set_attn_flags(ctypes.c_int(flags))
+                got = paged_attn.flashinfer_decode(qt, kct, vct, *meta, D ** -0.5, window_left=window)
+                _check(got.float().cpu().numpy(), want, dt)
+    finally:
+        lib().mrs_set_attn_flags(ctypes.c_int(0))
