@@ -63,11 +63,15 @@ int mrs_mmvq_fused(int ggml_type, int mode, int dt, const void *w0, const void *
                    int n0, int n1, int n2, int b_size, int activation, int pdl, void *stream);
 
 /* The same in two launches, for steps whose rows are many or long: the optional RMSNorm and the Q8_1 rows [b_size][K / 32] (36 bytes each, K %
- * 32 == 0, x and norm_w 16-byte aligned) by one, the GEMV over rows quantised so by the other.  The same bits as mrs_mmvq_fused; several
- * GEMVs may read the rows of one quantisation. */
+ * 32 == 0, x and norm_w 16-byte aligned) by one, the GEMV over rows quantised so by the other.  The same bits as mrs_mmvq_fused; from three
+ * rows over 8 MB of Q4_K, Q5_K, Q6_K or Q8_0 weights on, the same integer dots and scales, added up in f32 in another order.  Several GEMVs may
+ * read the rows of one quantisation. */
 int mrs_rms_quantize_q8_1(int dt, const void *x, const void *norm_w, float eps, int K, int b_size, void *q8, int pdl, void *stream);
 int mrs_mmvq_q8(int ggml_type, int mode, int dt, const void *w0, const void *w1, const void *w2, const void *q8, const void *residual,
                 void *dst0, void *dst1, void *dst2, int K, int n0, int n1, int n2, int b_size, int activation, int pdl, void *stream);
+/* Both in one call, without a norm: q8 holds b_size x K / 32 blocks. */
+int mrs_mmvq_rows(int ggml_type, int mode, int dt, const void *w0, const void *w1, const void *w2, const void *x, void *q8, void *dst0, void *dst1,
+                  void *dst2, int K, int n0, int n1, int n2, int b_size, int activation, void *stream);
 
 /* QKV projection where attn_v carries its own ggml type (llama.cpp's k-quant "M" recipes, e.g.
  * Q4_K_M: attn_q/attn_k Q4_K, attn_v Q6_K on half the layers): q||k rows and v rows read the same

@@ -24,6 +24,8 @@
 
 #include <stdio.h>
 
+extern "C" int32_t *mrs_mmq_timeout_flag(void);      // mmq_ts.cu: the device's word for waits that ran out
+
 namespace mrs {
 
 // CTA shape: NCW = 8 consumer warps + 1 producer warp, two CTAs per SM; a stage holds 2
@@ -63,6 +65,7 @@ struct MmvqParams {
   int K, stride_col_y, stride_col_dst, ncols;
   int mode, activation, dst_dtype;
   int nstages, vrows, pdl, flags;
+  int *timeouts;         // set when a wait of the tensor-core kernel runs out (page-locked host memory)
 #ifdef MRS_TIMELINE
   unsigned long long *dbg;  // dev build: [gridDim.x][16] globaltimer stamps of this launch
 #endif
@@ -117,6 +120,10 @@ __device__ __forceinline__ void resolve_row(const MmvqParams &p, int vrow, int w
     m = 0; row = vrow;
   }
 }
+
+}  // namespace mrs
+#include "mmvq_mma.cuh"
+namespace mrs {
 
 // accessor handed to QT::aux — d8/s8 of q8_1 block j relative to the weight block
 struct YGlobal {
@@ -638,6 +645,41 @@ static cudaError_t launch_one(MmvqParams p, cudaStream_t stream) {
   return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
+// Rows of Q8_1 activations from so many on, over at least so many bytes of weights: integer tensor-core products (mmvq_mma.cuh).  One B200, us
+// with the quantising launch, vector kernel / tensor cores: Q4_K 14336 x 4096 2 rows 15.3 / 16.8, 3 19.8 / 16.9, 4 20.2 / 17.1, 8 31.7 / 18.6;
+// 4096 x 14336 4 rows 22.2 / 18.6, 8 34.6 / 22.3; gate and up of 14336 x 4096 4 rows 32.8 / 25.3, 8 55.3 / 26.6; Q6_K 4096 x 14336 4 rows
+// 27.1 / 21.9, 8 38.4 / 28.3.  Below 8 MB launches and the fill of the rings are what is paid for.
+constexpr int MV_MIN_ROWS = 3;
+constexpr size_t MV_MIN_BYTES = 8u << 20;
+template <int T, int NC> static cudaError_t launch_mma(MmvqParams p, cudaStream_t stream) {
+  constexpr size_t STAGE = 16 * (size_t)MvFmt<T>::PITCH;
+  int32_t *const timeouts = mrs_mmq_timeout_flag();
+  if (timeouts == nullptr || *(volatile const int32_t *)timeouts != 0) return cudaErrorNotSupported;
+  const DevInfo &d = query_device();
+  const size_t fixed = 256 + (size_t)NC * (p.K + 32) + (size_t)p.K / 32 * NC * 8 + 2 * 8 * 128 * 4;
+  int per_sm = 2, nst = 0;
+  size_t budget = (size_t)d.max_smem / 2 - 1024;
+  if (fixed + 2 * STAGE > budget) { per_sm = 1; budget = (size_t)d.max_smem - 1024; }
+  while (nst < MAX_STAGES && fixed + (nst + 1) * STAGE <= budget) nst++;
+  if (nst < 2) return cudaErrorNotSupported;
+  p.nstages = nst;
+  p.timeouts = timeouts;
+  const int P = p.mode == MODE_GLU ? 8 : 16, passes = (p.vrows + P - 1) / P, most = per_sm * d.num_sms;
+  auto kern = mmvq_mma_kernel<T, NC>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, d.max_smem);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(passes < most ? passes : most);
+  cfg.blockDim = dim3(9 * 32);
+  cfg.dynamicSmemBytes = fixed + nst * STAGE;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
 template <int T> static bool rows_aligned(const MmvqParams &p) {
   using Q = QT<T>;
   const int row_bytes = (p.K / Q::QK) * Q::BYTES;
@@ -713,6 +755,12 @@ static cudaError_t launch_type(MmvqParams p, cudaStream_t stream) {
   for (int m = 0; m < 3; m++)
     if (p.w[m] != nullptr) wbytes += (size_t)p.nrows[m] * row_bytes;
   const int b = p.ncols;
+  if constexpr (MvFmt<T>::ok) {
+    if (b >= MV_MIN_ROWS && p.xkind == X_Q8_1 && p.K % 256 == 0 && fast && wbytes >= MV_MIN_BYTES && !(g_flags & 16)) {
+      const cudaError_t e = b <= 4 ? launch_mma<T, 4>(p, stream) : launch_mma<T, 8>(p, stream);
+      if (e != cudaErrorNotSupported) return e;
+    }
+  }
 #define MRS_DISPATCH(NC)                                                                          \
   do {                                                                                            \
     if constexpr (HasLong<T>::value) {                                                            \
@@ -812,7 +860,7 @@ using namespace mrs;
 static int g_mrs_pdl = 0;  // PDL on reference-shaped launchers is opt-in (mrs_set_pdl)
 
 extern "C" void mrs_set_pdl(int enabled) { g_mrs_pdl = enabled; }
-// flags: bit 3 = never use the long-segment variant; bits 8.. = long-segment threshold in MiB
+// flags: bit 3 = never use the long-segment variant; bit 4 = never the tensor-core kernel; bits 8.. = long-segment threshold in MiB
 extern "C" void mrs_set_mmvq_flags(int f) { g_flags = f & 0xff; if (f >> 8) g_long_min_bytes = (long long)(f >> 8) << 20; }
 extern "C" int mrs_mmvq_has_wide(void) { return 0; }
 extern "C" void mrs_set_mmvq_ctas_per_sm(int n) { g_ctas_per_sm = n < 1 ? 1 : (n > 3 ? 3 : n); }
@@ -923,14 +971,18 @@ extern "C" int mrs_mmvq_fused(int ggml_type, int mode, int dt, const void *w0, c
 
 // Q8_1 rows [b_size][K / 32] of [RMSNorm'd] activations, and the GEMV over rows quantised so: together what mrs_mmvq_fused does, for steps
 // whose rows are many or long (K % 32 == 0)
-extern "C" int mrs_rms_quantize_q8_1(int dt, const void *x, const void *norm_w, float eps, int K, int b_size, void *q8, int pdl, void *stream) {
+// follows: may start beside the grid before; leads: lets the grid behind start
+static int launch_rms_quantize(int dt, const void *x, const void *norm_w, float eps, int K, int b_size, void *q8, bool follows, bool leads, void *stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((K + RQ_COLS - 1) / RQ_COLS, b_size); cfg.blockDim = dim3(RQ_THREADS); cfg.stream = (cudaStream_t)stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = pdl ? 1 : 0;
-  return (int)cudaLaunchKernelEx(&cfg, rms_quantize_q8_1_kernel, x, norm_w, eps, dt, K, (block_q8_1 *)q8, pdl);
+  cfg.attrs = attr; cfg.numAttrs = follows ? 1 : 0;
+  return (int)cudaLaunchKernelEx(&cfg, rms_quantize_q8_1_kernel, x, norm_w, eps, dt, K, (block_q8_1 *)q8, (int)leads);
+}
+extern "C" int mrs_rms_quantize_q8_1(int dt, const void *x, const void *norm_w, float eps, int K, int b_size, void *q8, int pdl, void *stream) {
+  return launch_rms_quantize(dt, x, norm_w, eps, K, b_size, q8, pdl != 0, pdl != 0, stream);
 }
 extern "C" int mrs_mmvq_q8(int ggml_type, int mode, int dt, const void *w0, const void *w1, const void *w2, const void *q8, const void *residual,
                            void *dst0, void *dst1, void *dst2, int K, int n0, int n1, int n2, int b_size, int activation, int pdl, void *stream) {
@@ -943,6 +995,15 @@ extern "C" int mrs_mmvq_q8(int ggml_type, int mode, int dt, const void *w0, cons
   p.dst_dtype = dt; p.pdl = pdl;
   p.vrows = (mode == MODE_QKV) ? n0 + n1 + n2 : n0;
   return (int)mmvq_dispatch(ggml_type, p, (cudaStream_t)stream);
+}
+
+// Both for one call of a linear: rows of x into q8 (b_size x K / 32 blocks), then the GEMV, whose weights are on their way while the rows are
+// quantised.  (The first launch follows the stream as any other, so whatever wrote the weights has ended when the second reads them.)
+extern "C" int mrs_mmvq_rows(int ggml_type, int mode, int dt, const void *w0, const void *w1, const void *w2, const void *x, void *q8, void *dst0, void *dst1,
+                             void *dst2, int K, int n0, int n1, int n2, int b_size, int activation, void *stream) {
+  const int e = launch_rms_quantize(dt, x, nullptr, 0.0f, K, b_size, q8, false, true, stream);
+  if (e != 0) return e;
+  return mrs_mmvq_q8(ggml_type, mode, dt, w0, w1, w2, q8, nullptr, dst0, dst1, dst2, K, n0, n1, n2, b_size, activation, 1, stream);
 }
 
 static cudaError_t mmvq_dispatch_dual_entry(int t1, const MmvqParams &pa, int t2, const MmvqParams &pb, cudaStream_t stream) {

@@ -98,7 +98,7 @@ _WORKSPACE = {}
 def _workspace(device, nbytes):
     """Grow-never-free scratch keyed like fast_mmvq.rs:70-112 (stable addresses for graphs)."""
     cap = 1 << max(int(nbytes) - 1, 0).bit_length()
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream, cap)
+    key = (device.index, raw_stream(device), cap)
     buf = _WORKSPACE.get(key)
     if buf is None:
         buf = torch.empty(cap, dtype=torch.uint8, device=device)
@@ -197,12 +197,17 @@ def quantize_q8_1(xs: torch.Tensor, k_padded=None) -> torch.Tensor:
     return out
 
 
-def _quantize_into_workspace(xs, k, b_size):
-    k_padded = _pad(k, MATRIX_ROW_PADDING)
-    scratch = _workspace(xs.device, b_size * (k_padded // Q8_1_BLOCK_SIZE) * Q8_1_TYPE_SIZE)
-    fn = getattr(lib(), f"launch_mmvq_gguf_quantize_q8_1_{_DT_TAG[xs.dtype]}")
-    fn(_ptr(xs), _ptr(scratch), ctypes.c_int(k), ctypes.c_int(k_padded), ctypes.c_int(b_size), _stream_ptr(xs.device))
-    return scratch, k_padded // Q8_1_BLOCK_SIZE
+def _rows(mode, ws, xs, outs, k, b_size, activation=0):
+    """Rows quantised into the workspace, then the GEMV over them: two launches behind one call."""
+    n = [w.shape[0] for w in ws] + [0, 0]
+    wp = [w.data.data_ptr() for w in ws] + [0, 0]
+    op = [o.data_ptr() for o in outs] + [0, 0]
+    scratch = _workspace(xs.device, b_size * (k // Q8_1_BLOCK_SIZE) * Q8_1_TYPE_SIZE)
+    fn = typed("mrs_mmvq_rows", _I, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P)
+    rc = fn(_ggml_code(ws[0].dtype), mode, _DT_CODE[xs.dtype], wp[0], wp[1], wp[2], xs.data_ptr(), scratch.data_ptr(), op[0], op[1], op[2], k, n[0], n[1],
+            n[2], b_size, activation, raw_stream(xs.device))
+    if rc != 0:
+        raise RuntimeError(f"mrs_mmvq_rows failed with cudaError {rc}")
 
 
 def plain(w: QTensor, xs: torch.Tensor) -> torch.Tensor:
@@ -213,10 +218,7 @@ def plain(w: QTensor, xs: torch.Tensor) -> torch.Tensor:
     if _one_launch(b_size, k, nrows, xs):
         _fused_one_row(0, (w,), xs, (out,), k)
         return out
-    scratch, stride_col_y = _quantize_into_workspace(xs, k, b_size)
-    fn = getattr(lib(), f"launch_mmvq_gguf_{w.dtype}_{_DT_TAG[xs.dtype]}_plain")
-    fn(_ptr(w.data), _ptr(scratch), _ptr(out), ctypes.c_int(k), ctypes.c_int(nrows), ctypes.c_int(stride_col_y),
-       ctypes.c_int(nrows), ctypes.c_int(b_size), _stream_ptr(xs.device))
+    _rows(0, (w,), xs, (out,), k, b_size)
     return out
 
 
@@ -232,11 +234,7 @@ def fused_glu(gate_w: QTensor, up_w: QTensor, xs: torch.Tensor, activation: GluA
     if _one_launch(b_size, k, nrows, xs):
         _fused_one_row(1, (gate_w, up_w), xs, (out,), k, int(activation))
         return out
-    scratch, stride_col_y = _quantize_into_workspace(xs, k, b_size)
-    fn = getattr(lib(), f"launch_mmvq_gguf_{gate_w.dtype}_{_DT_TAG[xs.dtype]}_fused_glu")
-    fn(_ptr(gate_w.data), _ptr(up_w.data), _ptr(scratch), _ptr(out), ctypes.c_int(k), ctypes.c_int(nrows),
-       ctypes.c_int(stride_col_y), ctypes.c_int(nrows), ctypes.c_int(b_size), ctypes.c_int(int(activation)),
-       _stream_ptr(xs.device))
+    _rows(1, (gate_w, up_w), xs, (out,), k, b_size, int(activation))
     return out
 
 
@@ -252,11 +250,7 @@ def fused_qkv(q_w: QTensor, k_w: QTensor, v_w: QTensor, xs: torch.Tensor):
     if _one_launch(b_size, k, sum(w.shape[0] for w in (q_w, k_w, v_w)), xs):
         _fused_one_row(2, (q_w, k_w, v_w), xs, outs, k)
         return tuple(outs)
-    scratch, stride_col_y = _quantize_into_workspace(xs, k, b_size)
-    fn = getattr(lib(), f"launch_mmvq_gguf_{q_w.dtype}_{_DT_TAG[xs.dtype]}_fused_qkv")
-    fn(_ptr(q_w.data), _ptr(k_w.data), _ptr(v_w.data), _ptr(scratch), _ptr(outs[0]), _ptr(outs[1]), _ptr(outs[2]),
-       ctypes.c_int(k), ctypes.c_int(q_w.shape[0]), ctypes.c_int(k_w.shape[0]), ctypes.c_int(v_w.shape[0]),
-       ctypes.c_int(stride_col_y), ctypes.c_int(b_size), _stream_ptr(xs.device))
+    _rows(2, (q_w, k_w, v_w), xs, outs, k, b_size)
     return tuple(outs)
 
 

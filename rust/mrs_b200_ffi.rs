@@ -36,6 +36,7 @@ extern "C" {
     pub fn mrs_mmvq_fused(ggml_type: i32, mode: i32, dt: i32, w0: *const c_void, w1: *const c_void, w2: *const c_void, x: *const c_void, norm_w: *const c_void, eps: f32, residual: *const c_void, dst0: *mut c_void, dst1: *mut c_void, dst2: *mut c_void, K: i32, n0: i32, n1: i32, n2: i32, b_size: i32, activation: i32, pdl: i32, stream: *mut c_void) -> i32;
     pub fn mrs_rms_quantize_q8_1(dt: i32, x: *const c_void, norm_w: *const c_void, eps: f32, K: i32, b_size: i32, q8: *mut c_void, pdl: i32, stream: *mut c_void) -> i32;
     pub fn mrs_mmvq_q8(ggml_type: i32, mode: i32, dt: i32, w0: *const c_void, w1: *const c_void, w2: *const c_void, q8: *const c_void, residual: *const c_void, dst0: *mut c_void, dst1: *mut c_void, dst2: *mut c_void, K: i32, n0: i32, n1: i32, n2: i32, b_size: i32, activation: i32, pdl: i32, stream: *mut c_void) -> i32;
+    pub fn mrs_mmvq_rows(ggml_type: i32, mode: i32, dt: i32, w0: *const c_void, w1: *const c_void, w2: *const c_void, x: *const c_void, q8: *mut c_void, dst0: *mut c_void, dst1: *mut c_void, dst2: *mut c_void, K: i32, n0: i32, n1: i32, n2: i32, b_size: i32, activation: i32, stream: *mut c_void) -> i32;
     pub fn mrs_mmvq_fused_qkv_mixed(type_qk: i32, type_v: i32, dt: i32, wq: *const c_void, wk: *const c_void, wv: *const c_void, x: *const c_void, norm_w: *const c_void, eps: f32, q: *mut c_void, k: *mut c_void, v: *mut c_void, K: i32, nq: i32, nk: i32, nv: i32, b_size: i32, pdl: i32, stream: *mut c_void) -> i32;
     pub fn mrs_mmq_gguf(ggml_type: i32, w: *const c_void, x: *const c_void, y: *mut c_void, M: i32, N: i32, K: i32, dtype: i32, stream: *mut c_void) -> i32;
     pub fn mrs_mmq_set_weight_format(fmt: i32);

@@ -250,3 +250,34 @@ def test_one_row_captured_and_not(cuda, K, N):
     graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("dtype,N,K", [("q4_k", 6501, 2304), ("q5_k", 5297, 2304), ("q6_k", 4450, 2304), ("q8_0", 8193, 1024), ("q4_k", 1100, 14336),
+                                       ("q6_k", 1000, 11008), ("q8_0", 34000, 256)])
+@pytest.mark.parametrize("rows", [3, 4, 5, 8])
+def test_large_matrices_on_tensor_cores(cuda, dtype, rows, N, K):
+    """Three to eight rows over at least 8 MB of weights: integer products on the tensor cores against the vector kernel in every mode.  Integer dots
+    and their scales are exact in both; f32 sums of at most K / 16 terms in two orders, whose parts stay within 16 of the largest result, differ
+    by less than K x 2^-24 of that."""
+    import ctypes
+    from mistralrs_b200 import lib
+    gen = torch.Generator(device=cuda).manual_seed(N)
+    weight = lambda n, seed: quant.QTensor(to_dev(make_weight(dtype, n, K, seed).reshape(-1), cuda), dtype, (n, K))
+    x = torch.randn(rows, K, device=cuda, generator=gen)
+    ws = [weight(N, 1), weight(N, 2), weight(N - 7, 3)]
+    call = lambda t: [quant.plain(ws[0], t), *quant.fused_qkv(*ws, t), quant.fused_glu(ws[0], ws[1], t, quant.GluActivationType.Relu)]
+    results = []
+    try:
+        for flags in (16, 0):
+            lib().mrs_set_mmvq_flags(ctypes.c_int(flags))
+            results.append((call(x), call(x.to(torch.bfloat16))))
+    finally:
+        lib().mrs_set_mmvq_flags(ctypes.c_int(0))
+    (want, want16), (got, got16) = results
+    assert not all(torch.equal(a, b) for a, b in zip(got, want))        # two kernels
+    top = [w.abs().max() for w in want]
+    for a, b, s in zip(got, want, [*top[:4], 2 * top[1] * top[2]]):
+        assert ((a - b).abs() <= K * 2.0 ** -24 * s).all()
+    for a, b in zip(got16, want16):           # the same rounding but where a sum lies at its edge
+        assert ((a - b).abs() <= 2.0 ** -6 * b.abs().max()).all() and (a != b).float().mean() < 2e-2
+    assert lib().mrs_mmq_timeouts() == 0
