@@ -125,6 +125,10 @@ int marlin_awq_4bit_f16(const void *inputs, const int32_t *weight, const void *s
                         const void *out, int m, int k, int n, const void *workspace, int groupsize, int64_t stream);
 int marlin_awq_4bit_bf16(const void *inputs, const int32_t *weight, const void *scales, const void *zeros,
                          const void *out, int m, int k, int n, const void *workspace, int groupsize, int64_t stream);
+/* The same with dtype (activations, result) and scale_dtype (scales) each 0 f16 / 1 bf16: scales are rounded to the activation format as the
+ * kernel reads them.  Not reference ABI. */
+int mrs_marlin_4bit(const void *inputs, const int32_t *weight, const void *scales, const void *zeros, void *out, int m, int k, int n,
+                    int groupsize, int dtype, int scale_dtype, int is_awq, int64_t stream);
 /* weight: GPTQ [k/8, n] i32 / AWQ [k, n] i32 with n = out_dim/8; perm: argsort(g_idx) [k] i32 (GPTQ;
  * NULL = identity); bits must be 4 — REF kernels/marlin/marlin_repack.cu:255,473 */
 void gptq_marlin_repack(const void *weight, const void *perm, const void *result, int k, int n, int bits, int64_t stream);

@@ -55,16 +55,17 @@ struct TsParams {
   int nt, tiles_m, tiles_n;   // tokens per tile (multiple of 16), tiles
   int ksplit;                 // CTAs of a cluster that share K
   int rs, xs, xb;             // depths of the raw and the X ring; 64-k tiles of an X stage
-  // int4 checkpoints (TS_INT4): w in tiles [K/64][N][32 B] (csrc/w4a16.cu), scales [K/group][N] in the activation format
+  // int4 checkpoints (TS_INT4): w in tiles [K/64][N][32 B] (csrc/w4a16.cu), scales [K/group][N]
   const uint8_t *scales;
   const uint8_t *qzeros;      // AWQ [K/group][N/8] words, or null: zero point 8
   int group32, group_shift;   // weights of a group / 32, and its logarithm or -1
-  int scale_perm;             // columns 0 plain, 1 / 2 Marlin-permuted 64 / 32 wide
+  int scale_perm;             // columns 0 plain, 1 / 2 Marlin-permuted 64 / 32 wide; TS_SCALES_OTHER: scales in the other 16-bit format
   int pdl;                    // link of a programmatic-dependent-launch chain: x comes from, y may be read by, the grid before
 };
 // (eight bytes more, and every launch took the host 0.3 us longer)
 static_assert(sizeof(TsParams) <= 104, "parameters of a launch");
 
+constexpr int TS_SCALES_OTHER = 4;         // (of TsParams::scale_perm) f16 scales of bf16 rows, bf16 scales of f16 rows: rounded on the way
 constexpr int TS_INT4 = 200;               // block type of int4 checkpoints
 // SPAN: bytes of 256 weights of a row; PITCH: of a row in a raw stage, an odd multiple of 16 (16-byte reads of 8 consecutive rows
 // then fall on distinct banks) that also holds the bytes in front of and behind an unaligned span
@@ -689,8 +690,9 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
     if constexpr (TYPE == TS_INT4) {
       // inverses of the reference's scale-column permutations (REF gptq_cuda.rs:530-540 get_scale_perms), which stay inside a tile:
       // 64 wide perm[8 i + j] = i + 8 j, 32 wide perm[8 i + j] = 2 i + {0, 1, 8, 9, 16, 17, 24, 25}[j]
-      const int c = p.scale_perm == 1 ? (r & ~63) + 8 * (r & 7) + ((r & 63) >> 3)
-                  : p.scale_perm == 2 ? (r & ~31) + 8 * ((r & 7) >> 1) + 2 * ((r & 31) >> 3) + (r & 1) : r;
+      const int perm = p.scale_perm & 3;
+      const int c = perm == 1 ? (r & ~63) + 8 * (r & 7) + ((r & 63) >> 3)
+                  : perm == 2 ? (r & ~31) + 8 * ((r & 7) >> 1) + 2 * ((r & 31) >> 3) + (r & 1) : r;
       scale0 = smem_u32(r_ring) + (uint32_t)(TS_I4_SCALES + 2 * c);
       zero0 = smem_u32(r_ring) + (uint32_t)(TS_I4_ZEROS + 4 * (r >> 3));
       zero_shift = 4 * ((r & 1) ? 4 + ((r & 7) >> 1) : (r & 7) >> 1);        // nibble i of a word is column {0, 2, 4, 6, 1, 3, 5, 7}[i]
@@ -720,6 +722,10 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
           for (uint32_t h = 0; h < 2; h++) {
             const uint32_t g = (p.group_shift >= 0 ? (u1 + h) >> p.group_shift : (u1 + h) / (uint32_t)p.group32) - g0;
             u.s[h] = lds_u16s(scale0 + stage + g * (TS_BM * 2));
+            if (p.scale_perm & TS_SCALES_OTHER) {
+              if constexpr (BF) u.s[h] = __bfloat16_as_ushort(__float2bfloat16_rn(ts_h2f(u.s[h])));
+              else u.s[h] = __half_as_ushort(__float2half_rn(__uint_as_float(u.s[h] << 16)));
+            }
             u.z[h] = p.qzeros != nullptr ? (lds32(zero0 + stage + g * 64u) >> zero_shift) & 0xFu : 8u;
           }
           u.template half<0>(o);

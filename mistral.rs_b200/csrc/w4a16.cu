@@ -401,13 +401,13 @@ extern "C" int32_t mrs_dense_linear_pdl(const void *x, const void *w, void *y, i
 // permutation when group < K/8 (the reference passes in_dim / pack_factor as size_k), else the
 // 32-wide one; `workspace` (Marlin's lock array) is not needed.
 static int marlin_common(const void *inputs, const int32_t *weight, const void *scales, const void *zeros, void *out, int m,
-                         int k, int n, int groupsize, int dtype, int is_awq, int64_t stream) {
+                         int k, int n, int groupsize, int dtype, int is_awq, int64_t stream, int scales_other = 0) {
   cudaError_t status = cudaGetLastError();
   if (status != cudaSuccess) return (int)status;
   const int group = groupsize <= 0 ? k : groupsize;
   const int perm_kind = (groupsize > 0 && groupsize < k / 8) ? 1 : 2;
   const cudaError_t e = run_int4(inputs, weight, scales, is_awq ? (const int32_t *)zeros : nullptr, out, m, k, n, group,
-                               dtype, perm_kind, (cudaStream_t)stream);
+                               dtype, perm_kind | scales_other, (cudaStream_t)stream);
   return e == cudaSuccess ? (int)cudaGetLastError() : (int)e;
 }
 extern "C" int marlin_gptq_4bit_f16(const void *inputs, const int32_t *weight, const void *scales, const void *zeros,
@@ -429,6 +429,14 @@ extern "C" int marlin_awq_4bit_bf16(const void *inputs, const int32_t *weight, c
                                     const void *out, int m, int k, int n, const void *workspace, int groupsize, int64_t stream) {
   (void)workspace;
   return marlin_common(inputs, weight, scales, zeros, (void *)out, m, k, n, groupsize, MRS_BF16, 1, stream);
+}
+
+// The same with scales in their own 16-bit format (scale_dtype, 0 f16 / 1 bf16): a checkpoint's f16 scales under bf16 rows are rounded as the
+// kernel reads them, not by a pass of 3.7 us before each call.
+extern "C" int mrs_marlin_4bit(const void *inputs, const int32_t *weight, const void *scales, const void *zeros, void *out, int m, int k, int n,
+                               int groupsize, int dtype, int scale_dtype, int is_awq, int64_t stream) {
+  if (scale_dtype != MRS_F16 && scale_dtype != MRS_BF16) return (int)cudaErrorInvalidValue;
+  return marlin_common(inputs, weight, scales, zeros, out, m, k, n, groupsize, dtype, is_awq, stream, scale_dtype != dtype ? TS_SCALES_OTHER : 0);
 }
 
 // weight [k/8, n] i32, perm [k] i32 (argsort of g_idx; the reference always passes one), result: k*n/2 bytes

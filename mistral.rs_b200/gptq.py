@@ -16,6 +16,8 @@ import torch
 from . import lib
 from .quant import _I, _P, raw_stream, typed
 
+_CODE = {torch.float16: 0, torch.bfloat16: 1}
+
 
 class GptqLayer:
     def __init__(self, qweight, scales, qzeros=None, g_idx=None, bits=4, group_size=128, is_awq=False, bias=None,
@@ -123,13 +125,21 @@ class GptqMarlinLayer:
         if a.shape[-1] != self.k or a.dtype not in (torch.float16, torch.bfloat16):
             raise ValueError("GptqMarlinLayer: bad input shape/dtype")
         x = a.reshape(-1, self.k).contiguous()
-        scales = self.scales if self.scales.dtype == a.dtype else self.scales.to(a.dtype)
         out = x.new_empty((x.shape[0], self.n))
         name = f"marlin_{'awq' if self.is_awq else 'gptq'}_4bit_{'f16' if a.dtype == torch.float16 else 'bf16'}"
         fn = typed(name, _P, _P, _P, _P, _P, _I, _I, _I, _P, _I, ctypes.c_int64)
         groupsize = -1 if self.scales.shape[0] == 1 else self.k // self.scales.shape[0]
-        rc = fn(x.data_ptr(), self.q_weight.data_ptr(), scales.data_ptr(), self.qzeros.data_ptr() if self.qzeros is not None else 0, out.data_ptr(),
-                x.shape[0], self.k, self.n, self.workspace.data_ptr(), groupsize, raw_stream(a.device))
+        zeros, scales = self.qzeros.data_ptr() if self.qzeros is not None else 0, self.scales
+        if scales.dtype != a.dtype and scales.dtype in _CODE and scales.is_contiguous() and scales.data_ptr() % 16 == 0:
+            # the checkpoint's own 16-bit format, rounded inside the kernel
+            name = "mrs_marlin_4bit"
+            fn = typed(name, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, ctypes.c_int64)
+            rc = fn(x.data_ptr(), self.q_weight.data_ptr(), scales.data_ptr(), zeros, out.data_ptr(), x.shape[0], self.k, self.n, groupsize,
+                    _CODE[a.dtype], _CODE[scales.dtype], int(self.is_awq), raw_stream(a.device))
+        else:
+            scales = scales if scales.dtype == a.dtype else scales.to(a.dtype)
+            rc = fn(x.data_ptr(), self.q_weight.data_ptr(), scales.data_ptr(), zeros, out.data_ptr(), x.shape[0], self.k, self.n,
+                    self.workspace.data_ptr(), groupsize, raw_stream(a.device))
         if rc != 0:
             raise RuntimeError(f"{name} failed with status {rc}")
         out = out.reshape(*a.shape[:-1], self.n)

@@ -45,6 +45,7 @@ extern "C" {
     pub fn mrs_mmq_timeouts() -> i32;
     pub fn mrs_mmq_timeout_flag() -> *mut i32;
     pub fn mrs_gptq_gemm(x: *const c_void, qweight: *const i32, scales: *const c_void, qzeros: *const i32, g_idx: *const i32, y: *mut c_void, M: i32, K: i32, N: i32, group_size: i32, is_awq: i32, stream: *mut c_void) -> i32;
+    pub fn mrs_marlin_4bit(inputs: *const c_void, weight: *const i32, scales: *const c_void, zeros: *const c_void, out: *mut c_void, m: i32, k: i32, n: i32, groupsize: i32, dtype: i32, scale_dtype: i32, is_awq: i32, stream: i64) -> i32;
     pub fn mrs_w4a16_gemm(x: *const c_void, w_tiles: *const c_void, scales: *const c_void, qzeros: *const i32, y: *mut c_void, M: i32, K: i32, N: i32, group: i32, dtype: i32, scale_perm: i32, stream: *mut c_void) -> i32;
     pub fn mrs_dense_linear(x: *const c_void, w: *const c_void, y: *mut c_void, M: i32, K: i32, N: i32, dtype: i32, stream: *mut c_void) -> i32;
     pub fn mrs_gguf_affine_repack_f16(format: i32, source: *const c_void, payload: *mut c_void, scales: *mut c_void, offsets: *mut c_void, k: i32, n: i32, padded_n: i32, stream: usize) -> i32;

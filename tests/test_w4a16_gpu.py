@@ -105,3 +105,23 @@ def test_dense_linear(cuda, M, N, K):
     mag = x.double().abs() @ w.double().abs().t()
     tol = 2.0 ** -11 * ref.abs() * 1.01 + 2e-6 * mag + 1e-6
     assert bool(((y.double() - ref).abs() <= tol).all()), float(((y.double() - ref).abs() / tol).max())
+
+
+@pytest.mark.parametrize("K,N,group", [(64, 64, 32), (1024, 192, 128), (512, 128, 512), (4096, 1088, 64)])
+@pytest.mark.parametrize("awq", [False, True])
+def test_scales_in_the_other_format(cuda, awq, K, N, group):
+    """f16 scales under bf16 rows and bf16 scales under f16 rows: bit for bit what scales rounded before the call give."""
+    gen = torch.Generator(device=cuda).manual_seed(K + N)
+    ints = lambda *shape: torch.randint(-2 ** 31, 2 ** 31, shape, dtype=torch.int32, device=cuda, generator=gen)  # noqa: E731
+    qweight = ints(K, N // 8) if awq else ints(K // 8, N)
+    scales = torch.rand(K // group, N, device=cuda, generator=gen) * 0.02 + 1e-3
+    scales[0, :4] = torch.tensor([0.0, 6e-8, -3e-5, 1.5], device=cuda)
+    for rows, other in ((torch.bfloat16, torch.float16), (torch.float16, torch.bfloat16)):
+        layer = gptq.GptqMarlinLayer(qweight, scales.to(other), ints(K // group, N // 8) if awq else None, group_size=group, is_awq=awq)
+        for M in (1, 17, 130):
+            x = torch.randn(M, K, device=cuda, generator=gen).to(rows)
+            got, kept = layer.forward_raw(x), layer.scales
+            layer.scales = kept.to(rows)
+            want = layer.forward_raw(x)
+            layer.scales = kept
+            assert torch.equal(got.view(torch.int16), want.view(torch.int16))
