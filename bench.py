@@ -484,7 +484,7 @@ def bench_nisasun(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
             setattr(mod, name, g)
             return f
         names = ["embed_streams", "streams_read_norm", "streams_write", "glu_split", "gated_group_norm", "causal_conv", "ssm_steps",
-                 "linear_scan", "attention_prepare", "paged_attention", "fresh_prompt_attention", "scale_rows", "activate_cols", "moe_route", "moe_small", "moe_sort", "moe_gather", "moe_combine"]
+                 "linear_scan", "attention_prepare", "paged_attention", "fresh_prompt_attention", "scale_rows", "activate_cols", "moe_route", "moe_small", "moe_place", "moe_sort", "moe_gather", "moe_combine"]
         saved = {n: wrap(K, n) for n in names}
         saved_lin = wrap(mixers, "linear")
 
@@ -612,7 +612,7 @@ def bench_kilizen(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
     warmup, steps = max(3, warmup), max(1, steps)
     names = [n for n in ("embed_streams", "streams_read_norm", "streams_write", "glu_split", "gated_group_norm", "causal_conv", "ssm_steps", "linear_scan",
-                         "qk_norm_store", "window_attention", "fresh_prompt_attention", "scale_rows", "activate_cols", "moe_route", "moe_small", "moe_sort",
+                         "qk_norm_store", "window_attention", "fresh_prompt_attention", "scale_rows", "activate_cols", "moe_route", "moe_small", "moe_place", "moe_sort",
                          "moe_gather", "moe_combine", "tanh_norm_rows", "residual_tanh_norm", "rotation_table", "attention_prepare", "paged_attention",
                          "prompt_attention", "mlstm_gates", "append_ones", "mlstm_out_norm", "moe_route_top_softmax", "moe_small_ungated")]
 
@@ -795,7 +795,7 @@ def bench_fosulix(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
     names = ["embed_streams", "embed_scaled", "streams_read_norm", "rms_residual", "glu_split", "gated_group_norm", "causal_conv", "linear_scan",
              "activate_cols", "bounded_gate", "latent_prepare", "rotate_pairs", "latent_prompt_attention", "paged_attention", "prompt_attention",
              "fresh_prompt_attention", "attention_prepare", "rotation_table", "moe_route", "moe_route_scored", "moe_route_top_softmax", "moe_small",
-             "moe_small_ungated", "moe_sort", "moe_gather", "moe_combine", "tanh_norm_rows", "residual_tanh_norm", "mlstm_gates", "append_ones",
+             "moe_small_ungated", "moe_place", "moe_sort", "moe_gather", "moe_combine", "tanh_norm_rows", "residual_tanh_norm", "mlstm_gates", "append_ones",
              "mlstm_out_norm", "scale_rows"]
 
     def timed(fn, reps=steps):
@@ -1081,7 +1081,7 @@ def bench_kibotar(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
              "activate_cols", "bounded_gate", "power_gate", "latent_prepare", "rotate_pairs", "latent_prompt_attention", "paged_attention",
              "prompt_attention", "tc_attention", "attention_prepare", "rotation_table", "pool_blocks", "mix_heads", "gate_cols",
              "moe_route_scored", "moe_small",
-             "moe_sort", "moe_gather", "moe_combine", "scale_rows"]
+             "moe_place", "moe_sort", "moe_gather", "moe_combine", "scale_rows"]
     measure = engine_bench_tools(torch, dev, steps, warmup, prompt, decode_batches, names)
     out = {"metric": "kibotar_prefill_tok_s", "unit": "tok/s", "n_gpus": 1, "steps": steps, "warmup": warmup, "higher_is_better": True,
            "dtype": "bf16 (f32 residual, states, decays, norms, softmax and mixed weights)", "data": "synthetic", "sizes": []}
@@ -1363,7 +1363,7 @@ def bench_bafusun(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
     warmup, steps = max(3, warmup), max(1, steps)
     names = ["embed_scaled", "embed_streams", "rms_residual", "tanh_norm_rows", "residual_tanh_norm", "glu_split", "activate_cols", "gated_lookup", "rotation_table",
              "attention_prepare", "paged_attention", "prompt_attention", "tc_attention", "gather_rows", "router_logits", "moe_route_scored", "moe_route_top_softmax", "moe_small",
-             "moe_small_ungated", "moe_grouped", "moe_gemm", "moe_sort", "moe_gather", "moe_combine", "soft_cap"]
+             "moe_small_ungated", "moe_grouped", "moe_gemm", "moe_place", "moe_sort", "moe_gather", "moe_combine", "soft_cap"]
     measure = engine_bench_tools(torch, dev, steps, warmup, prompt, decode_batches, names)
     out = {"metric": "bafusun_prefill_tok_s", "unit": "tok/s", "n_gpus": 1, "steps": steps, "warmup": warmup, "higher_is_better": True,
            "dtype": "bf16 (f32 residual, norms, angles, softmax, router)", "data": "synthetic", "sizes": []}

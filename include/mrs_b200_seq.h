@@ -542,6 +542,13 @@ int mrs_seq_moe_combine(const void *sorted_y, int dtype, const int32_t *order, c
 int mrs_seq_moe_combine_some(const void *sorted_y, int dtype, const int32_t *order, const float *weights, const int32_t *experts,
                              const void *x, int n_ffn, int n_tok, int top, int width, int32_t *scratch_inverse, void *out,
                              int64_t stream);
+/* sort and gather in one launch where mrs_seq_moe_place_fits: rows of x sorted by expert, counts [n_experts], inverse [n_pairs] (the row of each
+ * pair), which mrs_seq_moe_combine_at takes (NULL there: the order of the pairs). */
+int mrs_seq_moe_place_fits(int n_pairs, int n_experts);
+int mrs_seq_moe_place(const int32_t *experts, int n_pairs, int n_experts, const void *x, int dtype, int top, int width, int32_t *counts,
+                      int32_t *inverse, void *sorted, int64_t stream);
+int mrs_seq_moe_combine_at(const void *sorted_y, int dtype, const int32_t *inverse, const float *weights, const int32_t *experts, const void *x,
+                           int n_ffn, int n_tok, int top, int width, void *out, int64_t stream);
 
 #ifdef __cplusplus
 }

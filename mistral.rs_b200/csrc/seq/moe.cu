@@ -86,7 +86,10 @@ __device__ __forceinline__ void route_token(const float *z, const mrs_seq_moe_ro
       if (gscore[e / per] != INFINITY) choice[e] = -INFINITY;
     __syncwarp();
   }
-  float wsum = 0.0f;
+  // (choice r waits in lane r: weights that went to memory and came back for the division made half of the kernel's time)
+  float wsum = 0.0f, my_w = 0.0f;
+  int my_e = 0;
+  const bool held = top <= 32;
   for (int r = 0; r < top; r++) {
     float bv = -INFINITY;
     int bi = 0x7fffffff;
@@ -101,13 +104,22 @@ __device__ __forceinline__ void route_token(const float *z, const mrs_seq_moe_ro
     }
     if (bi == 0x7fffffff) bi = 0;   // fewer eligible experts than `top`: weight 0
     const float wv = bv == -INFINITY ? 0.0f : score[bi];
+    if (lane == r) { my_e = bi; my_w = wv; }
     if (lane == 0) {
-      experts[r] = bi;
-      weights[r] = wv;
+      if (!held) { experts[r] = bi; weights[r] = wv; }
       if (bv != -INFINITY) choice[bi] = -INFINITY;
     }
     wsum += wv;
     __syncwarp();
+  }
+  if (held) {
+    if (lane < top) {
+      if (renorm && wsum + renorm_eps > 0.0f) my_w /= wsum + renorm_eps;
+      if (weight_scale != 1.0f) my_w *= weight_scale;
+      experts[lane] = my_e;
+      weights[lane] = my_w;
+    }
+    return;
   }
   if (renorm && lane == 0 && wsum + renorm_eps > 0.0f)
     for (int r = 0; r < top; r++) weights[r] /= wsum + renorm_eps;
@@ -409,6 +421,36 @@ __global__ void moe_inverse_kernel(const int32_t *__restrict__ order, int n_pair
   if (i < n_pairs) inverse[order[i]] = i;
 }
 
+// The three above for few pairs, in one launch: CTA i finds pair i's row (pairs of lower experts, and earlier ones of its own) by looking at
+// all pairs, copies its token there, and counts the pairs of expert i.  Bound by the launch: 128 pairs of 2048 columns took 6.5 us in three
+// launches (sort 1.9, gather 2.3, inverse 2.3) and as many calls from the host
+// (32 tokens to 4 of 16 experts, the whole layer: 107.3 us so, 100.5 now).  Each CTA reads all pairs: MOE_PLACE_PAIRS is the line.
+constexpr int MOE_PLACE_PAIRS = 2048;
+template <typename U>
+__global__ void __launch_bounds__(128) moe_place_kernel(const int32_t *__restrict__ experts, int n_pairs, int n_experts, const U *__restrict__ x, int top,
+                                                        int width, int32_t *__restrict__ counts, int32_t *__restrict__ inverse, U *__restrict__ sorted) {
+  __shared__ int32_t red[2][4];
+  const int i = blockIdx.x, own = i < n_pairs ? experts[i] : 0;
+  int before = 0, mine = 0;
+  for (int j = threadIdx.x; j < n_pairs; j += 128) {
+    const int e = experts[j];
+    before += e < own || (e == own && j < i);
+    mine += e == i;
+  }
+  before = __reduce_add_sync(0xffffffffu, before);
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = before; red[1][threadIdx.x >> 5] = mine; }
+  __syncthreads();
+  const int at = red[0][0] + red[0][1] + red[0][2] + red[0][3];
+  if (threadIdx.x == 0) {
+    if (i < n_experts) counts[i] = red[1][0] + red[1][1] + red[1][2] + red[1][3];
+    if (i < n_pairs) inverse[i] = at;
+  }
+  if (i >= n_pairs) return;
+  const U *from = x + (int64_t)(i / top) * width;
+  for (int c = threadIdx.x; c < width; c += 128) sorted[(int64_t)at * width + c] = from[c];
+}
+
 // inverse NULL: rows of sorted_y are in the order of the pairs.  experts NULL: every pair has a row in sorted_y; else pairs of experts from n_ffn on take their token's row of x
 template <typename T, int VEC>
 __global__ void moe_combine_kernel(const T *__restrict__ sorted_y, const int32_t *__restrict__ inverse, const float *__restrict__ weights,
@@ -584,6 +626,23 @@ extern "C" int mrs_seq_moe_sort(const int32_t *experts, int n_pairs, int n_exper
   return launch_status();
 }
 
+extern "C" int mrs_seq_moe_place_fits(int n_pairs, int n_experts) { return n_pairs > 0 && n_pairs <= MOE_PLACE_PAIRS && n_experts <= MOE_PLACE_PAIRS; }
+extern "C" int mrs_seq_moe_place(const int32_t *experts, int n_pairs, int n_experts, const void *x, int dtype, int top, int width, int32_t *counts,
+                                 int32_t *inverse, void *sorted, int64_t stream) {
+  if (!mrs_seq_moe_place_fits(n_pairs, n_experts)) return -2;
+  const int grid = n_pairs > n_experts ? n_pairs : n_experts;
+  const int64_t row_bytes = (int64_t)width * (dtype == MRS_SEQ_BF16 ? 2 : 4);
+  if (row_bytes % 16 == 0 && (((uintptr_t)x | (uintptr_t)sorted) & 15) == 0) {
+    moe_place_kernel<uint4><<<grid, 128, 0, (cudaStream_t)stream>>>(experts, n_pairs, n_experts, (const uint4 *)x, top, (int)(row_bytes / 16), counts,
+                                                                    inverse, (uint4 *)sorted);
+    return launch_status();
+  }
+  SEQ_DISPATCH_DTYPE(dtype, {
+    moe_place_kernel<T><<<grid, 128, 0, (cudaStream_t)stream>>>(experts, n_pairs, n_experts, (const T *)x, top, width, counts, inverse, (T *)sorted);
+  });
+  return launch_status();
+}
+
 extern "C" int mrs_seq_moe_gather(const void *x, int dtype, const int32_t *order, int n_pairs, int top, int width, void *sorted,
                                   int64_t stream) {
   if (n_pairs <= 0) return 0;
@@ -641,18 +700,15 @@ extern "C" int mrs_seq_moe_grouped(const mrs_seq_moe_grouped_args *args, int64_t
   return launch_status();
 }
 
-extern "C" int mrs_seq_moe_combine_some(const void *sorted_y, int dtype, const int32_t *order, const float *weights, const int32_t *experts,
-                                        const void *x, int n_ffn, int n_tok, int top, int width, int32_t *scratch_inverse, void *out,
-                                        int64_t stream) {
+// inverse: the row of each pair in sorted_y, or null: the order of the pairs
+extern "C" int mrs_seq_moe_combine_at(const void *sorted_y, int dtype, const int32_t *inverse, const float *weights, const int32_t *experts, const void *x,
+                                      int n_ffn, int n_tok, int top, int width, void *out, int64_t stream) {
   if (n_tok <= 0) return 0;
   if (experts && !x) return -2;
-  const int n_pairs = n_tok * top;
-  if (order) moe_inverse_kernel<<<(n_pairs + 255) / 256, 256, 0, (cudaStream_t)stream>>>(order, n_pairs, scratch_inverse);
-  else scratch_inverse = nullptr;
   const bool vec = width % 4 == 0 && (((uintptr_t)sorted_y | (uintptr_t)x | (uintptr_t)out) & 15) == 0;
   const int th = width >= 1024 ? 256 : 128;
 #define SEQ_COMBINE(V)                                                                                                            \
-  moe_combine_kernel<T, V><<<n_tok, th, 0, (cudaStream_t)stream>>>((const T *)sorted_y, scratch_inverse, weights, experts, (const T *)x, \
+  moe_combine_kernel<T, V><<<n_tok, th, 0, (cudaStream_t)stream>>>((const T *)sorted_y, inverse, weights, experts, (const T *)x,  \
                                                                    n_ffn, top, width, (T *)out)
   SEQ_DISPATCH_DTYPE(dtype, {
     if (vec) SEQ_COMBINE(4);
@@ -660,6 +716,15 @@ extern "C" int mrs_seq_moe_combine_some(const void *sorted_y, int dtype, const i
   });
 #undef SEQ_COMBINE
   return launch_status();
+}
+extern "C" int mrs_seq_moe_combine_some(const void *sorted_y, int dtype, const int32_t *order, const float *weights, const int32_t *experts,
+                                        const void *x, int n_ffn, int n_tok, int top, int width, int32_t *scratch_inverse, void *out,
+                                        int64_t stream) {
+  if (n_tok <= 0) return 0;
+  if (experts && !x) return -2;
+  const int n_pairs = n_tok * top;
+  if (order) moe_inverse_kernel<<<(n_pairs + 255) / 256, 256, 0, (cudaStream_t)stream>>>(order, n_pairs, scratch_inverse);
+  return mrs_seq_moe_combine_at(sorted_y, dtype, order ? scratch_inverse : nullptr, weights, experts, x, n_ffn, n_tok, top, width, out, stream);
 }
 
 extern "C" int mrs_seq_moe_combine(const void *sorted_y, int dtype, const int32_t *order, const float *weights, int n_tok, int top,

@@ -751,9 +751,14 @@ class RoutedExperts:
             small = K.moe_small if self.gated else K.moe_small_ungated
             out = small(h, self.w_gate_up, self.w_down, experts, weights, self.act)
         elif self.one_launch_products():
-            counts, order = K.moe_sort(experts, self.n_routes)
-            hid = K.moe_gemm(K.moe_gather(h, order, self.top), self.w_gate_up, counts, self.act, self.gated)
-            out = K.moe_combine(K.moe_gemm(hid, self.w_down, counts), order, weights, **self._identities(experts, h))
+            order = inverse = None
+            if K.moe_place_fits(experts.numel(), self.n_routes):
+                rows, counts, inverse = K.moe_place(h, experts, self.n_routes)
+            else:
+                counts, order = K.moe_sort(experts, self.n_routes)
+                rows = K.moe_gather(h, order, self.top)
+            hid = K.moe_gemm(rows, self.w_gate_up, counts, self.act, self.gated)
+            out = K.moe_combine(K.moe_gemm(hid, self.w_down, counts), order, weights, inverse=inverse, **self._identities(experts, h))
         else:
             counts, order = K.moe_sort(experts, self.n_routes)
             spans, at = [], 0

@@ -448,6 +448,22 @@ def moe_gather(x, order, top, n=None):
     return out
 
 
+def moe_place_fits(n_pairs, n_experts):
+    return bool(lib().mrs_seq_moe_place_fits(_i(n_pairs), _i(n_experts)))
+
+
+def moe_place(x, experts, n_experts):
+    """`moe_sort` and `moe_gather` in one launch for few pairs (`moe_place_fits`): -> (rows sorted by expert, in each by pair; counts [n_experts]; the
+    row of each pair, for `moe_combine`)."""
+    n, top, W = experts.numel(), experts.shape[1], x.shape[1]
+    ints = torch.empty(n_experts + n, dtype=torch.int32, device=x.device)
+    counts, inverse = ints[:n_experts], ints[n_experts:]
+    out = torch.empty(n, W, dtype=x.dtype, device=x.device)
+    _ok(lib().mrs_seq_moe_place(_p(experts), _i(n), _i(n_experts), _p(x), _i(DTYPE_CODE[x.dtype]), _i(top), _i(W), _p(counts), _p(inverse), _p(out),
+                                _st(x)), "moe_place")
+    return out, counts, inverse
+
+
 def moe_gemm_fits(dtype, width, ff, n_experts):
     """True when `moe_gemm` takes both products of experts of this size."""
     return dtype in DTYPE_CODE and all(lib().mrs_seq_moe_gemm_fits(_i(DTYPE_CODE[dtype]), _i(a), _i(b), _i(n_experts)) for a, b in ((ff, width), (width, ff)))
@@ -470,12 +486,17 @@ def moe_gemm_timeouts():
     return int(lib().mrs_seq_moe_gemm_timeouts())
 
 
-def moe_combine(sorted_y, order, weights, experts=None, x=None, n_ffn=0):
-    """order None: sorted_y is in pair order.  With experts and x: the pairs of experts from n_ffn on have no rows in sorted_y, they add their token's row of x."""
+def moe_combine(sorted_y, order, weights, experts=None, x=None, n_ffn=0, inverse=None):
+    """inverse: the row of each pair in sorted_y (`moe_place`); else order, the pair of each row (`moe_sort`); neither: sorted_y is in pair order.  With
+    experts and x: the pairs of experts from n_ffn on have no rows in sorted_y, they add their token's row of x."""
     T, top = weights.shape
     W = sorted_y.shape[1]
-    inverse = torch.empty(T * top, dtype=torch.int32, device=sorted_y.device) if order is not None else None
     out = torch.empty(T, W, dtype=sorted_y.dtype, device=sorted_y.device)
+    if inverse is not None:
+        _ok(lib().mrs_seq_moe_combine_at(_p(sorted_y), _i(DTYPE_CODE[sorted_y.dtype]), _p(inverse), _p(weights), _p(experts), _p(x), _i(n_ffn), _i(T),
+                                         _i(top), _i(W), _p(out), _st(sorted_y)), "moe_combine")
+        return out
+    inverse = torch.empty(T * top, dtype=torch.int32, device=sorted_y.device) if order is not None else None
     _ok(lib().mrs_seq_moe_combine_some(_p(sorted_y), _i(DTYPE_CODE[sorted_y.dtype]), _p(order), _p(weights), _p(experts), _p(x), _i(n_ffn), _i(T),
                                        _i(top), _i(W), _p(inverse), _p(out), _st(sorted_y)), "moe_combine")
     return out

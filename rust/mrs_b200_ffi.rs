@@ -116,4 +116,7 @@ extern "C" {
     pub fn mrs_seq_moe_gemm_timeouts() -> i32;
     pub fn mrs_seq_moe_combine(sorted_y: *const c_void, dtype: i32, order: *const i32, weights: *const f32, n_tok: i32, top: i32, width: i32, scratch_inverse: *mut i32, out: *mut c_void, stream: i64) -> i32;
     pub fn mrs_seq_moe_combine_some(sorted_y: *const c_void, dtype: i32, order: *const i32, weights: *const f32, experts: *const i32, x: *const c_void, n_ffn: i32, n_tok: i32, top: i32, width: i32, scratch_inverse: *mut i32, out: *mut c_void, stream: i64) -> i32;
+    pub fn mrs_seq_moe_place_fits(n_pairs: i32, n_experts: i32) -> i32;
+    pub fn mrs_seq_moe_place(experts: *const i32, n_pairs: i32, n_experts: i32, x: *const c_void, dtype: i32, top: i32, width: i32, counts: *mut i32, inverse: *mut i32, sorted: *mut c_void, stream: i64) -> i32;
+    pub fn mrs_seq_moe_combine_at(sorted_y: *const c_void, dtype: i32, inverse: *const i32, weights: *const f32, experts: *const i32, x: *const c_void, n_ffn: i32, n_tok: i32, top: i32, width: i32, out: *mut c_void, stream: i64) -> i32;
 }
