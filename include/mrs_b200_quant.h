@@ -64,7 +64,7 @@ int mrs_mmvq_fused(int ggml_type, int mode, int dt, const void *w0, const void *
 
 /* The same in two launches, for steps whose rows are many or long: the optional RMSNorm and the Q8_1 rows [b_size][K / 32] (36 bytes each, K %
  * 32 == 0, x and norm_w 16-byte aligned) by one, the GEMV over rows quantised so by the other.  The same bits as mrs_mmvq_fused; from three
- * rows over 8 MB of Q4_K, Q5_K, Q6_K or Q8_0 weights on, the same integer dots and scales, added up in f32 in another order.  Several GEMVs may
+ * rows (Q8_0: five) over 5 MB of Q4_K, Q5_K, Q6_K or Q8_0 weights on, the same integer dots and scales, added up in f32 in another order.  Several GEMVs may
  * read the rows of one quantisation. */
 int mrs_rms_quantize_q8_1(int dt, const void *x, const void *norm_w, float eps, int K, int b_size, void *q8, int pdl, void *stream);
 int mrs_mmvq_q8(int ggml_type, int mode, int dt, const void *w0, const void *w1, const void *w2, const void *q8, const void *residual,

@@ -648,9 +648,18 @@ static cudaError_t launch_one(MmvqParams p, cudaStream_t stream) {
 // Rows of Q8_1 activations from so many on, over at least so many bytes of weights: integer tensor-core products (mmvq_mma.cuh).  One B200, us
 // with the quantising launch, vector kernel / tensor cores: Q4_K 14336 x 4096 2 rows 15.3 / 16.8, 3 19.8 / 16.9, 4 20.2 / 17.1, 8 31.7 / 18.6;
 // 4096 x 14336 4 rows 22.2 / 18.6, 8 34.6 / 22.3; gate and up of 14336 x 4096 4 rows 32.8 / 25.3, 8 55.3 / 26.6; Q6_K 4096 x 14336 4 rows
-// 27.1 / 21.9, 8 38.4 / 28.3.  Below 8 MB launches and the fill of the rings are what is paid for.
-constexpr int MV_MIN_ROWS = 3;
-constexpr size_t MV_MIN_BYTES = 8u << 20;
+// 27.1 / 21.9, 8 38.4 / 28.3; Q5_K 14336 x 4096 4 rows 23.9 / 18.8, 8 42.0 / 20.7.  Q8_0, which the vector kernel need not unpack: 6144 x 4096 3 rows
+// 13.4 / 14.1, 4 13.4 / 14.2, 8 18.1 / 13.2, so from five rows on.  Small matrices: Q4_K 3072 x 3072 (5.3 MB) 3 rows 10.1 / 8.1, 8 14.8 / 9.1; Q6_K
+// 2560 x 2560 (5.4 MB) 11.2 / 9.0 and 15.1 / 9.9; smaller ones keep the vector kernel, and with it the bits of the fused launches.
+constexpr int MV_MIN_ROWS = 3, MV_MIN_ROWS_Q8_0 = 5;
+constexpr size_t MV_MIN_BYTES = 5u << 20;
+// whether rows that come quantised would go that way (up to alignment and room)
+bool mmvq_tensor_cores(int ggml_type, int rows, int K, int64_t nrows) {
+  const int bytes = ggml_type == MRS_Q4_K ? MvFmt<MRS_Q4_K>::BYTES : ggml_type == MRS_Q5_K ? MvFmt<MRS_Q5_K>::BYTES :
+                    ggml_type == MRS_Q6_K ? MvFmt<MRS_Q6_K>::BYTES : ggml_type == MRS_Q8_0 ? MvFmt<MRS_Q8_0>::BYTES : 0;
+  return rows >= (ggml_type == MRS_Q8_0 ? MV_MIN_ROWS_Q8_0 : MV_MIN_ROWS) && K % 256 == 0 && (size_t)(K / 256) * bytes * nrows >= MV_MIN_BYTES &&
+         !(g_flags & 16);
+}
 template <int T, int NC> static cudaError_t launch_mma(MmvqParams p, cudaStream_t stream) {
   constexpr size_t STAGE = 16 * (size_t)MvFmt<T>::PITCH;
   int32_t *const timeouts = mrs_mmq_timeout_flag();
@@ -756,7 +765,7 @@ static cudaError_t launch_type(MmvqParams p, cudaStream_t stream) {
     if (p.w[m] != nullptr) wbytes += (size_t)p.nrows[m] * row_bytes;
   const int b = p.ncols;
   if constexpr (MvFmt<T>::ok) {
-    if (b >= MV_MIN_ROWS && p.xkind == X_Q8_1 && p.K % 256 == 0 && fast && wbytes >= MV_MIN_BYTES && !(g_flags & 16)) {
+    if (p.xkind == X_Q8_1 && fast && mmvq_tensor_cores(T, b, p.K, (int64_t)p.nrows[0] + (p.w[1] ? p.nrows[1] : 0) + (p.w[2] ? p.nrows[2] : 0))) {
       const cudaError_t e = b <= 4 ? launch_mma<T, 4>(p, stream) : launch_mma<T, 8>(p, stream);
       if (e != cudaErrorNotSupported) return e;
     }

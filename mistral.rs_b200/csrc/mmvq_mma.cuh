@@ -1,4 +1,4 @@
-// mmvq_mma.cuh — streaming GEMV of mmvq.cu for three to eight rows of Q8_1 activations over large matrices: integer products on the tensor
+// mmvq_mma.cuh — streaming GEMV of mmvq.cu for three (Q8_0: five) to eight rows of Q8_1 activations over large matrices: integer products on the tensor
 // cores (mma.sync m16n8k32 / m16n8k16, s8).
 //
 // The vector kernel's dot products, and its reads of the activations from shared memory, grow with the rows: Q4_K 14336 x 4096 took 12 us for

@@ -252,11 +252,11 @@ def test_one_row_captured_and_not(cuda, K, N):
     assert all(torch.equal(a, b) for a, b in zip(got, want))
 
 
-@pytest.mark.parametrize("dtype,N,K", [("q4_k", 6501, 2304), ("q5_k", 5297, 2304), ("q6_k", 4450, 2304), ("q8_0", 8193, 1024), ("q4_k", 1100, 14336),
+@pytest.mark.parametrize("dtype,N,K", [("q4_k", 6501, 2304), ("q4_k", 4100, 2304), ("q5_k", 5297, 2304), ("q6_k", 4450, 2304), ("q8_0", 8193, 1024), ("q4_k", 1100, 14336),
                                        ("q6_k", 1000, 11008), ("q8_0", 34000, 256)])
 @pytest.mark.parametrize("rows", [3, 4, 5, 8])
 def test_large_matrices_on_tensor_cores(cuda, dtype, rows, N, K):
-    """Three to eight rows over at least 8 MB of weights: integer products on the tensor cores against the vector kernel in every mode.  Integer dots
+    """Three (Q8_0: five) to eight rows over at least 5 MB of weights: integer products on the tensor cores against the vector kernel in every mode.  Integer dots
     and their scales are exact in both; f32 sums of at most K / 16 terms in two orders, whose parts stay within 16 of the largest result, differ
     by less than K x 2^-24 of that."""
     import ctypes
@@ -274,7 +274,7 @@ def test_large_matrices_on_tensor_cores(cuda, dtype, rows, N, K):
     finally:
         lib().mrs_set_mmvq_flags(ctypes.c_int(0))
     (want, want16), (got, got16) = results
-    assert not all(torch.equal(a, b) for a, b in zip(got, want))        # two kernels
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) == (dtype == "q8_0" and rows < 5)        # two kernels
     top = [w.abs().max() for w in want]
     for a, b, s in zip(got, want, [*top[:4], 2 * top[1] * top[2]]):
         assert ((a - b).abs() <= K * 2.0 ** -24 * s).all()
