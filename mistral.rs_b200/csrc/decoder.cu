@@ -53,6 +53,7 @@ extern "C" int32_t flashinfer_decode(void *q, void *key_cache, void *value_cache
                                      cudaStream_t stream);
 
 namespace mrs {
+bool mmvq_tensor_cores(int ggml_type, int rows, int K, int64_t nrows);      // mmvq.cu
 
 __global__ void embedding_gather_kernel(int type, const uint8_t *__restrict__ table, int cols, int per,
                                         const int32_t *__restrict__ ids, void *__restrict__ out, int act_dtype) {
@@ -395,16 +396,23 @@ extern "C" int32_t mrs_llama_decode_step(const mrs_llama_step *s, void *stream) 
   // without it: four layers 4096 wide (K = 4096 and 14336), Q4_K_M, 2 sequences 358 (down projection alone) / 376, all products 402;
   // 3 sequences 484 (down alone) / 529, all 491; 4: 507 / 573; 8: 751 / 1028.  Six layers 2048 wide (K = 2048 and 5632): 2 sequences 298
   // (down alone) / 288; 3: 375 (down alone) / 384, all 416; 4: 408 (down alone) / 417, all 433; 5: 543 / 610; 8: 587 / 716.  (A single row
-  // stays fused, however long: behind the GEMV before it the launch is not free.)  The rows go to a buffer of their own: nothing else of the
+  // stays fused, however long: behind the GEMV before it the launch is not free.)  Three and four rows also where the product then runs on the
+  // tensor cores: the four layers take 465 us for 3 sequences (496 with the down projection alone apart), 457 for 4 (537); 491 for 5 and 495
+  // for 8, which were 715 and 757 on the vector kernels; six layers 2048 wide 393 for 3 (395), 407 for 4 (421), 473 for 5 (560), 487 for 8 (598).  The rows go to a buffer of their own: nothing else of the
   // step is overwritten, the last step's logits among them.
   const bool extended = s->extension == MRS_LLAMA_STEP_Q8 && ((uintptr_t)s->q8 & 3) == 0;
   void *const q8 = extended ? s->q8 : nullptr;
   const int64_t q8_bytes = q8 != nullptr ? s->q8_bytes : 0;
+  bool held = false;                       // q8 has the rows of the last product that was not told that they are there
   auto gemv = [&](const mrs_qweight &w0, int mode, const void *w1, const void *w2, const void *x, const void *norm_w, const void *residual, void *d0,
                   void *d1, void *d2, int K, int n0, int n1, int n2, bool quantised) -> int {
-    if (!((B >= 5 || (B >= 2 && (int64_t)B * K >= 16384)) && K % 32 == 0 && (int64_t)B * (K / 32) * 36 <= q8_bytes))
+    const int64_t rows = (int64_t)n0 + n1 + n2;
+    if (!((B >= 5 || (B >= 2 && (int64_t)B * K >= 16384) || mmvq_tensor_cores(w0.ggml_type, B, K, rows)) && K % 32 == 0 && (int64_t)B * (K / 32) * 36 <= q8_bytes)) {
+      if (!quantised) held = false;
       return mrs_mmvq_fused(w0.ggml_type, mode, dt, w0.data, w1, w2, x, norm_w, s->rms_eps, residual, d0, d1, d2, K, n0, n1, n2, B, 0, pdl, stream);
-    if (!quantised) MRS_TRY(mrs_rms_quantize_q8_1(dt, x, norm_w, s->rms_eps, K, B, q8, pdl, stream));
+    }
+    if (!quantised || !held) MRS_TRY(mrs_rms_quantize_q8_1(dt, x, norm_w, s->rms_eps, K, B, q8, pdl, stream));
+    held = true;
     return mrs_mmvq_q8(w0.ggml_type, mode, dt, w0.data, w1, w2, q8, residual, d0, d1, d2, K, n0, n1, n2, B, 0, pdl, stream);
   };
   MRS_TRY(mrs_embedding_gather(s->tok_embd.ggml_type, s->tok_embd.data, H, s->token_ids, B, s->x, dt, stream));
