@@ -92,17 +92,11 @@ constexpr int TS_I4_CHUNK = TS_BM * 32, TS_I4_SCALES = 4 * TS_I4_CHUNK, TS_I4_ZE
 template <int TYPE, bool ALIGNED> struct TsStage { static constexpr int BYTES = TS_BM * TsPitch<TYPE, ALIGNED>::value; };
 template <> struct TsStage<TS_INT4, true> { static constexpr int BYTES = TS_I4_STAGE; };
 
-// By the whole warp.  False when the phase did not complete within the limit: the caller then ends its part of the CTA.  The loop is one piece
-// with uniform branches: a vote over the lanes' answers in each round cost 2 to 5 % of a launch (14336 x 4096 of Q4_K, 24 tokens 18.1 us, 17.5
-// so), a loop that each lane leaves by itself more, and the issuer and the producers pass several waits in a span.
+// By the whole warp.  False when the phase did not complete within the limit: the caller then ends its part of the CTA.  (The issuer and the producers
+// pass several waits in a span: 2 to 5 % of a launch lies between this loop, vote inside, and one that leaves PTX to vote in each round: Q5_K 4096 x
+// 4096, 200 tokens in a graph 17.7 us and 18.2, int4 14336 x 4096, 32 tokens 15.7 and 16.1.)
 __device__ __forceinline__ bool ts_wait(uint64_t *bar, uint32_t parity, int *timeouts) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, %3;\n\t"
-      "WAIT_%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra.uni DONE_%=;\n\t"
-      "sub.u32 n, n, 1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra.uni WAIT_%=;\n\tDONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done) : "r"(smem_u32(bar)), "r"(parity), "n"(TS_WAIT_LIMIT) : "memory");
-  if (done) return true;
+  if (mbar_wait_warp(bar, parity, TS_WAIT_LIMIT)) return true;
   *(volatile int *)timeouts = 1;
   return false;
 }

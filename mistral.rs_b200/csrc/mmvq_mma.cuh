@@ -47,13 +47,7 @@ __device__ __forceinline__ float4 mv_ldsf4(uint32_t a) {
 // By the whole warp, with a limit.  A wait that runs out is reported, and the warp goes through its part without waiting again.
 constexpr uint32_t MV_WAIT_LIMIT = 1u << 22;
 __device__ __forceinline__ void mv_wait(uint64_t *bar, uint32_t parity, bool &dead, int *timeouts) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, %3;\n\t"
-      "WAIT_%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra.uni DONE_%=;\n\t"
-      "sub.u32 n, n, 1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra.uni WAIT_%=;\n\tDONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done) : "r"(smem_u32(bar)), "r"(parity), "r"(dead ? 1u : MV_WAIT_LIMIT) : "memory");
-  if (!done) {
+  if (!mbar_wait_warp(bar, parity, dead ? 1u : MV_WAIT_LIMIT)) {
     dead = true;
     *(volatile int *)timeouts = 1;
   }

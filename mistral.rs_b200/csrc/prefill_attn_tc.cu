@@ -100,17 +100,10 @@ __device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t *r) {
       : "memory");
 }
 
-// By the whole warp.  False when the phase did not complete within the limit: the caller then ends its part of the CTA.  (The loop in one
-// piece, with uniform branches: a vote over the lanes' answers cost 150 clocks on a barrier that had completed, and a tile passes six waits in
-// turn: 2900 tokens, 32 heads on 8, 81 us so, 75 as it is.)
+// By the whole warp.  False when the phase did not complete within the limit: the caller then ends its part of the CTA.  (A tile passes six waits in
+// turn; a loop that left PTX to vote in each round took 81 us for 2900 tokens, 32 heads on 8, this one 75.)
 __device__ __forceinline__ bool ft_wait(uint64_t *bar, uint32_t parity, int *timeouts) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, %3;\n\t"
-      "WAIT_%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra.uni DONE_%=;\n\t"
-      "sub.u32 n, n, 1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra.uni WAIT_%=;\n\tDONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done) : "r"(smem_u32(bar)), "r"(parity), "n"(FT_WAIT_LIMIT) : "memory");
-  if (done) return true;
+  if (mbar_wait_warp(bar, parity, FT_WAIT_LIMIT)) return true;
   *(volatile int *)timeouts = 1;
   return false;
 }
