@@ -230,6 +230,8 @@ __global__ void __launch_bounds__(9 * 32, 2) mmvq_mma_kernel(const MmvqParams p)
         }
       }
       for (int s = 0; s < nseg; s++) {
+        // (stages come free once the consumers have their activations: a limit does not count the grids before this one)
+        if (p.pdl && n == nst) pdl_wait();
         mv_wait(&empty[stage], phase ^ 1, dead, p.timeouts);
         if (dead) break;
         n++;
