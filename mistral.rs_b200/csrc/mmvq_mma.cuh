@@ -250,8 +250,8 @@ __global__ void __launch_bounds__(9 * 32, 2) mmvq_mma_kernel(const MmvqParams p)
         if (++stage == nst) { stage = 0; phase ^= 1; }
       }
     }
-    if (dead)                                // copies in flight land before the CTA may end (the consumers have waited for them otherwise)
-      for (int i = max(0, n - nst); i < n; i++) { bool gone = false; mv_wait(&full[i % nst], (i / nst) & 1, gone, p.timeouts); }
+    // copies in flight land before the CTA may end: the consumers have not waited for them where one of their waits ran out
+    for (int i = max(0, n - nst); i < n; i++) { bool gone = false; mv_wait(&full[i % nst], (i / nst) & 1, gone, p.timeouts); }
     return;
   }
 
