@@ -303,7 +303,8 @@ __global__ void __launch_bounds__(9 * 32, 2) mmvq_mma_kernel(const MmvqParams p)
                           xl + 256u * (uint32_t)k, dl + (uint32_t)(k * 8 * NC * 8), NC * 8u, t, acc);
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[stage]);
+      // (a warp whose wait ran out gives no stage back: its copies may be on their way still, and the producer's own wait ends that part)
+      if (lane == 0 && !dead) mbar_arrive(&empty[stage]);
       if (++stage == nst) { stage = 0; phase ^= 1; }
     }
     // partial tiles [warp][row][8 columns]
