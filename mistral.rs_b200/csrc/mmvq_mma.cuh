@@ -44,7 +44,7 @@ __device__ __forceinline__ float4 mv_ldsf4(uint32_t a) {
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
   return v;
 }
-// By the whole warp, with a limit.  A wait that runs out is reported, and the warp goes through its part without waiting again.
+// By the whole warp, with a limit.  A wait that runs out is reported, and the warp goes through its part without waiting again (and without a result).
 constexpr uint32_t MV_WAIT_LIMIT = 1u << 22;
 __device__ __forceinline__ void mv_wait(uint64_t *bar, uint32_t parity, bool &dead, int *timeouts) {
   if (!mbar_wait_warp(bar, parity, dead ? 1u : MV_WAIT_LIMIT)) {
@@ -307,7 +307,8 @@ __global__ void __launch_bounds__(9 * 32, 2) mmvq_mma_kernel(const MmvqParams p)
       if (lane == 0 && !dead) mbar_arrive(&empty[stage]);
       if (++stage == nst) { stage = 0; phase ^= 1; }
     }
-    // partial tiles [warp][row][8 columns]
+    // partial tiles [warp][row][8 columns]; NaN where a wait ran out, and so in every sum that lacks the tile
+    if (dead) acc[0] = acc[1] = acc[2] = acc[3] = __int_as_float(0x7fffffff);
     float *mine = red + (size_t)(buf * NCW + warp) * 128;
     *(float2 *)(mine + g * 8 + 2 * t) = make_float2(acc[0], acc[1]);
     *(float2 *)(mine + (g + 8) * 8 + 2 * t) = make_float2(acc[2], acc[3]);
