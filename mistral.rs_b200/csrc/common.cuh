@@ -133,8 +133,8 @@ __device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity) {
       ".reg .pred P1;\n\t"
       "WAIT_LOOP:\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 P1, [%0], %1;\n\t"
-      "@P1 bra.uni WAIT_DONE;\n\t"
-      "bra.uni WAIT_LOOP;\n\t"
+      "@P1 bra WAIT_DONE;\n\t"
+      "bra WAIT_LOOP;\n\t"
       "WAIT_DONE:\n\t"
       "}" ::"r"(smem_u32(bar)),
       "r"(parity)

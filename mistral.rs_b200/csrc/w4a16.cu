@@ -59,7 +59,7 @@ __device__ __forceinline__ void mbar_wait_cluster(uint64_t *bar, uint32_t parity
   asm volatile(
       "{\n\t.reg .pred P1;\n\tWAITC_LOOP:\n\t"
       "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P1, [%0], %1;\n\t"
-      "@P1 bra.uni WAITC_DONE;\n\tbra.uni WAITC_LOOP;\n\tWAITC_DONE:\n\t}" ::"r"(smem_u32(bar)),
+      "@P1 bra WAITC_DONE;\n\tbra WAITC_LOOP;\n\tWAITC_DONE:\n\t}" ::"r"(smem_u32(bar)),
       "r"(parity)
       : "memory");
 }
