@@ -93,9 +93,11 @@ void mrs_mmq_set_weight_format(int32_t fmt);
  * tensor memory; every type, w and x on 16-byte boundaries) and csrc/mmq_tc.cu (forced weight formats, and what the first refuses).
  * path 0: automatic (default); 1: mmq_tc.cu only.  mrs_mmq_gguf_ts is the first kernel's own entry point: it returns
  * cudaErrorNotSupported (801) when the launch does not fit it.
- * Waits inside that kernel, which the int4 linears below run on as well, have a limit.  A launch in which one runs out leaves its output
- * incomplete and sets a word in host memory: from then on calls on that device return cudaErrorLaunchTimeout (702).  mrs_mmq_timeouts
- * waits for the device and returns the word, mrs_mmq_timeout_flag returns its address (for graphs, whose replays pass no entry point). */
+ * Waits inside that kernel, which the int4 linears below run on as well, have a limit, and so have those of the tensor-core GEMV (three to eight
+ * rows, above) and of prompt attention.  A launch in which one runs out leaves its output incomplete and sets a word in host memory: from then on
+ * calls on that device that would run on one of the three return cudaErrorLaunchTimeout (702; launch_mmvq_gguf_*, which return nothing, print it and
+ * leave the result as it is).  mrs_mmq_timeouts waits for the device and returns the word, mrs_mmq_timeout_flag returns its address (for graphs,
+ * whose replays pass no entry point). */
 void mrs_mmq_set_path(int32_t path);
 int32_t mrs_mmq_gguf_ts(int32_t ggml_type, const void *w, const void *x, void *y, int32_t M, int32_t N, int32_t K,
                         int32_t dtype, void *stream);

@@ -663,7 +663,7 @@ bool mmvq_tensor_cores(int ggml_type, int rows, int K, int64_t nrows) {
 template <int T, int NC> static cudaError_t launch_mma(MmvqParams p, cudaStream_t stream) {
   constexpr size_t STAGE = 16 * (size_t)MvFmt<T>::PITCH;
   int32_t *const timeouts = mrs_mmq_timeout_flag();
-  if (timeouts == nullptr || *(volatile const int32_t *)timeouts != 0) return cudaErrorNotSupported;
+  if (timeouts == nullptr) return cudaErrorNotSupported;
   const DevInfo &d = query_device();
   const size_t fixed = 256 + (size_t)NC * (p.K + 32) + (size_t)p.K / 32 * NC * 8 + 2 * 8 * 128 * 4;
   int per_sm = 2, nst = 0;
@@ -671,6 +671,7 @@ template <int T, int NC> static cudaError_t launch_mma(MmvqParams p, cudaStream_
   if (fixed + 2 * STAGE > budget) { per_sm = 1; budget = (size_t)d.max_smem - 1024; }
   while (nst < MAX_STAGES && fixed + (nst + 1) * STAGE <= budget) nst++;
   if (nst < 2) return cudaErrorNotSupported;
+  if (*(volatile const int32_t *)timeouts != 0) return cudaErrorLaunchTimeout;      // (as the dequantising GEMM and prompt attention do)
   p.nstages = nst;
   p.timeouts = timeouts;
   const int P = p.mode == MODE_GLU ? 8 : 16, passes = (p.vrows + P - 1) / P, most = per_sm * d.num_sms;

@@ -34,15 +34,16 @@ def forward(w, xs: torch.Tensor) -> torch.Tensor:
 
 
 def check_timeouts(device):
-    """Raises when a wait inside the dequantising GEMM (ggml and int4 linears) ever ran out on `device`: results since then are incomplete.
-    Reads a word in host memory, so call it once the work in question is done.  Calls refuse to launch by themselves from then on; replays of a
+    """Raises when a wait inside a kernel that shares this word ever ran out on `device`: the dequantising GEMM (ggml and int4 linears), the tensor-core
+    GEMV (three to eight rows over large matrices) and prompt attention.  Results since then are incomplete.  Reads a word in host memory, so call
+    it once the work in question is done.  Calls that would run on one of these kernels are refused by themselves from then on; replays of a
     graph pass no entry point and need this."""
     with torch.cuda.device(device):
         fn = lib().mrs_mmq_timeout_flag
         fn.restype = ctypes.POINTER(ctypes.c_int32)
         flag = fn()
     if flag and flag[0]:
-        raise RuntimeError("a wait inside the dequantising GEMM ran out: the results of this device are incomplete")
+        raise RuntimeError("a wait inside a linear or prompt attention ran out: the results of this device are incomplete")
 
 
 def set_path(path: str):

@@ -281,3 +281,35 @@ def test_large_matrices_on_tensor_cores(cuda, dtype, rows, N, K):
     for a, b in zip(got16, want16):           # the same rounding but where a sum lies at its edge
         assert ((a - b).abs() <= 2.0 ** -6 * b.abs().max()).all() and (a != b).float().mean() < 2e-2
     assert lib().mrs_mmq_timeouts() == 0
+
+
+def test_tensor_core_calls_are_refused_once_a_wait_has_run_out(cuda):
+    """The word that a kernel sets when a wait runs out, set here by the host: three to eight rows over 5 MB of weights and prompt attention, whose
+    kernels set it too, refuse as the dequantising GEMM does; what runs on kernels without it (a row, small matrices, softcap) goes on."""
+    import ctypes
+    from mistralrs_b200 import lib, mmq, paged_attn
+    weight = lambda n, k: quant.QTensor(to_dev(make_weight("q4_k", n, k, 1).reshape(-1), cuda), "q4_k", (n, k))
+    large, small = weight(4608, 2304), weight(64, 256)
+    gen = torch.Generator(device=cuda).manual_seed(1)
+    x, y = torch.randn(4, 2304, device=cuda, generator=gen), torch.randn(4, 256, device=cuda, generator=gen)
+    q = {d: torch.randn(70, 2, d, device=cuda, generator=gen).to(torch.float16) for d in (64, 128)}
+    refused = [lambda: quant.plain(large, x), lambda: quant.fused_glu(large, large, x, quant.GluActivationType.Silu),
+               lambda: quant.fused_qkv(large, large, large, x)[0], lambda: paged_attn.prefill_attention(q[64], q[64], q[64], 0.125),
+               lambda: paged_attn.prefill_attention(q[128], q[128], q[128], 0.1, window_left=20)]
+    go_on = [lambda: quant.plain(large, x[:2]), lambda: quant.plain(small, y), lambda: paged_attn.prefill_attention(q[64], q[64], q[64], 0.125, softcap=20.0)]
+    want = [[call() for call in calls] for calls in (refused, go_on)]
+    assert lib().mrs_mmq_timeouts() == 0
+    fn = lib().mrs_mmq_timeout_flag
+    fn.restype = ctypes.POINTER(ctypes.c_int32)
+    flag = fn()
+    try:
+        flag[0] = 1
+        for call in refused:
+            with pytest.raises(RuntimeError, match="702"):
+                call()
+        assert all(torch.equal(call(), w) for call, w in zip(go_on, want[1]))
+        with pytest.raises(RuntimeError, match="ran out"):
+            mmq.check_timeouts(cuda)
+    finally:
+        flag[0] = 0
+    assert all(torch.equal(call(), w) for call, w in zip(refused, want[0]))
