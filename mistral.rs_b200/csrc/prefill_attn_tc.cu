@@ -134,11 +134,12 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   const int q0 = qt * FT_BM;
   const int q_hi = min(len, q0 + FT_BM) - 1;
   const int kv_end = p.causal ? (q_hi + 1) : len;
-  const int t0 = WINDOW ? max(0, q0 - p.window_left) / FT_BN : 0;      // first KV tile
-  const int nt = (kv_end + FT_BN - 1) / FT_BN - t0;
-  // Past its end a sequence's last tile holds the next one's rows: masked scores in S, but a value times a probability of zero, which is not
-  // zero where that value is no finite number.  The producer clears them.
-  const bool ragged = p.cu_seqlens != nullptr && (t0 + nt) * FT_BN > len;
+  // Tiles start at the first key that a row of the tile may see, wherever that lies (a tile's row needs no alignment): nothing before it is read.
+  const int first = WINDOW ? max(0, q0 - p.window_left) : 0;
+  const int nt = (kv_end - first + FT_BN - 1) / FT_BN;
+  // Past the last key that a row may see the last tile holds later tokens' rows or the next sequence's: masked scores in S, but a value times a
+  // probability of zero, which is not zero where that value is no finite number.  The producer clears them.
+  const bool ragged = (WINDOW || p.cu_seqlens != nullptr) && first + nt * FT_BN > kv_end;
 
   // The producer initialises the barriers and goes on to its first loads; the CTA barrier, which it does not wait for, orders that before the
   // others' first wait.
@@ -168,7 +169,7 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     int nk = 0, nv = 0;
     load(q_s, &tmap_q, h * D, seq0 + q0, q_full);
     for (int j = 0; j < nt; j++) {
-      const int ph = j & 1, row = seq0 + (t0 + j) * FT_BN;
+      const int ph = j & 1, row = seq0 + first + j * FT_BN;
       ok = ft_wait(k_empty, ph ^ 1, late);
       if (!ok) break;
       load(k_s, &tmap_k, kvh * D, row, k_full);
@@ -183,7 +184,7 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     if (nk > 0) ft_wait(k_full, (nk - 1) & 1, late);
     if (nv > 0) ft_wait(v_full, (nv - 1) & 1, late);
     if (ok && ragged) {
-      const int r0 = len - (t0 + nt - 1) * FT_BN;                            // rows r0 .. 127 of the last tile
+      const int r0 = kv_end - first - (nt - 1) * FT_BN;                            // rows r0 .. 127 of the last tile
       for (int i = lane; i < (FT_BN - r0) * 8 * BOXES; i += 32) {            // (a row of a box is 128 bytes wherever the swizzle puts its parts)
         const int x = i / ((FT_BN - r0) * 8), y = i - x * (FT_BN - r0) * 8;
         sts128(smem_u32(v_s) + (uint32_t)(x * BOX + r0 * 128 + y * 16), make_uint4(0u, 0u, 0u, 0u));
@@ -242,7 +243,7 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     for (int j = 0; j < nt; j++) {
       const int ph = j & 1;
       const uint32_t ts = t_s + lane_off;
-      const int kv0 = (t0 + j) * FT_BN;
+      const int kv0 = first + j * FT_BN;
       const int lim = min(p.causal ? qg : len - 1, len - 1) - kv0;                 // columns > lim are masked,
       const int low = WINDOW ? qg - p.window_left - kv0 : 0;                       // and those below low
       ok = ft_wait(s_full, ph, late);

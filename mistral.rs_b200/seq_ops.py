@@ -343,8 +343,8 @@ def scale_rows(x, row0, rows, col0, cols, scale):
 
 def fresh_prompt_attention(y, row0, rows, q_col, k_col, v_col, heads, kv_heads, d, scale, window, out, out_col):
     """Causal (windowed) attention of one sequence's first `rows` tokens over its own fresh q / k / v, through the
-    package's prompt-attention kernels (tcgen05 for head size 128 without a window, mma.sync otherwise; libmrs_b200.so,
-    built on first use).  q / k / v are column ranges of `y`; writes heads * d columns of `out` from out_col."""
+    package's prompt-attention kernels (tcgen05 for head sizes 64 and 128, windows too; mma.sync for strides that it declines;
+    libmrs_b200.so, built on first use).  q / k / v are column ranges of `y`; writes heads * d columns of `out` from out_col."""
     from . import LIB_PATH, lib as main_lib
     make_target(os.path.join(_HERE, "csrc"), LIB_PATH)
     ld, at = y.stride(0), row0 * y.stride(0)

@@ -1,4 +1,4 @@
-"""Prompt attention kernel (csrc/prefill_attn.cu) vs a plain fp64 torch reference of the same op:
+"""Prompt attention kernels (csrc/prefill_attn_tc.cu, csrc/prefill_attn.cu) vs a plain fp64 torch reference of the same op:
 causal, GQA, ragged lengths, var-len batches, sliding window, soft-cap, both dtypes and head sizes."""
 import numpy as np
 import pytest
@@ -71,7 +71,7 @@ def test_varlen_batch(cuda):
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
 def test_both_kernels_head_128(cuda, dt):
-    """Head size 128 without window / softcap runs on csrc/prefill_attn_tc.cu (tcgen05, S and P in tensor memory);
+    """Head sizes 64 and 128 without softcap run on csrc/prefill_attn_tc.cu (tcgen05, S and P in tensor memory);
     mrs_prefill_attn_tc_debug(0, ...) keeps the call on csrc/prefill_attn.cu (mma.sync).  Both against the fp64
     reference, on a ragged multi-tile prompt, causal and not."""
     import ctypes
@@ -125,3 +125,20 @@ def test_sequences_do_not_see_their_neighbours(cuda, D, window):
         kk, vv = torch.full_like(k, float("nan")), torch.full_like(v, float("inf"))
         kk[at], vv[at] = k[at], v[at]
         assert torch.equal(run(kk, vv)[at], clean[at])
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("varlen", [False, True])
+def test_values_outside_the_window_of_a_tile_leave_no_trace(cuda, D, varlen):
+    """Keys that no row of a tile of 128 queries may see, before its windows or behind its last row, are not multiplied: infinite values there change
+    no bit, wherever the windows start."""
+    T, H, KVH = 300, 4, 2
+    gen = torch.Generator(device=cuda).manual_seed(D)
+    q, k, v = (torch.randn(T, h, D, device=cuda, generator=gen).to(torch.bfloat16) for h in (H, KVH, KVH))
+    kw = dict(cu_seqlens=torch.tensor([0, T], dtype=torch.int32, device=cuda), max_seqlen=T) if varlen else {}
+    for window in (0, 1, 40, 64, 100, 127):
+        run = lambda vv: paged_attn.prefill_attention(q, k, vv, D ** -0.5, window_left=window, **kw)  # noqa: E731
+        clean, vv = run(v), v.clone()
+        vv[:128 - window] = float("inf")      # (of the second tile's rows, 128 .. 255)
+        vv[256:] = float("nan")
+        assert torch.equal(run(vv)[128:256], clean[128:256]), window
