@@ -12,8 +12,11 @@ import ctypes
 import torch
 
 from . import lib
+from .quant import _F, _I, _P, raw_stream, typed
 
+_L = ctypes.c_int64
 _DT_CODE = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}
+_PROMPT_CODE = {torch.float16: 0, torch.bfloat16: 1}
 _TAG = {torch.float16: "f16", torch.bfloat16: "bf16", torch.float32: "f32"}
 _SUPPORTED_HEAD_SIZES = (64, 80, 96, 112, 128, 192, 256)      # backend/paged_attention.rs:251-261
 PARTITION_SIZE = 512  # backend/paged_attention.rs:302
@@ -296,15 +299,14 @@ def prefill_attention(q, k, v, softmax_scale, causal=True, cu_seqlens=None, max_
     for t, name in ((q, "q"), (k, "k"), (v, "v")):
         if t.stride(2) != 1 or t.stride(1) != D:
             raise ValueError(f"prefill_attention: {name} must have dense heads")
+    if not q.is_cuda:
+        raise ValueError(f"prefill_attention: expected a cuda device, but got: {q.device}")
     out = torch.empty(T, H, D, dtype=q.dtype, device=q.device)
     batch = 0 if cu_seqlens is None else cu_seqlens.numel() - 1
-    rc = lib().mrs_prefill_attention(_p(q), _p(k), _p(v), _p(out), _p(cu_seqlens), ctypes.c_int(batch), ctypes.c_int(T),
-                                     ctypes.c_int(max_seqlen or T), ctypes.c_int(H), ctypes.c_int(KVH), ctypes.c_int(D),
-                                     ctypes.c_int64(q.stride(0)), ctypes.c_int64(k.stride(0)), ctypes.c_int64(out.stride(0)),
-                                     ctypes.c_float(softmax_scale), ctypes.c_int(int(causal)),
-                                     ctypes.c_int(-1 if window_left is None else window_left),
-                                     ctypes.c_float(0.0 if softcap is None else softcap),
-                                     ctypes.c_uint32({torch.float16: 0, torch.bfloat16: 1}[q.dtype]), _stream(q.device))
+    entry = typed("mrs_prefill_attention", _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _L, _L, _L, _F, _I, _I, _F, ctypes.c_uint32, _P)
+    rc = entry(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), None if cu_seqlens is None else cu_seqlens.data_ptr(), batch, T,
+               max_seqlen or T, H, KVH, D, q.stride(0), k.stride(0), out.stride(0), softmax_scale, int(causal), -1 if window_left is None else window_left,
+               0.0 if softcap is None else softcap, _PROMPT_CODE[q.dtype], raw_stream(q.device))
     if rc != 0:
         raise RuntimeError(f"mrs_prefill_attention failed with cudaError {rc}")
     return out

@@ -1,4 +1,6 @@
 """Decode-backend selection (host logic): REF mistralrs-core/src/flashinfer/mod.rs:257-273, perf_flags.rs:9-29."""
+import pytest
+
 from mistralrs_b200 import paged_attn as pa
 
 
@@ -23,3 +25,14 @@ def test_env_flag(monkeypatch):
         assert pa.flashinfer_decode_enabled() is want, v
     monkeypatch.setenv(pa.FLASHINFER_DECODE_ENV, "0")
     assert not pa.flashinfer_supports_layer(32, 8, 128, 128)
+
+
+def test_prompt_attention_refuses_what_it_cannot_read():
+    """Refused before anything is launched: host tensors, f32, heads that are not dense, shapes that do not agree."""
+    import torch
+    q, k = torch.zeros(4, 8, 64, dtype=torch.bfloat16), torch.zeros(4, 2, 64, dtype=torch.bfloat16)
+    for bad in ((q, k, k), (q[:, ::2], k, k), (q, k[:3], k[:3]), (q, k, k[:, :1]), (q[..., :32], k[..., :32], k[..., :32])):
+        with pytest.raises(ValueError):
+            pa.prefill_attention(*bad, 0.125)
+    with pytest.raises((KeyError, ValueError)):
+        pa.prefill_attention(q.float(), k.float(), k.float(), 0.125)
