@@ -19,6 +19,7 @@
 #include <cuda_fp8.h>
 #include <stdio.h>
 #include <stdlib.h>
+#include <atomic>
 #include <type_traits>
 
 namespace mrs {
@@ -604,15 +605,22 @@ __global__ void merge_partials_kernel(const T *__restrict__ tmp_o, const float *
 #include "paged_attn_mma.cuh"
 namespace mrs {
 
+constexpr int PA_MAX_DEVICES = 64;
 static int g_pa_flags = 0;   // bit 0: keep HND decode on the SIMT kernel (A/B, debugging); bit 2 / 3: never / always pairs of CTAs a tile; bit 4: merge late
 
 // Pairs of CTAs a tile, each with half of its tokens: at up to one and a half CTAs an SM.  There a tile's time is its chain of stages (load, scores,
 // soft-max, product: ~1 us each), and half as many of them take 11.3 us where the whole took 13.8 (1 sequence of 300 tokens, 32 query and 8 KV heads of
 // 128), 13.9 against 15.4 (1 of 3000), 13.9 against 15.5 (16 of 300), 12.7 against 14.0 (8 of 500).  With more CTAs the pairs no longer run at one time
 // and each adds a head and an exchange: 256 CTAs take 19.4 us against 15.2, 376 take 25.3 against 19.2.
-static bool pm_pairs(long long ctas) {
+static bool pm_pairs(long long ctas, int dev) {
   if (g_pa_flags & 12) return (g_pa_flags & 8) != 0;
-  return 2 * ctas <= 3 * 148;
+  static std::atomic<int> known[PA_MAX_DEVICES];
+  int sms = known[dev].load(std::memory_order_relaxed);
+  if (sms == 0) {
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    known[dev].store(sms, std::memory_order_relaxed);
+  }
+  return 2 * ctas <= 3LL * sms;
 }
 
 template <typename K>
@@ -669,7 +677,9 @@ static cudaError_t launch_decode_g(PagedParams p, int tiles, cudaStream_t st) {
         }
       }
       if constexpr (!FUSED) {
-        if (pm_pairs((long long)tiles * p.num_kv_heads * nsub)) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev >= 0 && dev < PA_MAX_DEVICES && pm_pairs((long long)tiles * p.num_kv_heads * nsub, dev)) {
           auto kern = paged_decode_mma_kernel<T, D, false, false, true>;
           const size_t dyn = pm_smem_bytes<D>(false, false);
           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
@@ -680,8 +690,20 @@ static cudaError_t launch_decode_g(PagedParams p, int tiles, cudaStream_t st) {
           attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
           attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
           attr[1].val.programmaticStreamSerializationAllowed = 1;
-          cfg.attrs = attr; cfg.numAttrs = p.pdl ? 2 : 1;
-          return cudaLaunchKernelEx(&cfg, kern, p);
+          cfg.attrs = attr; cfg.numAttrs = 1;
+          static std::atomic<int> feasible[PA_MAX_DEVICES];      // (as above; asked once per device)
+          int can = feasible[dev].load(std::memory_order_relaxed);
+          if (can == 0) {
+            int ncl = 0;
+            const cudaError_t qe = cudaOccupancyMaxActiveClusters(&ncl, kern, &cfg);
+            if (qe != cudaSuccess) (void)cudaGetLastError();
+            can = qe == cudaSuccess && ncl >= 1 ? 1 : -1;
+            feasible[dev].store(can, std::memory_order_relaxed);
+          }
+          if (can == 1) {
+            cfg.numAttrs = p.pdl ? 2 : 1;
+            return cudaLaunchKernelEx(&cfg, kern, p);
+          }
         }
       }
       return launch_pa(paged_decode_mma_kernel<T, D, FUSED, false>, grid, p, st, pm_smem_bytes<D>(FUSED, false), PM_THREADS);
