@@ -313,3 +313,58 @@ def test_tensor_core_calls_are_refused_once_a_wait_has_run_out(cuda):
     finally:
         flag[0] = 0
     assert all(torch.equal(call(), w) for call, w in zip(refused, want[0]))
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f16", "f32"])
+@pytest.mark.parametrize("dtype,N", [(t, 70) for t in ALL_TYPES] + [("q4_k", 4300), ("q5_k", 3500), ("q6_k", 2900), ("q8_0", 2300), ("q3_k", 5400)])
+def test_reference_shaped_launchers(cuda, dtype, N, dt):
+    """launch_mmvq_gguf_<type>_<dtype>_{plain,fused_glu,fused_qkv} as a caller of the C symbols has them: activation rows padded to 512 columns, results
+    with a stride of their own, one to eight rows, below and above 5 MB.  The bits of the Python calls; those against the oracle elsewhere here."""
+    import ctypes
+    from mistralrs_b200 import lib
+    K = 2304
+    gen = torch.Generator(device=cuda).manual_seed(N)
+    weight = lambda n, seed: quant.QTensor(to_dev(make_weight(dtype, n, K, seed).reshape(-1), cuda), dtype, (n, K))  # noqa: E731
+    ws = [weight(N, 1), weight(N, 2), weight(N - 7, 3)]
+    P, I = lambda t: ctypes.c_void_p(t.data_ptr()), ctypes.c_int  # noqa: E731
+    entry = lambda kind: getattr(lib(), f"launch_mmvq_gguf_{dtype}_{dt}_{kind}")  # noqa: E731
+    stream = ctypes.c_void_p(torch.cuda.current_stream(cuda).cuda_stream)
+    for rows in range(1, 9):
+        x = torch.randn(rows, K, device=cuda, generator=gen).to({"bf16": torch.bfloat16, "f16": torch.float16, "f32": torch.float32}[dt])
+        y, stride = quant.quantize_q8_1(x), 2560 // 32
+        plain, glu = (torch.full((rows, N + 5), -77.0, dtype=x.dtype, device=cuda) for _ in range(2))
+        qkv = [torch.empty(rows, w.shape[0], dtype=x.dtype, device=cuda) for w in ws]
+        entry("plain")(P(ws[0].data), P(y), P(plain), I(K), I(N), I(stride), I(N + 5), I(rows), stream)
+        entry("fused_glu")(P(ws[0].data), P(ws[1].data), P(y), P(glu), I(K), I(N), I(stride), I(N + 5), I(rows), I(0), stream)
+        entry("fused_qkv")(*(P(w.data) for w in ws), P(y), *(P(o) for o in qkv), I(K), *(I(w.shape[0]) for w in ws), I(stride), I(rows), stream)
+        assert torch.equal(plain[:, :N], quant.plain(ws[0], x)) and bool((plain[:, N:] == -77.0).all()), rows
+        assert torch.equal(glu[:, :N], quant.fused_glu(ws[0], ws[1], x, quant.GluActivationType.Silu)) and bool((glu[:, N:] == -77.0).all()), rows
+        assert all(torch.equal(a, b) for a, b in zip(qkv, quant.fused_qkv(*ws, x))), rows
+    assert lib().mrs_mmq_timeouts() == 0
+
+
+@pytest.mark.parametrize("dtype,N,K", [("q4_k", 4300, 2304), ("q5_k", 3500, 2304), ("q6_k", 2900, 2304), ("q6_k", 1000, 11008), ("q8_0", 2300, 2304)])
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+def test_tensor_core_rows_with_a_residual_against_the_oracle(cuda, dtype, N, K, dt):
+    """mmvq_mma_kernel on its own oracle, with the residual of a decode step's projections: the oracle's integer dots to 5e-6 in f32 (as the vector
+    kernel); in bf16 the product is rounded, and again after the residual is added."""
+    import ctypes
+    from mistralrs_b200 import GGML, lib
+    wb = make_weight(dtype, N, K, 5)
+    w = to_dev(wb.reshape(-1), cuda)
+    P, I = lambda t: ctypes.c_void_p(t.data_ptr() if t is not None else 0), ctypes.c_int  # noqa: E731
+    stream = ctypes.c_void_p(torch.cuda.current_stream(cuda).cuda_stream)
+    code = {"f32": 2, "bf16": 1}[dt]
+    for rows in (3, 5, 8):
+        y = quant.quantize_q8_1(to_dev(make_acts(rows, K, 6 + rows, dt), cuda, dt), k_padded=K)
+        ref = oracle.mmvq_q8_1(dtype, wb, y.cpu().numpy(), K, N, K // 32, rows)      # (over the rows as quantised: 16-bit inputs have ties)
+        scale = np.abs(ref).max()
+        residual = to_dev((np.random.default_rng(rows).standard_normal((rows, N)) * scale).astype(np.float32), cuda, dt)
+        for add in (None, residual):
+            out = torch.empty(rows, N, dtype=residual.dtype, device=cuda)
+            assert lib().mrs_mmvq_q8(I(GGML[dtype]), I(0), I(code), P(w), P(None), P(None), P(y), P(add), P(out), P(None), P(None), I(K), I(N), I(0), I(0),
+                                     I(rows), I(0), I(0), stream) == 0
+            want = ref + (0 if add is None else add.double().cpu().numpy())
+            err = np.abs(out.double().cpu().numpy() - want)
+            step = 0.0 if dt == "f32" else 2.0 ** -8 * (np.abs(want) + (0 if add is None else np.abs(ref)))      # half a place of each rounding, and more
+            assert (err <= 5e-6 * scale + 2.0 ** -23 * np.abs(want) + step).all(), (rows, add is None, err.max())

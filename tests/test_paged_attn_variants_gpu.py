@@ -125,3 +125,29 @@ def test_hnd_layout_fp8_f32_and_512(cuda, dt, cache, D):
         got = paged_attn.flashinfer_decode(q.to(cuda), kc, vc, d(indptr), d(indices), d(last), d(req), d(tile), d(oind), d(chunk),
                                            d(mask), scale, k_scale=ksc, v_scale=vsc).float().cpu().numpy()
         assert np.abs(got - want).max() <= TOL[dt] * np.abs(want).max(), (dt, cache, D, split)
+
+
+@pytest.mark.parametrize("dt,cache,D,BS", [(torch.bfloat16, torch.float8_e4m3fn, 128, 16), (torch.float16, torch.float8_e4m3fn, 64, 32),
+                                           (torch.bfloat16, torch.float8_e4m3fn, 80, 16), (torch.bfloat16, torch.float8_e4m3fn, 112, 8),
+                                           (torch.float32, torch.float32, 64, 16), (torch.float16, torch.float16, 96, 16),
+                                           (torch.bfloat16, torch.bfloat16, 192, 32), (torch.bfloat16, torch.bfloat16, 256, 16),
+                                           (torch.float16, torch.float16, 512, 16)])
+def test_hnd_windows_on_the_general_kernel(cuda, dt, cache, D, BS):
+    """Tiles that start at the window, so in the middle of a page, with fp8 and f32 caches and the head sizes besides 64 and 128 (paged_decode_kernel),
+    whole and in tiles of four pages, some of which lie before the window altogether."""
+    ctx = [1, 45, 129, 300]
+    q, kq, vq, kd, vd, tables, NB, max_blocks, ksc, vsc = _setup(cuda, dt, cache, D, ctx, BS=BS)
+    kc, vc = _fill_hnd(kq, vq, tables, NB, 2, D, BS, cache, cuda)
+    used = [t[:-(-c // BS)] for t, c in zip(tables, ctx)]
+    indptr, indices, last = kv_index.make_paged_kv_tensors(used, ctx, BS, sum(len(u) for u in used))
+    scale = D ** -0.5
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)  # noqa: E731
+    for window in (0, 1, 30, 63, 64, 127, 128, 200, 1000):
+        seen = [min(c, window + 1) for c in ctx]
+        want = _ref(q.float().numpy(), [k[len(k) - n:] for k, n in zip(kd, seen)], [v[len(v) - n:] for v, n in zip(vd, seen)], seen, scale)
+        for split in (None, 4):
+            padded = len(ctx) if split is None else sum(-(-len(u) // split) for u in used)
+            req, tile, oind, chunk, mask = kv_index.make_paged_kv_decode_tensors(used, ctx, BS, split, padded)
+            got = paged_attn.flashinfer_decode(q.to(cuda), kc, vc, d(indptr), d(indices), d(last), d(req), d(tile), d(oind), d(chunk),
+                                               d(mask), scale, window_left=window, k_scale=ksc, v_scale=vsc).float().cpu().numpy()
+            assert np.abs(got - want).max() <= TOL[dt] * np.abs(want).max(), (window, split)

@@ -142,3 +142,32 @@ def test_values_outside_the_window_of_a_tile_leave_no_trace(cuda, D, varlen):
         vv[:128 - window] = float("inf")      # (of the second tile's rows, 128 .. 255)
         vv[256:] = float("nan")
         assert torch.equal(run(vv)[128:256], clean[128:256]), window
+
+
+@pytest.fixture(params=[0, 1], ids=["mma.sync", "tcgen05"])
+def either_kernel(request):
+    """Both prompt kernels for what both take (softcap runs on csrc/prefill_attn.cu whatever is asked for)."""
+    import ctypes
+    from mistralrs_b200 import lib
+    lib().mrs_prefill_attn_tc_debug(ctypes.c_int32(request.param), ctypes.c_uint32(0), ctypes.c_uint32(0))
+    yield
+    lib().mrs_prefill_attn_tc_debug(ctypes.c_int32(1), ctypes.c_uint32(0), ctypes.c_uint32(0))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_ragged_batches_windows_and_softcap_on_either_kernel(cuda, either_kernel, dt, D):
+    """Sequences of several lengths (one of them empty) with every pair of window and softcap, causal and not, on each kernel: 3 ulp as above."""
+    lens, H, KVH = [5, 130, 0, 64, 257], 6, 2
+    gen = torch.Generator(device=cuda).manual_seed(D)
+    q, k, v = (torch.randn(sum(lens), h, D, device=cuda, generator=gen).to(dt) for h in (H, KVH, KVH))
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device=cuda)
+    scale, ulp = D ** -0.5, 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11
+    for causal in (True, False):
+        for window in (None, 0, 63, 70, 128):
+            for softcap in (None, 20.0):
+                got = paged_attn.prefill_attention(q, k, v, scale, causal=causal, cu_seqlens=cu, max_seqlen=max(lens), window_left=window, softcap=softcap).double()
+                for a, b in zip(cu[:-1].tolist(), cu[1:].tolist()):
+                    if a < b:
+                        want = _ref(q[a:b], k[a:b], v[a:b], scale, causal, window, softcap)
+                        assert (got[a:b] - want).abs().max().item() <= 3 * ulp * want.abs().max().item() + 1e-6, (causal, window, softcap, b - a)
