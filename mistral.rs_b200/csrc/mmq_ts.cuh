@@ -55,19 +55,21 @@ struct TsParams {
   int nt, tiles_m, tiles_n;   // tokens per tile (multiple of 16), tiles
   int ksplit;                 // CTAs of a cluster that share K
   int rs, xs, xb;             // depths of the raw and the X ring; 64-k tiles of an X stage
-  // int4 checkpoints (TS_INT4): w in tiles [K/64][N][32 B] (csrc/w4a16.cu), scales [K/group][N]
+  // int4 checkpoints: w in tiles [K/64][N][32 B] (csrc/w4a16.cu), scales [K/group][N]
   const uint8_t *scales;
   const uint8_t *qzeros;      // AWQ [K/group][N/8] words, or null: zero point 8
   int group32, group_shift;   // weights of a group / 32, and its logarithm or -1
-  int scale_perm;             // columns 0 plain, 1 / 2 Marlin-permuted 64 / 32 wide; TS_SCALES_OTHER: scales in the other 16-bit format
+  int scale_perm;             // columns 0 plain, 1 / 2 Marlin-permuted 64 / 32 wide
   int pdl;                    // link of a programmatic-dependent-launch chain: x comes from, y may be read by, the grid before
 };
 // (eight bytes more, and every launch took the host 0.3 us longer)
 static_assert(sizeof(TsParams) <= 104, "parameters of a launch");
 
-constexpr int TS_SCALES_OTHER = 4;         // (of TsParams::scale_perm) f16 scales of bf16 rows, bf16 scales of f16 rows: rounded on the way
-                                           // (4096 x 14336, 500 tokens: 54.6 us behind a launch that casts them, 50.5 so)
-constexpr int TS_INT4 = 200;               // block type of int4 checkpoints
+// block types of int4 checkpoints: scales in the activation format, and in the other 16-bit format (f16 scales of bf16 rows, bf16 scales of f16 rows),
+// rounded as they are read (4096 x 14336, 500 tokens: 54.6 us behind a launch that casts them, 50.5 so).  A type of its own: asked for at run time in the
+// inner loop the format cost every int4 call up to 1 % (14336 x 4096 at 32 tokens 15.31 us, 15.21 without; 4096 x 14336 at 500 49.5, 49.0).
+constexpr int TS_INT4 = 200, TS_INT4_OTHER = 201;
+constexpr bool ts_is_int4(int type) { return type == TS_INT4 || type == TS_INT4_OTHER; }
 // SPAN: bytes of 256 weights of a row; PITCH: of a row in a raw stage, an odd multiple of 16 (16-byte reads of 8 consecutive rows
 // then fall on distinct banks) that also holds the bytes in front of and behind an unaligned span
 template <int TYPE> struct TsFmt;
@@ -88,9 +90,11 @@ template <> struct TsPitch<MRS_Q5_0, true> { static constexpr int value = 176; }
 template <> struct TsPitch<MRS_Q8_0, true> { static constexpr int value = 272; };
 // int4 tiles: four chunks of [128 rows][32 B], then up to 8 rows of 128 scales (groups of 32 at least) and 8 of 16 zero-point words
 template <> struct TsFmt<TS_INT4> { static constexpr int SPAN = 0, PITCH = 32; };
+template <> struct TsFmt<TS_INT4_OTHER> : TsFmt<TS_INT4> {};
 constexpr int TS_I4_CHUNK = TS_BM * 32, TS_I4_SCALES = 4 * TS_I4_CHUNK, TS_I4_ZEROS = TS_I4_SCALES + 8 * TS_BM * 2, TS_I4_STAGE = TS_I4_ZEROS + 8 * 64;
 template <int TYPE, bool ALIGNED> struct TsStage { static constexpr int BYTES = TS_BM * TsPitch<TYPE, ALIGNED>::value; };
 template <> struct TsStage<TS_INT4, true> { static constexpr int BYTES = TS_I4_STAGE; };
+template <> struct TsStage<TS_INT4_OTHER, true> : TsStage<TS_INT4, true> {};
 
 // By the whole warp.  False when the phase did not complete within the limit: the caller then ends its part of the CTA.  (The issuer and the producers
 // pass several waits in a span: 2 to 5 % of a launch lies between this loop, vote inside, and one that leaves PTX to vote in each round: Q5_K 4096 x
@@ -588,7 +592,7 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
         if (p.pdl && it == RS) pdl_wait();             // the ring is full: from here on its stages are freed at the grid before's pace
         ok = ts_wait(raw_empty + st, ph ^ 1, late);
         if (!ok) break;
-        if constexpr (TYPE == TS_INT4) {
+        if constexpr (ts_is_int4(TYPE)) {
           const int k0 = s * TS_SPAN_K, rows = min(TS_BM, p.N - n0), chunks = min(4, (p.K - k0) >> 6), g0 = (k0 >> 5) / p.group32;
           const int groups = ((k0 + 64 * chunks - 1) >> 5) / p.group32 - g0 + 1;                // that the span's k touch
           const uint32_t dst = smem_u32(r_ring) + (uint32_t)st * RAW_BYTES, bar = smem_u32(raw_full + st);
@@ -682,12 +686,11 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
     const uint32_t ta0 = tmem_a + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(part * 32);
     uint32_t scale0 = 0u, zero0 = 0u;                  // int4: this row's first scale and zero-point word
     int zero_shift = 0;
-    if constexpr (TYPE == TS_INT4) {
+    if constexpr (ts_is_int4(TYPE)) {
       // inverses of the reference's scale-column permutations (REF gptq_cuda.rs:530-540 get_scale_perms), which stay inside a tile:
       // 64 wide perm[8 i + j] = i + 8 j, 32 wide perm[8 i + j] = 2 i + {0, 1, 8, 9, 16, 17, 24, 25}[j]
-      const int perm = p.scale_perm & 3;
-      const int c = perm == 1 ? (r & ~63) + 8 * (r & 7) + ((r & 63) >> 3)
-                  : perm == 2 ? (r & ~31) + 8 * ((r & 7) >> 1) + 2 * ((r & 31) >> 3) + (r & 1) : r;
+      const int c = p.scale_perm == 1 ? (r & ~63) + 8 * (r & 7) + ((r & 63) >> 3)
+                  : p.scale_perm == 2 ? (r & ~31) + 8 * ((r & 7) >> 1) + 2 * ((r & 31) >> 3) + (r & 1) : r;
       scale0 = smem_u32(r_ring) + (uint32_t)(TS_I4_SCALES + 2 * c);
       zero0 = smem_u32(r_ring) + (uint32_t)(TS_I4_ZEROS + 4 * (r >> 3));
       zero_shift = 4 * ((r & 1) ? 4 + ((r & 7) >> 1) : (r & 7) >> 1);        // nibble i of a word is column {0, 2, 4, 6, 1, 3, 5, 7}[i]
@@ -699,7 +702,7 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
       for (int s = s0; s < s1; s++, it++) {
         const int as = it % TS_AS;
         uint32_t phase;                                // of the span inside its 16-byte aligned copy
-        if constexpr (TYPE == TS_INT4) phase = 0u;
+        if constexpr (ts_is_int4(TYPE)) phase = 0u;
         else if constexpr (ALIGNED) phase = (uint32_t)(s * F::SPAN) & 15u;
         else phase = ((uint32_t)(n0 + r) * (uint32_t)p.row_bytes + (uint32_t)s * (uint32_t)F::SPAN) & 15u;
         ok = ts_wait(raw_full + st, ph, late);
@@ -707,8 +710,8 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
         const bool live = s * TS_SPAN_K + 64 * part < p.K;   // the last span of a 32-wide type may be ragged
         uint32_t o[16];
         const uint32_t stage = (uint32_t)st * RAW_BYTES;
-        typename std::conditional<TYPE == TS_INT4, TsInt4<BF>, TsUnit<TYPE, ALIGNED, BF>>::type u;
-        if constexpr (TYPE == TS_INT4) {
+        typename std::conditional<ts_is_int4(TYPE), TsInt4<BF>, TsUnit<TYPE, ALIGNED, BF>>::type u;
+        if constexpr (ts_is_int4(TYPE)) {
           u.a = lds128(row0 + stage + (uint32_t)(part * TS_I4_CHUNK)); u.b = lds128(row0 + stage + (uint32_t)(part * TS_I4_CHUNK) + 16u);
           // each 32 weights' group, counted from the span's first (uniform); in units of 32 weights, by shifts where a group is a power of two
           const uint32_t u0 = (uint32_t)(s * (TS_SPAN_K / 32)), u1 = u0 + 2u * (uint32_t)part;
@@ -717,7 +720,7 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
           for (uint32_t h = 0; h < 2; h++) {
             const uint32_t g = (p.group_shift >= 0 ? (u1 + h) >> p.group_shift : (u1 + h) / (uint32_t)p.group32) - g0;
             u.s[h] = lds_u16s(scale0 + stage + g * (TS_BM * 2));
-            if (p.scale_perm & TS_SCALES_OTHER) {
+            if constexpr (TYPE == TS_INT4_OTHER) {
               if constexpr (BF) u.s[h] = __bfloat16_as_ushort(__float2bfloat16_rn(ts_h2f(u.s[h])));
               else u.s[h] = __half_as_ushort(__float2half_rn(__uint_as_float(u.s[h] << 16)));
             }
@@ -738,7 +741,7 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
           for (int i = 0; i < 16; i++) o[i] = 0u;
         }
         tmem_st_32x16(ta, o);
-        if constexpr (TYPE == TS_INT4) u.template half<1>(o);
+        if constexpr (ts_is_int4(TYPE)) u.template half<1>(o);
         else u.template half<1>(part, o);
         if (!live) {
 #pragma unroll
@@ -841,7 +844,7 @@ struct TsCall {
   int nt, tiles_m, ksplit, sms;       // the plan
   int *timeouts;
   cudaStream_t stream;
-  const void *scales, *qzeros;        // TS_INT4
+  const void *scales, *qzeros;        // int4
   int group, scale_perm, pdl;
 };
 
@@ -852,7 +855,7 @@ template <int TYPE, bool ALIGNED> static cudaError_t ts_launch_as(const TsCall &
   if (enc == nullptr) return cudaErrorNotSupported;
   CUtensorMap tw, tx;
   if (!tc_make_map_2d(&tx, c.x, (uint64_t)c.M, (uint64_t)c.K, TS_XK, (uint32_t)c.nt, c.dtype)) return cudaErrorInvalidValue;
-  if (ALIGNED && TYPE != TS_INT4) {
+  if (ALIGNED && !ts_is_int4(TYPE)) {
     const cuuint64_t dims[2] = {(cuuint64_t)(c.row_bytes / 2), (cuuint64_t)c.N};
     const cuuint64_t strides[1] = {(cuuint64_t)c.row_bytes};
     const cuuint32_t box[2] = {(cuuint32_t)(PITCH / 2), (cuuint32_t)TS_BM};
@@ -907,11 +910,9 @@ template <int TYPE, bool ALIGNED> static cudaError_t ts_launch_as(const TsCall &
 }
 
 template <int TYPE> cudaError_t ts_launch(const TsCall &c) {
-  if constexpr (TYPE == TS_INT4) return ts_launch_as<TYPE, true>(c);
-  else
-  if (c.row_bytes % 16 == 0) return ts_launch_as<TYPE, true>(c);
+  if (ts_is_int4(TYPE) || c.row_bytes % 16 == 0) return ts_launch_as<TYPE, true>(c);
   // superblocks of 144 and 176 bytes make every row a multiple of 16
-  if constexpr (TYPE == MRS_Q4_K || TYPE == MRS_Q5_K) return cudaErrorNotSupported;
+  if constexpr (ts_is_int4(TYPE) || TYPE == MRS_Q4_K || TYPE == MRS_Q5_K) return cudaErrorNotSupported;
   else return ts_launch_as<TYPE, false>(c);
 }
 

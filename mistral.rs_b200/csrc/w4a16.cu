@@ -345,7 +345,7 @@ static cudaError_t run_dense(const void *x, const void *w, void *y, int M, int K
 }
 
 static cudaError_t run_int4(const void *x, const void *w, const void *scales, const int32_t *qzeros, void *y, int M, int K, int N, int group, int dtype,
-                            int scale_perm, cudaStream_t st, int pdl = 0) {
+                            int scale_perm, cudaStream_t st, int pdl = 0, bool scales_other = false) {
   if (M <= 0 || N <= 0) return cudaSuccess;
   cudaError_t e;
   if (K % WA_BK != 0 || (dtype != MRS_F16 && dtype != MRS_BF16)) return cudaErrorInvalidValue;
@@ -360,10 +360,11 @@ static cudaError_t run_int4(const void *x, const void *w, const void *scales, co
   // (a span of a row: 128 B of nibbles and its scales; 800: the dequantisers' weight in the plan's estimate, two operations a weight)
   const TsPlan plan = ts_plan(M, N, K, 128 + 2 * ((TS_SPAN_K + group - 1) / group), 800, 0, d);
   const TsCall c = {w, x, y, M, N, K, 0, dtype, plan.nt, plan.tiles_m, plan.ksplit, d.sms, d.timeouts, st, scales, qzeros, group, scale_perm, pdl ? 1 : 0};
-  return ts_launch<TS_INT4>(c);
+  return scales_other ? ts_launch<TS_INT4_OTHER>(c) : ts_launch<TS_INT4>(c);
 }
 
 template cudaError_t ts_launch<TS_INT4>(const TsCall &);
+template cudaError_t ts_launch<TS_INT4_OTHER>(const TsCall &);
 
 }  // namespace mrs
 
@@ -401,13 +402,13 @@ extern "C" int32_t mrs_dense_linear_pdl(const void *x, const void *w, void *y, i
 // permutation when group < K/8 (the reference passes in_dim / pack_factor as size_k), else the
 // 32-wide one; `workspace` (Marlin's lock array) is not needed.
 static int marlin_common(const void *inputs, const int32_t *weight, const void *scales, const void *zeros, void *out, int m,
-                         int k, int n, int groupsize, int dtype, int is_awq, int64_t stream, int scales_other = 0) {
+                         int k, int n, int groupsize, int dtype, int is_awq, int64_t stream, bool scales_other = false) {
   cudaError_t status = cudaGetLastError();
   if (status != cudaSuccess) return (int)status;
   const int group = groupsize <= 0 ? k : groupsize;
   const int perm_kind = (groupsize > 0 && groupsize < k / 8) ? 1 : 2;
   const cudaError_t e = run_int4(inputs, weight, scales, is_awq ? (const int32_t *)zeros : nullptr, out, m, k, n, group,
-                               dtype, perm_kind | scales_other, (cudaStream_t)stream);
+                               dtype, perm_kind, (cudaStream_t)stream, 0, scales_other);
   return e == cudaSuccess ? (int)cudaGetLastError() : (int)e;
 }
 extern "C" int marlin_gptq_4bit_f16(const void *inputs, const int32_t *weight, const void *scales, const void *zeros,
@@ -436,7 +437,7 @@ extern "C" int marlin_awq_4bit_bf16(const void *inputs, const int32_t *weight, c
 extern "C" int mrs_marlin_4bit(const void *inputs, const int32_t *weight, const void *scales, const void *zeros, void *out, int m, int k, int n,
                                int groupsize, int dtype, int scale_dtype, int is_awq, int64_t stream) {
   if (scale_dtype != MRS_F16 && scale_dtype != MRS_BF16) return (int)cudaErrorInvalidValue;
-  return marlin_common(inputs, weight, scales, zeros, out, m, k, n, groupsize, dtype, is_awq, stream, scale_dtype != dtype ? TS_SCALES_OTHER : 0);
+  return marlin_common(inputs, weight, scales, zeros, out, m, k, n, groupsize, dtype, is_awq, stream, scale_dtype != dtype);
 }
 
 // weight [k/8, n] i32, perm [k] i32 (argsort of g_idx; the reference always passes one), result: k*n/2 bytes

@@ -125,3 +125,26 @@ def test_scales_in_the_other_format(cuda, awq, K, N, group):
             want = layer.forward_raw(x)
             layer.scales = kept
             assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
+def test_scale_columns_other_than_permuted_are_plain(cuda):
+    """mrs_w4a16_gemm and its link of a launch chain: scale_perm 1 and 2 are permutations, every other value has always meant plain columns."""
+    import ctypes
+    from mistralrs_b200 import lib
+    K, N, M = 512, 128, 20
+    gen = torch.Generator(device=cuda).manual_seed(1)
+    qweight = torch.randint(-2 ** 31, 2 ** 31, (K // 8, N), dtype=torch.int32, device=cuda, generator=gen)
+    scales = (torch.rand(K // 128, N, device=cuda, generator=gen) * 0.02 + 1e-3).to(torch.float16)
+    layer = gptq.GptqMarlinLayer(qweight, scales, group_size=128)
+    x = torch.randn(M, K, device=cuda, generator=gen).to(torch.float16)
+    P, I = lambda t: ctypes.c_void_p(t.data_ptr()), ctypes.c_int  # noqa: E731
+    stream = ctypes.c_void_p(torch.cuda.current_stream(cuda).cuda_stream)
+
+    def call(perm, link):
+        y = torch.empty(M, N, dtype=torch.float16, device=cuda)
+        args = (P(x), P(layer.q_weight), P(scales), ctypes.c_void_p(0), P(y), I(M), I(K), I(N), I(128), I(0), I(perm))
+        assert (lib().mrs_w4a16_gemm_pdl(*args, I(0), stream) if link else lib().mrs_w4a16_gemm(*args, stream)) == 0
+        return y
+    want = call(0, False)
+    assert all(torch.equal(call(perm, link), want) for perm in (3, 4, 7, 8, -1) for link in (False, True))
+    assert not torch.equal(call(1, False), want) and not torch.equal(call(2, True), want)
