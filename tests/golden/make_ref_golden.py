@@ -1,6 +1,6 @@
-"""Runs the UNMODIFIED reference CUDA kernels (oracle/_ref/*.so, built from /root/reference by
-oracle/build_ref.sh) on seeded inputs and stores their outputs as golden vectors:
-    python tests/golden/make_ref_golden.py            (on the GPU box; writes gpurun_out/ref_golden.npz)
+"""Runs the UNMODIFIED reference CUDA kernels (oracle/_ref/*.so, built from the reference's sources by
+oracle/build_ref.sh) on seeded inputs and stores their outputs as golden vectors (needs a GPU):
+    python tests/golden/make_ref_golden.py [OUT.npz]            (default: ref_golden.npz beside this file)
 The committed copy tests/golden/ref_golden.npz pins the CPU oracle (tests/test_oracle_golden.py)
 against what the reference itself computes."""
 import ctypes
@@ -209,6 +209,6 @@ if La is not None:
         out[f"pa_out_v1_{name}"] = o.float().cpu().numpy()
 
 torch.cuda.synchronize()
-os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-np.savez_compressed(os.path.join(ROOT, "gpurun_out", "ref_golden.npz"), **out)
-print("wrote gpurun_out/ref_golden.npz with", len(out), "arrays")
+path = sys.argv[1] if len(sys.argv) > 1 else os.path.join(os.path.dirname(os.path.abspath(__file__)), "ref_golden.npz")
+np.savez_compressed(path, **out)
+print("wrote", path, "with", len(out), "arrays")

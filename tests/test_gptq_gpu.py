@@ -1,6 +1,6 @@
 """GPTQ / AWQ int4 linear (tcgen05 path, raw checkpoint tensors) vs the numpy oracle
 (w = (q-8)*s symmetric GPTQ incl. act-order g_idx; w = (q-z)*s AWQ), f16 compute.
-Synthetic tensors per SURVEY §8(d): qweight uniform u4, scales f16 2^U(-8,-6), g_idx = k/128 and a
+Synthetic tensors: qweight uniform u4, scales f16 2^U(-8,-6), g_idx = k/128 and a
 random permutation (act-order)."""
 import numpy as np
 import pytest

@@ -14,7 +14,7 @@ def test_basic_allocation_golden():  # block_pool.rs `test_basic_allocation`
     blocks = pool.get_new_blocks(2)
     assert len(blocks) == 2 and pool.num_free_blocks() == 1
     assert all(pool.block_ref_cnt(b) == 1 for b in blocks)
-    assert pool.null_block_id() == 0 and blocks == [1, 2]  # SURVEY §8 a12: fresh pool -> 1..n
+    assert pool.null_block_id() == 0 and blocks == [1, 2]  # fresh pool -> 1..n
 
 
 def test_free_returns_to_pool_golden():  # `test_free_returns_to_pool`
@@ -86,7 +86,7 @@ def test_slot_mapping_and_pad():
 
 
 def test_fresh_pool_single_sequence_blocks():
-    # SURVEY §8 a12: fresh pool, one sequence of length L -> blocks 1..ceil(L/BS)
+    # fresh pool, one sequence of length L -> blocks 1..ceil(L/BS)
     for L, bs in ((128, 32), (129, 32), (384, 16)):
         pool = kv_index.BlockPool(64)
         nb = -(-L // bs)

@@ -1,7 +1,7 @@
 """Pins the CPU oracle (no GPU needed):
   * block decoders vs gguf-py 0.19.0 (tests/golden/gguf_dequant.npz, make_gguf_golden.py) — bit-exact;
   * Q8_1 quantiser, MMVQ arithmetic, fused GLU, RoPE, add_rms_norm, KV-cache scatter and paged
-    attention vs OUTPUTS OF THE UNMODIFIED REFERENCE KERNELS compiled from /root/reference and
+    attention vs OUTPUTS OF THE UNMODIFIED REFERENCE KERNELS compiled from its sources and
     run on a B200 (tests/golden/ref_golden.npz, make_ref_golden.py)."""
 import os
 
@@ -109,7 +109,7 @@ def test_paged_attention_vs_reference_kernels(ref):
         assert np.abs(got - want).max() <= 2.5 * 2.0 ** -8 * np.abs(want).max(), (on, np.abs(got - want).max())
 
 
-# ---- round 2: the reference kernels' outputs for MMQ, Marlin and the paged-attention variants pin the oracle too ----
+# ---- the reference kernels' outputs for MMQ, Marlin and the paged-attention variants pin the oracle too ----
 def _need(ref, key):
     if key not in ref.files:
         pytest.skip(f"tests/golden/ref_golden.npz has no `{key}`")

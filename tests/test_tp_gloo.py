@@ -72,7 +72,7 @@ def test_kv_head_and_block_alignment_rules():
     sys.path.insert(0, ROOT)
     from mistralrs_b200 import model as M
     cfg = M.LlamaConfig.llama3_8b()
-    for w in (2, 4, 8):   # SURVEY §8(d): K shards stay multiples of the 256 super-block
+    for w in (2, 4, 8):   # K shards stay multiples of the 256 super-block
         assert (cfg.inter // w) % 256 == 0 and (cfg.n_heads * cfg.head_dim // w) % 256 == 0
         assert cfg.n_kv_heads % w == 0
     c70 = M.LlamaConfig.llama3_70b()
