@@ -52,6 +52,11 @@ __device__ __forceinline__ void mv_wait(uint64_t *bar, uint32_t parity, bool &de
     *(volatile int *)timeouts = 1;
   }
 }
+// Copies in flight land before a CTA may end: the last of `n` stages, where a wait has run out.  (Out of line: in the consumers' code it cost launches
+// of four rows 1 %.)
+__device__ __noinline__ void mv_land(uint64_t *full, int n, int nst, int *timeouts) {
+  for (int i = max(0, n - nst); i < n; i++) { bool gone = false; mv_wait(&full[i % nst], (i / nst) & 1, gone, timeouts); }
+}
 // the word at a 2-byte aligned shared address
 __device__ __forceinline__ uint32_t mv_word(uint32_t a) {
   const uint32_t w = a & ~3u;
@@ -250,8 +255,7 @@ __global__ void __launch_bounds__(9 * 32, 2) mmvq_mma_kernel(const MmvqParams p)
         if (++stage == nst) { stage = 0; phase ^= 1; }
       }
     }
-    // copies in flight land before the CTA may end: the consumers have not waited for them where one of their waits ran out
-    for (int i = max(0, n - nst); i < n; i++) { bool gone = false; mv_wait(&full[i % nst], (i / nst) & 1, gone, p.timeouts); }
+    if (dead) mv_land(full, n, nst, p.timeouts);      // (otherwise the consumers wait for the last copies, or see to them where their own wait ran out)
     return;
   }
 
@@ -338,6 +342,7 @@ __global__ void __launch_bounds__(9 * 32, 2) mmvq_mma_kernel(const MmvqParams p)
       }
     }
   }
+  if (dead) mv_land(full, (vr1 - vr0 + P - 1) / P * nseg, nst, p.timeouts);
 }
 
 }  // namespace mrs
