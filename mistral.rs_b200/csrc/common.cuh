@@ -140,16 +140,17 @@ __device__ __forceinline__ void mbar_wait(uint64_t *bar, uint32_t parity) {
       "r"(parity)
       : "memory");
 }
-// By the whole warp, at most `limit` tries (the same in all lanes).  False when the phase did not complete within them.  PTX does not promise a warp
-// one answer: the lanes vote on it inside the loop, so that its branches are uniform and the warp is converged behind it, where .aligned instructions
-// may follow.  (Against a loop that each lane leaves by itself and a bar.warp.sync behind it, all within 1 %: four rows of a feed-forward of 4096 x
-// 14336 51.6 us and 52.5, three prompts of up to 2900 tokens 178 and 178, Q5_K 4096 x 4096 at 200 tokens 17.7 and 17.6.)
+// By the whole warp, at most `limit` tries (the same in all lanes).  False when the phase did not complete within them.  Plain branches, since PTX does
+// not promise a warp one answer: a lane that asks once more than the others is joined at the loop's end, as behind any loop, before the .aligned
+// instructions that may follow.  What is relied on beyond that: a phase that has completed stays so until this warp has passed it, so all lanes leave
+// with one answer, unless it completes at the very try that the limit ends on, seconds later, in a launch that is lost by then.  (A vote on each
+// answer inside the loop cost 1 to 2 % of a launch: Q4_K 14336 x 4096 at 300 tokens 34.5 us, 33.9 so; Q6_K 4096 x 14336 47.4 and 47.0.)
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, uint32_t limit) {
   uint32_t done;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, %3;\n\t"
-      "WAIT_%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tvote.sync.all.pred p, p, 0xffffffff;\n\t@p bra.uni DONE_%=;\n\t"
-      "sub.u32 n, n, 1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra.uni WAIT_%=;\n\tDONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      "WAIT_%=:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE_%=;\n\t"
+      "sub.u32 n, n, 1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra WAIT_%=;\n\tDONE_%=:\n\tselp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(done) : "r"(smem_u32(bar)), "r"(parity), "r"(limit) : "memory");
   return done != 0;
 }

@@ -97,8 +97,8 @@ template <> struct TsStage<TS_INT4, true> { static constexpr int BYTES = TS_I4_S
 template <> struct TsStage<TS_INT4_OTHER, true> : TsStage<TS_INT4, true> {};
 
 // By the whole warp.  False when the phase did not complete within the limit: the caller then ends its part of the CTA.  (The issuer and the producers
-// pass several waits in a span: 2 to 5 % of a launch lies between this loop, vote inside, and one that leaves PTX to vote in each round: Q5_K 4096 x
-// 4096, 200 tokens in a graph 17.7 us and 18.2, int4 14336 x 4096, 32 tokens 15.7 and 16.1.)
+// pass several waits in a span: 2 to 5 % of a launch lies between this loop and one that leaves PTX to vote in each round: Q5_K 4096 x 4096, 200
+// tokens in a graph 17.5 us and 18.3, int4 14336 x 4096, 32 tokens 15.3 and 16.1.)
 __device__ __forceinline__ bool ts_wait(uint64_t *bar, uint32_t parity, int *timeouts) {
   if (mbar_wait_warp(bar, parity, TS_WAIT_LIMIT)) return true;
   *(volatile int *)timeouts = 1;
