@@ -21,8 +21,8 @@
 // then the tensor pipe and the power limit.  The issuer must not be the bound: with its operands in ordinary registers sixteen products took
 // 1900 clocks beside the dequantisers, with a warp index that the compiler knows to be uniform 500.  Measured on one B200, us before and
 // after (before: one kernel for Q8_0, Q4_K and Q6_K with 128 or 256 tokens a tile and K whole, per-element decoding for the other types,
-// a kernel with 8 dequantising warps for int4): Q4_K 14336 x 4096, 24 tokens 29.3 / 18.4; Q5_K 4096 x 4096, 200 tokens 2517 / 20; Q8_0
-// 14336 x 4096, 4096 tokens 475 / 421; int4 14336 x 4096, 32 tokens 21.9 / 18.4; int4 with zero points 4096 x 14336, 500 tokens 170 / 67.
+// a kernel with 8 dequantising warps for int4): Q4_K 14336 x 4096, 24 tokens 29.3 / 18.4; Q5_K 4096 x 4096, 200 tokens 2517 / 18.5; Q8_0
+// 14336 x 4096, 4096 tokens 475 / 418; int4 14336 x 4096, 32 tokens 21.9 / 16.5; int4 with zero points 4096 x 14336, 500 tokens 170 / 61.5.
 // Every wait has a limit; one that runs out ends the CTA and sets a word in host memory, after which the entry points refuse every call
 // on that device with cudaErrorLaunchTimeout (the word itself: mrs_mmq_timeout_flag, mrs_mmq_timeouts).  That launch's output is not valid:
 // a tile may be missing, or with K split lack a rank's part (telling the other ranks cost every split launch 1 to 6 %).  What a limit counts is this grid's

@@ -245,7 +245,8 @@ extern "C" int32_t mrs_prefill_attention(const void *q, const void *k, const voi
   if (total_tokens <= 0) return 0;
   {   // the tcgen05 kernel when the call fits it (no softcap), at every length: 32 / 4 heads of 64, one prompt, us in a graph, mma.sync / tcgen05:
       // 8 tokens 5.8 / 4.2, 64 6.0 / 4.6, 128 10.0 / 4.8, 512 26.9 / 9.5; 32 / 8 heads of 128, window 20: 7.1 / 6.0, 7.5 / 6.3, 12.3 / 6.7, 16.9 / 9.9.
-      // (Its three tensor maps cost the host 0.8 us, which a lone short call outside a graph feels: 51 tokens 15.3 -> 16.1.)
+      // Its launch costs the host 0.7 us more (three tensor maps, 464 bytes of parameters), which calls of some 50 tokens in a host-bound stream feel (11.5
+      // us a call on mma.sync, 12.2 here); alone, to the end on the device, they are the faster ones here too (23.2 / 22.1).
     const int32_t e = mrs_prefill_attention_tc(q, k, v, out, cu_seqlens, batch, total_tokens, max_seqlen, num_heads, num_kv_heads,
                                                head_dim, q_stride, kv_stride, o_stride, softmax_scale, causal, window_left, softcap,
                                                dtype, stream);
