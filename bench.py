@@ -1775,7 +1775,8 @@ def main():
             "launches_per_token": launches_per_token,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "algorithmic_bytes_per_launch": weight_bytes / n_gemv, "peak_source": peak_src,
-                         "kernel": "mmvq_stream_kernel (all quantized GEMVs of one token" + (", incl. the in-graph all-reduces)" if world > 1 else ")"),
+                         "kernel": "mmvq_stream_kernel (all quantized GEMVs of one token" + (", incl. the in-graph all-reduces)" if world > 1 else ")") +
+                                   (", timed as a chain of launches; whole tokens run as one step_resident_kernel" if (launches_per_token or 99) < 10 else ""),
                          "launches": n_gemv, "avg_launch_us": gemv_s / n_gemv * 1e6, "bytes_per_token": weight_bytes},
             "breakdown_us_per_token": {"gemv_chain": gemv_s * 1e6, "attention_chain": attn_s * 1e6, "whole_token": 1e6 / value},
             "step_hbm_frac": total_bytes * value / 1e9 / peak,

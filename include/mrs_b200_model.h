@@ -61,7 +61,7 @@ typedef struct {
   int32_t batch, padded_tiles, max_blocks_per_seq;
   int32_t skip_mask;         /* measurement only: bit0 skip rope/cache/attention, bit1 skip the GEMVs */
   int32_t fused_attention;   /* 1: mrs_paged_decode_fused; 0: rotary + reshape_and_cache + flashinfer_decode */
-  int32_t extension;         /* 0, or MRS_LLAMA_STEP_Q8: the fields behind `tp` are there */
+  int32_t extension;         /* 0, or MRS_LLAMA_STEP_Q8 / _RESIDENT: which fields behind `tp` are there */
   int32_t *token_ids;        /* [batch] in: token to process; out_token may alias it */
   int32_t *positions;        /* [batch] */
   int64_t *slot_mapping;     /* [batch] */
@@ -83,8 +83,14 @@ typedef struct {
    * GEMVs that read it; same bits, less time.  Where the buffer is absent or too small the fused launch serves.  The step uses none of its
    * other buffers for this: the logits of a step are valid until the next step's head writes them. */
   void *q8; int64_t q8_bytes;
+  /* Only read when `extension` is MRS_LLAMA_STEP_RESIDENT (which has q8 too).  Scratch of at least mrs_llama_resident_bytes bytes, zeroed once, 16-byte
+   * aligned, of this step alone: with it a step of one sequence may run as one resident grid (csrc/step_resident.cu, a cooperative launch) instead of a
+   * chain of launches: the same bits in the same buffers, but tmp_v, tmp_s and attn_counters are then left as they are. */
+  void *resident; int64_t resident_bytes;
 } mrs_llama_step;
 #define MRS_LLAMA_STEP_Q8 0x51380001
+#define MRS_LLAMA_STEP_RESIDENT 0x51380002
+int64_t mrs_llama_resident_bytes(int32_t n_heads, int32_t head_dim, int32_t padded_tiles);
 
 /* Enqueue one decode step (all layers + lm_head + argmax) on `stream`. Returns cudaError. */
 int32_t mrs_llama_decode_step(const mrs_llama_step *s, void *stream);

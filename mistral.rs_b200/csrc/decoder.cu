@@ -52,6 +52,8 @@ extern "C" int32_t flashinfer_decode(void *q, void *key_cache, void *value_cache
                                      float k_scale, float v_scale, uint32_t dtype, uint32_t cache_dtype,
                                      cudaStream_t stream);
 
+extern "C" int32_t mrs_llama_step_resident(const mrs_llama_step *s, void *stream);      // step_resident.cu
+
 namespace mrs {
 bool mmvq_tensor_cores(int ggml_type, int rows, int K, int64_t nrows);      // mmvq.cu
 
@@ -400,7 +402,7 @@ extern "C" int32_t mrs_llama_decode_step(const mrs_llama_step *s, void *stream) 
   // tensor cores: the four layers take 465 us for 3 sequences (496 with the down projection alone apart), 457 for 4 (537); 491 for 5 and 495
   // for 8, which were 715 and 757 on the vector kernels; six layers 2048 wide 393 for 3 (395), 407 for 4 (421), 473 for 5 (560), 487 for 8 (598).  The rows go to a buffer of their own: nothing else of the
   // step is overwritten, the last step's logits among them.
-  const bool extended = s->extension == MRS_LLAMA_STEP_Q8 && ((uintptr_t)s->q8 & 3) == 0;
+  const bool extended = (s->extension == MRS_LLAMA_STEP_Q8 || s->extension == MRS_LLAMA_STEP_RESIDENT) && ((uintptr_t)s->q8 & 3) == 0;
   void *const q8 = extended ? s->q8 : nullptr;
   const int64_t q8_bytes = q8 != nullptr ? s->q8_bytes : 0;
   bool held = false;                       // q8 has the rows of the last product that was not told that they are there
@@ -416,6 +418,11 @@ extern "C" int32_t mrs_llama_decode_step(const mrs_llama_step *s, void *stream) 
     return mrs_mmvq_q8(w0.ggml_type, mode, dt, w0.data, w1, w2, q8, residual, d0, d1, d2, K, n0, n1, n2, B, 0, pdl, stream);
   };
   MRS_TRY(mrs_embedding_gather(s->tok_embd.ggml_type, s->tok_embd.data, H, s->token_ids, B, s->x, dt, stream));
+  if (B == 1) {
+    const int e = mrs_llama_step_resident(s, stream);
+    if (e == 0) MRS_TRY(mrs_argmax(s->logits, B, s->vocab, dt, s->out_token, s->argmax_scratch, pdl, stream));
+    if (e != (int)cudaErrorNotSupported) return e;
+  }
   void *hidden = s->x, *hidden2 = s->x2;
   for (int l = 0; l < s->n_layers; l++) {
     const mrs_llama_layer &L = s->layers[l];

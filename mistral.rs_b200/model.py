@@ -132,10 +132,11 @@ class _Step(ctypes.Structure):
                                                "attn_out", "act", "logits", "tmp_v", "tmp_s", "out_token",
                                                "attn_counters", "argmax_scratch")] + \
                [("all_reduce", _AR_FN), ("all_reduce_user", ctypes.c_void_p), ("tp", ctypes.c_void_p),
-                ("q8", ctypes.c_void_p), ("q8_bytes", ctypes.c_int64)]
+                ("q8", ctypes.c_void_p), ("q8_bytes", ctypes.c_int64), ("resident", ctypes.c_void_p), ("resident_bytes", ctypes.c_int64)]
 
 
 STEP_Q8 = 0x51380001       # MRS_LLAMA_STEP_Q8: q8 and q8_bytes are set
+STEP_RESIDENT = 0x51380002  # MRS_LLAMA_STEP_RESIDENT: and resident, resident_bytes
 
 
 class _TpCtx(ctypes.Structure):
@@ -586,6 +587,11 @@ class LlamaRunner:
         # the projections' inputs as Q8_1 rows (36 bytes for 32 columns), quantised once for a step of several sequences
         self.q8 = torch.empty(batch * max(H, self.n_heads * cfg.head_dim, cfg.inter // tp) // 32 * 36, dtype=torch.uint8, device=dev)
         s.extension, s.q8, s.q8_bytes = STEP_Q8, self.q8.data_ptr(), self.q8.numel()
+        if batch == 1:           # a step of one sequence as one resident grid: its barrier words and the attention's partial sums
+            nbytes = lib().mrs_llama_resident_bytes
+            nbytes.restype = ctypes.c_int64
+            self.resident = torch.zeros(nbytes(ctypes.c_int32(self.n_heads), ctypes.c_int32(cfg.head_dim), ctypes.c_int32(self.padded_tiles)), dtype=torch.uint8, device=dev)
+            s.extension, s.resident, s.resident_bytes = STEP_RESIDENT, self.resident.data_ptr(), self.resident.numel()
         self._ar_cb, self._peer = None, peer_allreduce
         if peer_allreduce is not None:     # in-graph peer-memory sum (takes precedence over the callback)
             s.tp = peer_allreduce.pointer()

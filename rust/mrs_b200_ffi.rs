@@ -7,6 +7,7 @@ use std::ffi::c_void;
 extern "C" {
     // ---- mrs_b200_model.h
     pub fn mrs_tp_allreduce_residual(ctx: *const c_void, slot: i32, residual: *const c_void, out: *mut c_void, count: i32, dtype: i32, pdl: i32, stream: *mut c_void) -> i32;
+    pub fn mrs_llama_resident_bytes(n_heads: i32, head_dim: i32, padded_tiles: i32) -> i64;
     pub fn mrs_llama_decode_step(s: *const c_void, stream: *mut c_void) -> i32;
     pub fn mrs_decode_advance(block_tables: *const i32, max_blocks_per_seq: i32, context_lens: *mut i32, batch: i32, block_size: i32, split_pages: i32, padded_tiles: i32, positions: *mut i32, slot_mapping: *mut i64, kv_indptr: *mut i32, kv_indices: *mut i32, kv_last_page_len: *mut i32, request_indices: *mut i32, kv_tile_indices: *mut i32, o_indptr: *mut i32, kv_chunk_size: *mut i32, block_valid_mask: *mut u8, max_pos: i32, error_flag: *mut i32, stream: *mut c_void) -> i32;
     pub fn mrs_embedding_gather(ggml_type: i32, table: *const c_void, cols: i32, ids: *const i32, n: i32, out: *mut c_void, act_dtype: i32, stream: *mut c_void) -> i32;

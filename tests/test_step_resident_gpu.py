@@ -1,0 +1,118 @@
+"""One-sequence decode steps as a resident grid (csrc/step_resident.cu) against the chain of launches that serves every other step: the same operations in
+the same order, so the same bits in every vector, cache row and logit."""
+import pytest
+import torch
+
+from mistralrs_b200 import model as M
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = {      # width, inner, heads, KV heads, head size
+    "gqa4": (2560, 1536, 16, 4, 128),         # ten blocks a row: a span and a part of one
+    "mha": (2560, 2816, 16, 16, 128),         # one query head a KV head, nine tiles at most; 176 and 80 blocks of Q8_0 a row
+    "gqa2_64": (3072, 512, 32, 16, 64),
+    "gqa7": (3584, 1024, 28, 4, 128),         # heads that do not fill the warps' groups; Q6_K rows off 16-byte boundaries
+    "gqa8_64": (2560, 768, 64, 8, 64),
+}
+
+
+def _pair(cuda, monkeypatch, shape, quant, dtype, layers=1, neox=True, block=16, vocab=1001, types=None, ctx=700):
+    hidden, inter, heads, kv, dim = SHAPES[shape]
+    if types is not None:
+        monkeypatch.setattr(M, "tensor_type", types)
+    cfg = M.LlamaConfig.tiny_test(quant=quant, n_layers=layers, hidden=hidden, inter=inter, n_heads=heads, n_kv_heads=kv, head_dim=dim, vocab=vocab,
+                                  rope_neox=neox, block_size=block, max_pos=4096, synth_scale_exp=(-15.5, -14.5))
+    w = M.LlamaWeights(cfg, cuda, dtype=dtype, fast_synth=True)
+    resident, chain = (M.LlamaRunner(w, batch=1, max_ctx=ctx) for _ in range(2))
+    chain.step_struct.extension = M.STEP_Q8
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for a, b in zip(resident.k_cache + resident.v_cache, chain.k_cache + chain.v_cache):
+        a.copy_(torch.randn(a.shape, device="cuda", generator=g))
+        b.copy_(a)
+    return resident, chain
+
+
+def _ran_resident(run):
+    """Tiles leave their sums in the scratch of the resident grid; nothing else writes there."""
+    return bool(run.resident[256:].any())
+
+
+def _step(run, at, token=11):
+    run.reset(at)
+    run.set_tokens([token])
+    run.step()
+    torch.cuda.synchronize()
+    return {k: run.buf[k].clone() for k in ("q", "k", "v", "attn_out", "x2", "act", "x", "logits", "out_token")}
+
+
+def _same(resident, chain, at):
+    a, b = _step(resident, at), _step(chain, at)
+    assert bool(torch.isfinite(b["logits"].float()).all()) and bool(b["logits"].any())
+    for k in a:
+        assert torch.equal(a[k], b[k]), (at, k, float((a[k].double() - b[k].double()).norm() / b[k].double().norm()))
+    assert all(torch.equal(x, y) for x, y in zip(resident.k_cache + resident.v_cache, chain.k_cache + chain.v_cache)), at
+
+
+@pytest.mark.parametrize("ctx", [60, 500, 1500])
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("quant,dtype", [("q4_k_m", torch.float16), ("q8_0", torch.bfloat16)])
+def test_step_equals_chain(cuda, monkeypatch, shape, quant, dtype, ctx):
+    """One tile a head, up to eight (a cluster's sums) and more (rounded partial results); contexts around a warp's, a step's and a tile's tokens."""
+    resident, chain = _pair(cuda, monkeypatch, shape, quant, dtype, neox=shape != "gqa4", ctx=ctx)
+    for at in (0, 1, 15, 16, 59, 63, 64, 65, 127, 128, 200, 497, 640, 1499):
+        if at < ctx:
+            _same(resident, chain, at)
+    assert (resident.padded_tiles == 1 or _ran_resident(resident)) and not _ran_resident(chain)
+
+
+@pytest.mark.parametrize("block", [8, 24, 32])
+def test_types_a_matrix_and_page_sizes(cuda, monkeypatch, block):
+    """q and k in Q6_K, v in Q8_0, o_proj in Q6_K, gate and up in Q8_0, down in Q4_K, the head in Q6_K with an odd number of rows; pages of other sizes."""
+    kinds = {"attn_q": "q6_k", "attn_k": "q6_k", "attn_v": "q8_0", "attn_output": "q6_k", "ffn_gate": "q8_0", "ffn_up": "q8_0", "output": "q6_k"}
+    resident, chain = _pair(cuda, monkeypatch, "gqa4", "q4_k_m", torch.float16, block=block, types=lambda cfg, name, layer=0: kinds.get(name, "q4_k"))
+    for at in (5, 100, 501):
+        _same(resident, chain, at)
+    assert _ran_resident(resident)
+
+
+def test_generation_in_a_graph(cuda, monkeypatch):
+    """Replays follow one another as eager steps do, bit for bit, and leave the words of the grid's barriers as they were."""
+    eager, graph = _pair(cuda, monkeypatch, "gqa4", "q4_k_m", torch.bfloat16, layers=2)
+    graph.step_struct.extension = M.STEP_RESIDENT
+    graph.capture()
+    for a, b in zip(eager.k_cache + eager.v_cache, graph.k_cache + graph.v_cache):      # (the capture's warm-up step wrote position 0)
+        b.copy_(a)
+    for run in (eager, graph):
+        run.reset(60)
+        run.set_tokens([7])
+    for _ in range(40):
+        eager.step()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(eager.logits(), graph.logits())
+    assert all(torch.equal(a, b) for a, b in zip(eager.k_cache + eager.v_cache, graph.k_cache + graph.v_cache))
+    assert not bool(graph.resident[:256].any()) and _ran_resident(graph)
+
+
+def test_more_layers_than_a_launch_holds(cuda, monkeypatch):
+    resident, chain = _pair(cuda, monkeypatch, "gqa2_64", "q4_k_m", torch.bfloat16, layers=33)
+    _same(resident, chain, 100)
+    assert _ran_resident(resident)
+
+
+def test_what_the_grid_declines(cuda, monkeypatch):
+    """Other block types, a sequence at the end of its context, a scratch that is too small, and the measuring switches: the chain's own bits or its rules."""
+    resident, chain = _pair(cuda, monkeypatch, "gqa4", "q4_k_m", torch.float16, types=lambda cfg, name, layer=0: "q4_0" if name == "ffn_down" else "q4_k")
+    assert torch.equal(_step(resident, 100)["logits"], _step(chain, 100)["logits"]) and not _ran_resident(resident)
+    monkeypatch.undo()
+    resident, chain = _pair(cuda, monkeypatch, "gqa4", "q4_k_m", torch.float16, ctx=160)
+    resident.step_struct.resident_bytes -= 16
+    assert torch.equal(_step(resident, 50)["logits"], _step(chain, 50)["logits"]) and not _ran_resident(resident)
+    resident.step_struct.resident_bytes += 16
+    before = [t.clone() for t in resident.k_cache + resident.v_cache]
+    resident.context_lens.fill_(160)          # full: attends, writes no cache row, sets the flag
+    resident.step()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(before, resident.k_cache + resident.v_cache))
+    assert int(resident.error_flag.item()) & 1 and _ran_resident(resident)
+    assert bool(torch.isfinite(resident.logits().float()).all())
