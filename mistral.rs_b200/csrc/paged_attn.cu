@@ -568,7 +568,7 @@ static cudaError_t launch_decode_g(PagedParams p, int tiles, cudaStream_t st) {
         int dev = 0;
         cudaGetDevice(&dev);
         if (dev >= 0 && dev < PA_MAX_DEVICES && pm_pairs((long long)tiles * p.num_kv_heads * nsub, dev)) {
-          auto kern = paged_decode_mma_kernel<T, D, false, false, true>;
+          auto kern = p.heads_per_cta <= 8 ? paged_decode_mma_kernel<T, D, false, false, true, true> : paged_decode_mma_kernel<T, D, false, false, true, false>;
           const size_t dyn = pm_smem_bytes<D>(false, false);
           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
           cudaLaunchConfig_t cfg = {};
@@ -593,6 +593,9 @@ static cudaError_t launch_decode_g(PagedParams p, int tiles, cudaStream_t st) {
             return cudaLaunchKernelEx(&cfg, kern, p);
           }
         }
+      }
+      if constexpr (!FUSED) {
+        if (p.heads_per_cta <= 8) return launch_pa(paged_decode_mma_kernel<T, D, false, false, false, true>, grid, p, st, pm_smem_bytes<D>(false, false), PM_THREADS);
       }
       return launch_pa(paged_decode_mma_kernel<T, D, FUSED, false>, grid, p, st, pm_smem_bytes<D>(FUSED, false), PM_THREADS);
     }

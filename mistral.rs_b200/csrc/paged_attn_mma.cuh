@@ -47,7 +47,24 @@ __device__ __forceinline__ void pm_st_cluster_f32(const float *local_ptr, uint32
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
 }
 
-template <typename T, int D, bool FUSED, bool CLUSTER, bool SPLIT = false>
+// 8 x 8 16-bit values (lane: row lane / 4, columns 2 (lane % 4), + 1) transposed
+__device__ __forceinline__ uint32_t pm_transpose(uint32_t v) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(v));
+  return d;
+}
+__device__ __forceinline__ float pm_exp2(float x) {
+  float d;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(d) : "f"(x));
+  return d;
+}
+
+// SWAP (up to eight heads a CTA, not FUSED): tokens are the products' M and heads their N, so that eight instead of sixteen products a head dimension of 128
+// make the scores of 16 tokens, eight the sums, and half as many accumulators are scaled, and only where a maximum has grown; a warp's 16 tokens that lie in
+// one page are copied from one address.  The instructions of 16 tokens, 870 before, were what bound the kernel (issue 44 % on average, 59 % on the SM with
+// the most tiles, HBM 51 %).  One B200, with the merge, before / now: 16 sequences of 1000 to 4000 tokens, 32 heads on 8, 48.1 / 36.5 us; 64 of 250 to 1000
+// 52.5 / 37.1; one of 300 10.9 / 8.9, of 8000 20.4 / 15.8; 32 heads on 32 82.8 / 62.0; 14 heads of 64 on 2, 33 sequences 11.5 / 10.1.
+template <typename T, int D, bool FUSED, bool CLUSTER, bool SPLIT = false, bool SWAP = false>
 __global__ void __launch_bounds__(PM_THREADS, 3) paged_decode_mma_kernel(const PagedParams p) {
   constexpr int KSTEPS = D / 16, DT = D / 8, CPR = D / 8, LPT = D / 8;
   constexpr int TILE_BYTES = PM_BN * D * 2;
@@ -61,6 +78,7 @@ __global__ void __launch_bounds__(PM_THREADS, 3) paged_decode_mma_kernel(const P
   __shared__ int sm_last;
 
   static_assert(!SPLIT || (!FUSED && !CLUSTER), "a tile's pair of CTAs merges for itself");
+  static_assert(!SWAP || (!FUSED && !CLUSTER), "the step's own kernels keep their products");
   const int tile = SPLIT ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, kvh = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if ((p.pdl || p.leads) && tid == 0) pdl_launch_dependents();
@@ -109,8 +127,33 @@ __global__ void __launch_bounds__(PM_THREADS, 3) paged_decode_mma_kernel(const P
   const int lrow = lane / CPR, lch = lane % CPR;
   const T *kbase = kc + (int64_t)kvh * p.kv_head_stride + lch * 8, *vbase = vc + (int64_t)kvh * p.kv_head_stride + lch * 8;
   const int psh = p.page_shift;
+  // SWAP: the 16 tokens of a warp's step lie in one page
+  const bool in_page = SWAP && (p.page_size & 15) == 0 && (t_begin & 15) == 0;
   auto load_tile = [&](int it, int buf) {       // cached tokens t_begin + 64 it + 16 warp .. +15 of the chunk
     const int row0 = 16 * warp + lrow, t0 = t_begin + it * PM_BN + row0;
+    if constexpr (SWAP) {
+      if (in_page) {
+        const int tw = t0 - lrow;
+        if (tw >= t_cache_end) {          // nothing: the step's products are not made
+          cp_async_commit();
+          return;
+        }
+        const int pgi = psh >= 0 ? tw >> psh : tw / p.page_size, in = psh >= 0 ? tw & (p.page_size - 1) : tw - pgi * p.page_size;
+        const int64_t goff = (pages_in_smem ? st_pages[pgi - pg0] : pages[pgi]) * p.kv_block_stride + (int64_t)(in + lrow) * D;
+        // (tile_off: rows RPP apart differ in the bits of RPP * i, which the swizzle takes by exclusive or)
+        const uint32_t dk = smem_u32(sk[buf]) + tile_off<D>(row0, lch), dv = smem_u32(sv[buf]) + tile_off<D>(row0, lch);
+        const T *const gk = kbase + goff, *const gv = vbase + goff;
+#pragma unroll
+        for (int i = 0; i < 16 / RPP; i++) {
+          const uint32_t x = (uint32_t)((i * RPP) & 7) << 4, at = (uint32_t)(i * RPP * D * 2);
+          const int sz = t0 + i * RPP < t_cache_end ? 16 : 0;
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((dk ^ x) + at), "l"(gk + i * RPP * D), "r"(sz) : "memory");
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((dv ^ x) + at), "l"(gv + i * RPP * D), "r"(sz) : "memory");
+        }
+        cp_async_commit();
+        return;
+      }
+    }
 #pragma unroll
     for (int i = 0; i < 16 / RPP; i++) {
       const int row = row0 + i * RPP, t = t0 + i * RPP;
@@ -171,6 +214,97 @@ __global__ void __launch_bounds__(PM_THREADS, 3) paged_decode_mma_kernel(const P
   }
   __syncthreads();
 
+  const float scale_log2 = p.sm_scale * 1.4426950408889634f;
+  float *mo = (float *)pm_smem;                    // [PM_WARPS][16][D] f32 (the K/V buffers are free at the end)
+  float *mm = mo + PM_WARPS * 16 * D, *ml = mm + PM_WARPS * 16;
+  if constexpr (SWAP) {
+    // lane: heads h = 2 (lane % 4), + 1 and tokens (sums: dimensions) lane / 4, + 8 of a product
+    uint32_t qb[KSTEPS][2];
+#pragma unroll
+    for (int ks = 0; ks < KSTEPS; ks++) {
+      const uint8_t *at = sq + tile_off<D>(lane >> 2, 2 * ks) + 4 * (lane & 3), *next = sq + tile_off<D>(lane >> 2, 2 * ks + 1) + 4 * (lane & 3);
+      qb[ks][0] = *(const uint32_t *)at;
+      qb[ks][1] = *(const uint32_t *)next;
+    }
+    float oacc[D / 16][4];
+#pragma unroll
+    for (int i = 0; i < D / 16; i++) { oacc[i][0] = oacc[i][1] = oacc[i][2] = oacc[i][3] = 0.f; }
+    float m_ref[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+    const int krow = 16 * warp + (lane & 15), vrow = 16 * warp + (lane & 7) + ((lane >> 4) << 3);
+    for (int it = 0; it < ntiles; it++) {
+      const int buf = it & 1;
+      if (it + 1 < ntiles) load_tile(it + 1, buf ^ 1);
+      else cp_async_commit();
+      cp_async_wait<1>();
+      __syncwarp();                                        // the warp's rows are there
+      const int tw = t_begin + it * PM_BN + 16 * warp;
+      if (tw < t_cache_end) {                              // warp-uniform
+        float s[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};      // (two chains of products)
+#pragma unroll
+        for (int ks = 0; ks < KSTEPS; ks++) {
+          uint32_t a[4];
+          ldsm_x4(smem_u32(sk[buf] + tile_off<D>(krow, 2 * ks + (lane >> 4))), a[0], a[1], a[2], a[3]);
+          mma16816<T>(ks & 1 ? s2 : s, a, qb[ks][0], qb[ks][1]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          s[e] += s2[e];
+          if (p.softcap > 0.f) s[e] = p.softcap * tanhf(s[e] * p.sm_scale / p.softcap) * 1.4426950408889634f;
+          else s[e] *= scale_log2;
+        }
+        if (tw + 16 > t_cache_end) {
+#pragma unroll
+          for (int e = 0; e < 4; e++) if (tw + (lane >> 2) + 8 * (e >> 1) >= t_cache_end) s[e] = -INFINITY;
+        }
+        // (the running maximum itself, not one that lags: its probability is one, exactly, and the largest weights of a tile round least: errors 0.00262 and
+        // 0.00277 of 16 sequences' results; the accumulators are only touched where it has grown)
+        float top[2] = {fmaxf(s[0], s[2]), fmaxf(s[1], s[3])};
+#pragma unroll
+        for (int m = 4; m < 32; m <<= 1) {
+          top[0] = fmaxf(top[0], __shfl_xor_sync(0xffffffffu, top[0], m));
+          top[1] = fmaxf(top[1], __shfl_xor_sync(0xffffffffu, top[1], m));
+        }
+        if (__any_sync(0xffffffffu, top[0] > m_ref[0] || top[1] > m_ref[1])) {
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            top[h] = fmaxf(top[h], m_ref[h]);
+            const float corr = top[h] == -INFINITY ? 1.f : pm_exp2(m_ref[h] - top[h]);
+            m_ref[h] = top[h];
+            l_run[h] *= corr;
+#pragma unroll
+            for (int i = 0; i < D / 16; i++) { oacc[i][h] *= corr; oacc[i][2 + h] *= corr; }
+          }
+        }
+        const float m0 = m_ref[0] == -INFINITY ? 0.f : m_ref[0], m1 = m_ref[1] == -INFINITY ? 0.f : m_ref[1];
+        const float p0 = pm_exp2(s[0] - m0), p1 = pm_exp2(s[1] - m1), p2 = pm_exp2(s[2] - m0), p3 = pm_exp2(s[3] - m1);
+        l_run[0] += p0 + p2;
+        l_run[1] += p1 + p3;
+        const uint32_t b0 = pm_transpose(pack2<T>(p0, p1)), b1 = pm_transpose(pack2<T>(p2, p3));
+#pragma unroll
+        for (int i = 0; i < D / 16; i++) {
+          uint32_t a[4];
+          ldsm_x4_t(smem_u32(sv[buf] + tile_off<D>(vrow, 2 * i + ((lane >> 3) & 1))), a[0], a[1], a[2], a[3]);
+          mma16816<T>(oacc[i], a, b0, b1);
+        }
+      }
+      __syncwarp();                                        // and read: the next copy may overwrite them
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int m = 4; m < 32; m <<= 1) l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], m);
+    __syncthreads();                                 // every warp has left its buffers
+    const int h = 2 * (lane & 3);
+#pragma unroll
+    for (int i = 0; i < D / 16; i++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) mo[((size_t)warp * 16 + h + (e & 1)) * D + 16 * i + (lane >> 2) + 8 * (e >> 1)] = oacc[i][e];
+    if (lane < 4) {
+#pragma unroll
+      for (int e = 0; e < 2; e++) { mm[warp * 16 + h + e] = m_ref[e]; ml[warp * 16 + h + e] = l_run[e]; }
+    }
+  } else {
   uint32_t qa[KSTEPS][4];
 #pragma unroll
   for (int ks = 0; ks < KSTEPS; ks++)
@@ -180,7 +314,6 @@ __global__ void __launch_bounds__(PM_THREADS, 3) paged_decode_mma_kernel(const P
 #pragma unroll
   for (int i = 0; i < DT; i++) { oacc[i][0] = oacc[i][1] = oacc[i][2] = oacc[i][3] = 0.f; }
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-  const float scale_log2 = p.sm_scale * 1.4426950408889634f;
 
   // one warp step over 16 tokens held in rows row0..row0+15 of (kt, vt); token of row j is t_first + j,
   // live when win_lo <= t < t_hi
@@ -269,8 +402,6 @@ __global__ void __launch_bounds__(PM_THREADS, 3) paged_decode_mma_kernel(const P
 
   __syncthreads();                                 // every warp has left its buffers
   // ---- merge the four warp states: rows 0..7 of the m16 tile live in (c0, c1), rows 8..15 in (c2, c3)
-  float *mo = (float *)pm_smem;                    // [PM_WARPS][16][D] f32 (the K/V buffers are free now)
-  float *mm = mo + PM_WARPS * 16 * D, *ml = mm + PM_WARPS * 16;
   {
     const int r0 = lane >> 2;
 #pragma unroll
@@ -283,6 +414,7 @@ __global__ void __launch_bounds__(PM_THREADS, 3) paged_decode_mma_kernel(const P
       mm[warp * 16 + r0] = m_run[0]; mm[warp * 16 + r0 + 8] = m_run[1];
       ml[warp * 16 + r0] = l_run[0]; ml[warp * 16 + r0 + 8] = l_run[1];
     }
+  }
   }
   __syncthreads();
   uint32_t crank = 0;
