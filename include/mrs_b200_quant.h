@@ -101,6 +101,10 @@ void mrs_mmq_set_weight_format(int32_t fmt);
 void mrs_mmq_set_path(int32_t path);
 int32_t mrs_mmq_gguf_ts(int32_t ggml_type, const void *w, const void *x, void *y, int32_t M, int32_t N, int32_t K,
                         int32_t dtype, void *stream);
+/* y_i = x . w_i^T for two or three matrices (n2 = 0: two) of a type and as many columns, as one launch of the first kernel (Q4_K, Q5_K, Q6_K, Q8_0, all
+ * pointers on 16-byte boundaries); cudaErrorNotSupported (801), and nothing launched, where it does not fit. */
+int32_t mrs_mmq_gguf_multi(int32_t ggml_type, const void *w0, const void *w1, const void *w2, const void *x, void *y0, void *y1, void *y2,
+                           int32_t M, int32_t n0, int32_t n1, int32_t n2, int32_t K, int32_t dtype, void *stream);
 int32_t mrs_mmq_timeouts(void);
 int32_t *mrs_mmq_timeout_flag(void);
 

@@ -487,6 +487,7 @@ static int tc_row_bytes(int type, int K) {
 // dtype 0 = f16, 1 = bf16.  K must be a multiple of 64 (and of the type's block size).
 static int g_tc_b_fmt = -1;  // -1: same 16-bit format as the activations; 0 force f16; 1 force bf16
 extern "C" void mrs_mmq_set_weight_format(int32_t fmt) { g_tc_b_fmt = fmt; }
+namespace mrs { bool mmq_format_is_forced() { return g_tc_b_fmt >= 0; } }
 
 extern "C" int32_t mrs_mmq_gguf_ts(int32_t ggml_type, const void *w, const void *x, void *y, int32_t M, int32_t N, int32_t K,
                                    int32_t dtype, void *stream);   // mmq_ts.cu

@@ -95,7 +95,7 @@ TsPlan ts_plan(int M, int N, int K, int span_bytes, int dequant_clocks, int spli
       if (span < stream) span = stream;
       const double each = ((spans + ks - 1) / ks) * span;
       const double cost = ks > 1 ? waves * (START + each + SPLIT_END + 8.0 * nt) : START + waves * (each + TILE_END) + 8.0 * nt;
-      if (cost < best_cost) { best_cost = cost; best = {nt, tm, ks}; }
+      if (cost < best_cost) { best_cost = cost; best = {nt, tm, ks, (int)waves, cost}; }
     }
   }
   return best;
@@ -135,10 +135,55 @@ extern "C" int32_t mrs_mmq_gguf_ts(int32_t ggml_type, const void *w, const void 
   // the dequantisers' weight in the plan's estimate
   const int clocks = ggml_type == MRS_Q6_K ? 1500 : ggml_type == MRS_Q5_K || ggml_type == MRS_Q3_K || ggml_type == MRS_Q5_0 || ggml_type == MRS_Q5_1 ? 1350 : 1150;
   const TsPlan plan = ts_plan(M, N, K, bytes * (256 / elems), clocks, TS_SPLIT_MIN_ROWS, d);
-  const TsCall c = {w, x, y, M, N, K, K / elems * bytes, dtype, plan.nt, plan.tiles_m, plan.ksplit, d.sms, d.timeouts, (cudaStream_t)stream, nullptr, nullptr, 0, 0, 0};
+  const TsCall c = {w, x, y, M, N, K, K / elems * bytes, dtype, plan.nt, plan.tiles_m, plan.ksplit, d.sms, d.timeouts, (cudaStream_t)stream, nullptr, nullptr, 0, 0, 0, 1, {}, {}, {}};
   switch (ggml_type) {
 #define MRS_TS_CASE(T) case T: return (int32_t)ts_launch<T>(c);
   MRS_TS_TYPES(MRS_TS_CASE)
+  default: return (int32_t)cudaErrorNotSupported;
+  }
+}
+
+namespace mrs { bool mmq_format_is_forced(); }      // mmq_tc.cu
+
+// y_i = x . w_i^T for two or three matrices of a type and as many columns (n2 = 0: two), as one launch.  cudaErrorNotSupported, and nothing launched,
+// where that does not fit this kernel: the caller launches them one by one.
+extern "C" int32_t mrs_mmq_gguf_multi(int32_t ggml_type, const void *w0, const void *w1, const void *w2, const void *x, void *y0, void *y1, void *y2, int32_t M,
+                                      int32_t n0, int32_t n1, int32_t n2, int32_t K, int32_t dtype, void *stream) {
+  if (g_mmq_path == 1 || mmq_format_is_forced()) return (int32_t)cudaErrorNotSupported;
+  const int elems = blk_elems(ggml_type), bytes = blk_bytes(ggml_type);
+  if (bytes == 0 || M <= 0 || n0 <= 0 || n1 <= 0 || n2 < 0 || K <= 0 || K % elems != 0 || K % 64 != 0 || (K / elems * bytes) % 16 != 0 || (dtype != 0 && dtype != 1))
+    return (int32_t)cudaErrorNotSupported;
+  const void *const ptrs[] = {w0, w1, n2 > 0 ? w2 : w1, x, y0, y1, n2 > 0 ? y2 : y1};
+  for (const void *q : ptrs) if (q == nullptr || ((uintptr_t)q & 15)) return (int32_t)cudaErrorNotSupported;
+  if ((int64_t)n0 + n1 + n2 > 0x7fffff00) return (int32_t)cudaErrorNotSupported;
+  const TsDevice &d = ts_device();
+  const cudaError_t refused = ts_refused(d);
+  if (refused != cudaSuccess) return (int32_t)refused;
+  const int clocks = ggml_type == MRS_Q6_K ? 1500 : ggml_type == MRS_Q5_K ? 1350 : 1150, pad = TS_BM - 1;
+  const int rows = (n0 + pad) / TS_BM * TS_BM + (n1 + pad) / TS_BM * TS_BM + (n2 + pad) / TS_BM * TS_BM;
+  const bool split = n0 >= TS_SPLIT_MIN_ROWS && n1 >= TS_SPLIT_MIN_ROWS && (n2 == 0 || n2 >= TS_SPLIT_MIN_ROWS);      // (as each alone)
+  const TsPlan plan = ts_plan(M, rows, K, bytes * (256 / elems), clocks, split ? TS_SPLIT_MIN_ROWS : 0x7fffffff, d);
+  // Where one launch is worth it, by the plan's estimate: it saves a start and a drain a matrix, and waves where matrices leave SMs idle.  For many tokens only
+  // saved waves count: a wave that fills the GPU takes a tenth longer than one that does not.  One B200, us alone / together: Q4_K 4096 + 1024 + 1024 of 4096 at
+  // 24, 300, 1000 tokens 23.5 / 12.2, 43.1 / 19.2, 63.2 / 39.1; 2 x 14336 at 24, 200 tokens 34.5 / 30.7, 46.1 / 42.7, and with Q8_0 at 300, 1000 (left alone)
+  // 78.5 / 81.1, 195 / 213; Q6_K 2 x 14336 at 512 (alone) 112 / 130; 3 x 4096 at 1000 (alone) 90 / 101; 2 x 5632 of 2048 at 1000 60.2 / 45.8.
+  double alone = 0.0;
+  int waves = 0;
+  const int each[] = {n0, n1, n2};
+  for (int n : each) {
+    if (n == 0) continue;
+    const TsPlan one = ts_plan(M, n, K, bytes * (256 / elems), clocks, TS_SPLIT_MIN_ROWS, d);
+    alone += one.cost;
+    waves += one.waves;
+  }
+  if (plan.cost > 0.92 * alone || (M > 320 && plan.waves >= waves)) return (int32_t)cudaErrorNotSupported;
+  const TsCall c = {w0, x, y0, M, n0, K, K / elems * bytes, dtype, plan.nt, plan.tiles_m, plan.ksplit, d.sms, d.timeouts, (cudaStream_t)stream, nullptr, nullptr, 0, 0, 0,
+                    n2 > 0 ? 3 : 2, {w1, w2}, {y1, y2}, {n1, n2}};
+  switch (ggml_type) {
+  case MRS_Q4_K: return (int32_t)ts_launch<MRS_Q4_K>(c);
+  case MRS_Q5_K: return (int32_t)ts_launch<MRS_Q5_K>(c);
+  case MRS_Q6_K: return (int32_t)ts_launch<MRS_Q6_K>(c);
+  case MRS_Q8_0: return (int32_t)ts_launch<MRS_Q8_0>(c);
   default: return (int32_t)cudaErrorNotSupported;
   }
 }

@@ -530,9 +530,25 @@ __device__ __forceinline__ bool ts_issue_span(uint32_t acc, uint32_t a, uint32_t
   return true;
 }
 
-template <int TYPE, bool ALIGNED, bool BF>
-__global__ void __launch_bounds__(TS_THREADS, 1)
-mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const TsParams p) {
+// Up to three matrices of a type that read the same activations, as one grid: their row tiles follow one another (p.N, p.y and the map of the launch are the
+// first one's).  Alone each pays for its start, its drain and its last wave: q, k and v of an 8B model (Q4_K, 4096 + 1024 + 1024 rows) at 300 tokens.
+struct TsMore {
+  CUtensorMap w[2];
+  void *y[2];
+  int n[2], first[2];                    // rows, and the first row tile, of the second and the third matrix
+};
+
+// of row `r` of row tile tn: the row in its matrix, the matrix's rows and results
+__device__ __forceinline__ void ts_place(const TsMore *more, int tn, int r, int &nrow, int &N, void *&out) {
+  if (tn < more->first[0]) return;
+  const int k = tn >= more->first[1] ? 1 : 0;
+  nrow = (tn - more->first[k]) * TS_BM + r;
+  N = more->n[k];
+  out = more->y[k];
+}
+
+template <int TYPE, bool ALIGNED, bool BF, bool MULTI>
+__device__ __forceinline__ void ts_grid(const CUtensorMap &tmap_w, const CUtensorMap &tmap_x, const TsParams &p, const TsMore *more) {
   using F = TsFmt<TYPE>;
   constexpr int PITCH = TsPitch<TYPE, ALIGNED>::value, RAW_BYTES = TsStage<TYPE, ALIGNED>::BYTES;
   constexpr int LOADERS = ALIGNED ? 1 : 64;           // arrivals that fill a raw stage
@@ -587,7 +603,12 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
     int it = 0, st = 0, ph = 0;
     bool ok = true;
     for (int t = first; ok && t < n_tiles; t += step) {
-      const int n0 = (t % p.tiles_n) * TS_BM;
+      int n0 = (t % p.tiles_n) * TS_BM;
+      const CUtensorMap *map = &tmap_w;
+      if constexpr (MULTI) {
+        const int tn = t % p.tiles_n, k = tn >= more->first[1] ? 1 : 0;
+        if (tn >= more->first[0]) { n0 = (tn - more->first[k]) * TS_BM; map = &more->w[k]; }
+      }
       for (int s = s0; s < s1; s++, it++) {
         if (p.pdl && it == RS) pdl_wait();             // the ring is full: from here on its stages are freed at the grid before's pace
         ok = ts_wait(raw_empty + st, ph ^ 1, late);
@@ -607,7 +628,7 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
         } else if constexpr (ALIGNED) {
           // (a box starts on a 16-byte boundary: the aligned address below the span; the dequantisers read from the phase on)
           mbar_arrive_expect_tx_warp(raw_full + st, RAW_BYTES);
-          tma_load_2d_warp(r_ring + (size_t)st * RAW_BYTES, &tmap_w, ((s * F::SPAN) & ~15) / 2, n0, raw_full + st);
+          tma_load_2d_warp(r_ring + (size_t)st * RAW_BYTES, map, ((s * F::SPAN) & ~15) / 2, n0, raw_full + st);
         } else {
           constexpr int CH = (F::SPAN + 14 + 15) / 16;                     // 16-byte chunks that cover a span at any phase
           const uint32_t dst = smem_u32(r_ring) + (uint32_t)st * RAW_BYTES;
@@ -763,7 +784,10 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
     if (p.pdl) pdl_wait();                   // y may still be read by the grid before
     int j = 0;
     for (int t = first; t < n_tiles; t += step, j++) {
-      const int b = j % n_acc, m0 = (t / p.tiles_n) * p.nt, nrow = (t % p.tiles_n) * TS_BM + q4 * 32 + lane;
+      const int b = j % n_acc, m0 = (t / p.tiles_n) * p.nt;
+      int nrow = (t % p.tiles_n) * TS_BM + q4 * 32 + lane, N = p.N;
+      void *out = p.y;
+      if constexpr (MULTI) ts_place(more, t % p.tiles_n, q4 * 32 + lane, nrow, N, out);
       if (!ts_wait(acc_full + b, (j / n_acc) & 1, late)) break;
       tc_fence_after();
       const int cols = min(p.nt, p.M - m0);
@@ -776,8 +800,8 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
           __syncwarp();
           if (lane == 0) mbar_arrive(acc_empty + b);
         }
-        if (nrow < p.N) {
-          uint16_t *y = (uint16_t *)p.y + (size_t)(m0 + c0) * p.N + nrow;
+        if (nrow < N) {
+          uint16_t *y = (uint16_t *)out + (size_t)(m0 + c0) * N + nrow;
 #pragma unroll
           for (int c = 0; c < 32; c++) {
             if (c0 + c < cols) {
@@ -785,7 +809,7 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
               if constexpr (BF) *(__nv_bfloat16 *)y = __float2bfloat16_rn(v);
               else *(__half *)y = __float2half_rn(v);
             }
-            y += p.N;
+            y += N;
           }
         }
       }
@@ -819,21 +843,34 @@ mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
       }
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    const int m0 = (first / p.tiles_n) * p.nt + rank * C, nrow = (first % p.tiles_n) * TS_BM + row;
-    if (warp >= 4 && ok && nrow < p.N) {
+    const int m0 = (first / p.tiles_n) * p.nt + rank * C;
+    int nrow = (first % p.tiles_n) * TS_BM + row, N = p.N;
+    void *out = p.y;
+    if constexpr (MULTI) ts_place(more, first % p.tiles_n, row, nrow, N, out);
+    if (warp >= 4 && ok && nrow < N) {
       const int cols = min(min(C, p.nt - rank * C), p.M - m0);
       for (int c = g; c < cols; c += G) {
         float v = red[(size_t)c * TS_BM + row];
         for (int s = 1; s < p.ksplit; s++) v += red[((size_t)s * C + c) * TS_BM + row];
-        const size_t at = (size_t)(m0 + c) * p.N + nrow;
-        if constexpr (BF) ((__nv_bfloat16 *)p.y)[at] = __float2bfloat16_rn(v);
-        else ((__half *)p.y)[at] = __float2half_rn(v);
+        const size_t at = (size_t)(m0 + c) * N + nrow;
+        if constexpr (BF) ((__nv_bfloat16 *)out)[at] = __float2bfloat16_rn(v);
+        else ((__half *)out)[at] = __float2half_rn(v);
       }
     }
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem_base, 512);
+}
+template <int TYPE, bool ALIGNED, bool BF>
+__global__ void __launch_bounds__(TS_THREADS, 1)
+mmq_ts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const TsParams p) {
+  ts_grid<TYPE, ALIGNED, BF, false>(tmap_w, tmap_x, p, nullptr);
+}
+template <int TYPE, bool BF>
+__global__ void __launch_bounds__(TS_THREADS, 1)
+mmq_ts_multi_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const TsParams p, const __grid_constant__ TsMore more) {
+  ts_grid<TYPE, true, BF, true>(tmap_w, tmap_x, p, &more);
 }
 
 // ---- host ---------------------------------------------------------------------------------------
@@ -846,23 +883,30 @@ struct TsCall {
   cudaStream_t stream;
   const void *scales, *qzeros;        // int4
   int group, scale_perm, pdl;
+  int matrices;                       // more than one: w, y and N are the first's
+  const void *w2[2];
+  void *y2[2];
+  int n2[2];
 };
 
+template <int TYPE> static bool ts_map_weights(CUtensorMap *map, const void *w, int N, int row_bytes) {
+  const cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / 2), (cuuint64_t)N};
+  const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
+  const cuuint32_t box[2] = {(cuuint32_t)(TsPitch<TYPE, true>::value / 2), (cuuint32_t)TS_BM};
+  const cuuint32_t estr[2] = {1, 1};
+  return tc_get_encode()(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 template <int TYPE, bool ALIGNED> static cudaError_t ts_launch_as(const TsCall &c) {
-  using F = TsFmt<TYPE>;
-  constexpr int PITCH = TsPitch<TYPE, ALIGNED>::value, RAW_BYTES = TsStage<TYPE, ALIGNED>::BYTES;
-  PFN_encodeTiled enc = tc_get_encode();
-  if (enc == nullptr) return cudaErrorNotSupported;
+  constexpr int RAW_BYTES = TsStage<TYPE, ALIGNED>::BYTES;
+  // types that files hold side by side: q, k and v, gate and up
+  constexpr bool GROUPS = ALIGNED && (TYPE == MRS_Q4_K || TYPE == MRS_Q5_K || TYPE == MRS_Q6_K || TYPE == MRS_Q8_0);
+  if (c.matrices > 1 && !GROUPS) return cudaErrorNotSupported;
+  if (tc_get_encode() == nullptr) return cudaErrorNotSupported;
   CUtensorMap tw, tx;
   if (!tc_make_map_2d(&tx, c.x, (uint64_t)c.M, (uint64_t)c.K, TS_XK, (uint32_t)c.nt, c.dtype)) return cudaErrorInvalidValue;
   if (ALIGNED && !ts_is_int4(TYPE)) {
-    const cuuint64_t dims[2] = {(cuuint64_t)(c.row_bytes / 2), (cuuint64_t)c.N};
-    const cuuint64_t strides[1] = {(cuuint64_t)c.row_bytes};
-    const cuuint32_t box[2] = {(cuuint32_t)(PITCH / 2), (cuuint32_t)TS_BM};
-    const cuuint32_t estr[2] = {1, 1};
-    if (enc(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(c.w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return cudaErrorInvalidValue;
+    if (!ts_map_weights<TYPE>(&tw, c.w, c.N, c.row_bytes)) return cudaErrorInvalidValue;
   } else {
     tw = tx;                          // not read
   }
@@ -884,9 +928,20 @@ template <int TYPE, bool ALIGNED> static cudaError_t ts_launch_as(const TsCall &
   if (p.xb == 4 && p.xs > 4) p.xs = 4;
   p.rs = (BUDGET - p.xs * stage) / RAW_BYTES;
   if (p.rs > TS_RS_MAX) p.rs = TS_RS_MAX;
+  TsMore more;
+  if (c.matrices > 1) {
+    for (int i = 0; i < 2; i++) {
+      const bool there = i + 1 < c.matrices;
+      if (there && !ts_map_weights<TYPE>(&more.w[i], c.w2[i], c.n2[i], c.row_bytes)) return cudaErrorInvalidValue;
+      more.first[i] = there ? p.tiles_n : 1 << 30;
+      more.n[i] = there ? c.n2[i] : 0;
+      more.y[i] = there ? c.y2[i] : nullptr;
+      if (!there) more.w[i] = tx;     // not read
+      if (there) p.tiles_n += (c.n2[i] + TS_BM - 1) / TS_BM;
+    }
+  }
   const int tiles = p.tiles_m * p.tiles_n;
   auto kern = c.dtype == 1 ? mmq_ts_kernel<TYPE, ALIGNED, true> : mmq_ts_kernel<TYPE, ALIGNED, false>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM_MAX);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = p.ksplit > 1 ? dim3(p.ksplit, tiles) : dim3(1, tiles < c.sms ? tiles : c.sms);
   cfg.blockDim = dim3(TS_THREADS);
@@ -906,6 +961,14 @@ template <int TYPE, bool ALIGNED> static cudaError_t ts_launch_as(const TsCall &
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
+  if constexpr (GROUPS) {
+    if (c.matrices > 1) {
+      auto multi = c.dtype == 1 ? mmq_ts_multi_kernel<TYPE, true> : mmq_ts_multi_kernel<TYPE, false>;
+      cudaFuncSetAttribute(multi, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM_MAX);
+      return cudaLaunchKernelEx(&cfg, multi, tw, tx, p, more);
+    }
+  }
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TS_SMEM_MAX);
   return cudaLaunchKernelEx(&cfg, kern, tw, tx, p);
 }
 
@@ -921,7 +984,7 @@ struct TsDevice { int sms, clusters[9]; int *timeouts; int32_t *flag; };   // th
 const TsDevice &ts_device();
 // cudaErrorLaunchTimeout once a wait has run out on the device, cudaErrorNotSupported when there is no word to report it in
 cudaError_t ts_refused(const TsDevice &d);
-struct TsPlan { int nt, tiles_m, ksplit; };
+struct TsPlan { int nt, tiles_m, ksplit, waves; double cost; };
 TsPlan ts_plan(int M, int N, int K, int span_bytes, int dequant_clocks, int split_min_rows, const TsDevice &d);
 
 // clusters of n CTAs of this kernel that the device holds at once, n = 2 .. 8 (every type's kernel takes a whole SM)

@@ -12,8 +12,7 @@ from .quant import _I, _P, raw_stream, typed
 _DT_CODE = {torch.float16: 0, torch.bfloat16: 1}
 
 
-def forward(w, xs: torch.Tensor) -> torch.Tensor:
-    """w: quant.QTensor [N, K]; xs [..., K] bf16/f16 -> [..., N]."""
+def _check(w, xs):
     if xs.dtype not in _DT_CODE:
         raise ValueError(f"fast_mmq: input dtype must be BF16 or F16, got {xs.dtype}")
     nrows, ncols = w.shape
@@ -23,6 +22,12 @@ def forward(w, xs: torch.Tensor) -> torch.Tensor:
         raise ValueError("fast_mmq: input and weight are on different devices")
     if ncols % 64:
         raise ValueError("fast_mmq: K must be a multiple of 64")
+    return nrows, ncols
+
+
+def forward(w, xs: torch.Tensor) -> torch.Tensor:
+    """w: quant.QTensor [N, K]; xs [..., K] bf16/f16 -> [..., N]."""
+    nrows, ncols = _check(w, xs)
     xs = xs.contiguous()
     M = xs.numel() // ncols
     out = xs.new_empty((*xs.shape[:-1], nrows))
@@ -30,6 +35,38 @@ def forward(w, xs: torch.Tensor) -> torch.Tensor:
     rc = entry(GGML[w.dtype], w.data.data_ptr(), xs.data_ptr(), out.data_ptr(), M, nrows, ncols, _DT_CODE[xs.dtype], raw_stream(xs.device))
     if rc != 0:
         raise RuntimeError(f"mrs_mmq_gguf failed with cudaError {rc}")
+    return out
+
+
+_NOT_SUPPORTED = 801        # cudaErrorNotSupported: nothing was launched, alone is faster or what is possible
+
+
+def forward_many(ws, xs: torch.Tensor):
+    """[forward(w, xs) for w in ws], neighbours of one type as one launch (up to three) where that is faster."""
+    for w in ws:
+        _check(w, xs)
+    xs = xs.contiguous()
+    out, i = [], 0
+    while i < len(ws):
+        n = 1
+        while n < 3 and i + n < len(ws) and ws[i + n].dtype == ws[i].dtype:
+            n += 1
+        group = ws[i:i + n]
+        i += n
+        M = xs.numel() // xs.shape[-1]
+        if n > 1 and M > 0:
+            ys = [xs.new_empty((*xs.shape[:-1], w.shape[0])) for w in group]
+            data, rows, to = [w.data.data_ptr() for w in group], [w.shape[0] for w in group], [y.data_ptr() for y in ys]
+            if n == 2:
+                data.append(None), rows.append(0), to.append(None)
+            entry = typed("mrs_mmq_gguf_multi", _I, *[_P] * 7, *[_I] * 6, _P)
+            rc = entry(GGML[group[0].dtype], *data, xs.data_ptr(), *to, M, *rows, xs.shape[-1], _DT_CODE[xs.dtype], raw_stream(xs.device))
+            if rc == 0:
+                out += ys
+                continue
+            if rc != _NOT_SUPPORTED:
+                raise RuntimeError(f"mrs_mmq_gguf_multi failed with cudaError {rc}")
+        out += [forward(w, xs) for w in group]
     return out
 
 
@@ -65,14 +102,14 @@ def plain(w, xs: torch.Tensor) -> torch.Tensor:
 
 
 def fused_qkv(q_w, k_w, v_w, xs: torch.Tensor):
-    return forward(q_w, xs), forward(k_w, xs), forward(v_w, xs)
+    return tuple(forward_many([q_w, k_w, v_w], xs))
 
 
 def fused_glu(gate_w, up_w, xs: torch.Tensor, activation) -> torch.Tensor:
     if tuple(gate_w.shape) != tuple(up_w.shape):
         raise ValueError(f"fast_mmq fused_glu: gate/up shape mismatch {tuple(gate_w.shape)} vs {tuple(up_w.shape)}")
     from . import ops
-    return ops.fused_glu(forward(gate_w, xs), forward(up_w, xs), activation)
+    return ops.fused_glu(*forward_many([gate_w, up_w], xs), activation)
 
 
 def fused_ffn(gate_w, up_w, down_w, xs: torch.Tensor, activation) -> torch.Tensor:

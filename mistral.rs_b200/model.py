@@ -721,16 +721,13 @@ class LlamaPrefill:
         scale = 1.0 / float(np.sqrt(D))
         h = ops.rms_norm(x, w.layers[0]["attn_norm"], cfg.rms_eps)
         for l, L in enumerate(w.layers):
-            q = mmq.forward(qt(L["attn_q"]), h).view(T, H, D)
-            k = mmq.forward(qt(L["attn_k"]), h).view(T, KVH, D)
-            v = mmq.forward(qt(L["attn_v"]), h).view(T, KVH, D)
+            q, k, v = (t.view(T, -1, D) for t in mmq.forward_many([qt(L[n]) for n in ("attn_q", "attn_k", "attn_v")], h))
             ops.apply_rotary_qk(q, k, w.rope_cos, w.rope_sin, None, is_neox=cfg.rope_neox)
             attn = paged_attn.prefill_attention(q, k, v, scale)
             paged_attn.reshape_and_cache_flashinfer(k, v, self.k_cache[l], self.v_cache[l], slots)
             o = mmq.forward(qt(L["attn_output"]), attn.view(T, H * D))
             x, h2 = ops.add_rms_norm(o, x, L["ffn_norm"], cfg.rms_eps)       # x = o + x ; h2 = norm(x)
-            gate = mmq.forward(qt(L["ffn_gate"]), h2)
-            up = mmq.forward(qt(L["ffn_up"]), h2)
+            gate, up = mmq.forward_many([qt(L["ffn_gate"]), qt(L["ffn_up"])], h2)
             d = mmq.forward(qt(L["ffn_down"]), ops.fused_glu(gate, up, 0))
             nxt = w.layers[l + 1]["attn_norm"] if l + 1 < cfg.n_layers else w.output_norm
             x, h = ops.add_rms_norm(d, x, nxt, cfg.rms_eps)                   # x = d + x ; h = next norm(x)

@@ -43,6 +43,7 @@ extern "C" {
     pub fn mrs_mmq_set_weight_format(fmt: i32);
     pub fn mrs_mmq_set_path(path: i32);
     pub fn mrs_mmq_gguf_ts(ggml_type: i32, w: *const c_void, x: *const c_void, y: *mut c_void, M: i32, N: i32, K: i32, dtype: i32, stream: *mut c_void) -> i32;
+    pub fn mrs_mmq_gguf_multi(ggml_type: i32, w0: *const c_void, w1: *const c_void, w2: *const c_void, x: *const c_void, y0: *mut c_void, y1: *mut c_void, y2: *mut c_void, M: i32, n0: i32, n1: i32, n2: i32, K: i32, dtype: i32, stream: *mut c_void) -> i32;
     pub fn mrs_mmq_timeouts() -> i32;
     pub fn mrs_mmq_timeout_flag() -> *mut i32;
     pub fn mrs_gptq_gemm(x: *const c_void, qweight: *const i32, scales: *const c_void, qzeros: *const i32, g_idx: *const i32, y: *mut c_void, M: i32, K: i32, N: i32, group_size: i32, is_awq: i32, stream: *mut c_void) -> i32;
