@@ -43,6 +43,8 @@ _NOT_SUPPORTED = 801        # cudaErrorNotSupported: nothing was launched, alone
 
 def forward_many(ws, xs: torch.Tensor):
     """[forward(w, xs) for w in ws], neighbours of one type as one launch (up to three) where that is faster."""
+    if not xs.is_cuda:                     # (refused there)
+        return [forward(w, xs) for w in ws]
     for w in ws:
         _check(w, xs)
     xs = xs.contiguous()
