@@ -534,6 +534,10 @@ int mrs_seq_moe_gather(const void *x, int dtype, const int32_t *order, int n_pai
 int mrs_seq_moe_gemm(const void *sorted, const void *weights, const int32_t *counts, int n_rows, int n_ffn, int n, int k, int gated,
                      const mrs_seq_glu_rule *rule, void *out, int64_t stream);
 int mrs_seq_moe_gemm_fits(int dtype, int n, int k, int n_ffn);
+/* Both products of the experts: hidden [n_rows, ff] = the first with up [n_ffn, gated ? 2 * ff : ff, width], out [n_rows, width] = hidden by
+ * down [n_ffn, width, ff]; the same results as two calls.  The second launch reads counts and begins on down while the first one runs. */
+int mrs_seq_moe_products(const void *sorted, const void *up, const void *down, const int32_t *counts, int n_rows, int n_ffn, int width, int ff,
+                         int gated, const mrs_seq_glu_rule *rule, void *hidden, void *out, int64_t stream);
 int mrs_seq_moe_gemm_timeouts(void);
 int mrs_seq_moe_combine(const void *sorted_y, int dtype, const int32_t *order, const float *weights, int n_tok, int top,
                         int width, int32_t *scratch_inverse, void *out, int64_t stream);

@@ -132,6 +132,8 @@ __global__ void moe_route_kernel(const mrs_seq_moe_route_args a) {
   extern __shared__ float sm[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int t = blockIdx.x * nw + wib;
+  wait_for_previous();
+  let_next_start();
   if (t >= a.n_tok) return;
   float *score = sm + (size_t)wib * (2 * a.n_experts + a.n_groups), *choice = score + a.n_experts, *gscore = choice + a.n_experts;
   route_token(a.logits + (int64_t)t * (a.logits_ld > 0 ? a.logits_ld : a.n_experts), a, score, choice, gscore, lane, a.experts + (int64_t)t * a.top, a.weights + (int64_t)t * a.top);
@@ -141,6 +143,7 @@ __global__ void moe_route_kernel(const mrs_seq_moe_route_args a) {
 template <typename T, int VEC>
 __global__ void __launch_bounds__(128) router_logits_kernel(const T *__restrict__ x, const float *__restrict__ w, int width, int n_experts, float *__restrict__ logits) {
   __shared__ float red[33];
+  let_next_start();
   const float *wr = w + (int64_t)blockIdx.x * width;
   const T *xr = x + (int64_t)blockIdx.y * width;
   float s = 0.0f;
@@ -189,6 +192,8 @@ __global__ void moe_route_top_softmax_kernel(const float *__restrict__ logits, i
   extern __shared__ float sm[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int t = blockIdx.x * nw + wib;
+  wait_for_previous();
+  let_next_start();
   if (t >= n_tok) return;
   float *z = sm + (size_t)wib * n_experts;
   for (int e = lane; e < n_experts; e += 32) z[e] = logits[(int64_t)t * n_experts + e];
@@ -424,12 +429,14 @@ __global__ void moe_inverse_kernel(const int32_t *__restrict__ order, int n_pair
 // The three above for few pairs, in one launch: CTA i finds pair i's row (pairs of lower experts, and earlier ones of its own) by looking at
 // all pairs, copies its token there, and counts the pairs of expert i.  Bound by the launch: 128 pairs of 2048 columns took 6.5 us in three
 // launches (sort 1.9, gather 2.3, inverse 2.3) and as many calls from the host
-// (32 tokens to 4 of 16 experts, the whole layer: 107.3 us so, 100.5 now).  Each CTA reads all pairs: MOE_PLACE_PAIRS is the line.
+// (32 tokens to 4 of 16 experts, the whole layer: 107.3 us so, 100.5 with the one).  Each CTA reads all pairs: MOE_PLACE_PAIRS is the line.
 constexpr int MOE_PLACE_PAIRS = 2048;
 template <typename U>
 __global__ void __launch_bounds__(128) moe_place_kernel(const int32_t *__restrict__ experts, int n_pairs, int n_experts, const U *__restrict__ x, int top,
                                                         int width, int32_t *__restrict__ counts, int32_t *__restrict__ inverse, U *__restrict__ sorted) {
   __shared__ int32_t red[2][4];
+  wait_for_previous();
+  let_next_start();
   const int i = blockIdx.x, own = i < n_pairs ? experts[i] : 0;
   int before = 0, mine = 0;
   for (int j = threadIdx.x; j < n_pairs; j += 128) {
@@ -456,6 +463,7 @@ template <typename T, int VEC>
 __global__ void moe_combine_kernel(const T *__restrict__ sorted_y, const int32_t *__restrict__ inverse, const float *__restrict__ weights,
                                    const int32_t *__restrict__ experts, const T *__restrict__ x, int n_ffn, int top, int width,
                                    T *__restrict__ out) {
+  wait_for_previous();
   const int t = blockIdx.x;
   for (int c = threadIdx.x * VEC; c < width; c += blockDim.x * VEC) {
     float acc[VEC];
@@ -524,8 +532,7 @@ extern "C" int mrs_seq_moe_route_general(const mrs_seq_moe_route_args *args, int
   if (!route_args_ok(a)) return -2;
   const int warps = 4;
   const size_t bytes = (size_t)warps * (2 * n_experts + n_groups) * sizeof(float);
-  moe_route_kernel<<<(n_tok + warps - 1) / warps, warps * 32, bytes, (cudaStream_t)stream>>>(a);
-  return launch_status();
+  return launch_after(moe_route_kernel, (n_tok + warps - 1) / warps, warps * 32, bytes, (cudaStream_t)stream, a);
 }
 
 extern "C" int mrs_seq_moe_route_top_softmax(const float *logits, int n_tok, int n_experts, int top, int32_t *experts, float *weights,
@@ -533,9 +540,8 @@ extern "C" int mrs_seq_moe_route_top_softmax(const float *logits, int n_tok, int
   if (n_tok <= 0) return 0;
   if (n_experts < 1 || n_experts > ROUTE_MAX_EXPERTS || top < 1 || top > n_experts) return -2;
   const int warps = 4;
-  moe_route_top_softmax_kernel<<<(n_tok + warps - 1) / warps, warps * 32, (size_t)warps * n_experts * sizeof(float), (cudaStream_t)stream>>>(
-      logits, n_tok, n_experts, top, experts, weights);
-  return launch_status();
+  return launch_after(moe_route_top_softmax_kernel, (n_tok + warps - 1) / warps, warps * 32, (size_t)warps * n_experts * sizeof(float),
+                      (cudaStream_t)stream, logits, n_tok, n_experts, top, experts, weights);
 }
 
 extern "C" int mrs_seq_moe_up(const void *x, const void *up, int dtype, const int32_t *experts, int n_tok, int top, int width, int ff,
@@ -633,12 +639,12 @@ extern "C" int mrs_seq_moe_place(const int32_t *experts, int n_pairs, int n_expe
   const int grid = n_pairs > n_experts ? n_pairs : n_experts;
   const int64_t row_bytes = (int64_t)width * (dtype == MRS_SEQ_BF16 ? 2 : 4);
   if (row_bytes % 16 == 0 && (((uintptr_t)x | (uintptr_t)sorted) & 15) == 0) {
-    moe_place_kernel<uint4><<<grid, 128, 0, (cudaStream_t)stream>>>(experts, n_pairs, n_experts, (const uint4 *)x, top, (int)(row_bytes / 16), counts,
-                                                                    inverse, (uint4 *)sorted);
-    return launch_status();
+    return launch_after(moe_place_kernel<uint4>, grid, 128, 0, (cudaStream_t)stream, experts, n_pairs, n_experts, (const uint4 *)x, top,
+                             (int)(row_bytes / 16), counts, inverse, (uint4 *)sorted);
   }
   SEQ_DISPATCH_DTYPE(dtype, {
-    moe_place_kernel<T><<<grid, 128, 0, (cudaStream_t)stream>>>(experts, n_pairs, n_experts, (const T *)x, top, width, counts, inverse, (T *)sorted);
+    return launch_after(moe_place_kernel<T>, grid, 128, 0, (cudaStream_t)stream, experts, n_pairs, n_experts, (const T *)x, top, width, counts,
+                             inverse, (T *)sorted);
   });
   return launch_status();
 }
@@ -707,9 +713,9 @@ extern "C" int mrs_seq_moe_combine_at(const void *sorted_y, int dtype, const int
   if (experts && !x) return -2;
   const bool vec = width % 4 == 0 && (((uintptr_t)sorted_y | (uintptr_t)x | (uintptr_t)out) & 15) == 0;
   const int th = width >= 1024 ? 256 : 128;
-#define SEQ_COMBINE(V)                                                                                                            \
-  moe_combine_kernel<T, V><<<n_tok, th, 0, (cudaStream_t)stream>>>((const T *)sorted_y, inverse, weights, experts, (const T *)x,  \
-                                                                   n_ffn, top, width, (T *)out)
+#define SEQ_COMBINE(V)                                                                                                        \
+  return launch_after(moe_combine_kernel<T, V>, n_tok, th, 0, (cudaStream_t)stream, (const T *)sorted_y, inverse,        \
+                           weights, experts, (const T *)x, n_ffn, top, width, (T *)out)
   SEQ_DISPATCH_DTYPE(dtype, {
     if (vec) SEQ_COMBINE(4);
     else SEQ_COMBINE(1);

@@ -13,6 +13,10 @@
 // weight tiles.  Rows past an expert's last belong to its neighbour (or are zeros): each accumulator row depends on its own
 // input row alone and is stored only where it belongs.
 //
+// In a step of few rows the weights' bytes are the bound, and the launches around the two products are half as long as one of them
+// (16 experts of 25 MB, 32 tokens to 4 of them, in a graph: 81 us of 94).  So every launch of the chain may begin while the one before
+// it runs, and the second product fetches the first weights of its tiles before it waits for the hidden rows: 86 us.
+//
 // Every wait has a limit; a wait that runs out sets a device flag (mrs_seq_moe_gemm_timeouts) and ends the CTA.
 #include "seq_common.cuh"
 #include "seq_tc.cuh"
@@ -31,6 +35,7 @@ struct Params {
   int n_ffn, n, k;             // experts; output columns per expert (GATED: 2 n weight rows, gate rows then up rows); length of a dot
   mrs_seq_glu_rule rule;
   __nv_bfloat16 *out;          // [sorted rows][n]
+  bool early;                  // the launch before this one is not the writer of counts and weights: they are read while it still runs
 };
 
 __device__ int g_timeouts = 0;
@@ -75,7 +80,9 @@ __global__ void __launch_bounds__(THREADS, 1) moe_gemm_kernel(const __grid_const
   constexpr int cols = GATED ? BN / 2 : BN;                // output columns of a tile
   const int n_tiles = (p.n + cols - 1) / cols;
 
+  if (!p.early) seq::wait_for_previous();
   if (smem_u32(smem) & 1023) {               // the swizzled boxes need it; never seen
+    seq::wait_for_previous();
     if (threadIdx.x == 0) atomicExch(&g_timeouts, 2);
     return;
   }
@@ -128,19 +135,30 @@ __global__ void __launch_bounds__(THREADS, 1) moe_gemm_kernel(const __grid_const
 
   if (warp == 0) {
     // ===================== TMA producer =====================
-    int it = 0;
+    auto load_weights = [&](const Tile &x, int ks, int s) {
+      uint8_t *b_s = smem + s * STAGE_BYTES + A_BYTES;
+      mbar_arrive_expect_tx_warp(full + s, STAGE_BYTES);
+      tma_load_2d_warp(b_s, &tmap_b, ks * BK, x.b_row0, full + s);
+      tma_load_2d_warp(b_s + B_BYTES / 2, &tmap_b, ks * BK, x.b_row1, full + s);
+    };
+    int it = 0, ahead = 0;                   // ahead: stages whose weights are on their way
+    if (p.early && (int)blockIdx.x < total) {
+      const Tile x = tile_of(blockIdx.x);
+      for (; ahead < min(STAGES, k_steps); ahead++) load_weights(x, ahead, ahead);
+    }
+    seq::wait_for_previous();
+    seq::let_next_start();
     bool ok = true;
     for (int t = blockIdx.x; ok && t < total; t += gridDim.x) {
       const Tile x = tile_of(t);
       for (int ks = 0; ks < k_steps; ks++, it++) {
         const int s = it % STAGES;
-        ok = wait(empty + s, ((it / STAGES) & 1) ^ 1);
-        if (!ok) break;
-        uint8_t *a_s = smem + s * STAGE_BYTES, *b_s = a_s + A_BYTES;
-        mbar_arrive_expect_tx_warp(full + s, STAGE_BYTES);
-        tma_load_2d_warp(a_s, &tmap_a, ks * BK, x.a_row, full + s);
-        tma_load_2d_warp(b_s, &tmap_b, ks * BK, x.b_row0, full + s);
-        tma_load_2d_warp(b_s + B_BYTES / 2, &tmap_b, ks * BK, x.b_row1, full + s);
+        if (it >= ahead) {
+          ok = wait(empty + s, ((it / STAGES) & 1) ^ 1);
+          if (!ok) break;
+          load_weights(x, ks, s);
+        }
+        tma_load_2d_warp(smem + s * STAGE_BYTES, &tmap_a, ks * BK, x.a_row, full + s);
       }
     }
     // copies in flight land before the CTA may end
@@ -151,6 +169,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_gemm_kernel(const __grid_const
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
     int it = 0, j = 0;
     bool ok = true;
+    seq::wait_for_previous();
     for (int t = blockIdx.x; ok && t < total; t += gridDim.x, j++) {
       const uint32_t t_acc = tmem_base + (uint32_t)((j & 1) * BN);
       ok = wait(acc_empty + (j & 1), ((j >> 1) & 1) ^ 1);
@@ -177,6 +196,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_gemm_kernel(const __grid_const
     const int q4 = warp & 3, r = q4 * 32 + lane, part = (warp - 2) >> 2;      // a warp reads its own quarter of the TMEM lanes
     const uint32_t lane_off = (uint32_t)(q4 * 32) << 16;
     int j = 0;
+    seq::wait_for_previous();
     for (int t = blockIdx.x; t < total; t += gridDim.x, j++) {
       const Tile x = tile_of(t);
       const bool ok = __all_sync(0xffffffffu, wait(acc_full + (j & 1), (j >> 1) & 1));
@@ -228,15 +248,16 @@ extern "C" int mrs_seq_moe_gemm_timeouts(void) {
   return e == cudaSuccess ? v : -(int)e;
 }
 
-extern "C" int mrs_seq_moe_gemm(const void *sorted, const void *weights, const int32_t *counts, int n_rows, int n_ffn, int n, int k, int gated,
-                                const mrs_seq_glu_rule *rule, void *out, int64_t stream) {
-  using namespace seqg;
-  if (n_rows <= 0) return 0;
+namespace seqg {
+static int launch(const void *sorted, const void *weights, const int32_t *counts, int n_rows, int n_ffn, int n, int k, int gated, const mrs_seq_glu_rule *rule,
+                  void *out, bool early, int64_t stream) {
   if (!sorted || !weights || !counts || !out || !rule || !mrs_seq_moe_gemm_fits(MRS_SEQ_BF16, n, k, n_ffn)) return -2;
   if (((uintptr_t)sorted | (uintptr_t)weights | (uintptr_t)out) & 15) return -3;
   CUtensorMap ta, tb;
+  // weights: the next 64 columns of a row are wanted next, and one 256-byte fetch brings both.  16 experts of 25 MB, 32 tokens to 4 of
+  // them: 88.1 us with fetches of 128 bytes, 86.0 so (16 sorted rows at a time instead of 128 made no difference at all)
   if (!tc_make_map_2d(&ta, sorted, (uint64_t)n_rows, (uint64_t)k, BK, BM, 1) ||
-      !tc_make_map_2d(&tb, weights, (uint64_t)n_ffn * n * (gated ? 2 : 1), (uint64_t)k, BK, BN / 2, 1))
+      !tc_make_map_2d(&tb, weights, (uint64_t)n_ffn * n * (gated ? 2 : 1), (uint64_t)k, BK, BN / 2, 1, CU_TENSOR_MAP_L2_PROMOTION_L2_256B))
     return -4;
   static bool raised = false;
   if (!raised) {
@@ -246,11 +267,25 @@ extern "C" int mrs_seq_moe_gemm(const void *sorted, const void *weights, const i
     raised = true;
   }
   Params p = {};
-  p.counts = counts; p.n_ffn = n_ffn; p.n = n; p.k = k; p.rule = *rule; p.out = (__nv_bfloat16 *)out;
+  p.counts = counts; p.n_ffn = n_ffn; p.n = n; p.k = k; p.rule = *rule; p.out = (__nv_bfloat16 *)out; p.early = early;
   const int cols = gated ? BN / 2 : BN;
   const int64_t most = ((int64_t)(n_rows + BM - 1) / BM + (n_ffn < n_rows ? n_ffn : n_rows)) * ((n + cols - 1) / cols);      // tiles at any split of the rows
   const int grid = (int)(most < 148 ? most : 148);
-  if (gated) moe_gemm_kernel<true><<<grid, THREADS, SMEM, (cudaStream_t)stream>>>(ta, tb, p);
-  else moe_gemm_kernel<false><<<grid, THREADS, SMEM, (cudaStream_t)stream>>>(ta, tb, p);
-  return (int)cudaGetLastError();
+  return seq::launch_after(gated ? moe_gemm_kernel<true> : moe_gemm_kernel<false>, grid, THREADS, SMEM, (cudaStream_t)stream, ta, tb, p);
+}
+}  // namespace seqg
+
+extern "C" int mrs_seq_moe_gemm(const void *sorted, const void *weights, const int32_t *counts, int n_rows, int n_ffn, int n, int k, int gated,
+                                const mrs_seq_glu_rule *rule, void *out, int64_t stream) {
+  return n_rows <= 0 ? 0 : seqg::launch(sorted, weights, counts, n_rows, n_ffn, n, k, gated, rule, out, false, stream);
+}
+
+// The second launch may read counts and its weights early: the first one began after all that came before it had ended.
+extern "C" int mrs_seq_moe_products(const void *sorted, const void *up, const void *down, const int32_t *counts, int n_rows, int n_ffn, int width, int ff,
+                                    int gated, const mrs_seq_glu_rule *rule, void *hidden, void *out, int64_t stream) {
+  if (n_rows <= 0) return 0;
+  if (!down || !out || (((uintptr_t)down | (uintptr_t)out) & 15) || !mrs_seq_moe_gemm_fits(MRS_SEQ_BF16, width, ff, n_ffn)) return -2;
+  const mrs_seq_glu_rule none = {};
+  const int rc = seqg::launch(sorted, up, counts, n_rows, n_ffn, ff, width, gated, rule, hidden, false, stream);
+  return rc != 0 ? rc : seqg::launch(hidden, down, counts, n_rows, n_ffn, width, ff, 0, &none, out, true, stream);
 }

@@ -11,6 +11,29 @@
 
 namespace seq {
 
+// ---- launches that overlap ------------------------------------------------------------------------------
+// A kernel of `launch_after` may begin while the one before it in the stream still runs, once every CTA of that one has called
+// let_next_start or ended.  It calls wait_for_previous, in every CTA, before it touches what anything before it reads or writes:
+// the wait ends when the one before has ended and its writes are visible.  A kernel that calls both calls the wait first: what begins
+// during a kernel then finds everything before that kernel ended.  (A kernel without these calls keeps the usual order.)
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+inline int launch_after(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr[1] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  return (int)(e == cudaSuccess ? cudaGetLastError() : e);
+}
+
 // ---- storage types ----------------------------------------------------------------------------------
 template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }

@@ -757,8 +757,8 @@ class RoutedExperts:
             else:
                 counts, order = K.moe_sort(experts, self.n_routes)
                 rows = K.moe_gather(h, order, self.top)
-            hid = K.moe_gemm(rows, self.w_gate_up, counts, self.act, self.gated)
-            out = K.moe_combine(K.moe_gemm(hid, self.w_down, counts), order, weights, inverse=inverse, **self._identities(experts, h))
+            ys = K.moe_products(rows, self.w_gate_up, self.w_down, counts, self.act, self.gated)
+            out = K.moe_combine(ys, order, weights, inverse=inverse, **self._identities(experts, h))
         else:
             counts, order = K.moe_sort(experts, self.n_routes)
             spans, at = [], 0

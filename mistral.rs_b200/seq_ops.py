@@ -481,6 +481,17 @@ def moe_gemm(rows, weights, counts, act=ACT_NONE, gated=False):
     return out
 
 
+def moe_products(rows, up, down, counts, act, gated):
+    """`moe_gemm` of up and, on its result, of down: [n, W].  The second launch begins on its weights while the first one runs."""
+    n, W = rows.shape
+    ff = down.shape[2]
+    hidden, out = (torch.empty(n, c, dtype=rows.dtype, device=rows.device) for c in (ff, W))
+    rule = GluRule.of(act)
+    _ok(lib().mrs_seq_moe_products(_p(rows), _p(up), _p(down), _p(counts), _i(n), _i(up.shape[0]), _i(W), _i(ff), _i(int(gated)), ctypes.byref(rule),
+                                   _p(hidden), _p(out), _st(rows)), "moe_products")
+    return out
+
+
 def moe_gemm_timeouts():
     """Non-zero when a wait inside `moe_gemm`'s kernel ever ran out (synchronises)."""
     return int(lib().mrs_seq_moe_gemm_timeouts())

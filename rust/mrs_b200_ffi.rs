@@ -115,6 +115,7 @@ extern "C" {
     pub fn mrs_seq_moe_gather(x: *const c_void, dtype: i32, order: *const i32, n_pairs: i32, top: i32, width: i32, sorted: *mut c_void, stream: i64) -> i32;
     pub fn mrs_seq_moe_gemm(sorted: *const c_void, weights: *const c_void, counts: *const i32, n_rows: i32, n_ffn: i32, n: i32, k: i32, gated: i32, rule: *const c_void, out: *mut c_void, stream: i64) -> i32;
     pub fn mrs_seq_moe_gemm_fits(dtype: i32, n: i32, k: i32, n_ffn: i32) -> i32;
+    pub fn mrs_seq_moe_products(sorted: *const c_void, up: *const c_void, down: *const c_void, counts: *const i32, n_rows: i32, n_ffn: i32, width: i32, ff: i32, gated: i32, rule: *const c_void, hidden: *mut c_void, out: *mut c_void, stream: i64) -> i32;
     pub fn mrs_seq_moe_gemm_timeouts() -> i32;
     pub fn mrs_seq_moe_combine(sorted_y: *const c_void, dtype: i32, order: *const i32, weights: *const f32, n_tok: i32, top: i32, width: i32, scratch_inverse: *mut i32, out: *mut c_void, stream: i64) -> i32;
     pub fn mrs_seq_moe_combine_some(sorted_y: *const c_void, dtype: i32, order: *const i32, weights: *const f32, experts: *const i32, x: *const c_void, n_ffn: i32, n_tok: i32, top: i32, width: i32, scratch_inverse: *mut i32, out: *mut c_void, stream: i64) -> i32;
