@@ -484,7 +484,7 @@ def bench_nisasun(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
             setattr(mod, name, g)
             return f
         names = ["embed_streams", "streams_read_norm", "streams_write", "glu_split", "gated_group_norm", "causal_conv", "ssm_steps",
-                 "linear_scan", "attention_prepare", "paged_attention", "fresh_prompt_attention", "scale_rows", "activate_cols", "moe_route", "moe_small", "moe_place", "moe_sort", "moe_gather", "moe_combine"]
+                 "linear_scan", "attention_prepare", "paged_attention", "fresh_prompt_attention", "scale_rows", "activate_cols", "moe_route", "moe_block", "moe_small", "moe_place", "moe_sort", "moe_gather", "moe_combine"]
         saved = {n: wrap(K, n) for n in names}
         saved_lin = wrap(mixers, "linear")
 
@@ -612,7 +612,7 @@ def bench_kilizen(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
     warmup, steps = max(3, warmup), max(1, steps)
     names = [n for n in ("embed_streams", "streams_read_norm", "streams_write", "glu_split", "gated_group_norm", "causal_conv", "ssm_steps", "linear_scan",
-                         "qk_norm_store", "window_attention", "fresh_prompt_attention", "scale_rows", "activate_cols", "moe_route", "moe_small", "moe_place", "moe_sort",
+                         "qk_norm_store", "window_attention", "fresh_prompt_attention", "scale_rows", "activate_cols", "moe_route", "moe_block", "moe_small", "moe_place", "moe_sort",
                          "moe_gather", "moe_combine", "tanh_norm_rows", "residual_tanh_norm", "rotation_table", "attention_prepare", "paged_attention",
                          "prompt_attention", "mlstm_gates", "append_ones", "mlstm_out_norm", "moe_route_top_softmax", "moe_small_ungated")]
 
@@ -795,7 +795,7 @@ def bench_fosulix(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
     names = ["embed_streams", "embed_scaled", "streams_read_norm", "rms_residual", "glu_split", "gated_group_norm", "causal_conv", "linear_scan",
              "activate_cols", "bounded_gate", "latent_prepare", "rotate_pairs", "latent_prompt_attention", "paged_attention", "prompt_attention",
              "fresh_prompt_attention", "attention_prepare", "rotation_table", "moe_route", "moe_route_scored", "moe_route_top_softmax", "moe_small",
-             "moe_small_ungated", "moe_place", "moe_sort", "moe_gather", "moe_combine", "tanh_norm_rows", "residual_tanh_norm", "mlstm_gates", "append_ones",
+             "moe_small_ungated", "moe_block", "moe_place", "moe_sort", "moe_gather", "moe_combine", "tanh_norm_rows", "residual_tanh_norm", "mlstm_gates", "append_ones",
              "mlstm_out_norm", "scale_rows"]
 
     def timed(fn, reps=steps):
@@ -1080,7 +1080,7 @@ def bench_kibotar(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
     names = ["embed_scaled", "embed_pair", "streams_read_norm", "rms_residual", "glu_split", "gated_group_norm", "causal_conv", "linear_scan",
              "activate_cols", "bounded_gate", "power_gate", "latent_prepare", "rotate_pairs", "latent_prompt_attention", "paged_attention",
              "prompt_attention", "tc_attention", "attention_prepare", "rotation_table", "pool_blocks", "mix_heads", "gate_cols",
-             "moe_route_scored", "moe_small",
+             "moe_route_scored", "moe_block", "moe_small",
              "moe_place", "moe_sort", "moe_gather", "moe_combine", "scale_rows"]
     measure = engine_bench_tools(torch, dev, steps, warmup, prompt, decode_batches, names)
     out = {"metric": "kibotar_prefill_tok_s", "unit": "tok/s", "n_gpus": 1, "steps": steps, "warmup": warmup, "higher_is_better": True,
@@ -1363,7 +1363,7 @@ def bench_bafusun(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
     warmup, steps = max(3, warmup), max(1, steps)
     names = ["embed_scaled", "embed_streams", "rms_residual", "tanh_norm_rows", "residual_tanh_norm", "glu_split", "activate_cols", "gated_lookup", "rotation_table",
              "attention_prepare", "paged_attention", "prompt_attention", "tc_attention", "gather_rows", "router_logits", "moe_route_scored", "moe_route_top_softmax", "moe_small",
-             "moe_small_ungated", "moe_grouped", "moe_gemm", "moe_place", "moe_sort", "moe_gather", "moe_combine", "soft_cap"]
+             "moe_small_ungated", "moe_grouped", "moe_products", "moe_block", "moe_place", "moe_sort", "moe_gather", "moe_combine", "soft_cap"]
     measure = engine_bench_tools(torch, dev, steps, warmup, prompt, decode_batches, names)
     out = {"metric": "bafusun_prefill_tok_s", "unit": "tok/s", "n_gpus": 1, "steps": steps, "warmup": warmup, "higher_is_better": True,
            "dtype": "bf16 (f32 residual, norms, angles, softmax, router)", "data": "synthetic", "sizes": []}
@@ -1419,9 +1419,9 @@ def bench_bafusun(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
                                                            "like_ms": kops.get("moe_combine"), "like_hbm_frac": gbs(n * T * (top + 1) * W * 2, kops.get("moe_combine"))}
         roof["moe_sort"] = {"ms": ops.get("moe_sort"), "like": "moe_sort", "like_ms": kops.get("moe_sort")}
         eflop, keflop = 2.0 * W * ffn * 3 * ff, 2.0 * W * n * T * top * 2 * ff
-        roof["moe_gemm (16 experts; halves joined in the epilogue)"] = {
-            "ms": ops.get("moe_gemm"), "tflops": tfl(eflop, ops.get("moe_gemm")), "tensor_frac": tfrac(eflop, ops.get("moe_gemm")), "like": "moe_gemm (no gate)",
-            "like_ms": kops.get("moe_gemm"), "like_tflops": tfl(keflop, kops.get("moe_gemm")), "like_tensor_frac": tfrac(keflop, kops.get("moe_gemm"))}
+        roof["moe_products (16 experts; halves joined in the epilogue)"] = {
+            "ms": ops.get("moe_products"), "tflops": tfl(eflop, ops.get("moe_products")), "tensor_frac": tfrac(eflop, ops.get("moe_products")), "like": "moe_products (no gate)",
+            "like_ms": kops.get("moe_products"), "like_tflops": tfl(keflop, kops.get("moe_products")), "like_tensor_frac": tfrac(keflop, kops.get("moe_products"))}
         roof["glu_split (capped; shared expert)"] = {"ms": ops.get("glu_split"), "hbm_frac": gbs(n * T * sf * 6, ops.get("glu_split")), "like": "activate_cols",
                                                      "like_ms": kops.get("activate_cols"), "like_hbm_frac": gbs(n * T * sf * 4, kops.get("activate_cols"))}
         roof["gated_lookup (with its product)"] = {"ms": ops.get("gated_lookup"), "hbm_frac": gbs(n * (T * W * 2 + T * side * 2 * 4), ops.get("gated_lookup"))}
@@ -1437,9 +1437,9 @@ def bench_bafusun(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
                                                           "like_ms": dk[1].get("paged_attention"), "like_hbm_frac": gbs(kv, dk[1].get("paged_attention"))}
             used = lambda routes: E * (1.0 - (1.0 - top / routes) ** b)            # experts that at least one of b tokens chooses, if the choice is even
             mb, kmb = n * used(E + I) * 3 * ff * W * 2, n * used(E) * 2 * ff * W * 2
-            mine, theirs = ("moe_grouped", "moe_grouped") if dk[0].get("moe_grouped") else ("moe_small", "moe_small_ungated")
-            roof["%s (decode, b=%d)" % (mine, b)] = {"ms": dk[0].get(mine), "hbm_frac": gbs(mb, dk[0].get(mine)), "like": theirs + " (no gate)",
-                                                     "like_ms": dk[1].get(theirs), "like_hbm_frac": gbs(kmb, dk[1].get(theirs))}
+            block = "moe_block"                      # the router, the rule, both products and the sum
+            roof["%s (decode, b=%d)" % (block, b)] = {"ms": dk[0].get(block), "hbm_frac": gbs(mb, dk[0].get(block)), "like": block + " (no gate)",
+                                                      "like_ms": dk[1].get(block), "like_hbm_frac": gbs(kmb, dk[1].get(block))}
         row["roofline"] = roof
         out["sizes"].append(row)
     out["value"] = out["sizes"][0]["prefill_tok_s"]

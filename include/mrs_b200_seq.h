@@ -476,6 +476,10 @@ typedef struct {
   int64_t logits_ld;      /* floats between the rows of logits; 0: n_experts */
 } mrs_seq_moe_route_args;
 int mrs_seq_moe_route_general(const mrs_seq_moe_route_args *args, int64_t stream);
+/* mrs_seq_router_logits and the rule above in one launch, for steps of few tokens and few experts (_fits): x [n_tok, width], w f32
+ * [n_experts, width]; args->logits and logits_ld are not read.  The same experts and weights as the two. */
+int mrs_seq_moe_router(const void *x, int dtype, const float *w, int width, const mrs_seq_moe_route_args *args, int64_t stream);
+int mrs_seq_moe_router_fits(int width, int n_experts, int n_tok);
 /* The router's product for few tokens: logits[t][e] = w[e] . x[t] in f32 (x [n_tok, width] of the activation type, w f32
  * [n_experts, width], logits f32 [n_tok, n_experts]). */
 int mrs_seq_router_logits(const void *x, int dtype, const float *w, int width, int n_experts, int n_tok, float *logits, int64_t stream);
@@ -553,6 +557,28 @@ int mrs_seq_moe_place(const int32_t *experts, int n_pairs, int n_experts, const 
                       int32_t *inverse, void *sorted, int64_t stream);
 int mrs_seq_moe_combine_at(const void *sorted_y, int dtype, const int32_t *inverse, const float *weights, const int32_t *experts, const void *x,
                            int n_ffn, int n_tok, int top, int width, void *out, int64_t stream);
+/* A routed-expert block in one call: the router's product, the rule, the experts and the weighted sum, by the entries above (the same results).
+ * logits [n_tok, logits_ld], or NULL: formed from router [n_routes, width].  route: the score of the grouped rule, or the softmax over the chosen
+ * logits (contiguous rows; the grouped rule's fields are not read).  products: which entries take the experts.  up [n_ffn, gated ? 2 * ff : ff,
+ * width], down [n_ffn, width, ff]; routes from n_ffn on are identities.  scratch: 16-byte aligned, at least (2 * width + ff) * pairs elements of the
+ * activation type + 4 * (3 * pairs + n_routes + n_tok * n_routes) bytes + 2048 (pairs = n_tok * top); -3: too little.  One-launch products take
+ * bf16 and what mrs_seq_moe_place_fits and mrs_seq_moe_gemm_fits allow. */
+enum { MRS_SEQ_ROUTE_SOFTMAX = 0, MRS_SEQ_ROUTE_SIGMOID = 1, MRS_SEQ_ROUTE_TOP_SOFTMAX = 2 };
+enum { MRS_SEQ_PRODUCTS_ONE_LAUNCH = 0, MRS_SEQ_PRODUCTS_GROUPED = 1, MRS_SEQ_PRODUCTS_STREAMED = 2 };
+typedef struct {
+  const void *x;
+  const float *router, *logits;
+  int64_t logits_ld;
+  const float *correction;
+  const void *up, *down;
+  void *scratch;
+  int64_t scratch_bytes;
+  void *out;
+  int dtype, n_tok, width, ff, n_routes, n_ffn, top, gated, route, products, n_groups, keep_groups, renorm, group_top;
+  float weight_scale, renorm_eps;
+  mrs_seq_glu_rule rule;
+} mrs_seq_moe_block_args;
+int mrs_seq_moe_block(const mrs_seq_moe_block_args *args, int64_t stream);
 
 #ifdef __cplusplus
 }

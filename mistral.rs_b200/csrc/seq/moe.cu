@@ -160,6 +160,43 @@ __global__ void __launch_bounds__(128) router_logits_kernel(const T *__restrict_
   if (threadIdx.x == 0) logits[(int64_t)blockIdx.y * n_experts + blockIdx.x] = s;
 }
 
+// The two steps above in one launch for few tokens and few experts: one CTA per token, 128 threads per product, each product summed in
+// the order of router_logits_kernel (the same bits), then the routing rule by the first warp.  Bound by latency: the router's rows come
+// to every CTA from L2 at one SM's rate, and a group of 128 threads takes its products one after the other, so their size and number draw
+// the line.  us of two launches / one, 1, 8 and 32 tokens: 8 experts of 1024 columns 5.5 / 4.4, 5.8 / 4.5, 5.9 / 4.5; 16 of 2048 5.6 / 5.2, 5.8 /
+// 5.4, 6.1 / 5.5; beyond it 16 of 4096 5.8 / 6.2, 6.2 / 6.3, 6.6 / 6.5, 32 of 1024 5.3 / 6.3, 5.7 / 6.4, 6.1 / 6.6.
+constexpr int ROUTE_FUSED_GROUPS = 8, ROUTE_FUSED_EXPERTS = 16, ROUTE_FUSED_TOKENS = 64, ROUTE_FUSED_WEIGHTS = 32768;
+template <typename T, int VEC>
+__global__ void __launch_bounds__(128 * ROUTE_FUSED_GROUPS) router_route_kernel(const T *__restrict__ x, const float *__restrict__ w, int width,
+                                                                                const mrs_seq_moe_route_args a) {
+  constexpr int E = ROUTE_FUSED_EXPERTS;
+  __shared__ float part[E][4], z[E], score[E], choice[E], gscore[E];
+  const int t = blockIdx.x, group = threadIdx.x >> 7, i = threadIdx.x & 127, lane = threadIdx.x & 31, warp = i >> 5;
+  const T *xr = x + (int64_t)t * width;
+  wait_for_previous();
+  let_next_start();
+  for (int e = group; e < a.n_experts; e += ROUTE_FUSED_GROUPS) {
+    const float *wr = w + (int64_t)e * width;
+    float s = 0.0f;
+#pragma unroll 4
+    for (int c = i * VEC; c < width; c += 128 * VEC) {
+      if (VEC == 4) {
+        const float4 p = *(const float4 *)(wr + c), q = load4<T>(xr + c);
+        s = fmaf(p.x, q.x, fmaf(p.y, q.y, fmaf(p.z, q.z, fmaf(p.w, q.w, s))));
+      } else {
+        s = fmaf(wr[c], to_f32<T>(xr[c]), s);
+      }
+    }
+    s = warp_sum(s);
+    if (lane == 0) part[e][warp] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  for (int e = lane; e < a.n_experts; e += 32) z[e] = (part[e][0] + part[e][2]) + (part[e][1] + part[e][3]);
+  __syncwarp();
+  route_token(z, a, score, choice, gscore, lane, a.experts + (int64_t)t * a.top, a.weights + (int64_t)t * a.top);
+}
+
 // hidden[t][k][r] = act(gate_up[e][r] . x_t) * (gate_up[e][ff + r] . x_t): one warp per output element;
 // blockIdx.y is the (token, k) pair, pairs laid out [token][k]
 template <typename T>
@@ -535,6 +572,24 @@ extern "C" int mrs_seq_moe_route_general(const mrs_seq_moe_route_args *args, int
   return launch_after(moe_route_kernel, (n_tok + warps - 1) / warps, warps * 32, bytes, (cudaStream_t)stream, a);
 }
 
+extern "C" int mrs_seq_moe_router_fits(int width, int n_experts, int n_tok) {
+  return width > 0 && n_experts >= 1 && n_experts <= ROUTE_FUSED_EXPERTS && n_tok >= 0 && n_tok <= ROUTE_FUSED_TOKENS &&
+         (int64_t)width * n_experts <= ROUTE_FUSED_WEIGHTS;
+}
+
+extern "C" int mrs_seq_moe_router(const void *x, int dtype, const float *w, int width, const mrs_seq_moe_route_args *args, int64_t stream) {
+  const mrs_seq_moe_route_args &a = *args;
+  if (a.n_tok <= 0) return 0;
+  if (!x || !w || !a.experts || !a.weights || !route_args_ok(a) || !mrs_seq_moe_router_fits(width, a.n_experts, a.n_tok)) return -2;
+  const bool vec = width % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
+  constexpr int threads = 128 * ROUTE_FUSED_GROUPS;
+  SEQ_DISPATCH_DTYPE(dtype, {
+    return vec ? launch_after(router_route_kernel<T, 4>, a.n_tok, threads, 0, (cudaStream_t)stream, (const T *)x, w, width, a)
+               : launch_after(router_route_kernel<T, 1>, a.n_tok, threads, 0, (cudaStream_t)stream, (const T *)x, w, width, a);
+  });
+  return launch_status();
+}
+
 extern "C" int mrs_seq_moe_route_top_softmax(const float *logits, int n_tok, int n_experts, int top, int32_t *experts, float *weights,
                                              int64_t stream) {
   if (n_tok <= 0) return 0;
@@ -736,4 +791,71 @@ extern "C" int mrs_seq_moe_combine_some(const void *sorted_y, int dtype, const i
 extern "C" int mrs_seq_moe_combine(const void *sorted_y, int dtype, const int32_t *order, const float *weights, int n_tok, int top,
                                    int width, int32_t *scratch_inverse, void *out, int64_t stream) {
   return mrs_seq_moe_combine_some(sorted_y, dtype, order, weights, nullptr, nullptr, 0, n_tok, top, width, scratch_inverse, out, stream);
+}
+
+// The whole block behind one call: the steps are the entries above, their buffers one piece of scratch.  For calls from the host, whose
+// six calls of a front end with a tensor each took longer than the kernels of small experts (32 experts of 5 MB, 8 tokens: 79 us of which
+// the kernels make 43).
+extern "C" int mrs_seq_moe_block(const mrs_seq_moe_block_args *args, int64_t stream) {
+  const mrs_seq_moe_block_args &a = *args;
+  if (a.n_tok <= 0) return 0;
+  if (!a.x || !a.up || !a.down || !a.out || !a.scratch || (!a.router && !a.logits) || a.width <= 0 || a.ff <= 0 || a.top < 1 || a.n_ffn < 1 ||
+      a.n_routes < a.n_ffn || (a.dtype != MRS_SEQ_BF16 && a.dtype != MRS_SEQ_F32))
+    return -2;
+  const int64_t pairs = (int64_t)a.n_tok * a.top, elem = a.dtype == MRS_SEQ_BF16 ? 2 : 4;
+  if (pairs > INT_MAX) return -2;
+  int64_t used = 0;
+  auto piece = [&](int64_t bytes) {
+    void *at = (uint8_t *)a.scratch + used;
+    used += (bytes + 255) / 256 * 256;
+    return at;
+  };
+  const bool fused = !a.logits && a.route != MRS_SEQ_ROUTE_TOP_SOFTMAX && mrs_seq_moe_router_fits(a.width, a.n_routes, a.n_tok);
+  float *logits = a.logits || fused ? nullptr : (float *)piece((int64_t)a.n_tok * a.n_routes * 4);
+  int32_t *experts = (int32_t *)piece(pairs * 4);
+  float *weights = (float *)piece(pairs * 4);
+  const bool streams = a.products == MRS_SEQ_PRODUCTS_STREAMED;
+  int32_t *counts = streams ? nullptr : (int32_t *)piece((int64_t)a.n_routes * 4), *at = streams ? nullptr : (int32_t *)piece(pairs * 4);
+  void *hidden = piece(pairs * a.ff * elem), *y = streams ? nullptr : piece(pairs * a.width * elem);
+  void *rows = a.products == MRS_SEQ_PRODUCTS_ONE_LAUNCH ? piece(pairs * a.width * elem) : nullptr;
+  if (used > a.scratch_bytes || ((uintptr_t)a.scratch & 15)) return -3;
+
+  int rc = 0;
+  const mrs_seq_moe_route_args r = {a.logits ? a.logits : logits, a.correction, a.n_tok, a.n_routes, a.n_groups, a.keep_groups, a.top, a.renorm,
+                                    a.route == MRS_SEQ_ROUTE_SIGMOID ? MRS_SEQ_SCORE_SIGMOID : MRS_SEQ_SCORE_SOFTMAX, a.group_top, a.weight_scale,
+                                    a.renorm_eps, experts, weights, a.logits ? a.logits_ld : 0};
+  if (logits) rc = mrs_seq_router_logits(a.x, a.dtype, a.router, a.width, a.n_routes, a.n_tok, logits, stream);
+  if (rc != 0) return rc;
+  if (fused) rc = mrs_seq_moe_router(a.x, a.dtype, a.router, a.width, &r, stream);
+  else if (a.route != MRS_SEQ_ROUTE_TOP_SOFTMAX) rc = mrs_seq_moe_route_general(&r, stream);
+  else if (a.logits && a.logits_ld != a.n_routes) return -2;
+  else rc = mrs_seq_moe_route_top_softmax(r.logits, a.n_tok, a.n_routes, a.top, experts, weights, stream);
+  if (rc != 0) return rc;
+
+  const bool identities = a.n_routes > a.n_ffn;
+  if (streams) {
+    if (a.gated) {
+      const mrs_seq_moe_small_args s = {a.x, a.up, a.down, a.dtype, experts, weights, a.n_tok, a.top, a.width, a.ff, a.n_ffn, a.rule, hidden, a.out};
+      return mrs_seq_moe_small(&s, stream);
+    }
+    if (identities) return -2;
+    rc = mrs_seq_moe_up(a.x, a.up, a.dtype, experts, a.n_tok, a.top, a.width, a.ff, a.rule.act, hidden, stream);
+    return rc != 0 ? rc : mrs_seq_moe_down(hidden, a.down, a.dtype, experts, weights, a.n_tok, a.top, a.width, a.ff, a.out, stream);
+  }
+  const int32_t *inverse = nullptr;
+  if (a.products == MRS_SEQ_PRODUCTS_GROUPED) {
+    rc = mrs_seq_moe_sort(experts, (int)pairs, a.n_routes, counts, at, stream);
+    if (rc != 0) return rc;
+    const mrs_seq_moe_grouped_args g = {a.x, a.up, a.down, a.dtype, counts, at, a.n_tok, a.top, a.width, a.ff, a.n_ffn, a.gated, a.rule, hidden, y};
+    rc = mrs_seq_moe_grouped(&g, stream);
+  } else {
+    if (a.dtype != MRS_SEQ_BF16) return -2;
+    rc = mrs_seq_moe_place(experts, (int)pairs, a.n_routes, a.x, a.dtype, a.top, a.width, counts, at, rows, stream);
+    if (rc != 0) return rc;
+    inverse = at;
+    rc = mrs_seq_moe_products(rows, a.up, a.down, counts, (int)pairs, a.n_ffn, a.width, a.ff, a.gated, &a.rule, hidden, y, stream);
+  }
+  return rc != 0 ? rc
+                 : mrs_seq_moe_combine_at(y, a.dtype, inverse, weights, identities ? experts : nullptr, identities ? a.x : nullptr, identities ? a.n_ffn : 0,
+                                          a.n_tok, a.top, a.width, a.out, stream);
 }

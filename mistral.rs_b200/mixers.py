@@ -684,10 +684,11 @@ class RoutedExperts:
     # 2 above that.
     GROUPED_MIN_TOKENS, GROUPED_PER_EXPERT, GROUPED_PAIR_BYTES = 4, 8, 700 << 20
     SMALL_EXPERT_BYTES = 32 << 20
+    ROUTES = {"grouped_softmax": K.ROUTE_SOFTMAX, "grouped_sigmoid": K.ROUTE_SIGMOID, "top_softmax": K.ROUTE_TOP_SOFTMAX}
 
     def __init__(self, w_router, correction, w_gate_up, w_down, top, n_groups, keep_groups, act, renorm=False, rule="grouped_softmax",
                  gated=True, shared=None, group_top=1, weight_scale=1.0, renorm_eps=0.0):
-        if rule not in ("grouped_softmax", "grouped_sigmoid", "top_softmax"):
+        if rule not in self.ROUTES:
             raise ValueError(f"unknown routing rule {rule!r}")
         self.group_top, self.weight_scale = int(group_top), float(weight_scale)
         self.w_router, self.correction, self.w_gate_up, self.w_down = w_router, correction, w_gate_up, w_down
@@ -733,32 +734,38 @@ class RoutedExperts:
         return n_tok * self.top <= per_expert * self.n_experts and not (self.grouped_fits() and self.outgrows_groups(n_tok))
 
     def route(self, h):
-        logits = K.router_logits(h, self.w_router, self.w_router16)
         if self.rule == "top_softmax":
-            return K.moe_route_top_softmax(logits.contiguous(), self.top)
+            return K.moe_route_top_softmax(K.router_logits(h, self.w_router, self.w_router16).contiguous(), self.top)
         fn = K.SCORE_SIGMOID if self.rule == "grouped_sigmoid" else K.SCORE_SOFTMAX
-        return K.moe_route_scored(logits, self.correction, self.n_groups, self.keep_groups, self.top, self.renorm, fn, self.group_top,
-                                  self.weight_scale, self.renorm_eps)
+        rule = (self.correction, self.n_groups, self.keep_groups, self.top, self.renorm, fn, self.group_top, self.weight_scale, self.renorm_eps)
+        if K.moe_router_fits(h.shape[1], self.n_routes, h.shape[0]):
+            return K.moe_router(h, self.w_router, *rule)
+        return K.moe_route_scored(K.router_logits(h, self.w_router, self.w_router16), *rule)
 
     def _identities(self, experts, h):
         return {"experts": experts, "x": h, "n_ffn": self.n_experts} if self.n_routes > self.n_experts else {}
 
     def forward(self, h):
+        n_tok, products = h.shape[0], None
+        if self.groups_weights(n_tok):
+            products = K.GROUPED
+        elif self.streams_weights(n_tok):           # few pairs: every pair streams its expert
+            products = K.STREAMED
+        elif self.one_launch_products() and K.moe_place_fits(n_tok * self.top, self.n_routes):
+            products = K.ONE_LAUNCH
+        if products is not None:
+            logits = K.router_logits(h, self.w_router, self.w_router16) if n_tok > K.ROUTER_SPREAD else None
+            if logits is not None and self.rule == "top_softmax":
+                logits = logits.contiguous()
+            out = K.moe_block(h, self.w_router, logits, self.correction, self.w_gate_up, self.w_down, self.top, self.gated, self.act,
+                              self.ROUTES[self.rule], products, self.n_groups, self.keep_groups, self.renorm, self.group_top, self.weight_scale,
+                              self.renorm_eps)
+            return out if self.shared is None else self.shared.forward_added_to(h, out)
         experts, weights = self.route(h)
-        if self.groups_weights(h.shape[0]):
-            out = K.moe_grouped(h, self.w_gate_up, self.w_down, experts, weights, self.n_routes, self.act, self.gated)
-        elif self.streams_weights(h.shape[0]):      # few pairs: every pair streams its expert
-            small = K.moe_small if self.gated else K.moe_small_ungated
-            out = small(h, self.w_gate_up, self.w_down, experts, weights, self.act)
-        elif self.one_launch_products():
-            order = inverse = None
-            if K.moe_place_fits(experts.numel(), self.n_routes):
-                rows, counts, inverse = K.moe_place(h, experts, self.n_routes)
-            else:
-                counts, order = K.moe_sort(experts, self.n_routes)
-                rows = K.moe_gather(h, order, self.top)
-            ys = K.moe_products(rows, self.w_gate_up, self.w_down, counts, self.act, self.gated)
-            out = K.moe_combine(ys, order, weights, inverse=inverse, **self._identities(experts, h))
+        if self.one_launch_products():
+            counts, order = K.moe_sort(experts, self.n_routes)
+            ys = K.moe_products(K.moe_gather(h, order, self.top), self.w_gate_up, self.w_down, counts, self.act, self.gated)
+            out = K.moe_combine(ys, order, weights, **self._identities(experts, h))
         else:
             counts, order = K.moe_sort(experts, self.n_routes)
             spans, at = [], 0

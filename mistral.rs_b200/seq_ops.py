@@ -154,6 +154,14 @@ class MoeGroupedArgs(ctypes.Structure):
                 ("n_ffn", ctypes.c_int), ("gated", ctypes.c_int), ("rule", GluRule), ("hidden", ctypes.c_void_p), ("y", ctypes.c_void_p)]
 
 
+class MoeBlockArgs(ctypes.Structure):
+    _fields_ = ([(n, ctypes.c_void_p) for n in ("x", "router", "logits")] + [("logits_ld", ctypes.c_int64)]
+                + [(n, ctypes.c_void_p) for n in ("correction", "up", "down", "scratch")] + [("scratch_bytes", ctypes.c_int64), ("out", ctypes.c_void_p)]
+                + [(n, ctypes.c_int) for n in ("dtype", "n_tok", "width", "ff", "n_routes", "n_ffn", "top", "gated", "route", "products", "n_groups",
+                                               "keep_groups", "renorm", "group_top")]
+                + [("weight_scale", ctypes.c_float), ("renorm_eps", ctypes.c_float), ("rule", GluRule)])
+
+
 class LatentAttentionArgs(ctypes.Structure):
     _fields_ = [("q", ctypes.c_void_p), ("q_ld", ctypes.c_int64), ("cache", ctypes.c_void_p), ("cache_row", ctypes.c_int64),
                 ("out", ctypes.c_void_p), ("out_ld", ctypes.c_int64), ("portions", ctypes.c_void_p), ("cu_tok", ctypes.c_void_p),
@@ -368,14 +376,32 @@ def moe_route_scored(logits, correction, n_groups, keep_groups, top, renorm=Fals
                      renorm_eps=0.0):
     """`moe_route` with its choices open: softmax or sigmoid scores, a group scored by the sum of its group_top largest
     choices, renormalising by (sum + renorm_eps), weights times weight_scale."""
-    T, E = logits.shape
-    experts = torch.empty(T, top, dtype=torch.int32, device=logits.device)
-    weights = torch.empty(T, top, dtype=torch.float32, device=logits.device)
+    a, experts, weights = _route_args(logits.device, *logits.shape, correction, n_groups, keep_groups, top, renorm, score_fn, group_top, weight_scale,
+                                      renorm_eps)
+    a.logits, a.logits_ld = _p(logits).value, logits.stride(0)
+    _ok(lib().mrs_seq_moe_route_general(ctypes.byref(a), _st(logits)), "moe_route_scored")
+    return experts, weights
+
+
+def _route_args(device, n_tok, n_experts, correction, n_groups, keep_groups, top, renorm, score_fn, group_top, weight_scale, renorm_eps):
+    experts = torch.empty(n_tok, top, dtype=torch.int32, device=device)
+    weights = torch.empty(n_tok, top, dtype=torch.float32, device=device)
     a = MoeRouteArgs()
-    a.logits, a.correction, a.n_tok, a.n_experts, a.logits_ld = _p(logits).value, _p(correction).value, T, E, logits.stride(0)
+    a.correction, a.n_tok, a.n_experts = _p(correction).value, n_tok, n_experts
     a.n_groups, a.keep_groups, a.top, a.renorm, a.score_fn, a.group_top = n_groups, keep_groups, top, int(renorm), score_fn, group_top
     a.weight_scale, a.renorm_eps, a.experts, a.weights = float(weight_scale), float(renorm_eps), _p(experts).value, _p(weights).value
-    _ok(lib().mrs_seq_moe_route_general(ctypes.byref(a), _st(logits)), "moe_route_scored")
+    return a, experts, weights
+
+
+def moe_router_fits(width, n_experts, n_tok):
+    return bool(lib().mrs_seq_moe_router_fits(_i(width), _i(n_experts), _i(n_tok)))
+
+
+def moe_router(x, w, correction, n_groups, keep_groups, top, renorm=False, score_fn=SCORE_SOFTMAX, group_top=1, weight_scale=1.0, renorm_eps=0.0):
+    """`router_logits` and `moe_route_scored` in one launch (`moe_router_fits`): the same experts and weights."""
+    T, W = x.shape
+    a, experts, weights = _route_args(x.device, T, w.shape[0], correction, n_groups, keep_groups, top, renorm, score_fn, group_top, weight_scale, renorm_eps)
+    _ok(lib().mrs_seq_moe_router(_p(x), _i(DTYPE_CODE[x.dtype]), _p(w), _i(W), ctypes.byref(a), _st(x)), "moe_router")
     return experts, weights
 
 
@@ -489,6 +515,27 @@ def moe_products(rows, up, down, counts, act, gated):
     rule = GluRule.of(act)
     _ok(lib().mrs_seq_moe_products(_p(rows), _p(up), _p(down), _p(counts), _i(n), _i(up.shape[0]), _i(W), _i(ff), _i(int(gated)), ctypes.byref(rule),
                                    _p(hidden), _p(out), _st(rows)), "moe_products")
+    return out
+
+
+ROUTE_SOFTMAX, ROUTE_SIGMOID, ROUTE_TOP_SOFTMAX = 0, 1, 2
+ONE_LAUNCH, GROUPED, STREAMED = 0, 1, 2
+
+
+def moe_block(x, router, logits, correction, up, down, top, gated, act, route, products, n_groups=1, keep_groups=1, renorm=False, group_top=1,
+              weight_scale=1.0, renorm_eps=0.0):
+    """A routed-expert block in one call: router [routes, W] (or logits [T, routes], already formed), the rule, the experts' products by the
+    kernels `products` names, the weighted sum: [T, W].  The same results as the calls it stands for."""
+    T, W = x.shape
+    ff, n_routes, pairs, code = down.shape[2], router.shape[0], T * top, DTYPE_CODE[x.dtype]
+    out = torch.empty(T, W, dtype=x.dtype, device=x.device)
+    size = pairs * (2 * W + ff) * x.element_size() + 4 * (3 * pairs + n_routes + T * n_routes) + 2048
+    scratch = torch.empty(size, dtype=torch.uint8, device=x.device)
+    a = MoeBlockArgs(x.data_ptr(), router.data_ptr(), logits.data_ptr() if logits is not None else None, logits.stride(0) if logits is not None else 0,
+                     correction.data_ptr() if correction is not None else None, up.data_ptr(), down.data_ptr(), scratch.data_ptr(), size, out.data_ptr(),
+                     code, T, W, ff, n_routes, up.shape[0], top, int(gated), route, products, n_groups, keep_groups, int(renorm), group_top, weight_scale,
+                     renorm_eps, GluRule.of(act))
+    _ok(lib().mrs_seq_moe_block(ctypes.byref(a), _st(x)), "moe_block")
     return out
 
 

@@ -102,6 +102,8 @@ extern "C" {
     pub fn mrs_seq_moe_route(logits: *const f32, correction: *const f32, n_tok: i32, n_experts: i32, n_groups: i32, keep_groups: i32, top: i32, renorm: i32, experts: *mut i32, weights: *mut f32, stream: i64) -> i32;
     pub fn mrs_seq_moe_route_scored(logits: *const f32, correction: *const f32, n_tok: i32, n_experts: i32, n_groups: i32, keep_groups: i32, top: i32, renorm: i32, score_fn: i32, group_top: i32, weight_scale: f32, experts: *mut i32, weights: *mut f32, stream: i64) -> i32;
     pub fn mrs_seq_moe_route_general(args: *const c_void, stream: i64) -> i32;
+    pub fn mrs_seq_moe_router(x: *const c_void, dtype: i32, w: *const f32, width: i32, args: *const c_void, stream: i64) -> i32;
+    pub fn mrs_seq_moe_router_fits(width: i32, n_experts: i32, n_tok: i32) -> i32;
     pub fn mrs_seq_router_logits(x: *const c_void, dtype: i32, w: *const f32, width: i32, n_experts: i32, n_tok: i32, logits: *mut f32, stream: i64) -> i32;
     pub fn mrs_seq_moe_gate_up(x: *const c_void, gate_up: *const c_void, dtype: i32, experts: *const i32, n_tok: i32, top: i32, width: i32, ff: i32, act: i32, hidden: *mut c_void, stream: i64) -> i32;
     pub fn mrs_seq_moe_down(hidden: *const c_void, down: *const c_void, dtype: i32, experts: *const i32, weights: *const f32, n_tok: i32, top: i32, width: i32, ff: i32, out: *mut c_void, stream: i64) -> i32;
@@ -122,4 +124,5 @@ extern "C" {
     pub fn mrs_seq_moe_place_fits(n_pairs: i32, n_experts: i32) -> i32;
     pub fn mrs_seq_moe_place(experts: *const i32, n_pairs: i32, n_experts: i32, x: *const c_void, dtype: i32, top: i32, width: i32, counts: *mut i32, inverse: *mut i32, sorted: *mut c_void, stream: i64) -> i32;
     pub fn mrs_seq_moe_combine_at(sorted_y: *const c_void, dtype: i32, inverse: *const i32, weights: *const f32, experts: *const i32, x: *const c_void, n_ffn: i32, n_tok: i32, top: i32, width: i32, out: *mut c_void, stream: i64) -> i32;
+    pub fn mrs_seq_moe_block(args: *const c_void, stream: i64) -> i32;
 }
