@@ -673,16 +673,17 @@ class RoutedExperts:
     those behind them are identity experts, which hand the sublayer's input back and have no weights."""
 
     # Where `seq_ops.moe_grouped` takes the sizes: steps of at least GROUPED_MIN_TOKENS tokens with up to GROUPED_PER_EXPERT pairs per
-    # expert on average run on it; smaller ones stream the weights once per pair.  Its arithmetic grows with the pairs (about 0.054 us
-    # per megabyte of weights that a pair reads), the one-launch products' does not: above one pair per expert and GROUPED_PAIR_BYTES they take
-    # over.  One B200, us of the block, grouped / one-launch: 16 experts, top 4, width and ff 2048 (25 MB each): 4 tokens 84 / 95,
-    # 8: 113 / 102, 16: 154 / 106, 32: 242 / 107; 8 experts, top 2, 2048 x 1024 (13 MB): 16 tokens 69 / 88, 32: 91 / 89; 32 experts, top 2,
-    # 1024 x 768 (5 MB): 64 tokens 100 / 89, 128: 140 / 99; 16 experts, top 4, 4096 x 2048 (50 MB): 4 tokens 127 / 147, 8: 165 / 164.  At the
-    # line (805 MB) with few experts the two are even for calls from the host (8 experts of 25 MB, top 8, 4 tokens: 91 / 92) and the one-launch
-    # products ahead in a graph (79 / 67).  The same line for steps that stream per pair: 8 experts of 100 MB, top 8, 2 tokens 657 / 186.
+    # expert on average run on it; smaller ones stream the weights once per pair.  Its arithmetic grows with the pairs, the one-launch
+    # products' does not: they take over at two pairs per expert (one, from 32 experts on) and ONE_LAUNCH_PAIRS pairs, or above one pair per
+    # expert and GROUPED_PAIR_BYTES of weights that the pairs read.  One B200, us of the block in a graph, grouped / one-launch: 16 experts,
+    # top 4, width and ff 2048 (25 MB each): 4 tokens 78 / 77, 6: 96 / 92, 8: 104 / 82, 32: 252 / 88; 8 experts, top 2, 2048 x 768 (9 MB): 4
+    # tokens 35 / 41, 6: 39 / 41, 12: 53 / 43, 32: 86 / 43; 8 experts, top 2, 1024 x 768 (5 MB): 8 tokens 31 / 35, 12: 35 / 35, 16: 43 / 35;
+    # 16 experts, top 2, 1024 x 768: 8 tokens 41 / 37, 12: 41 / 39, 32: 61 / 37; 32 experts, top 2, 1024 x 768: 8 tokens 41 / 39, 16: 53 / 43, 64:
+    # 92 / 49; 32 experts, top 4, 2048 x 2048: 4 tokens 92 / 96, 8: 135 / 115; 16 experts, top 4, 4096 x 2048 (50 MB): 4 tokens 139 / 133, 6: 158 /
+    # 150.  The bytes' line for steps that stream per pair: 8 experts of 100 MB, top 8, 2 tokens 657 / 186.
     # Elsewhere weights are streamed per pair up to 4 pairs per expert while an expert is small enough that repeated reads hit L2, up to
     # 2 above that.
-    GROUPED_MIN_TOKENS, GROUPED_PER_EXPERT, GROUPED_PAIR_BYTES = 4, 8, 700 << 20
+    GROUPED_MIN_TOKENS, GROUPED_PER_EXPERT, GROUPED_PAIR_BYTES, ONE_LAUNCH_PAIRS = 4, 8, 700 << 20, 20
     SMALL_EXPERT_BYTES = 32 << 20
     ROUTES = {"grouped_softmax": K.ROUTE_SOFTMAX, "grouped_sigmoid": K.ROUTE_SIGMOID, "top_softmax": K.ROUTE_TOP_SOFTMAX}
 
@@ -713,8 +714,9 @@ class RoutedExperts:
 
     def outgrows_groups(self, n_tok):
         """True when the one-launch products are the faster of the two for this many tokens."""
-        return (n_tok * self.top > self.n_experts and n_tok * self.top * self.expert_bytes() > self.GROUPED_PAIR_BYTES
-                and self.one_launch_products())
+        pairs, E = n_tok * self.top, self.n_experts
+        many = n_tok >= self.GROUPED_MIN_TOKENS and pairs >= max(self.ONE_LAUNCH_PAIRS, E if E >= 32 else 2 * E)
+        return (many or (pairs > E and pairs * self.expert_bytes() > self.GROUPED_PAIR_BYTES)) and self.one_launch_products()
 
     def expert_bytes(self):
         # (from the shapes: indexing two tensors took 3 us of the host, a twentieth of a small block's time)
