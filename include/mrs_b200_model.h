@@ -156,6 +156,8 @@ void mrs_add_rms_norm_pdl(const void *x, const void *residual, const void *weigh
                           int32_t nrows, int32_t ncols, float eps, int32_t dtype, int32_t pdl, void *stream);
 void mrs_split_glu_pdl(const void *input, void *output, uint32_t rows, uint32_t split_size, int32_t activation,
                        int32_t dtype, int32_t pdl, void *stream);
+void mrs_fused_glu_pdl(const void *a, const void *b, void *output, uint32_t rows, uint32_t cols, uint32_t a_row_stride, uint32_t b_row_stride,
+                       int32_t activation, int32_t dtype, int32_t pdl, void *stream);
 
 #ifdef __cplusplus
 }

@@ -105,6 +105,11 @@ int32_t mrs_mmq_gguf_ts(int32_t ggml_type, const void *w, const void *x, void *y
  * pointers on 16-byte boundaries); cudaErrorNotSupported (801), and nothing launched, where it does not fit. */
 int32_t mrs_mmq_gguf_multi(int32_t ggml_type, const void *w0, const void *w1, const void *w2, const void *x, void *y0, void *y1, void *y2,
                            int32_t M, int32_t n0, int32_t n1, int32_t n2, int32_t K, int32_t dtype, void *stream);
+/* The same two as links of a programmatic-dependent-launch chain: they may begin on the weights while the launch before them in the stream
+ * runs, so that launch must not write the weights, nor may one before it that has not ended; x and y are touched once it has ended. */
+int32_t mrs_mmq_gguf_chained(int32_t ggml_type, const void *w, const void *x, void *y, int32_t M, int32_t N, int32_t K, int32_t dtype, void *stream);
+int32_t mrs_mmq_gguf_multi_chained(int32_t ggml_type, const void *w0, const void *w1, const void *w2, const void *x, void *y0, void *y1, void *y2,
+                           int32_t M, int32_t n0, int32_t n1, int32_t n2, int32_t K, int32_t dtype, void *stream);
 int32_t mrs_mmq_timeouts(void);
 int32_t *mrs_mmq_timeout_flag(void);
 

@@ -393,6 +393,11 @@ extern "C" void mrs_add_rms_norm_pdl(const void *x, const void *residual, const 
   if (dtype == MRS_F16) launch_rms<__half>(x, residual, weight, residual_dst, norm_dst, nrows, ncols, eps, (cudaStream_t)stream, pdl);
   else if (dtype == MRS_BF16) launch_rms<__nv_bfloat16>(x, residual, weight, residual_dst, norm_dst, nrows, ncols, eps, (cudaStream_t)stream, pdl);
 }
+extern "C" void mrs_fused_glu_pdl(const void *a, const void *b, void *output, uint32_t rows, uint32_t cols, uint32_t a_row_stride, uint32_t b_row_stride,
+                                  int32_t activation, int32_t dtype, int32_t pdl, void *stream) {
+  if (dtype == MRS_F16) launch_glu<__half>(a, b, output, rows, cols, a_row_stride, b_row_stride, activation, (cudaStream_t)stream, pdl);
+  else if (dtype == MRS_BF16) launch_glu<__nv_bfloat16>(a, b, output, rows, cols, a_row_stride, b_row_stride, activation, (cudaStream_t)stream, pdl);
+}
 extern "C" void mrs_split_glu_pdl(const void *input, void *output, uint32_t rows, uint32_t split_size, int32_t activation,
                                   int32_t dtype, int32_t pdl, void *stream) {
   if (dtype == MRS_F16)

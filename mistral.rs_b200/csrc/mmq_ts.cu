@@ -120,8 +120,7 @@ extern "C" int32_t mrs_mmq_timeouts(void) {
 extern "C" int32_t *mrs_mmq_timeout_flag(void) { return ts_device().flag; }
 
 // returns cudaErrorNotSupported when the launch does not fit this kernel (the caller falls back to mmq_tc.cu)
-extern "C" int32_t mrs_mmq_gguf_ts(int32_t ggml_type, const void *w, const void *x, void *y, int32_t M, int32_t N, int32_t K,
-                                   int32_t dtype, void *stream) {
+static int32_t gguf_ts(int32_t ggml_type, const void *w, const void *x, void *y, int32_t M, int32_t N, int32_t K, int32_t dtype, int pdl, void *stream) {
   if (g_mmq_path == 1) return (int32_t)cudaErrorNotSupported;
   const int elems = blk_elems(ggml_type), bytes = blk_bytes(ggml_type);
   if (bytes == 0 || M <= 0 || N <= 0 || K <= 0 || K % elems != 0 || K % 64 != 0 || (dtype != 0 && dtype != 1)) return (int32_t)cudaErrorNotSupported;
@@ -135,7 +134,7 @@ extern "C" int32_t mrs_mmq_gguf_ts(int32_t ggml_type, const void *w, const void 
   // the dequantisers' weight in the plan's estimate
   const int clocks = ggml_type == MRS_Q6_K ? 1500 : ggml_type == MRS_Q5_K || ggml_type == MRS_Q3_K || ggml_type == MRS_Q5_0 || ggml_type == MRS_Q5_1 ? 1350 : 1150;
   const TsPlan plan = ts_plan(M, N, K, bytes * (256 / elems), clocks, TS_SPLIT_MIN_ROWS, d);
-  const TsCall c = {w, x, y, M, N, K, K / elems * bytes, dtype, plan.nt, plan.tiles_m, plan.ksplit, d.sms, d.timeouts, (cudaStream_t)stream, nullptr, nullptr, 0, 0, 0, 1, {}, {}, {}};
+  const TsCall c = {w, x, y, M, N, K, K / elems * bytes, dtype, plan.nt, plan.tiles_m, plan.ksplit, d.sms, d.timeouts, (cudaStream_t)stream, nullptr, nullptr, 0, 0, pdl, 1, {}, {}, {}};
   switch (ggml_type) {
 #define MRS_TS_CASE(T) case T: return (int32_t)ts_launch<T>(c);
   MRS_TS_TYPES(MRS_TS_CASE)
@@ -143,12 +142,29 @@ extern "C" int32_t mrs_mmq_gguf_ts(int32_t ggml_type, const void *w, const void 
   }
 }
 
+extern "C" int32_t mrs_mmq_gguf_ts(int32_t ggml_type, const void *w, const void *x, void *y, int32_t M, int32_t N, int32_t K,
+                                   int32_t dtype, void *stream) {
+  return gguf_ts(ggml_type, w, x, y, M, N, K, dtype, 0, stream);
+}
+
 namespace mrs { bool mmq_format_is_forced(); }      // mmq_tc.cu
+extern "C" int32_t mrs_mmq_gguf(int32_t ggml_type, const void *w, const void *x, void *y, int32_t M, int32_t N, int32_t K, int32_t dtype, void *stream);
+
+// A link of a programmatic-dependent-launch chain: begins on the weights while the launch before it runs.  A layer of a prompt call is ten
+// launches of 5 to 50 us, whose starts (tensor memory, first weights, 2 to 3 us) and ends were paid one after the other: eight layers of
+// 4096 x 14336, 300 tokens, 1716 to 1765 us so, 1622 with the products, the GLU and the norms as links.
+extern "C" int32_t mrs_mmq_gguf_chained(int32_t ggml_type, const void *w, const void *x, void *y, int32_t M, int32_t N, int32_t K, int32_t dtype, void *stream) {
+  if (M > 0 && N > 0 && !mmq_format_is_forced()) {
+    const int32_t e = gguf_ts(ggml_type, w, x, y, M, N, K, dtype, 1, stream);
+    if (e != (int32_t)cudaErrorNotSupported) return e;
+  }
+  return mrs_mmq_gguf(ggml_type, w, x, y, M, N, K, dtype, stream);
+}
 
 // y_i = x . w_i^T for two or three matrices of a type and as many columns (n2 = 0: two), as one launch.  cudaErrorNotSupported, and nothing launched,
 // where that does not fit this kernel: the caller launches them one by one.
-extern "C" int32_t mrs_mmq_gguf_multi(int32_t ggml_type, const void *w0, const void *w1, const void *w2, const void *x, void *y0, void *y1, void *y2, int32_t M,
-                                      int32_t n0, int32_t n1, int32_t n2, int32_t K, int32_t dtype, void *stream) {
+static int32_t gguf_multi(int32_t ggml_type, const void *w0, const void *w1, const void *w2, const void *x, void *y0, void *y1, void *y2, int32_t M, int32_t n0,
+                          int32_t n1, int32_t n2, int32_t K, int32_t dtype, int pdl, void *stream) {
   if (g_mmq_path == 1 || mmq_format_is_forced()) return (int32_t)cudaErrorNotSupported;
   const int elems = blk_elems(ggml_type), bytes = blk_bytes(ggml_type);
   if (bytes == 0 || M <= 0 || n0 <= 0 || n1 <= 0 || n2 < 0 || K <= 0 || K % elems != 0 || K % 64 != 0 || (K / elems * bytes) % 16 != 0 || (dtype != 0 && dtype != 1))
@@ -177,7 +193,7 @@ extern "C" int32_t mrs_mmq_gguf_multi(int32_t ggml_type, const void *w0, const v
     waves += one.waves;
   }
   if (plan.cost > 0.92 * alone || (M > 320 && plan.waves >= waves)) return (int32_t)cudaErrorNotSupported;
-  const TsCall c = {w0, x, y0, M, n0, K, K / elems * bytes, dtype, plan.nt, plan.tiles_m, plan.ksplit, d.sms, d.timeouts, (cudaStream_t)stream, nullptr, nullptr, 0, 0, 0,
+  const TsCall c = {w0, x, y0, M, n0, K, K / elems * bytes, dtype, plan.nt, plan.tiles_m, plan.ksplit, d.sms, d.timeouts, (cudaStream_t)stream, nullptr, nullptr, 0, 0, pdl,
                     n2 > 0 ? 3 : 2, {w1, w2}, {y1, y2}, {n1, n2}};
   switch (ggml_type) {
   case MRS_Q4_K: return (int32_t)ts_launch<MRS_Q4_K>(c);
@@ -186,4 +202,13 @@ extern "C" int32_t mrs_mmq_gguf_multi(int32_t ggml_type, const void *w0, const v
   case MRS_Q8_0: return (int32_t)ts_launch<MRS_Q8_0>(c);
   default: return (int32_t)cudaErrorNotSupported;
   }
+}
+
+extern "C" int32_t mrs_mmq_gguf_multi(int32_t ggml_type, const void *w0, const void *w1, const void *w2, const void *x, void *y0, void *y1, void *y2, int32_t M,
+                                      int32_t n0, int32_t n1, int32_t n2, int32_t K, int32_t dtype, void *stream) {
+  return gguf_multi(ggml_type, w0, w1, w2, x, y0, y1, y2, M, n0, n1, n2, K, dtype, 0, stream);
+}
+extern "C" int32_t mrs_mmq_gguf_multi_chained(int32_t ggml_type, const void *w0, const void *w1, const void *w2, const void *x, void *y0, void *y1, void *y2,
+                                              int32_t M, int32_t n0, int32_t n1, int32_t n2, int32_t K, int32_t dtype, void *stream) {
+  return gguf_multi(ggml_type, w0, w1, w2, x, y0, y1, y2, M, n0, n1, n2, K, dtype, 1, stream);
 }

@@ -27,24 +27,34 @@ def _check(w, xs):
 
 def forward(w, xs: torch.Tensor) -> torch.Tensor:
     """w: quant.QTensor [N, K]; xs [..., K] bf16/f16 -> [..., N]."""
+    return _linear("mrs_mmq_gguf", w, xs)
+
+
+def forward_chained(w, xs: torch.Tensor) -> torch.Tensor:
+    """`forward` for weights that nothing in flight writes: begins on them while the launch before it runs."""
+    return _linear("mrs_mmq_gguf_chained", w, xs)
+
+
+def _linear(name, w, xs):
     nrows, ncols = _check(w, xs)
     xs = xs.contiguous()
     M = xs.numel() // ncols
     out = xs.new_empty((*xs.shape[:-1], nrows))
-    entry = typed("mrs_mmq_gguf", _I, _P, _P, _P, _I, _I, _I, _I, _P)
+    entry = typed(name, _I, _P, _P, _P, _I, _I, _I, _I, _P)
     rc = entry(GGML[w.dtype], w.data.data_ptr(), xs.data_ptr(), out.data_ptr(), M, nrows, ncols, _DT_CODE[xs.dtype], raw_stream(xs.device))
     if rc != 0:
-        raise RuntimeError(f"mrs_mmq_gguf failed with cudaError {rc}")
+        raise RuntimeError(f"{name} failed with cudaError {rc}")
     return out
 
 
 _NOT_SUPPORTED = 801        # cudaErrorNotSupported: nothing was launched, alone is faster or what is possible
 
 
-def forward_many(ws, xs: torch.Tensor):
-    """[forward(w, xs) for w in ws], neighbours of one type as one launch (up to three) where that is faster."""
+def forward_many(ws, xs: torch.Tensor, chained=False):
+    """[forward(w, xs) for w in ws], neighbours of one type as one launch (up to three) where that is faster.  chained: as `forward_chained`."""
+    one = forward_chained if chained else forward
     if not xs.is_cuda:                     # (refused there)
-        return [forward(w, xs) for w in ws]
+        return [one(w, xs) for w in ws]
     for w in ws:
         _check(w, xs)
     xs = xs.contiguous()
@@ -61,14 +71,14 @@ def forward_many(ws, xs: torch.Tensor):
             data, rows, to = [w.data.data_ptr() for w in group], [w.shape[0] for w in group], [y.data_ptr() for y in ys]
             if n == 2:
                 data.append(None), rows.append(0), to.append(None)
-            entry = typed("mrs_mmq_gguf_multi", _I, *[_P] * 7, *[_I] * 6, _P)
+            entry = typed("mrs_mmq_gguf_multi_chained" if chained else "mrs_mmq_gguf_multi", _I, *[_P] * 7, *[_I] * 6, _P)
             rc = entry(GGML[group[0].dtype], *data, xs.data_ptr(), *to, M, *rows, xs.shape[-1], _DT_CODE[xs.dtype], raw_stream(xs.device))
             if rc == 0:
                 out += ys
                 continue
             if rc != _NOT_SUPPORTED:
                 raise RuntimeError(f"mrs_mmq_gguf_multi failed with cudaError {rc}")
-        out += [forward(w, xs) for w in group]
+        out += [one(w, xs) for w in group]
     return out
 
 

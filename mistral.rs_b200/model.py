@@ -721,16 +721,16 @@ class LlamaPrefill:
         scale = 1.0 / float(np.sqrt(D))
         h = ops.rms_norm(x, w.layers[0]["attn_norm"], cfg.rms_eps)
         for l, L in enumerate(w.layers):
-            q, k, v = (t.view(T, -1, D) for t in mmq.forward_many([qt(L[n]) for n in ("attn_q", "attn_k", "attn_v")], h))
+            q, k, v = (t.view(T, -1, D) for t in mmq.forward_many([qt(L[n]) for n in ("attn_q", "attn_k", "attn_v")], h, chained=True))
             ops.apply_rotary_qk(q, k, w.rope_cos, w.rope_sin, None, is_neox=cfg.rope_neox)
             attn = paged_attn.prefill_attention(q, k, v, scale)
             paged_attn.reshape_and_cache_flashinfer(k, v, self.k_cache[l], self.v_cache[l], slots)
-            o = mmq.forward(qt(L["attn_output"]), attn.view(T, H * D))
-            x, h2 = ops.add_rms_norm(o, x, L["ffn_norm"], cfg.rms_eps)       # x = o + x ; h2 = norm(x)
-            gate, up = mmq.forward_many([qt(L["ffn_gate"]), qt(L["ffn_up"])], h2)
-            d = mmq.forward(qt(L["ffn_down"]), ops.fused_glu(gate, up, 0))
+            o = mmq.forward_chained(qt(L["attn_output"]), attn.view(T, H * D))
+            x, h2 = ops.add_rms_norm_chained(o, x, L["ffn_norm"], cfg.rms_eps)       # x = o + x ; h2 = norm(x)
+            gate, up = mmq.forward_many([qt(L["ffn_gate"]), qt(L["ffn_up"])], h2, chained=True)
+            d = mmq.forward_chained(qt(L["ffn_down"]), ops.fused_glu_chained(gate, up, 0))
             nxt = w.layers[l + 1]["attn_norm"] if l + 1 < cfg.n_layers else w.output_norm
-            x, h = ops.add_rms_norm(d, x, nxt, cfg.rms_eps)                   # x = d + x ; h = next norm(x)
+            x, h = ops.add_rms_norm_chained(d, x, nxt, cfg.rms_eps)                   # x = d + x ; h = next norm(x)
         if all_logits:
             return mmq.forward(qt(w.output), h)
         return quant.plain(qt(w.output), h[T - 1:T].contiguous())[0]

@@ -9,7 +9,9 @@ import numpy as np
 import torch
 
 from . import lib
+from .quant import _F, _I, _P, raw_stream, typed
 
+_U = ctypes.c_uint32
 _TAG = {torch.float16: "f16", torch.bfloat16: "bf16", torch.float32: "f32"}
 _DT_CODE = {torch.float16: 0, torch.bfloat16: 1, torch.float32: 2}
 
@@ -36,6 +38,25 @@ def fused_glu(a, b, activation):
                                                   ctypes.c_uint32(a2.stride(0)), ctypes.c_uint32(b2.stride(0)),
                                                   ctypes.c_int(int(activation)), ctypes.c_void_p(_stream(a.device)))
     return out
+
+
+def fused_glu_chained(a, b, activation):
+    """`fused_glu` of contiguous 16-bit rows as a link of a chain of launches: the next one may begin while it runs."""
+    cols = a.shape[-1]
+    out = torch.empty_like(a)
+    entry = typed("mrs_fused_glu_pdl", _P, _P, _P, _U, _U, _U, _U, _I, _I, _I, _P)
+    entry(a.data_ptr(), b.data_ptr(), out.data_ptr(), a.numel() // cols, cols, cols, cols, int(activation), _DT_CODE[a.dtype], 1, raw_stream(a.device))
+    return out
+
+
+def add_rms_norm_chained(x, residual, weight, eps):
+    """`add_rms_norm` of contiguous 16-bit rows as a link of a chain of launches."""
+    cols = x.shape[-1]
+    s, n = torch.empty_like(x), torch.empty_like(x)
+    entry = typed("mrs_add_rms_norm_pdl", _P, _P, _P, _P, _P, _I, _I, _F, _I, _I, _P)
+    entry(x.data_ptr(), residual.data_ptr(), weight.data_ptr(), s.data_ptr(), n.data_ptr(), x.numel() // cols, cols, eps, _DT_CODE[x.dtype], 1,
+          raw_stream(x.device))
+    return s, n
 
 
 def fused_split_glu(x, activation):
