@@ -127,4 +127,8 @@ def fused_glu(gate_w, up_w, xs: torch.Tensor, activation) -> torch.Tensor:
 def fused_ffn(gate_w, up_w, down_w, xs: torch.Tensor, activation) -> torch.Tensor:
     if tuple(gate_w.shape) != tuple(up_w.shape):
         raise ValueError(f"fast_mmq fused_ffn: gate/up shape mismatch {tuple(gate_w.shape)} vs {tuple(up_w.shape)}")
-    return forward(down_w, fused_glu(gate_w, up_w, xs, activation))
+    if not xs.is_cuda:                     # (refused there)
+        return forward(down_w, fused_glu(gate_w, up_w, xs, activation))
+    # the first launch is a plain one: nothing that was in flight before it runs beside the links
+    from . import ops
+    return forward_chained(down_w, ops.fused_glu_chained(*forward_many([gate_w, up_w], xs), activation))
