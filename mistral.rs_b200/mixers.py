@@ -667,7 +667,7 @@ class RoutedExperts:
     `seq_ops.GluRule` (how gate and up are joined).  Experts are GLU feed-forwards (`gated`: w_up holds gate | up rows) or plain down(act(up h)); a
     `shared` feed-forward, when given, runs for every token and is added.  A few tokens: two
     weight-streaming kernels per (token, expert) pair.  A few tokens per expert: the same with every expert's weights read once for
-    all its pairs.  Many: rows sorted by expert, both products of all experts as one tcgen05 launch each (`seq_ops.moe_gemm`; the first
+    all its pairs.  Many: rows sorted by expert, both products of all experts as one tcgen05 launch each (`seq_ops.moe_products`; the first
     joins its halves), weighted combine in f32; in f32, or at sizes it does not take, one library product pair per expert that
     has rows (the per-expert row counts then cross to the host once per layer).  The router may have more outputs than there are experts:
     those behind them are identity experts, which hand the sublayer's input back and have no weights."""
