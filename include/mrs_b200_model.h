@@ -85,12 +85,16 @@ typedef struct {
   void *q8; int64_t q8_bytes;
   /* Only read when `extension` is MRS_LLAMA_STEP_RESIDENT (which has q8 too).  Scratch of at least mrs_llama_resident_bytes bytes, zeroed once, 16-byte
    * aligned, of this step alone: with it a step of one sequence may run as one resident grid (csrc/step_resident.cu, a cooperative launch) instead of a
-   * chain of launches: the same bits in the same buffers, but tmp_v, tmp_s and attn_counters are then left as they are. */
+   * chain of launches: the same bits in the same buffers, but tmp_v, tmp_s and attn_counters are then left as they are.  A grid whose wait ran out leaves
+   * NaN in its logits, sets the device's word (mrs_mmq_timeout_flag) and leaves the first word of the scratch at 0x80000000: every later launch with it,
+   * replays of a graph among them, then ends at once in the same way.  The scratch serves again once it is zeroed, with no step in flight. */
   void *resident; int64_t resident_bytes;
 } mrs_llama_step;
 #define MRS_LLAMA_STEP_Q8 0x51380001
 #define MRS_LLAMA_STEP_RESIDENT 0x51380002
 int64_t mrs_llama_resident_bytes(int32_t n_heads, int32_t head_dim, int32_t padded_tiles);
+/* 1 where mrs_llama_decode_step would now run this step as a resident grid. */
+int32_t mrs_llama_step_is_resident(const mrs_llama_step *s);
 
 /* Enqueue one decode step (all layers + lm_head + argmax) on `stream`. Returns cudaError. */
 int32_t mrs_llama_decode_step(const mrs_llama_step *s, void *stream);

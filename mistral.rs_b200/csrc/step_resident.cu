@@ -10,8 +10,10 @@
 //   warps 16..19  producers, one for four consumers: lane = (consumer warp, row of its pair), one cp.async.bulk a row segment into the group's ring
 //
 // A layer has five grid barriers: q / k / v, attention, o_proj, gate and up, down.  The grid is launched as a cooperative one, so all its CTAs run at
-// the same time.  Every wait has a limit; one that runs out ends the grid (each CTA sees its copies land first) and sets the device's word
-// (mrs_mmq_timeout_flag), after which steps are launched as a chain again; graph replays are told by mmq.check_timeouts.
+// the same time.  Every wait has a limit; one that runs out ends the grid (each CTA sees its copies land first), leaves NaN in the logits of each CTA that
+// it stopped and sets the device's word (mrs_mmq_timeout_flag), after which steps are launched as a chain again.  The grid's own word of arrivals then
+// stays RS_DEAD: a later launch with the same scratch (a replay passes no host code) leaves at its first meeting, its logits NaN, and sets the device's word
+// again.  A runner's replay and mmq.check_timeouts look at that word.
 //
 // Every operation is the chain's, in its order, so the bits of logits and caches are the chain's too.  (They have to be: the 8-bit quants of a layer's five
 // products blow up any difference, f32 sums in another order left eight layers' logits as far from the chain's as from exact ones.)
@@ -48,6 +50,7 @@ constexpr int RS_HEADER = 1024;          // barriers, offsets, small exchanges
 // 263 / 281; 8 KV heads, 892 tokens 236 / 213).
 constexpr int RS_MIN_HIDDEN = 2560, RS_MAX_KV_HEADS = 16, RS_MAX_TILE = 8192;      // tile: tokens x KV heads
 constexpr uint32_t RS_COPY_LIMIT = 1u << 22, RS_GRID_LIMIT = 1u << 22;      // polls (seconds)
+constexpr uint32_t RS_DEAD = 1u << 31;   // in the word of arrivals: a wait of this step ran out, now or in a launch before (arrivals stay far below)
 
 struct RsLayer {
   const uint8_t *w[7];                   // q, k, v, o, gate, up, down
@@ -64,7 +67,7 @@ struct RsParams {
   const int32_t *kv_indptr, *kv_indices, *last_page, *tile_ends, *tile_size;
   void *x, *x2, *q, *k, *v, *attn, *act, *logits;
   float *part;                           // [tiles][heads][D], then two words a tile and head
-  uint32_t *sync;                        // arrivals, CTAs that are done, tiles of each KV head: zero between launches
+  uint32_t *sync;                        // arrivals (or RS_DEAD), CTAs that are done, tiles of each KV head: zero between launches
   int *timeouts;
   float eps, scale_log2;
   int layers, hidden, inter, nq, nkv, heads, kv_heads, page_size, page_shift, vocab, head_type, interleaved, tiles;
@@ -344,13 +347,26 @@ __device__ __forceinline__ bool rs_meet(const RsParams &p, RsShared &sh, uint32_
     uint32_t n = *(volatile int *)&sh.stop ? RS_GRID_LIMIT : 0u, seen;
     for (;; n++) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(p.sync) : "memory");
-      if (n >= RS_GRID_LIMIT || (int32_t)(seen - round) >= 0) break;
+      if (n >= RS_GRID_LIMIT || (seen & RS_DEAD) || seen >= round) break;
     }
-    if (n >= RS_GRID_LIMIT) { *(volatile int *)p.timeouts = 1; *(volatile int *)&sh.stop = 1; }
-    sh.go = n < RS_GRID_LIMIT;          // (one thread's finding: all of the CTA's threads leave, or none)
+    sh.go = n < RS_GRID_LIMIT && !(seen & RS_DEAD);          // (one thread's finding: all of the CTA's threads leave, or none)
   }
   rs_bar();
   return *(volatile int *)&sh.go != 0;
+}
+
+// The CTA leaves a step that is lost: its own copies have landed (the producers see to theirs), its rows of the logits are NaN, and the word of arrivals
+// sends the other CTAs, and launches to come, the same way.  A lost step is not counted as done, so nothing makes the word zero again.
+__device__ __forceinline__ void rs_lost(const RsParams &p, RsShared &sh, int dt, int tid) {
+  if (tid == 0) {
+    *(volatile int *)&sh.stop = 1;
+    *(volatile int *)p.timeouts = 1;
+    atomicExch(p.sync, RS_DEAD);
+  }
+  cp_async_wait<0>();
+  if (p.head == nullptr) return;         // (the launch behind this one has the head)
+  const RsOp o = rs_op(p, 5 * p.layers);
+  for (int row = 2 * o.first + tid; row < min(2 * (o.first + o.count), p.vocab); row += RS_CT) store_act(p.logits, row, __int_as_float(0x7FC00000), dt);
 }
 
 template <typename T> __device__ __forceinline__ void rs_unpack8(const uint4 &v, float *f) {
@@ -376,10 +392,9 @@ template <int TYPE> __device__ __forceinline__ void rs_store_chunk(uint8_t *img,
   U::side(e, d, isum16, img + (size_t)npos * 16 * U::WORDS, npos, pos);
 }
 
-__device__ __forceinline__ void rs_landed(const RsParams &p, RsShared &sh, RsRing &rr, int group, int slot) {
+__device__ __forceinline__ void rs_landed(RsShared &sh, RsRing &rr, int group, int slot) {
   if (!mbar_wait_warp(&sh.full[group][slot], (rr.at.seq / RS_DEPTH) & 1, rr.dead ? 1u : RS_COPY_LIMIT)) {
     rr.dead = true;
-    *(volatile int *)p.timeouts = 1;
     *(volatile int *)&sh.stop = 1;
   }
 }
@@ -402,7 +417,7 @@ __device__ __forceinline__ void rs_gemv(const RsParams &p, const RsOp &o, RsShar
     if (mine + RS_WARPS * j >= o.count) {        // a round without rows for this warp
       for (int s = 0; s < nseg; s++) {
         const int slot = (int)(rr.at.seq & (RS_DEPTH - 1));
-        rs_landed(p, sh, rr, group, slot);
+        rs_landed(sh, rr, group, slot);
         if (lane == 0) mbar_arrive(&sh.empty[group][slot]);
         rr.at.pos = rs_place(rr.at, size, p.ring) + size; rr.at.seq++;
       }
@@ -420,7 +435,7 @@ __device__ __forceinline__ void rs_gemv(const RsParams &p, const RsOp &o, RsShar
     for (int s = 0; s < nseg; s++) {
       const int slot = (int)(rr.at.seq & (RS_DEPTH - 1));
       const uint32_t at = rs_place(rr.at, size, p.ring), sp = (uint32_t)(s * G::SEG_BYTES);
-      rs_landed(p, sh, rr, group, slot);
+      rs_landed(sh, rr, group, slot);
       const uint8_t *wp0 = ring + at + rows_at + (G::ALIGNED ? 0u : ((ph0 + sp) & 15u));
       const uint8_t *wp1 = ring + at + rows_at + G::SLOT + (G::ALIGNED ? 0u : ((ph1 + sp) & 15u));
       if (s * G::SEG_BLOCKS + lblk < nblocks) {
@@ -826,6 +841,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) step_resident_kernel(const __gr
   RsRing rr = {{0u, 0u}, false};
   uint32_t round = 0;
   const int ops = 5 * p.layers + (p.head != nullptr ? 1 : 0);
+  constexpr int DT = std::is_same<T, __half>::value ? MRS_F16 : MRS_BF16;
   for (int i = 0; i < ops; i++) {
     const RsOp o = rs_op(p, i);
     const RsLayer &L = p.L[min(i / 5, p.layers - 1)];
@@ -837,10 +853,10 @@ __global__ void __launch_bounds__(RS_THREADS, 1) step_resident_kernel(const __gr
       uint4 nw0 = make_uint4(0u, 0u, 0u, 0u);
       if (norm_w != nullptr && tid < (o.K >> 3)) nw0 = __ldg((const uint4 *)norm_w + tid);
       if (o.kind == RS_O) {
-        if (!rs_attend<T, D>(p, L, sh, img, round, tiles, chunk, kv_len, page0, tid, warp, lane)) return;
+        if (!rs_attend<T, D>(p, L, sh, img, round, tiles, chunk, kv_len, page0, tid, warp, lane)) return rs_lost(p, sh, DT, tid);
         rs_arrive(p, tid);
       }
-      if (i > 0 && !rs_meet(p, sh, round, tid)) return;
+      if (i > 0 && !rs_meet(p, sh, round, tid)) return rs_lost(p, sh, DT, tid);
       rs_quantise<T>(p, o, sh, o.kind == RS_QK ? L.type[RS_V] : o.type, norm_w, nw0, img, tid, warp, lane);
     }
     switch (o.type) {
@@ -852,6 +868,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) step_resident_kernel(const __gr
   }
   // the last CTA leaves the words as it found them
   rs_bar();
+  if (*(volatile int *)&sh.stop) return rs_lost(p, sh, DT, tid);
   if (tid == 0) {
     __threadfence();
     if (atomicAdd(p.sync + 1, 1u) == gridDim.x - 1) { p.sync[0] = 0u; p.sync[1] = 0u; }
@@ -882,28 +899,27 @@ extern "C" int64_t mrs_llama_resident_bytes(int32_t heads, int32_t head_dim, int
   return 256 + (int64_t)padded_tiles * heads * (head_dim + 2) * 4;
 }
 
-// Layers and head of a step, its first hidden state in s->x.  cudaErrorNotSupported, and nothing launched, where the step is not of the kind described
-// above: the caller launches its chain.
-extern "C" int32_t mrs_llama_step_resident(const mrs_llama_step *s, void *stream) {
-  const int no = (int)cudaErrorNotSupported, D = s->head_dim, dt = s->act_dtype;
+// The launch's parameters but for the layers, its CTAs and their shared memory; false where the step is not of the kind described above.
+static bool rs_plan(const mrs_llama_step *s, RsParams &p, int &sms, size_t &smem) {
+  const int D = s->head_dim, dt = s->act_dtype;
   if (s->extension != MRS_LLAMA_STEP_RESIDENT || s->resident == nullptr || ((uintptr_t)s->resident & 15) || s->batch != 1 || s->skip_mask != 0 ||
       !s->fused_attention || s->tp != nullptr || s->all_reduce != nullptr || (D != 64 && D != 128) || (dt != MRS_F16 && dt != MRS_BF16) || s->n_layers < 1)
-    return no;
+    return false;
   if (s->n_kv_heads < 1 || s->n_heads % s->n_kv_heads != 0 || s->n_heads / s->n_kv_heads > 8 || s->n_kv_heads > RS_MAX_KV_HEADS ||
       s->hidden % 256 != 0 || s->hidden < RS_MIN_HIDDEN || s->block_size < 1 || s->vocab < 1 ||
       s->padded_tiles < 1 || s->padded_tiles > RS_TILES || s->tmp_v == nullptr || s->resident_bytes < mrs_llama_resident_bytes(s->n_heads, D, s->padded_tiles))
-    return no;
-  if ((int64_t)s->max_blocks_per_seq * s->block_size / s->padded_tiles * s->n_kv_heads > RS_MAX_TILE) return no;
-  int dev = 0, sms = 0, most = 0, coop = 0;
+    return false;
+  if ((int64_t)s->max_blocks_per_seq * s->block_size / s->padded_tiles * s->n_kv_heads > RS_MAX_TILE) return false;
+  int dev = 0, most = 0, coop = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   int32_t *const timeouts = mrs_mmq_timeout_flag();
-  if (!coop || (int64_t)s->padded_tiles * s->n_kv_heads > sms || timeouts == nullptr || *(volatile const int32_t *)timeouts != 0) return no;
+  if (!coop || (int64_t)s->padded_tiles * s->n_kv_heads > sms || timeouts == nullptr || *(volatile const int32_t *)timeouts != 0) return false;
 
   const int nq = s->n_heads * D, nkv = s->n_kv_heads * D, inter = s->layers[0].w_down.cols;
-  RsParams p = {};
+  p = {};
   p.x_bytes = D == 64 ? rs_attend_bytes<64>() : rs_attend_bytes<128>();
   int widest = 0;
   auto usable = [&](const mrs_qweight &w, int rows, int K) {
@@ -916,25 +932,25 @@ extern "C" int32_t mrs_llama_step_resident(const mrs_llama_step *s, void *stream
   };
   auto image = [&](int bytes) { if (bytes > p.x_bytes) p.x_bytes = bytes; };
   const void *aligned[] = {s->x, s->x2, s->q, s->k, s->v, s->attn_out, s->act, s->final_norm, s->rope_cos, s->rope_sin};
-  for (const void *a : aligned) if (a == nullptr || ((uintptr_t)a & 15)) return no;
+  for (const void *a : aligned) if (a == nullptr || ((uintptr_t)a & 15)) return false;
   for (int l = 0; l < s->n_layers; l++) {
     const mrs_llama_layer &L = s->layers[l];
     if (!usable(L.wq, nq, s->hidden) || !usable(L.wk, nkv, s->hidden) || !usable(L.wv, nkv, s->hidden) || !usable(L.wo, s->hidden, nq) ||
         !usable(L.w_gate, inter, s->hidden) || !usable(L.w_up, inter, s->hidden) || !usable(L.w_down, s->hidden, inter) ||
         L.wq.ggml_type != L.wk.ggml_type || L.w_gate.ggml_type != L.w_up.ggml_type)
-      return no;
+      return false;
     const void *ptrs[] = {L.attn_norm, L.ffn_norm, L.k_cache, L.v_cache};
-    for (const void *a : ptrs) if (a == nullptr || ((uintptr_t)a & 15)) return no;
+    for (const void *a : ptrs) if (a == nullptr || ((uintptr_t)a & 15)) return false;
     image(rs_image(L.wq.ggml_type, s->hidden) + (L.wv.ggml_type != L.wq.ggml_type ? rs_image(L.wv.ggml_type, s->hidden) : 0));
     image(rs_image(L.wo.ggml_type, nq));
     image(rs_image(L.w_gate.ggml_type, s->hidden));
     image(rs_image(L.w_down.ggml_type, inter));
   }
-  if (!usable(s->lm_head, s->vocab, s->hidden)) return no;
+  if (!usable(s->lm_head, s->vocab, s->hidden)) return false;
   image(rs_image(s->lm_head.ggml_type, s->hidden));
   p.x_bytes = (p.x_bytes + 127) & ~127;
   p.ring = (most - RS_HEADER - p.x_bytes) / RS_PRODUCERS & ~15;
-  if (p.ring < 4 * RS_GROUP * widest) return no;                 // two stages at least
+  if (p.ring < 4 * RS_GROUP * widest) return false;                 // two stages at least
 
   p.final_norm = s->final_norm; p.rope_cos = s->rope_cos; p.rope_sin = s->rope_sin;
   p.positions = s->positions; p.slots = s->slot_mapping;
@@ -950,7 +966,26 @@ extern "C" int32_t mrs_llama_step_resident(const mrs_llama_step *s, void *stream
   p.page_shift = -1;
   for (int i = 0; i < 31; i++) if (s->block_size == 1 << i) p.page_shift = i;
   p.vocab = s->vocab; p.head_type = s->lm_head.ggml_type; p.interleaved = s->rope_neox ? 0 : 1;
-  const size_t smem = RS_HEADER + p.x_bytes + (size_t)RS_PRODUCERS * p.ring;
+  smem = RS_HEADER + p.x_bytes + (size_t)RS_PRODUCERS * p.ring;
+  return true;
+}
+
+// 1 where mrs_llama_decode_step would run this step as a resident grid.
+extern "C" int32_t mrs_llama_step_is_resident(const mrs_llama_step *s) {
+  RsParams p;
+  int sms = 0;
+  size_t smem = 0;
+  return rs_plan(s, p, sms, smem) ? 1 : 0;
+}
+
+// Layers and head of a step, its first hidden state in s->x.  cudaErrorNotSupported, and nothing launched, where the step is not of the kind described
+// above: the caller launches its chain.
+extern "C" int32_t mrs_llama_step_resident(const mrs_llama_step *s, void *stream) {
+  const int no = (int)cudaErrorNotSupported, D = s->head_dim, dt = s->act_dtype;
+  RsParams p;
+  int sms = 0;
+  size_t smem = 0;
+  if (!rs_plan(s, p, sms, smem)) return no;
   for (int l0 = 0; l0 < s->n_layers; l0 += RS_LAYERS) {
     p.layers = s->n_layers - l0 < RS_LAYERS ? s->n_layers - l0 : RS_LAYERS;
     p.head = l0 + p.layers == s->n_layers ? (const uint8_t *)s->lm_head.data : nullptr;

@@ -82,17 +82,22 @@ def forward_many(ws, xs: torch.Tensor, chained=False):
     return out
 
 
-def check_timeouts(device):
-    """Raises when a wait inside a kernel that shares this word ever ran out on `device`: the dequantising GEMM (ggml and int4 linears), the tensor-core
-    GEMV (three to eight rows over large matrices) and prompt attention.  Results since then are incomplete.  Reads a word in host memory, so call
-    it once the work in question is done.  Calls that would run on one of these kernels are refused by themselves from then on; replays of a
-    graph pass no entry point and need this."""
+def timeout_word(device):
+    """The word that a kernel sets when a wait of its runs out on `device`: an int32 in host memory, as a ctypes pointer."""
     with torch.cuda.device(device):
         fn = lib().mrs_mmq_timeout_flag
         fn.restype = ctypes.POINTER(ctypes.c_int32)
-        flag = fn()
+        return fn()
+
+
+def check_timeouts(device):
+    """Raises when a wait inside a kernel that shares this word ever ran out on `device`: the dequantising GEMM (ggml and int4 linears), the tensor-core
+    GEMV (three to eight rows over large matrices), prompt attention and the resident grid of one-sequence decode steps.  Results since then are
+    incomplete.  Reads a word in host memory, so call it once the work in question is done.  Calls that would run on one of these kernels are refused by
+    themselves from then on (decode steps of one sequence run as a chain of launches instead); replays of a graph pass no entry point and need this."""
+    flag = timeout_word(device)
     if flag and flag[0]:
-        raise RuntimeError("a wait inside a linear or prompt attention ran out: the results of this device are incomplete")
+        raise RuntimeError("a wait inside a linear, prompt attention or a resident decode step ran out: the results of this device are incomplete")
 
 
 def set_path(path: str):

@@ -599,7 +599,7 @@ class LlamaRunner:
             self._ar_cb = _AR_FN(comm)
             s.all_reduce = self._ar_cb
         self.step_struct = s
-        self.graph = None
+        self.graph, self._lost = None, None       # _lost: the device's word for waits that ran out, where the graph holds a resident grid
 
     # ---- eager pieces -------------------------------------------------------------------
     def _stream(self):
@@ -623,6 +623,10 @@ class LlamaRunner:
         if rc != 0:
             raise RuntimeError(f"mrs_llama_decode_step failed: cudaError {rc}")
 
+    def is_resident(self):
+        """True where a step runs as one resident grid (csrc/step_resident.cu) and not as a chain of launches."""
+        return bool(lib().mrs_llama_step_is_resident(ctypes.byref(self.step_struct)))
+
     def step(self):
         """advance the KV metadata for the token in `token_ids`, run the stack, argmax -> token_ids."""
         if self.steps_taken >= self.max_ctx and not torch.cuda.is_current_stream_capturing():
@@ -637,21 +641,25 @@ class LlamaRunner:
 
     def replay(self):
         """one captured decode step; raises before a sequence would run past the allocated context
-        (the kernels freeze such a sequence and set error_flag, but a caller should never get there)"""
+        (the kernels freeze such a sequence and set error_flag, but a caller should never get there), and once a wait on this
+        device has run out where the captured step is a resident grid, which does not run any more then (capture again: a chain of launches)"""
         if self.steps_taken >= self.max_ctx:
             raise RuntimeError(f"LlamaRunner: context exhausted ({self.max_ctx} tokens: block table / RoPE table)")
+        if self._lost and self._lost[0]:
+            mmq.check_timeouts(self.dev)
         self.steps_taken += 1
         self.graph.replay()
 
     def check_overflow(self):
         if int(self.error_flag.item()) & 1:
             raise RuntimeError("LlamaRunner: a sequence ran past its allocated context (KV write skipped)")
-        mmq.check_timeouts(self.dev)      # (of prompts read on the same device; the flag above was read behind them)
+        mmq.check_timeouts(self.dev)      # (of resident steps, and of prompts read on the same device; the flag above was read behind them)
 
     def capture(self):
         self.step(); self.reset()  # warm-up outside capture (module load, attributes)
         torch.cuda.synchronize()
         g = torch.cuda.CUDAGraph(keep_graph=True)   # keep_graph: the kernel nodes can be counted afterwards
+        self._lost = mmq.timeout_word(self.dev) if self.is_resident() else None
         with torch.cuda.graph(g):
             self.step()
         self.reset()

@@ -3,7 +3,7 @@ the same order, so the same bits in every vector, cache row and logit."""
 import pytest
 import torch
 
-from mistralrs_b200 import model as M
+from mistralrs_b200 import mmq, model as M
 
 pytestmark = pytest.mark.gpu
 
@@ -116,3 +116,73 @@ def test_what_the_grid_declines(cuda, monkeypatch):
     assert all(torch.equal(a, b) for a, b in zip(before, resident.k_cache + resident.v_cache))
     assert int(resident.error_flag.item()) & 1 and _ran_resident(resident)
     assert bool(torch.isfinite(resident.logits().float()).all())
+
+
+def test_steps_go_on_as_a_chain_once_a_wait_has_run_out(cuda, monkeypatch):
+    """The device's word, set here by the host: eager steps are the chain's and leave the scratch alone, replays of a resident grid are refused, and a
+    step that is captured then is a chain."""
+    resident, chain = _pair(cuda, monkeypatch, "gqa4", "q4_k_m", torch.float16)
+    resident.capture()
+    chain.capture()                          # (a capture's warm-up step writes position 0)
+    assert resident.is_resident() and not chain.is_resident()
+    flag = mmq.timeout_word(cuda)
+    try:
+        flag[0] = 1
+        scratch = resident.resident.clone()
+        _same(resident, chain, 100)
+        assert torch.equal(resident.resident, scratch) and not resident.is_resident()
+        with pytest.raises(RuntimeError, match="ran out"):
+            resident.replay()
+        chain.reset(101)
+        chain.replay()                       # (no kernel of this graph knows the word)
+        resident.capture()
+        chain.capture()
+        for run in (resident, chain):
+            run.reset(120)
+            run.set_tokens([5])
+            run.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(resident.logits(), chain.logits()) and torch.equal(resident.resident, scratch)
+    finally:
+        flag[0] = 0
+    assert resident.is_resident()
+
+
+@pytest.mark.parametrize("layers", [1, 33])
+def test_a_lost_grid_stays_lost(cuda, monkeypatch, layers):
+    """What a grid whose wait ran out leaves in its scratch, put there by the host: launches with it, replays and eager ones, end at their first meeting with
+    NaN for logits, no cache row written and the device's word set, in one launch and in two; zeroed, the scratch serves again."""
+    run, _ = _pair(cuda, monkeypatch, "gqa2_64", "q4_k_m", torch.bfloat16, layers=layers)
+    run.capture()
+
+    def replay():
+        run.reset(100)
+        run.set_tokens([9])
+        run.replay()
+        torch.cuda.synchronize()
+        return run.logits().clone()
+
+    want, flag = replay(), mmq.timeout_word(cuda)
+    word = run.resident[:4].view(torch.int32)
+    assert bool(torch.isfinite(want.float()).all()) and int(word) == 0 and flag[0] == 0
+    caches = [t.clone() for t in run.k_cache + run.v_cache]
+    try:
+        word.fill_(-2 ** 31)
+        for launch in (run.replay, run.step, run.replay):
+            flag[0] = 0                      # (only then does a call reach the grid)
+            run.reset(200)
+            run.set_tokens([9])
+            run.logits().zero_()
+            launch()
+            torch.cuda.synchronize()
+            assert flag[0] == 1 and int(word) == -2 ** 31
+            assert bool(torch.isnan(run.logits()).all()) and 0 <= int(run.meta["token_ids"][0]) < run.cfg.vocab
+            assert all(torch.equal(a, b) for a, b in zip(caches, run.k_cache + run.v_cache))
+        with pytest.raises(RuntimeError, match="ran out"):
+            run.replay()
+        with pytest.raises(RuntimeError, match="ran out"):
+            run.check_overflow()
+    finally:
+        flag[0] = 0
+        run.resident[:256].zero_()
+    assert torch.equal(replay(), want) and int(word) == 0
