@@ -332,7 +332,7 @@ __device__ __forceinline__ void rs_produce(const RsParams &p, RsShared &sh, uint
 }
 
 // ---------------------------------------------------------------- consumers
-struct RsRing { RsStage at; bool dead; };      // where the warp reads; a wait of its own ran out
+struct RsRing { RsStage at; uint32_t polls; bool gives; };      // where the warp reads; its waits' limit; the lane gives stages back (the first, until a wait ran out)
 
 __device__ __forceinline__ void rs_bar() { asm volatile("bar.sync 1, %0;" ::"n"(RS_CT) : "memory"); }
 
@@ -392,9 +392,11 @@ template <int TYPE> __device__ __forceinline__ void rs_store_chunk(uint8_t *img,
   U::side(e, d, isum16, img + (size_t)npos * 16 * U::WORDS, npos, pos);
 }
 
+// (a lane whose wait ran out gives no stage back from then on: copies may be on their way still, and the producer waits for them at its end)
 __device__ __forceinline__ void rs_landed(RsShared &sh, RsRing &rr, int group, int slot) {
-  if (!mbar_wait_warp(&sh.full[group][slot], (rr.at.seq / RS_DEPTH) & 1, rr.dead ? 1u : RS_COPY_LIMIT)) {
-    rr.dead = true;
+  if (!mbar_wait_warp(&sh.full[group][slot], (rr.at.seq / RS_DEPTH) & 1, rr.polls)) {
+    rr.polls = 1u;
+    rr.gives = false;
     *(volatile int *)&sh.stop = 1;
   }
 }
@@ -418,7 +420,7 @@ __device__ __forceinline__ void rs_gemv(const RsParams &p, const RsOp &o, RsShar
       for (int s = 0; s < nseg; s++) {
         const int slot = (int)(rr.at.seq & (RS_DEPTH - 1));
         rs_landed(sh, rr, group, slot);
-        if (lane == 0) mbar_arrive(&sh.empty[group][slot]);
+        if (rr.gives) mbar_arrive(&sh.empty[group][slot]);
         rr.at.pos = rs_place(rr.at, size, p.ring) + size; rr.at.seq++;
       }
       continue;
@@ -448,7 +450,7 @@ __device__ __forceinline__ void rs_gemv(const RsParams &p, const RsOp &o, RsShar
         U::add(acc1, wp1, t, x);
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sh.empty[group][slot]);
+      if (rr.gives) mbar_arrive(&sh.empty[group][slot]);
       rr.at.pos = at + size; rr.at.seq++;
     }
     // both rows' sums in one butterfly: lanes 0..15 the first's, 16..31 the second's
@@ -838,7 +840,7 @@ __global__ void __launch_bounds__(RS_THREADS, 1) step_resident_kernel(const __gr
   const int page0 = p.kv_indptr[0], kv_len = (p.kv_indptr[1] - page0 - 1) * p.page_size + p.last_page[0];
   // the tiles of the step's plan
   const int tiles = p.tiles > 1 ? p.tile_ends[1] : 1, chunk = p.tiles > 1 ? *p.tile_size : kv_len;
-  RsRing rr = {{0u, 0u}, false};
+  RsRing rr = {{0u, 0u}, RS_COPY_LIMIT, lane == 0};
   uint32_t round = 0;
   const int ops = 5 * p.layers + (p.head != nullptr ? 1 : 0);
   constexpr int DT = std::is_same<T, __half>::value ? MRS_F16 : MRS_BF16;
