@@ -43,3 +43,15 @@ def test_chained_block_is_the_plain_one(cuda, kind, down, tokens, dtype):
     want, got = turns(False), turns(True)
     mmq.check_timeouts(cuda)
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and bool(torch.isfinite(want[1].float()).all())
+
+
+def test_links_refuse_what_their_kernels_do_not_take(cuda):
+    x, w = torch.ones(40, 512, dtype=torch.float16, device=cuda), torch.ones(512, dtype=torch.float16, device=cuda)
+    for a, b in ((x.float(), x.float()), (x, x.bfloat16()), (x, x[:2]), (x, x.cpu()), (x[:, ::2], x[:, ::2])):
+        with pytest.raises(ValueError, match="fused_glu_chained"):
+            ops.fused_glu_chained(a, b, 0)
+        with pytest.raises(ValueError, match="add_rms_norm_chained"):
+            ops.add_rms_norm_chained(a, b, w, 1e-5)
+    for weight in (w.float(), w[:256], w.cpu(), torch.ones(1024, dtype=torch.float16, device=cuda)[::2]):
+        with pytest.raises(ValueError, match="weight"):
+            ops.add_rms_norm_chained(x, x, weight, 1e-5)

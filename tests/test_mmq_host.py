@@ -37,3 +37,13 @@ def test_shape_mismatch_messages(cpu_kernels):
         mmq.fused_glu(_w(64, 32, 1), _w(48, 32, 2), x, 0)
     with pytest.raises(ValueError, match="fused_ffn: gate/up shape mismatch"):
         mmq.fused_ffn(_w(64, 32, 1), _w(48, 32, 2), _w(32, 64, 3), x, 0)
+
+
+def test_links_of_a_chain_refuse_what_their_kernels_do_not_take():
+    """Other types (the kernels' entries launch nothing for f32), shapes that differ, rows with gaps, host memory: refused before anything is launched."""
+    x, w = torch.ones(4, 16, dtype=torch.bfloat16), torch.ones(16, dtype=torch.bfloat16)
+    for a, b in ((x.float(), x.float()), (x, x.half()), (x, x[:2]), (x, x[:, :8]), (x[:, ::2], x[:, ::2]), (x, x)):
+        with pytest.raises(ValueError, match="fused_glu_chained"):
+            ops.fused_glu_chained(a, b, 0)
+        with pytest.raises(ValueError, match="add_rms_norm_chained"):
+            ops.add_rms_norm_chained(a, b, w, 1e-5)
