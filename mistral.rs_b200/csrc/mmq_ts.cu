@@ -166,8 +166,9 @@ extern "C" int32_t mrs_mmq_gguf_chained(int32_t ggml_type, const void *w, const 
 static int32_t gguf_multi(int32_t ggml_type, const void *w0, const void *w1, const void *w2, const void *x, void *y0, void *y1, void *y2, int32_t M, int32_t n0,
                           int32_t n1, int32_t n2, int32_t K, int32_t dtype, int pdl, void *stream) {
   if (g_mmq_path == 1 || mmq_format_is_forced()) return (int32_t)cudaErrorNotSupported;
+  if (ggml_type != MRS_Q4_K && ggml_type != MRS_Q5_K && ggml_type != MRS_Q6_K && ggml_type != MRS_Q8_0) return (int32_t)cudaErrorNotSupported;
   const int elems = blk_elems(ggml_type), bytes = blk_bytes(ggml_type);
-  if (bytes == 0 || M <= 0 || n0 <= 0 || n1 <= 0 || n2 < 0 || K <= 0 || K % elems != 0 || K % 64 != 0 || (K / elems * bytes) % 16 != 0 || (dtype != 0 && dtype != 1))
+  if (M <= 0 || n0 <= 0 || n1 <= 0 || n2 < 0 || K <= 0 || K % elems != 0 || K % 64 != 0 || (K / elems * bytes) % 16 != 0 || (dtype != 0 && dtype != 1))
     return (int32_t)cudaErrorNotSupported;
   const void *const ptrs[] = {w0, w1, n2 > 0 ? w2 : w1, x, y0, y1, n2 > 0 ? y2 : y1};
   for (const void *q : ptrs) if (q == nullptr || ((uintptr_t)q & 15)) return (int32_t)cudaErrorNotSupported;

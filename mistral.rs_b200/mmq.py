@@ -38,8 +38,11 @@ def forward_chained(w, xs: torch.Tensor) -> torch.Tensor:
 def _linear(name, w, xs):
     nrows, ncols = _check(w, xs)
     xs = xs.contiguous()
-    M = xs.numel() // ncols
-    out = xs.new_empty((*xs.shape[:-1], nrows))
+    return _launch(name, w, xs, xs.numel() // ncols, xs.new_empty((*xs.shape[:-1], nrows)))
+
+
+def _launch(name, w, xs, M, out):
+    nrows, ncols = w.shape
     entry = typed(name, _I, _P, _P, _P, _I, _I, _I, _I, _P)
     rc = entry(GGML[w.dtype], w.data.data_ptr(), xs.data_ptr(), out.data_ptr(), M, nrows, ncols, _DT_CODE[xs.dtype], raw_stream(xs.device))
     if rc != 0:
@@ -48,38 +51,40 @@ def _linear(name, w, xs):
 
 
 _NOT_SUPPORTED = 801        # cudaErrorNotSupported: nothing was launched, alone is faster or what is possible
+_GROUPED = ("q4_k", "q5_k", "q6_k", "q8_0")
 
 
 def forward_many(ws, xs: torch.Tensor, chained=False):
     """[forward(w, xs) for w in ws], neighbours of one type as one launch (up to three) where that is faster.  chained: as `forward_chained`."""
-    one = forward_chained if chained else forward
     if not xs.is_cuda:                     # (refused there)
-        return [one(w, xs) for w in ws]
-    for w in ws:
-        _check(w, xs)
+        return [(forward_chained if chained else forward)(w, xs) for w in ws]
+    rows = [_check(w, xs)[0] for w in ws]
     xs = xs.contiguous()
-    out, i = [], 0
+    ncols = xs.shape[-1]
+    M = xs.numel() // ncols
+    ys = [xs.new_empty((*xs.shape[:-1], n)) for n in rows]
+    one, many = ("mrs_mmq_gguf_chained", "mrs_mmq_gguf_multi_chained") if chained else ("mrs_mmq_gguf", "mrs_mmq_gguf_multi")
+    i = 0
     while i < len(ws):
-        n = 1
-        while n < 3 and i + n < len(ws) and ws[i + n].dtype == ws[i].dtype:
+        kind, n = ws[i].dtype, 1
+        while n < 3 and i + n < len(ws) and ws[i + n].dtype == kind and kind in _GROUPED and M > 0:
             n += 1
-        group = ws[i:i + n]
-        i += n
-        M = xs.numel() // xs.shape[-1]
-        if n > 1 and M > 0:
-            ys = [xs.new_empty((*xs.shape[:-1], w.shape[0])) for w in group]
-            data, rows, to = [w.data.data_ptr() for w in group], [w.shape[0] for w in group], [y.data_ptr() for y in ys]
+        j = i + n
+        if n > 1:
+            data, to, sizes = [w.data.data_ptr() for w in ws[i:j]], [y.data_ptr() for y in ys[i:j]], rows[i:j]
             if n == 2:
-                data.append(None), rows.append(0), to.append(None)
-            entry = typed("mrs_mmq_gguf_multi_chained" if chained else "mrs_mmq_gguf_multi", _I, *[_P] * 7, *[_I] * 6, _P)
-            rc = entry(GGML[group[0].dtype], *data, xs.data_ptr(), *to, M, *rows, xs.shape[-1], _DT_CODE[xs.dtype], raw_stream(xs.device))
+                data.append(None), sizes.append(0), to.append(None)
+            entry = typed(many, _I, *[_P] * 7, *[_I] * 6, _P)
+            rc = entry(GGML[kind], *data, xs.data_ptr(), *to, M, *sizes, ncols, _DT_CODE[xs.dtype], raw_stream(xs.device))
             if rc == 0:
-                out += ys
+                i = j
                 continue
             if rc != _NOT_SUPPORTED:
-                raise RuntimeError(f"mrs_mmq_gguf_multi failed with cudaError {rc}")
-        out += [one(w, xs) for w in group]
-    return out
+                raise RuntimeError(f"{many} failed with cudaError {rc}")
+        for k in range(i, j):
+            _launch(one, ws[k], xs, M, ys[k])
+        i = j
+    return ys
 
 
 def timeout_word(device):

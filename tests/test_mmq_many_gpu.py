@@ -81,3 +81,20 @@ def test_what_one_launch_declines(cuda):
     assert [tuple(y.shape) for y in mmq.forward_many(pair, x[:0])] == [(0, 512), (0, 512)]
     with pytest.raises(ValueError):
         mmq.forward_many([pair[0], six[0]], x)
+
+
+@pytest.mark.parametrize("kind,tokens,asked", [("q4_0", 24, 0), ("q8_0", 400, 1), ("q4_k", 24, 1)])
+def test_what_a_list_costs_the_host(cuda, monkeypatch, kind, tokens, asked):
+    """Each matrix is looked at once and each result allocated once, whether the list becomes one launch or is declined; types that never group are not asked for."""
+    g = torch.Generator(device=cuda).manual_seed(1)
+    ws = [_matrix(kind, 8192, 2048, cuda, g) for _ in range(2)]
+    x = torch.randn(tokens, 2048, device=cuda, generator=g).to(torch.bfloat16)
+    want = [mmq.forward(w, x) for w in ws]
+    seen, check, typed = [], mmq._check, mmq.typed
+    monkeypatch.setattr(mmq, "_check", lambda w, xs: seen.append("check") or check(w, xs))
+    monkeypatch.setattr(mmq, "typed", lambda name, *a: seen.append(name) or typed(name, *a))
+    before = torch.cuda.memory_stats(cuda)["allocation.all.allocated"]
+    ys = mmq.forward_many(ws, x)
+    assert torch.cuda.memory_stats(cuda)["allocation.all.allocated"] - before == 2
+    assert seen.count("check") == 2 and seen.count("mrs_mmq_gguf_multi") == asked
+    assert all(float((y.double() - w.double()).norm()) <= 2.0 ** -10 * float(w.double().norm()) for y, w in zip(ys, want))
