@@ -5,6 +5,10 @@
 
 namespace mrs {
 
+// Decode attention: tiles of one sequence that a cluster merges as sums.  More leave rounded results, which are merged in memory.  The resident decode step
+// (step_resident.cu) does the same by the same line, so that its bits are the attention kernel's (paged_attn_mma.cuh).
+constexpr int PM_CL_MAX = 8;
+
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool pred) {
   const uint32_t s = smem_u32(smem);
   const int sz = pred ? 16 : 0;   // src-size 0 -> zero fill

@@ -25,7 +25,6 @@
 namespace mrs {
 
 constexpr int PM_WARPS = 4, PM_THREADS = PM_WARPS * 32, PM_BN = 64;
-constexpr int PM_CL_MAX = 8;    // tiles of one sequence per cluster
 constexpr int PM_CL_G = 8;      // heads per CTA supported by the cluster merge buffer
 
 template <int D> constexpr size_t pm_smem_bytes(bool fused, bool cluster) {

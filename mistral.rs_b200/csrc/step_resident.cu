@@ -38,7 +38,6 @@ extern "C" int32_t *mrs_mmq_timeout_flag(void);      // mmq_ts.cu: the device's 
 
 namespace mrs {
 
-constexpr int PM_CL_MAX = 8;             // (paged_attn_mma.cuh) tiles that a cluster of the decode attention kernel merges
 constexpr int RS_WARPS = 16, RS_CT = RS_WARPS * 32, RS_GROUP = 4, RS_PRODUCERS = RS_WARPS / RS_GROUP, RS_THREADS = RS_CT + 32 * RS_PRODUCERS;
 constexpr int RS_LAYERS = 32;            // layers of a launch (its parameters hold their pointers); longer models take several
 constexpr int RS_DEPTH = 8;              // stages of a group's ring in flight
