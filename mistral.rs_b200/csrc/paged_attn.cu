@@ -568,7 +568,8 @@ static cudaError_t launch_decode_g(PagedParams p, int tiles, cudaStream_t st) {
         int dev = 0;
         cudaGetDevice(&dev);
         if (dev >= 0 && dev < PA_MAX_DEVICES && pm_pairs((long long)tiles * p.num_kv_heads * nsub, dev)) {
-          auto kern = p.heads_per_cta <= 8 ? paged_decode_mma_kernel<T, D, false, false, true, true> : paged_decode_mma_kernel<T, D, false, false, true, false>;
+          const bool swap = p.heads_per_cta <= 8;
+          auto kern = swap ? paged_decode_mma_kernel<T, D, false, false, true, true> : paged_decode_mma_kernel<T, D, false, false, true, false>;
           const size_t dyn = pm_smem_bytes<D>(false, false);
           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
           cudaLaunchConfig_t cfg = {};
@@ -579,14 +580,14 @@ static cudaError_t launch_decode_g(PagedParams p, int tiles, cudaStream_t st) {
           attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
           attr[1].val.programmaticStreamSerializationAllowed = 1;
           cfg.attrs = attr; cfg.numAttrs = 1;
-          static std::atomic<int> feasible[PA_MAX_DEVICES];      // (as above; asked once per device)
-          int can = feasible[dev].load(std::memory_order_relaxed);
+          static std::atomic<int> feasible[2][PA_MAX_DEVICES];      // (as above; asked once per kernel and device)
+          int can = feasible[swap][dev].load(std::memory_order_relaxed);
           if (can == 0) {
             int ncl = 0;
             const cudaError_t qe = cudaOccupancyMaxActiveClusters(&ncl, kern, &cfg);
             if (qe != cudaSuccess) (void)cudaGetLastError();
             can = qe == cudaSuccess && ncl >= 1 ? 1 : -1;
-            feasible[dev].store(can, std::memory_order_relaxed);
+            feasible[swap][dev].store(can, std::memory_order_relaxed);
           }
           if (can == 1) {
             cfg.numAttrs = p.pdl ? 2 : 1;
