@@ -497,9 +497,11 @@ constexpr int PA_MAX_DEVICES = 64;
 static int g_pa_flags = 0;   // bit 0: keep HND decode on the SIMT kernel (A/B, debugging); bit 2 / 3: never / always pairs of CTAs a tile; bit 4: merge late
 
 // Pairs of CTAs a tile, each with half of its tokens: at up to one and a half CTAs an SM.  There a tile's time is its chain of stages (load, scores,
-// soft-max, product: ~1 us each), and half as many of them take 11.3 us where the whole took 13.8 (1 sequence of 300 tokens, 32 query and 8 KV heads of
-// 128), 13.9 against 15.4 (1 of 3000), 13.9 against 15.5 (16 of 300), 12.7 against 14.0 (8 of 500).  With more CTAs the pairs no longer run at one time
-// and each adds a head and an exchange: 256 CTAs take 19.4 us against 15.2, 376 take 25.3 against 19.2.
+// soft-max, product: ~1 us each).  Drawn for the kernel with heads as rows (more than eight heads a KV head run on it), 32 heads on 8 of 128: half as many
+// stages 11.3 us where the whole took 13.8 (1 sequence of 300 tokens), 13.9 against 15.4 (1 of 3000), 13.9 against 15.5 (16 of 300), 12.7 against 14.0
+// (8 of 500).  With more CTAs the pairs no longer run at one time and each adds a head and an exchange: 256 CTAs take 19.4 us against 15.2, 376 25.3 against
+// 19.2.  With tokens as rows (SWAP) the stages are short enough that the pairs gain nothing any more, pairs / whole 8.9 / 8.8, 11.1 / 10.5, 10.6 / 10.0 and
+// 10.0 / 9.0 on the same four, 14 heads of 64 on 2, 33 sequences of 600 tokens 9.5 / 8.6; beyond the line 240 CTAs 15.9 / 10.5, 344 36.6 / 32.8.
 static bool pm_pairs(long long ctas, int dev) {
   if (g_pa_flags & 12) return (g_pa_flags & 8) != 0;
   static std::atomic<int> known[PA_MAX_DEVICES];
