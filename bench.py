@@ -59,7 +59,7 @@ def algorithmic_bytes_per_token(cfg, M, tp=1):
 
 
 class ClockSampler:
-    """nvidia-smi clocks + throttle reasons during the timed region (B200_PROFILING.md)."""
+    """nvidia-smi clocks + throttle reasons during the timed region."""
 
     def __init__(self, gpu_index=0):
         self.proc, self.lines, self.gpu = None, [], gpu_index
@@ -123,7 +123,7 @@ def cpu_decode_samples(cfg, M, seconds=10.0, min_tokens=2, threads=0, nsamples=1
     from DRAM each token, attention / norms / GLU included, one pinned thread per usable host core
     (oracle/cpu_decode_bench.c).  Compiled where it runs, with -O3 -march=native.
     `nsamples` timed samples of about `seconds` each share ONE model allocation (one short-lived child process).
-    Returns ([tok/s per sample], threads, description)."""
+    Returns ([tok/s per sample], threads, description, [seconds per sample])."""
     src = os.path.join(ROOT, "oracle", "cpu_decode_bench.c")
     out_dir = os.path.join(tempfile.gettempdir(), f"mrs_cpu_bench_{os.getuid()}")
     os.makedirs(out_dir, exist_ok=True)
@@ -169,11 +169,11 @@ def cpu_decode_samples(cfg, M, seconds=10.0, min_tokens=2, threads=0, nsamples=1
     sample = (f"{r['tokens'][-1]} whole tokens (all {cfg.n_layers} layers + lm_head, {r['weight_bytes'] / 1e9:.2f} GB of weights streamed "
               f"from DRAM per token, attention over {arg['ctx']} cached tokens, norms and GLU included), decode batch 1, "
               f"-O3 -march=native, {r['threads']} pinned threads (pool size chosen by a short probe over {len(os.sched_getaffinity(0))} visible CPUs)")
-    return r["tok_s"], r["threads"], sample
+    return r["tok_s"], r["threads"], sample, [n / v for n, v in zip(r["tokens"], r["tok_s"])]
 
 
 def cpu_decode_tokens_per_s(cfg, M, seconds=10.0, min_tokens=2, threads=0):
-    vals, th, sample = cpu_decode_samples(cfg, M, seconds=seconds, min_tokens=min_tokens, threads=threads, nsamples=1)
+    vals, th, sample, _ = cpu_decode_samples(cfg, M, seconds=seconds, min_tokens=min_tokens, threads=threads, nsamples=1)
     return vals[0], th, sample
 
 
@@ -196,12 +196,12 @@ def run_reference(args):
     # warm-up samples and timed samples share one model allocation and one pool-size probe: the run is
     # (warmup + steps) x budget seconds plus ~30 s of set-up, whatever --steps says
     nw = max(args.warmup, 0)
-    allv, threads, sample = cpu_decode_samples(cfg, M, seconds=budget, nsamples=nw + steps)
-    vals = allv[nw:]
+    allv, threads, sample, took = cpu_decode_samples(cfg, M, seconds=budget, nsamples=nw + steps)
+    vals, took = allv[nw:], took[nw:]
     value = sum(vals) / len(vals)
     print(json.dumps({
         "impl": "reference", "metric": "decode_tok_s", "value": value, "unit": "tok/s", "n_gpus": args.gpus,
-        "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 / value * (GEN_LEN - 1), "higher_is_better": True,
+        "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * sum(took) / len(took), "higher_is_better": True,
         "scaling": "strong", "vs_baseline": None, "dtype": "int8 (Q8_K / Q8_0) activations x ggml block dots, f32 accumulate", "data": "synthetic",
         "config": {"workload": "Llama-3-8B GGUF Q4_K_M decode batch=1 (CPU, whole tokens; each step a bounded sample)"},
         "cpu_baseline": {"value": value, "unit": "tok/s", "cores": threads, "kind": "port", "sample": sample},
@@ -484,7 +484,8 @@ def bench_nisasun(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
             setattr(mod, name, g)
             return f
         names = ["embed_streams", "streams_read_norm", "streams_write", "glu_split", "gated_group_norm", "causal_conv", "ssm_steps",
-                 "linear_scan", "attention_prepare", "paged_attention", "fresh_prompt_attention", "scale_rows", "activate_cols", "moe_route", "moe_block", "moe_small", "moe_place", "moe_sort", "moe_gather", "moe_combine"]
+                 "linear_scan", "attention_prepare", "paged_attention", "fresh_prompt_attention", "scale_rows", "activate_cols", "moe_route_scored", "moe_block", "moe_products", "moe_sort", "moe_gather",
+                 "moe_combine"]
         saved = {n: wrap(K, n) for n in names}
         saved_lin = wrap(mixers, "linear")
 
@@ -612,9 +613,9 @@ def bench_kilizen(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
     warmup, steps = max(3, warmup), max(1, steps)
     names = [n for n in ("embed_streams", "streams_read_norm", "streams_write", "glu_split", "gated_group_norm", "causal_conv", "ssm_steps", "linear_scan",
-                         "qk_norm_store", "window_attention", "fresh_prompt_attention", "scale_rows", "activate_cols", "moe_route", "moe_block", "moe_small", "moe_place", "moe_sort",
+                         "qk_norm_store", "window_attention", "fresh_prompt_attention", "scale_rows", "activate_cols", "moe_route_scored", "moe_block", "moe_products", "moe_sort",
                          "moe_gather", "moe_combine", "tanh_norm_rows", "residual_tanh_norm", "rotation_table", "attention_prepare", "paged_attention",
-                         "prompt_attention", "mlstm_gates", "append_ones", "mlstm_out_norm", "moe_route_top_softmax", "moe_small_ungated")]
+                         "prompt_attention", "mlstm_gates", "append_ones", "mlstm_out_norm", "moe_route_top_softmax")]
 
     def timed(fn, reps=steps):
         for _ in range(warmup):
@@ -794,8 +795,8 @@ def bench_fosulix(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
     warmup, steps = max(3, warmup), max(1, steps)
     names = ["embed_streams", "embed_scaled", "streams_read_norm", "rms_residual", "glu_split", "gated_group_norm", "causal_conv", "linear_scan",
              "activate_cols", "bounded_gate", "latent_prepare", "rotate_pairs", "latent_prompt_attention", "paged_attention", "prompt_attention",
-             "fresh_prompt_attention", "attention_prepare", "rotation_table", "moe_route", "moe_route_scored", "moe_route_top_softmax", "moe_small",
-             "moe_small_ungated", "moe_block", "moe_place", "moe_sort", "moe_gather", "moe_combine", "tanh_norm_rows", "residual_tanh_norm", "mlstm_gates", "append_ones",
+             "fresh_prompt_attention", "attention_prepare", "rotation_table", "moe_route_scored", "moe_route_top_softmax", "moe_block",
+             "moe_products", "moe_sort", "moe_gather", "moe_combine", "tanh_norm_rows", "residual_tanh_norm", "mlstm_gates", "append_ones",
              "mlstm_out_norm", "scale_rows"]
 
     def timed(fn, reps=steps):
@@ -1080,8 +1081,8 @@ def bench_kibotar(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
     names = ["embed_scaled", "embed_pair", "streams_read_norm", "rms_residual", "glu_split", "gated_group_norm", "causal_conv", "linear_scan",
              "activate_cols", "bounded_gate", "power_gate", "latent_prepare", "rotate_pairs", "latent_prompt_attention", "paged_attention",
              "prompt_attention", "tc_attention", "attention_prepare", "rotation_table", "pool_blocks", "mix_heads", "gate_cols",
-             "moe_route_scored", "moe_block", "moe_small",
-             "moe_place", "moe_sort", "moe_gather", "moe_combine", "scale_rows"]
+             "moe_route_scored", "moe_block", "moe_products",
+             "moe_sort", "moe_gather", "moe_combine", "scale_rows"]
     measure = engine_bench_tools(torch, dev, steps, warmup, prompt, decode_batches, names)
     out = {"metric": "kibotar_prefill_tok_s", "unit": "tok/s", "n_gpus": 1, "steps": steps, "warmup": warmup, "higher_is_better": True,
            "dtype": "bf16 (f32 residual, states, decays, norms, softmax and mixed weights)", "data": "synthetic", "sizes": []}
@@ -1362,8 +1363,8 @@ def bench_bafusun(torch, dev, peaks, steps=3, warmup=3, widths=(2048, 4096), pro
     tpeak = peaks.get("bf16_tflops_sustained", 1400.0)
     warmup, steps = max(3, warmup), max(1, steps)
     names = ["embed_scaled", "embed_streams", "rms_residual", "tanh_norm_rows", "residual_tanh_norm", "glu_split", "activate_cols", "gated_lookup", "rotation_table",
-             "attention_prepare", "paged_attention", "prompt_attention", "tc_attention", "gather_rows", "router_logits", "moe_route_scored", "moe_route_top_softmax", "moe_small",
-             "moe_small_ungated", "moe_grouped", "moe_products", "moe_block", "moe_place", "moe_sort", "moe_gather", "moe_combine", "soft_cap"]
+             "attention_prepare", "paged_attention", "prompt_attention", "tc_attention", "gather_rows", "router_logits", "moe_route_scored", "moe_route_top_softmax",
+             "moe_products", "moe_block", "moe_sort", "moe_gather", "moe_combine", "soft_cap"]
     measure = engine_bench_tools(torch, dev, steps, warmup, prompt, decode_batches, names)
     out = {"metric": "bafusun_prefill_tok_s", "unit": "tok/s", "n_gpus": 1, "steps": steps, "warmup": warmup, "higher_is_better": True,
            "dtype": "bf16 (f32 residual, norms, angles, softmax, router)", "data": "synthetic", "sizes": []}
@@ -1675,9 +1676,12 @@ def main():
     value = ntok * len(times) / sum(times)
     e2e_value = ntok * len(e2e_times) / sum(e2e_times)
 
-    # ---- roofline of the dominant kernel (mmvq_stream_kernel: every quantized GEMV of a token), measured live:
-    # a CUDA graph of ONE token's GEMV chain only (attention-side kernels skipped), CUDA events on the launching
-    # stream; weights (4.6 GB) >> L2 so every launch streams from HBM.  Under TP the chain includes the all-reduces.
+    runner.check_overflow()               # (replays pass no entry point: neither a full context nor a wait that ran out shows in them)
+    # ---- roofline of the dominant kernel.  Where a token is one resident grid (step_resident_kernel, layers and head), the timed tokens themselves.
+    # Else, and beside it, the chain of launches: a CUDA graph of ONE token's GEMVs (mmvq_stream_kernel; attention-side kernels skipped) and one of
+    # its attention side, CUDA events on the launching stream; weights (4.6 GB) >> L2 so every launch streams from HBM.  Under TP the GEMVs' chain
+    # includes the all-reduces.
+    resident = runner.is_resident()
     runner.step_struct.skip_mask = 1
     gg = torch.cuda.CUDAGraph(keep_graph=True)
     runner.reset(PROMPT_LEN + GEN_LEN // 2)
@@ -1701,13 +1705,27 @@ def main():
         head = cfg.vocab * cfg.hidden * BLOCK_BYTES[t] // BLOCK_ELEMS[t]
         weight_bytes = (weight_bytes - head) + head   # algorithmic_bytes_per_token already keeps the head whole per rank
     n_gemv = sum(4 if M.tensor_type(cfg, "attn_v", l) == M.tensor_type(cfg, "attn_q", l) else 5 for l in range(cfg.n_layers)) + 1
-    achieved = weight_bytes / gemv_s / 1e9
     traffic = None
     try:   # DRAM bytes per launch from the committed ncu --set full capture of this kernel (single-GPU shapes only)
         tr = json.load(open(os.path.join(ROOT, "profiles", "r02_traffic.json")))
         traffic = tr["dram_bytes_per_launch"] if (world == 1 and not big and not args.layers) else None
     except Exception:
         pass
+
+    def hbm(kernel, launches, seconds, traffic):
+        gbs = weight_bytes / seconds / 1e9
+        return {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak, "traffic": traffic,
+                "algorithmic_bytes_per_launch": weight_bytes / launches, "peak_source": peak_src, "kernel": kernel, "launches": launches,
+                "avg_launch_us": seconds / launches * 1e6, "bytes_per_token": weight_bytes}
+
+    chain = hbm("mmvq_stream_kernel (all quantized GEMVs of one token" + (", incl. the in-graph all-reduces)" if world > 1 else ")"), n_gemv, gemv_s, traffic)
+    chain_us = {"gemv_chain": gemv_s * 1e6, "attention_chain": attn_s * 1e6}
+    if resident:
+        roofline = hbm("step_resident_kernel (all layers and the head of one token, attention included)", -(-cfg.n_layers // 32), 1.0 / value, None)
+        breakdown = {"whole_token": 1e6 / value}
+        chain = dict(chain, us_per_token=chain_us, what="the launches that serve a step where the resident grid does not: timed apart, not part of `value`")
+    else:
+        roofline, chain, breakdown = chain, None, dict(chain_us, whole_token=1e6 / value)
 
     # ---- GPU reference arm: the unmodified reference kernels (oracle/_ref) chained as mistral.rs chains them, one
     # CUDA graph per token, same weights, same box (scripts/gpu_reference_chain.py)
@@ -1732,7 +1750,7 @@ def main():
             sec = e0.elapsed_time(e1) / 1e3
             gpu_ref = {"decode_tok_s": (GEN_LEN - 1) / sec, "launches_per_token": count_graph_kernels(rg),
                        "what": "unmodified reference kernels (mmvq_gguf, rotary, add_rms_norm, reshape_and_cache_flashinfer, flashinfer_decode; "
-                               "built from /root/reference with its own flags) chained per layer as mistral.rs does, CUDA graph per token, "
+                               "built with its own flags) chained per layer as mistral.rs does, CUDA graph per token, "
                                "reference split-KV policy; same synthetic weights, same decode window"}
             del rc_, rg
         except Exception as e:
@@ -1773,18 +1791,16 @@ def main():
                     "ttft_ms": None if ttft_e2e is None else ttft_e2e * 1e3},
             "gpu_launches": None if launches_per_token is None else launches_per_token * ntok,
             "launches_per_token": launches_per_token,
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": traffic, "algorithmic_bytes_per_launch": weight_bytes / n_gemv, "peak_source": peak_src,
-                         "kernel": "mmvq_stream_kernel (all quantized GEMVs of one token" + (", incl. the in-graph all-reduces)" if world > 1 else ")") +
-                                   (", timed as a chain of launches; whole tokens run as one step_resident_kernel" if (launches_per_token or 99) < 10 else ""),
-                         "launches": n_gemv, "avg_launch_us": gemv_s / n_gemv * 1e6, "bytes_per_token": weight_bytes},
-            "breakdown_us_per_token": {"gemv_chain": gemv_s * 1e6, "attention_chain": attn_s * 1e6, "whole_token": 1e6 / value},
+            "roofline": roofline,
+            "breakdown_us_per_token": breakdown,
             "step_hbm_frac": total_bytes * value / 1e9 / peak,
             "clocks": clocks,
         }
         if ttft_dev is not None:
             out["prompt"] = {"tokens": PROMPT_LEN, "ttft_ms": ttft_dev * 1e3, "prefill_tok_s": PROMPT_LEN / ttft_dev,
                              "note": "the 128-token prompt of this workload: one prefill pass (tcgen05 dequant-GEMMs + prompt attention + KV scatter) + first sample"}
+        if chain:
+            out["chain_of_launches"] = chain
         if gpu_ref:
             out["gpu_reference"] = gpu_ref
             if "decode_tok_s" in gpu_ref:
