@@ -37,6 +37,16 @@ def _ran_resident(run):
     return bool(run.resident[256:].any())
 
 
+def _launches(run, at):
+    """Kernels of one step, counted on a captured one: the grid's are one for 32 layers (and the embedding, the argmax, the advance)."""
+    import bench
+    run.reset(at)
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        run.step()
+    return bench.count_graph_kernels(g)
+
+
 def _step(run, at, token=11):
     run.reset(at)
     run.set_tokens([token])
@@ -57,12 +67,62 @@ def _same(resident, chain, at):
 @pytest.mark.parametrize("shape", SHAPES)
 @pytest.mark.parametrize("quant,dtype", [("q4_k_m", torch.float16), ("q8_0", torch.bfloat16)])
 def test_step_equals_chain(cuda, monkeypatch, shape, quant, dtype, ctx):
-    """One tile a head, up to eight (a cluster's sums) and more (rounded partial results); contexts around a warp's, a step's and a tile's tokens."""
+    """One tile a head (which leaves nothing in the scratch: the launches tell), up to eight (a cluster's sums) and more (rounded partial results);
+    contexts around a warp's, a step's and a tile's tokens."""
     resident, chain = _pair(cuda, monkeypatch, shape, quant, dtype, neox=shape != "gqa4", ctx=ctx)
     for at in (0, 1, 15, 16, 59, 63, 64, 65, 127, 128, 200, 497, 640, 1499):
         if at < ctx:
             _same(resident, chain, at)
-    assert (resident.padded_tiles == 1 or _ran_resident(resident)) and not _ran_resident(chain)
+    assert resident.is_resident() and not chain.is_resident()
+    assert _ran_resident(resident) == (resident.padded_tiles > 1) and not _ran_resident(chain)
+    assert _launches(resident, 1) == 4 < _launches(chain, 1)
+
+
+@pytest.mark.parametrize("shape,dtype", [("gqa4", torch.bfloat16), ("gqa7", torch.float16)])
+def test_more_tiles_than_a_warp_has_lanes(cuda, monkeypatch, shape, dtype):
+    """From the 33rd tile on a lane holds two tiles' states: on both sides of it, of a tile's end and of the context's."""
+    resident, chain = _pair(cuda, monkeypatch, shape, "q4_k_m", dtype, ctx=37 * 64)
+    assert resident.is_resident() and resident.padded_tiles > 33
+    tile = resident.split_pages * resident.cfg.block_size
+    for at in (31 * tile, 32 * tile - 2, 32 * tile - 1, 32 * tile, 32 * tile + 1, 33 * tile - 1, 33 * tile, 2200, 37 * 64 - 1):
+        _same(resident, chain, at)
+    assert _ran_resident(resident)
+
+
+def test_two_runners_on_two_streams(cuda, monkeypatch):
+    """Grids that each want all SMs, from graphs on streams of their own, beside a third stream's products: they run one after the other, with their bits."""
+    a, b = _pair(cuda, monkeypatch, "gqa4", "q4_k_m", torch.bfloat16, layers=2)
+    b.step_struct.extension = M.STEP_RESIDENT
+    for run in (a, b):
+        run.capture()
+    for x, y in zip(a.k_cache + a.v_cache, b.k_cache + b.v_cache):
+        y.copy_(x)
+
+    def start():
+        for run, token in ((a, 7), (b, 8)):
+            run.reset(60)
+            run.set_tokens([token])
+        torch.cuda.synchronize()
+
+    start()
+    for run in (a, b):
+        for _ in range(60):
+            run.replay()
+        torch.cuda.synchronize()
+    want = [(run.logits().clone(), [t.clone() for t in run.k_cache + run.v_cache]) for run in (a, b)]
+    start()
+    streams, m = [torch.cuda.Stream() for _ in range(3)], torch.randn(2048, 2048, device=cuda, dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+    for i in range(60):
+        for run, stream in zip((a, b), streams):
+            with torch.cuda.stream(stream):
+                run.replay()
+        with torch.cuda.stream(streams[2]):
+            m @ m
+    torch.cuda.synchronize()
+    mmq.check_timeouts(cuda)
+    for run, (logits, caches) in zip((a, b), want):
+        assert torch.equal(run.logits(), logits) and all(torch.equal(x, y) for x, y in zip(run.k_cache + run.v_cache, caches))
 
 
 @pytest.mark.parametrize("block", [8, 24, 32])
@@ -101,7 +161,8 @@ def test_more_layers_than_a_launch_holds(cuda, monkeypatch):
 
 
 def test_what_the_grid_declines(cuda, monkeypatch):
-    """Other block types, a sequence at the end of its context, a scratch that is too small, and the measuring switches: the chain's own bits or its rules."""
+    """Other block types, a scratch that is too small, the measuring switches: the chain, by its bits and its launches.  (A sequence at the end of its
+    context stays on the grid, by the chain's rules.)"""
     resident, chain = _pair(cuda, monkeypatch, "gqa4", "q4_k_m", torch.float16, types=lambda cfg, name, layer=0: "q4_0" if name == "ffn_down" else "q4_k")
     assert torch.equal(_step(resident, 100)["logits"], _step(chain, 100)["logits"]) and not _ran_resident(resident)
     monkeypatch.undo()
@@ -109,6 +170,13 @@ def test_what_the_grid_declines(cuda, monkeypatch):
     resident.step_struct.resident_bytes -= 16
     assert torch.equal(_step(resident, 50)["logits"], _step(chain, 50)["logits"]) and not _ran_resident(resident)
     resident.step_struct.resident_bytes += 16
+    for mask in (1, 2):
+        assert resident.is_resident()
+        for run in (resident, chain):
+            run.step_struct.skip_mask = mask
+        assert not resident.is_resident() and _launches(resident, 50) == _launches(chain, 50) and not _ran_resident(resident)
+        for run in (resident, chain):
+            run.step_struct.skip_mask = 0
     before = [t.clone() for t in resident.k_cache + resident.v_cache]
     resident.context_lens.fill_(160)          # full: attends, writes no cache row, sets the flag
     resident.step()
