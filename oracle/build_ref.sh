@@ -1,6 +1,6 @@
 #!/usr/bin/env bash
 # TEST INFRASTRUCTURE ONLY — builds the UNMODIFIED reference CUDA kernels of the hot path
-# straight from /root/reference (sources are never copied into this repo) into
+# straight from the reference's tree (sources are never copied into this repo) into
 # oracle/_ref/*.so.  These shared objects are the GPU-side oracle ("what does the
 # reference itself compute on these inputs?") and the "beat this" timing baseline.
 #
@@ -17,7 +17,7 @@ HERE="$(cd "$(dirname "$0")" && pwd)"
 OUT="$HERE/_ref"
 mkdir -p "$OUT"
 if [ ! -d "$REF" ]; then
-  echo "build_ref: $REF not present (GPU box?) - using prebuilt oracle/_ref/*.so if any"; exit 0
+  echo "build_ref: $REF not present - using prebuilt oracle/_ref/*.so if any"; exit 0
 fi
 NVCC=${NVCC:-/usr/local/cuda/bin/nvcc}
 COMMON=(-std=c++17 -O3 -U__CUDA_NO_HALF_OPERATORS__ -U__CUDA_NO_HALF_CONVERSIONS__

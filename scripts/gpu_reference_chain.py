@@ -1,4 +1,4 @@
-"""GPU reference arm: the UNMODIFIED reference kernels (oracle/_ref/*.so, compiled from /root/reference by
+"""GPU reference arm: the UNMODIFIED reference kernels (oracle/_ref/*.so, compiled from its sources by
 oracle/build_ref.sh with the reference's own flags) chained per decoder layer the way mistral.rs chains them
 (REF mistralrs-core/src/models/llama.rs:243-260 Block::forward, core/src/ops.rs:5036,5081 qkv_projections /
 quantized_ffn -> mistralrs-quant/src/gguf/fast_mmvq.rs:299,472,682), captured in one CUDA graph per token like

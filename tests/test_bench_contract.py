@@ -1,5 +1,5 @@
 """bench.py's reference arm runs without a GPU (the CPU port on whole tokens): check, offline, that the line it prints
-carries the keys the driver reads (`impl`, metric / unit / value, `cpu_baseline` with kind / cores / sample, `e2e` with
+carries the keys of its contract (`impl`, metric / unit / value, `cpu_baseline` with kind / cores / sample, `e2e` with
 zero host<->device bytes) and that the numbers are sane.  A one-layer model and a two-second sample keep it short."""
 import json
 import os

@@ -1,4 +1,4 @@
-"""Tensor parallel decode on real GPUs (needs >= 2 devices; skipped on a single-GPU box)."""
+"""Tensor parallel decode on real GPUs (needs >= 2 devices; skipped with one)."""
 import os
 import subprocess
 import sys
