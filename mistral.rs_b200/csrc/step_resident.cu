@@ -21,8 +21,10 @@
 // One B200, bf16, us a step in a graph, chain / resident: eight layers 4096 x 14336 with a 32000 head, Q4_K_M, 500 tokens of context 535 / 439; 32 layers
 // with a 128256 head 1878 / 1624; two layers at 100, 1000, 4000, 16000 tokens 164 / 151, 182 / 152, 195 / 170, 236 / 213, Q8_0 178 / 174, 197 / 179, 209 / 192,
 // 249 / 234; four layers 3072 x 8192 at 20, 500, 3000 tokens 221 / 200, 235 / 205, 270 / 225.
-// A layer of the first takes 88000 clocks: gate and up 19000 (5.4 TB/s with what the ring held), down 9000 (Q6_K 19000), q / k / v 5000, o_proj 3300;
-// attention 15000, a chain of loads and meetings; each meeting 4000 to 6000 from the last row to the next input, quantising it 2500 to 6000.
+// A layer of the first takes 91000 clocks (v and down in Q6_K: 102000), by stamps of each CTA: products until its last warp is done 55000 (65000), that is
+// q / k / v 10100 (11600), o_proj 7200, gate and up 24700 (5.3 TB/s with what the ring held), down 12700 (21500); attention and the meetings on both sides
+// of it 15500, a chain of loads in 56 of the CTAs that the others wait for; quantising the four inputs 14000 (1900 to 5200 each), in every CTA; the other
+// meetings 6700.
 // Tried: one producer warp for all rings (a copy took it 110 clocks: 713 us); consumers that ask for their own segments (480); vectors as words with tags
 // instead of barriers (all CTAs polling the same lines took L2 from the weights: 530); rows brought into L2 ahead of the ring (nothing).
 #include "mma_common.cuh"

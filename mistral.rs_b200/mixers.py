@@ -680,7 +680,9 @@ class RoutedExperts:
     # tokens 35 / 41, 6: 39 / 41, 12: 53 / 43, 32: 86 / 43; 8 experts, top 2, 1024 x 768 (5 MB): 8 tokens 31 / 35, 12: 35 / 35, 16: 43 / 35;
     # 16 experts, top 2, 1024 x 768: 8 tokens 41 / 37, 12: 41 / 39, 32: 61 / 37; 32 experts, top 2, 1024 x 768: 8 tokens 41 / 39, 16: 53 / 43, 64:
     # 92 / 49; 32 experts, top 4, 2048 x 2048: 4 tokens 92 / 96, 8: 135 / 115; 16 experts, top 4, 4096 x 2048 (50 MB): 4 tokens 139 / 133, 6: 158 /
-    # 150.  The bytes' line for steps that stream per pair: 8 experts of 100 MB, top 8, 2 tokens 657 / 186.
+    # 150.  More experts, one pair per expert and two: 32 experts of 13 MB 70 / 77 and 98 / 79; 64 of 17 MB, top 8, 177 / 145 and 267 / 155; 64 of 5 MB 65 /
+    # 56 and 96 / 65; 128 of 9 MB, top 8, 176 / 122 and 284 / 159; 128 of 3 MB 102 / 63 and 120 / 69; 256 of 6 MB, top 8, 573 / 121 and 1058 / 165; 512 of
+    # 6 MB, top 8, 1684 / 160 and 3271 / 170.  The bytes' line for steps that stream per pair: 8 experts of 100 MB, top 8, 2 tokens 657 / 186.
     # Elsewhere weights are streamed per pair up to 4 pairs per expert while an expert is small enough that repeated reads hit L2, up to
     # 2 above that.
     GROUPED_MIN_TOKENS, GROUPED_PER_EXPERT, GROUPED_PAIR_BYTES, ONE_LAUNCH_PAIRS = 4, 8, 700 << 20, 20

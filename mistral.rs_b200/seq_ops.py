@@ -422,6 +422,8 @@ def router_logits(x, w, w16=None):
     return out
 
 
+# `moe_block` calls the entries of the products below in C.  They stand here for callers with experts and weights of their own choosing, and for the tests, which
+# hold the block to them bit for bit: `moe_grouped`, `moe_small`, `moe_small_ungated`, `moe_place`, `moe_gemm`.
 def moe_grouped_fits(dtype, width, ff):
     """True when `moe_grouped` takes experts of this size."""
     return bool(lib().mrs_seq_moe_grouped_fits(_i(DTYPE_CODE[dtype]), _i(width), _i(ff)))
