@@ -141,4 +141,4 @@ def fused_ffn(gate_w, up_w, down_w, xs: torch.Tensor, activation) -> torch.Tenso
         return forward(down_w, fused_glu(gate_w, up_w, xs, activation))
     # the first launch is a plain one: nothing that was in flight before it runs beside the links
     from . import ops
-    return forward_chained(down_w, ops.fused_glu_chained(*forward_many([gate_w, up_w], xs), activation))
+    return forward_chained(down_w, ops._glu_link(*forward_many([gate_w, up_w], xs), activation))

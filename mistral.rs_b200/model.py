@@ -734,11 +734,11 @@ class LlamaPrefill:
             attn = paged_attn.prefill_attention(q, k, v, scale)
             paged_attn.reshape_and_cache_flashinfer(k, v, self.k_cache[l], self.v_cache[l], slots)
             o = mmq.forward_chained(qt(L["attn_output"]), attn.view(T, H * D))
-            x, h2 = ops.add_rms_norm_chained(o, x, L["ffn_norm"], cfg.rms_eps)       # x = o + x ; h2 = norm(x)
+            x, h2 = ops._add_rms_norm_link(o, x, L["ffn_norm"], cfg.rms_eps)       # x = o + x ; h2 = norm(x)
             gate, up = mmq.forward_many([qt(L["ffn_gate"]), qt(L["ffn_up"])], h2, chained=True)
-            d = mmq.forward_chained(qt(L["ffn_down"]), ops.fused_glu_chained(gate, up, 0))
+            d = mmq.forward_chained(qt(L["ffn_down"]), ops._glu_link(gate, up, 0))
             nxt = w.layers[l + 1]["attn_norm"] if l + 1 < cfg.n_layers else w.output_norm
-            x, h = ops.add_rms_norm_chained(d, x, nxt, cfg.rms_eps)                   # x = d + x ; h = next norm(x)
+            x, h = ops._add_rms_norm_link(d, x, nxt, cfg.rms_eps)                   # x = d + x ; h = next norm(x)
         if all_logits:
             return mmq.forward(qt(w.output), h)
         return quant.plain(qt(w.output), h[T - 1:T].contiguous())[0]

@@ -40,19 +40,30 @@ def fused_glu(a, b, activation):
     return out
 
 
-def _check_link(name, *tensors):
-    """What a link of a launch chain takes as it is: rows of one shape, type and device, contiguous, 16 bit, on the GPU."""
-    first = tensors[0]
-    for t in tensors:
-        if t.shape != first.shape or t.dtype != first.dtype or t.device != first.device:
-            raise ValueError(f"{name}: shape/dtype/device mismatch")
-        if not t.is_cuda or t.dtype not in (torch.float16, torch.bfloat16) or not t.is_contiguous():
-            raise ValueError(f"{name}: contiguous f16 or bf16 rows on the GPU")
+def _check_link(name, a, b):
+    if a.dtype not in (torch.float16, torch.bfloat16) or a.dtype is not b.dtype or a.shape != b.shape or a.device != b.device:
+        raise ValueError(f"{name}: f16 or bf16 rows of one shape, type and device")
+    if not (a.is_cuda and a.is_contiguous() and b.is_contiguous()):
+        raise ValueError(f"{name}: contiguous rows on the GPU")
 
 
 def fused_glu_chained(a, b, activation):
     """`fused_glu` of contiguous 16-bit rows as a link of a chain of launches: the next one may begin while it runs."""
     _check_link("fused_glu_chained", a, b)
+    return _glu_link(a, b, activation)
+
+
+def add_rms_norm_chained(x, residual, weight, eps):
+    """`add_rms_norm` of contiguous 16-bit rows as a link of a chain of launches."""
+    _check_link("add_rms_norm_chained", x, residual)
+    if weight.shape != x.shape[-1:] or weight.dtype is not x.dtype or weight.device != x.device or not weight.is_contiguous():
+        raise ValueError("add_rms_norm_chained: the weight is a row of the inputs' type")
+    return _add_rms_norm_link(x, residual, weight, eps)
+
+
+# The two above for rows that the package's own launches have just written: nothing is looked at.  (The host bounds short prompts, and the checks took it 10 us
+# a layer: two layers 2048 wide, 148 tokens 385 us with them, 365 without.)
+def _glu_link(a, b, activation):
     cols = a.shape[-1]
     out = torch.empty_like(a)
     entry = typed("mrs_fused_glu_pdl", _P, _P, _P, _U, _U, _U, _U, _I, _I, _I, _P)
@@ -60,12 +71,8 @@ def fused_glu_chained(a, b, activation):
     return out
 
 
-def add_rms_norm_chained(x, residual, weight, eps):
-    """`add_rms_norm` of contiguous 16-bit rows as a link of a chain of launches."""
-    _check_link("add_rms_norm_chained", x, residual)
+def _add_rms_norm_link(x, residual, weight, eps):
     cols = x.shape[-1]
-    if weight.shape != (cols,) or weight.dtype != x.dtype or weight.device != x.device or not weight.is_contiguous():
-        raise ValueError("add_rms_norm_chained: the weight is a row of the inputs' type")
     s, n = torch.empty_like(x), torch.empty_like(x)
     entry = typed("mrs_add_rms_norm_pdl", _P, _P, _P, _P, _P, _I, _I, _F, _I, _I, _P)
     entry(x.data_ptr(), residual.data_ptr(), weight.data_ptr(), s.data_ptr(), n.data_ptr(), x.numel() // cols, cols, eps, _DT_CODE[x.dtype], 1,
