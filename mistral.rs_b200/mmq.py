@@ -27,18 +27,21 @@ def _check(w, xs):
 
 def forward(w, xs: torch.Tensor) -> torch.Tensor:
     """w: quant.QTensor [N, K]; xs [..., K] bf16/f16 -> [..., N]."""
-    return _linear("mrs_mmq_gguf", w, xs)
+    nrows, ncols = _check(w, xs)
+    xs = xs.contiguous()
+    out = xs.new_empty((*xs.shape[:-1], nrows))
+    entry = typed("mrs_mmq_gguf", _I, _P, _P, _P, _I, _I, _I, _I, _P)
+    rc = entry(GGML[w.dtype], w.data.data_ptr(), xs.data_ptr(), out.data_ptr(), xs.numel() // ncols, nrows, ncols, _DT_CODE[xs.dtype], raw_stream(xs.device))
+    if rc != 0:
+        raise RuntimeError(f"mrs_mmq_gguf failed with cudaError {rc}")
+    return out
 
 
 def forward_chained(w, xs: torch.Tensor) -> torch.Tensor:
     """`forward` for weights that nothing in flight writes: begins on them while the launch before it runs."""
-    return _linear("mrs_mmq_gguf_chained", w, xs)
-
-
-def _linear(name, w, xs):
     nrows, ncols = _check(w, xs)
     xs = xs.contiguous()
-    return _launch(name, w, xs, xs.numel() // ncols, xs.new_empty((*xs.shape[:-1], nrows)))
+    return _launch("mrs_mmq_gguf_chained", w, xs, xs.numel() // ncols, xs.new_empty((*xs.shape[:-1], nrows)))
 
 
 def _launch(name, w, xs, M, out):
