@@ -184,6 +184,9 @@ static int32_t gguf_multi(int32_t ggml_type, const void *w0, const void *w1, con
   // saved waves count: a wave that fills the GPU takes a tenth longer than one that does not.  One B200, us alone / together: Q4_K 4096 + 1024 + 1024 of 4096 at
   // 24, 300, 1000 tokens 23.5 / 12.2, 43.1 / 19.2, 63.2 / 39.1; 2 x 14336 at 24, 200 tokens 34.5 / 30.7, 46.1 / 42.7, and with Q8_0 at 300, 1000 (left alone)
   // 78.5 / 81.1, 195 / 213; Q6_K 2 x 14336 at 512 (alone) 112 / 130; 3 x 4096 at 1000 (alone) 90 / 101; 2 x 5632 of 2048 at 1000 60.2 / 45.8.
+  // A plan with more waves than the matrices have alone (finer token tiles, a split K) pays in dequantising, which the estimate makes little of, so it has to
+  // promise more, alone / together: 2 x 11008 of 4096 at 256 tokens Q5_K (0.91 of the estimate alone) 54.6 / 65.2, Q4_K (0.79) 53.5 / 48.7, at 224 tokens (0.89) 48.6 / 48.2; 2 x
+  // 13824 of 5120 at 256 Q8_0 76.5 / 84.0.
   double alone = 0.0;
   int waves = 0;
   const int each[] = {n0, n1, n2};
@@ -193,7 +196,7 @@ static int32_t gguf_multi(int32_t ggml_type, const void *w0, const void *w1, con
     alone += one.cost;
     waves += one.waves;
   }
-  if (plan.cost > 0.92 * alone || (M > 320 && plan.waves >= waves)) return (int32_t)cudaErrorNotSupported;
+  if (plan.cost > (plan.waves > waves ? 0.85 : 0.92) * alone || (M > 320 && plan.waves >= waves)) return (int32_t)cudaErrorNotSupported;
   const TsCall c = {w0, x, y0, M, n0, K, K / elems * bytes, dtype, plan.nt, plan.tiles_m, plan.ksplit, d.sms, d.timeouts, (cudaStream_t)stream, nullptr, nullptr, 0, 0, pdl,
                     n2 > 0 ? 3 : 2, {w1, w2}, {y1, y2}, {n1, n2}};
   switch (ggml_type) {

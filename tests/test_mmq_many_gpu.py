@@ -98,3 +98,17 @@ def test_what_a_list_costs_the_host(cuda, monkeypatch, kind, tokens, asked):
     assert torch.cuda.memory_stats(cuda)["allocation.all.allocated"] - before == 2
     assert seen.count("check") == 2 and seen.count("mrs_mmq_gguf_multi") == asked
     assert all(float((y.double() - w.double()).norm()) <= 2.0 ** -10 * float(w.double().norm()) for y, w in zip(ys, want))
+
+
+@pytest.mark.parametrize("kind,rows,cols,tokens,one", [("q5_k", 11008, 4096, 256, False), ("q8_0", 13824, 5120, 256, False), ("q5_k", 11008, 4096, 200, True),
+                                                       ("q4_k", 11008, 4096, 256, True), ("q5_k", 16384, 4096, 256, True)])
+def test_more_waves_than_alone(cuda, kind, rows, cols, tokens, one):
+    """Lists whose one launch has more waves than the matrices have alone are grouped only where that promises much."""
+    g = torch.Generator(device=cuda).manual_seed(rows)
+    ws = [_matrix(kind, rows, cols, cuda, g) for _ in range(2)]
+    x = torch.randn(tokens, cols, device=cuda, generator=g).to(torch.bfloat16)
+    rc, _ = _entry(ws, x)
+    assert rc == (0 if one else 801)
+    for y, w in zip(mmq.forward_many(ws, x), ws):
+        want = mmq.forward(w, x)
+        assert float((y.double() - want.double()).norm()) <= 2.0 ** -10 * float(want.double().norm())
