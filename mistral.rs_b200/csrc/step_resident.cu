@@ -48,8 +48,11 @@ constexpr int RS_HEADER = 1024;          // barriers, offsets, small exchanges
 // Narrower models: the meetings take longer than the chain's links (four layers 2048 wide at 20 tokens 155 us, 160 so).  Long tiles: their steps of 64 tokens
 // are copied one at a time, two in the chain's kernel, so where KV heads leave a tile many tokens the chain is faster (two layers, chain / resident: 16 KV heads,
 // 451 tokens a tile 183 / 176, Q8_0 195 / 196; 1784 tokens 257 / 261; 32 KV heads, 58 tokens 155 / 149, Q8_0 164 / 167, 268 tokens 176 / 182, 2016 tokens
-// 263 / 281; 8 KV heads, 892 tokens 236 / 213).
-constexpr int RS_MIN_HIDDEN = 2560, RS_MAX_KV_HEADS = 16, RS_MAX_TILE = 8192;      // tile: tokens x KV heads
+// 263 / 281; 8 KV heads, 892 tokens 236 / 213).  Heads of 64: half the bytes a step for the same chain of loads, so half the tile (8 KV heads, three layers, resident /
+// chain: 500 tokens a tile 0.99 at 2560 x 6912, 0.97 at 2560 x 10240 and 0.94 at 4096 x 14336, 778 tokens 1.03, 1.00 and 0.95, 1000 tokens 1.04, 1.02 and 0.96;
+// Q8_0 0.03 to 0.06 above).  Close to the line Q8_0 may lose a few in a hundred: 2560 x 6912, 32 heads of 64 on 8, 1.00 to 1.05 at any length, and where the whole
+// context is two tiles 1.02 to 1.08 up to 2816 wide or with heads of 64; 20 heads of 128 on 4 0.78 to 0.97.
+constexpr int RS_MIN_HIDDEN = 2560, RS_MAX_KV_HEADS = 16, RS_MAX_TILE = 64;      // tile: tokens x KV heads for each element of a head
 constexpr uint32_t RS_COPY_LIMIT = 1u << 22, RS_GRID_LIMIT = 1u << 22;      // polls (seconds)
 constexpr uint32_t RS_DEAD = 1u << 31;   // in the word of arrivals: a wait of this step ran out, now or in a launch before (arrivals stay far below)
 
@@ -912,7 +915,7 @@ static bool rs_plan(const mrs_llama_step *s, RsParams &p, int &sms, size_t &smem
       s->hidden % 256 != 0 || s->hidden < RS_MIN_HIDDEN || s->block_size < 1 || s->vocab < 1 ||
       s->padded_tiles < 1 || s->padded_tiles > RS_TILES || s->tmp_v == nullptr || s->resident_bytes < mrs_llama_resident_bytes(s->n_heads, D, s->padded_tiles))
     return false;
-  if ((int64_t)s->max_blocks_per_seq * s->block_size / s->padded_tiles * s->n_kv_heads > RS_MAX_TILE) return false;
+  if ((int64_t)s->max_blocks_per_seq * s->block_size / s->padded_tiles * s->n_kv_heads > (int64_t)RS_MAX_TILE * D) return false;
   int dev = 0, most = 0, coop = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

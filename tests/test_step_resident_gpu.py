@@ -161,11 +161,16 @@ def test_more_layers_than_a_launch_holds(cuda, monkeypatch):
 
 
 def test_what_the_grid_declines(cuda, monkeypatch):
-    """Other block types, a scratch that is too small, the measuring switches: the chain, by its bits and its launches.  (A sequence at the end of its
+    """Other block types, long tiles, a scratch that is too small, the measuring switches: the chain, by its bits and its launches.  (A sequence at the end of its
     context stays on the grid, by the chain's rules.)"""
     resident, chain = _pair(cuda, monkeypatch, "gqa4", "q4_k_m", torch.float16, types=lambda cfg, name, layer=0: "q4_0" if name == "ffn_down" else "q4_k")
     assert torch.equal(_step(resident, 100)["logits"], _step(chain, 100)["logits"]) and not _ran_resident(resident)
     monkeypatch.undo()
+    for shape, ctx, grid in (("gqa8_64", 9 * 1024, True), ("gqa8_64", 10 * 1024, False), ("gqa2_64", 2304, True), ("gqa2_64", 2512, False), ("mha", 4096, True)):
+        resident, chain = _pair(cuda, monkeypatch, shape, "q4_k_m", torch.float16, ctx=ctx)       # tokens x KV heads a tile: 64 for each element of a head
+        assert resident.is_resident() == grid, (shape, ctx)
+        _same(resident, chain, 300)
+        assert _ran_resident(resident) == grid
     resident, chain = _pair(cuda, monkeypatch, "gqa4", "q4_k_m", torch.float16, ctx=160)
     resident.step_struct.resident_bytes -= 16
     assert torch.equal(_step(resident, 50)["logits"], _step(chain, 50)["logits"]) and not _ran_resident(resident)
